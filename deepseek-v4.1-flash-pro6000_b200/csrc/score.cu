@@ -1,11 +1,17 @@
 // Score reporting on device logits: log-normaliser, first maximum and the top-N ids with their log-probabilities, the
 // caller-visible outputs the reference computes with host passes over the vocabulary (engine/src/server.cpp:178-183
-// log_normalizer, :730-737 top_order, used at :450-461 and :603-612).  One CTA per row; the row is read from L2/HBM
-// 2 + N times, which is what a reporting path (a few rows per request, N <= 32) needs, not a decode-rate kernel.
+// log_normalizer, :730-737 top_order, used at :450-461 and :603-612).
 //   logsumexp   = m + log(sum_i exp(double(x_i) - m)), m = the row maximum (the reference sums sequentially; here the
 //                 sum is a fixed-order tree, so the value agrees to a few units in the last place, not bit for bit)
 //   top ids     = the first N ids in the order (logit descending, id ascending): exact
 //   top_logprob = double(x_id) - logsumexp
+// One cluster of up to eight CTAs per row, each with a contiguous slice that it reads twice (the second time from L2):
+// maximum and finiteness first, then the exponentials and, in the same pass, every id that can be among the first N.  The
+// first pass leaves one maximum per thread; N of them at or above a value prove N ids at or above it, so the slices'
+// own thresholds bound the N-th id of the row from below and a few dozen ids per row reach the final ranking.
+// A request has a few rows, so what bounds the kernel is the latency of two passes over a slice and three exchanges
+// between CTAs: 5 rows x 129280, N = 20 in 22.5 us a call (833 us with one CTA per row and a pass over the row per
+// listed id).
 #include "ds41_b200.h"
 #include "host_error.h"
 #include "row_core.cuh"
@@ -15,97 +21,201 @@ namespace {
 
 constexpr int kScoreThreads = 512;
 constexpr int kScoreWarps = kScoreThreads / 32;
+constexpr int kScoreList = 1024;       // ids that can be ranked by counting
+constexpr int kScoreBisect = 14;       // steps of the threshold search
 
-// (value, id) maximum under "larger value, then lower id" over the CTA; every thread gets the result.
-__device__ __forceinline__ void score_argmax(float &v, int &id, float *sv, int *si) {
+__device__ __forceinline__ uint32_t score_ordered(float v) {  // order-preserving; -0 and +0 are the same logit
+  const uint32_t bits = __float_as_uint(v == 0.f ? 0.f : v);
+  return bits ^ ((bits >> 31) ? 0xffffffffu : 0x80000000u);
+}
+__device__ __forceinline__ float score_value(uint32_t o) { return __uint_as_float(o ^ ((o >> 31) ? 0x80000000u : 0xffffffffu)); }
+// ascending key = (logit descending, id ascending)
+__device__ __forceinline__ unsigned long long score_key(float v, int id) {
+  return (unsigned long long)(~score_ordered(v)) << 32 | uint32_t(id);
+}
+
+struct ScoreSlot { unsigned long long key; double z; uint32_t threshold; int bad; };
+struct ScoreSmem {
+  ScoreSlot slots[kMaxCluster];        // one per CTA of the cluster, written by its owner
+  unsigned long long list[kScoreList]; // rank 0: candidate keys
+  unsigned long long red_q[kScoreWarps];
+  double red_d[kScoreWarps];
+  int count;
+};
+
+__device__ __forceinline__ unsigned long long score_block_min(ScoreSmem &s, unsigned long long v) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, id, o);
-    if (ov > v || (ov == v && oi < id)) { v = ov; id = oi; }
+  for (int o = 16; o; o >>= 1) { const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o); v = w < v ? w : v; }
+  if (lane == 0) s.red_q[warp] = v;
+  __syncthreads();
+  v = s.red_q[lane & (kScoreWarps - 1)];
+#pragma unroll
+  for (int o = kScoreWarps / 2; o; o >>= 1) { const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o); v = w < v ? w : v; }
+  __syncthreads();
+  return v;
+}
+
+// f(value, id, id's parity within a vector) over this CTA's slice [begin, end) of the row: 16-byte loads where the row's alignment allows, eight of
+// them in flight per thread.
+template <class F>
+__device__ __forceinline__ void score_slice(const float *x, int begin, int end, F f) {
+  const int misaligned = int((reinterpret_cast<uintptr_t>(x + begin) >> 2) & 3u);
+  const int head = min(end, begin + ((4 - misaligned) & 3)), vecs = (end - head) >> 2;
+  const float4 *v4 = reinterpret_cast<const float4 *>(x + head);
+  for (int i = begin + threadIdx.x; i < head; i += kScoreThreads) f(__ldg(x + i), i, 0);
+  int v = threadIdx.x;
+  for (; v + 7 * kScoreThreads < vecs; v += 8 * kScoreThreads) {
+    float4 q[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) q[k] = __ldg(v4 + v + k * kScoreThreads);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int id = head + 4 * (v + k * kScoreThreads);
+      f(q[k].x, id, 0); f(q[k].y, id + 1, 1); f(q[k].z, id + 2, 0); f(q[k].w, id + 3, 1);
+    }
   }
-  if (lane == 0) { sv[warp] = v; si[warp] = id; }
-  __syncthreads();
-  v = sv[0]; id = si[0];
-  for (int w = 1; w < kScoreWarps; ++w)
-    if (sv[w] > v || (sv[w] == v && si[w] < id)) { v = sv[w]; id = si[w]; }
-  __syncthreads();
+#pragma unroll 4
+  for (; v < vecs; v += kScoreThreads) {
+    const float4 q = __ldg(v4 + v);
+    const int id = head + 4 * v;
+    f(q.x, id, 0); f(q.y, id + 1, 1); f(q.z, id + 2, 0); f(q.w, id + 3, 1);
+  }
+  for (int i = head + 4 * vecs + threadIdx.x; i < end; i += kScoreThreads) f(__ldg(x + i), i, 0);
 }
 
 __global__ void __launch_bounds__(kScoreThreads) score_kernel(ds41_b200_score_args a) {
-  __shared__ float sv[kScoreWarps];
-  __shared__ int si[kScoreWarps];
-  __shared__ double sd[kScoreWarps];
-  const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ ScoreSmem s;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = int(cluster.block_rank()), nranks = int(cluster.num_blocks());
+  const int row = int(blockIdx.x) / nranks, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float *x = a.logits + size_t(row) * a.logits_stride;
-  // first maximum and finiteness
-  float best = -CUDART_INF_F;
-  int best_id = 0x7fffffff, bad = 0;
-  for (int i = tid; i < a.vocab; i += kScoreThreads) {
-    const float v = __ldg(x + i);
-    if ((__float_as_uint(v) & 0x7f800000u) == 0x7f800000u) bad = 1;
-    if (v > best) { best = v; best_id = i; }
+  const int slice = (((a.vocab + nranks - 1) / nranks) + 3) & ~3;
+  const int begin = min(a.vocab, rank * slice), end = min(a.vocab, begin + slice);
+  if (tid == 0) s.count = 0;
+  // ---- first maximum, finiteness; `own` stays in this thread as the sample of its ids
+  float own = -CUDART_INF_F;
+  int own_id = 0x7fffffff;
+  float poison = 0.f;
+  score_slice(x, begin, end, [&](float v, int id, int) {
+    poison = fmaf(v, 0.f, poison);      // NaN once any logit is NaN or infinite
+    if (v > own) { own = v; own_id = id; }
+  });
+  const uint32_t own_key = own_id == 0x7fffffff ? 0u : score_ordered(own);   // 0: no id at all
+  const bool bad_here = __syncthreads_or(!(poison == 0.f));
+  const unsigned long long first = score_block_min(s, own_id == 0x7fffffff ? ~0ull : score_key(own, own_id));
+  // a value that at least `want` of this CTA's thread maxima reach (0: it has none).  Bisection on the ordered bits,
+  // below the CTA's maximum; any such value is valid, more steps only shorten the list
+  const int groups = min(nranks, 4), want = (a.top_n + groups - 1) / groups;
+  uint32_t threshold = 0;
+  if (a.top_n > 0 && !bad_here) {
+    uint32_t lo = 0, hi = uint32_t(~first >> 32);
+    // start a few units of the logit's own scale below the maximum: a window that usually holds the answer
+    const uint32_t near = score_ordered(score_value(hi) - 16.f);
+    if (hi && near < hi && __syncthreads_count(own_key >= near) >= want) lo = near;
+    for (int k = 0; k < kScoreBisect && lo < hi; ++k) {
+      const uint32_t mid = lo + (hi - lo + 1) / 2;
+      if (__syncthreads_count(own_key >= mid && own_key != 0u) >= want) lo = mid; else hi = mid - 1;
+    }
+    threshold = lo;
   }
-  bad = __syncthreads_or(bad);
-  if (bad) {  // the reference rejects non-finite logits (engine/src/sampling.cpp:133-139)
-    if (tid == 0) {
-      a.status[row] = DS41_B200_ROW_NONFINITE;
-      a.logsumexp[row] = CUDART_NAN;
-      if (a.top1) a.top1[row] = -1;
+  if (tid < nranks) *cluster.map_shared_rank(&s.slots[rank], tid) = ScoreSlot{first, 0.0, threshold, bad_here ? 1 : 0};
+  cluster.sync();
+  unsigned long long best = ~0ull;
+  int bad = 0;
+  uint32_t cutoff = 0;  // the `groups`-th largest of the CTAs' thresholds: that many CTAs hold `want` ids each above it
+  for (int r = 0; r < nranks; ++r) {
+    best = min(best, s.slots[r].key);
+    bad |= s.slots[r].bad;
+    int above = 0;
+    for (int q = 0; q < nranks; ++q)
+      above += (s.slots[q].threshold > s.slots[r].threshold || (s.slots[q].threshold == s.slots[r].threshold && q < r)) ? 1 : 0;
+    if (above == groups - 1) cutoff = s.slots[r].threshold;
+  }
+  if (bad) {  // the reference rejects non-finite logits (engine/src/sampling.cpp:133-139); the same answer in every CTA
+    if (rank == 0) {
+      if (tid == 0) {
+        a.status[row] = DS41_B200_ROW_NONFINITE;
+        a.logsumexp[row] = CUDART_NAN;
+        if (a.top1) a.top1[row] = -1;
+      }
+      for (int k = tid; k < a.top_n; k += kScoreThreads) {
+        a.top_ids[size_t(row) * a.top_n + k] = -1;
+        a.top_logprob[size_t(row) * a.top_n + k] = CUDART_NAN;
+      }
     }
-    for (int k = tid; k < a.top_n; k += kScoreThreads) {
-      a.top_ids[size_t(row) * a.top_n + k] = -1;
-      a.top_logprob[size_t(row) * a.top_n + k] = CUDART_NAN;
-    }
+    cluster.sync();  // (no CTA leaves while another may still write its slots)
     return;
   }
-  score_argmax(best, best_id, sv, si);
-  // normaliser: lanes stride the row, fixed-order tree
-  const double m = double(best);
-  double z = 0;
-  for (int i = tid; i < a.vocab; i += kScoreThreads) z += exp_nonpos(double(__ldg(x + i)) - m);
+  // ---- normaliser (fixed order: a thread's ids, the warp, the block, the cluster) and the candidates
+  const float best_value = score_value(uint32_t(~best >> 32));
+  const double m = double(best_value);
+  double zs[2] = {0, 0};   // two chains of additions
+  int *count0 = cluster.map_shared_rank(&s.count, 0);
+  unsigned long long *list0 = cluster.map_shared_rank(s.list, 0);
+  const bool listing = a.top_n > 0;
+  const float cut = cutoff ? score_value(cutoff) : -CUDART_INF_F;
+  score_slice(x, begin, end, [&](float v, int id, int k) {
+    zs[k] += exp_nonpos(double(v) - m);
+    if (listing && v >= cut) {
+      const int slot = atomicAdd(count0, 1);
+      if (slot < kScoreList) list0[slot] = score_key(v, id);
+    }
+  });
+  double z = zs[0] + zs[1];
 #pragma unroll
   for (int o = 16; o; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-  if (lane == 0) sd[warp] = z;
+  if (lane == 0) s.red_d[warp] = z;
   __syncthreads();
   z = 0;
-  for (int w = 0; w < kScoreWarps; ++w) z += sd[w];
+  for (int w = 0; w < kScoreWarps; ++w) z += s.red_d[w];
+  if (tid < nranks) cluster.map_shared_rank(&s.slots[rank], tid)->z = z;
+  cluster.sync();
+  z = 0;
+  for (int r = 0; r < nranks; ++r) z += s.slots[r].z;
   const double lse = m + log(z);
-  if (tid == 0) {
+  if (rank == 0 && tid == 0) {
     a.status[row] = 0;
     a.logsumexp[row] = lse;
-    if (a.top1) a.top1[row] = best_id;
+    if (a.top1) a.top1[row] = int(uint32_t(best));
   }
-  // top-N by repeated selection of the next id in the order (logit descending, id ascending)
-  float prev_v = best;
-  int prev_id = best_id;
-  for (int k = 0; k < a.top_n; ++k) {
-    float v = -CUDART_INF_F;
-    int id = 0x7fffffff;
-    if (k == 0) { v = best; id = best_id; }
-    else {
-      for (int i = tid; i < a.vocab; i += kScoreThreads) {
-        const float y = __ldg(x + i);
-        const bool after = y < prev_v || (y == prev_v && i > prev_id);  // strictly after the previous pick
-        if (after && (y > v || (y == v && i < id))) { v = y; id = i; }
+  if (!listing) return;
+  auto publish = [&](int k, unsigned long long key) {   // key ~0: the row has fewer ids
+    const bool is = key != ~0ull;
+    a.top_ids[size_t(row) * a.top_n + k] = is ? int(uint32_t(key)) : -1;
+    a.top_logprob[size_t(row) * a.top_n + k] = is ? double(score_value(uint32_t(~key >> 32))) - lse : CUDART_NAN;
+  };
+  const int listed = *count0;          // complete since the barrier above; the same in every CTA
+  if (listed <= kScoreList) {
+    if (rank == 0) {                   // exact rank by counting (the keys are distinct)
+      for (int i = tid; i < listed; i += kScoreThreads) {
+        const unsigned long long mine = s.list[i];
+        int pos = 0;
+        for (int k = 0; k < listed; ++k) pos += s.list[k] < mine ? 1 : 0;
+        if (pos < a.top_n) publish(pos, mine);
       }
-      score_argmax(v, id, sv, si);
+      for (int k = listed + tid; k < a.top_n; k += kScoreThreads) publish(k, ~0ull);
     }
-    if (id == 0x7fffffff) id = -1;  // fewer than top_n ids in the row
-    if (tid == 0) {
-      a.top_ids[size_t(row) * a.top_n + k] = id;
-      a.top_logprob[size_t(row) * a.top_n + k] = id >= 0 ? double(v) - lse : CUDART_NAN;
-    }
-    prev_v = v; prev_id = id;
-    if (id < 0) {
-      for (int k2 = k + 1 + tid; k2 < a.top_n; k2 += kScoreThreads) {
-        a.top_ids[size_t(row) * a.top_n + k2] = -1;
-        a.top_logprob[size_t(row) * a.top_n + k2] = CUDART_NAN;
-      }
-      break;
+  } else {
+    // more than kScoreList ids at or above the cutoff (a plateau of ties): the next id in the order, one at a time
+    unsigned long long previous = best;
+    if (rank == 0 && tid == 0) publish(0, best);
+    for (int k = 1; k < a.top_n; ++k) {
+      unsigned long long next = ~0ull;
+      score_slice(x, begin, end, [&](float v, int id, int) {
+        const unsigned long long key = score_key(v, id);
+        if (key > previous && key < next) next = key;
+      });
+      next = score_block_min(s, next);
+      cluster.sync();                  // everybody has read the previous step's slots
+      if (tid < nranks) cluster.map_shared_rank(&s.slots[rank], tid)->key = next;
+      cluster.sync();
+      for (int r = 0; r < nranks; ++r) next = min(next, s.slots[r].key);
+      if (rank == 0 && tid == 0) publish(k, next);
+      previous = next;
     }
   }
+  cluster.sync();                      // rank 0's counter has been read by every CTA
 }
 
 }  // namespace
@@ -119,8 +229,18 @@ extern "C" int ds41_b200_score_logits(const ds41_b200_score_args *p, cudaStream_
     return invalid("score args: rows / vocab / buffers");
   if (p->top_n < 0 || p->top_n > DS41_B200_SCORE_MAX_TOP || (p->top_n > 0 && (!p->top_ids || !p->top_logprob)))
     return invalid("score args: top_n out of range or missing output buffers");
-  score_kernel<<<p->rows, kScoreThreads, 0, stream>>>(*p);
-  return int(cudaGetLastError());
+  // CTAs per row: enough that a thread's share of a slice stays at 32 ids or fewer, up to the portable cluster size
+  int cl = 1;
+  while (cl < kMaxCluster && p->vocab > cl * 16 * kScoreThreads) cl <<= 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(p->rows) * unsigned(cl));
+  cfg.blockDim = dim3(kScoreThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(cl); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  return int(cudaLaunchKernelEx(&cfg, score_kernel, *p));
 }
 
 // ---------------------------------------------------------------------------------------------------------------
