@@ -85,6 +85,15 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, u
       : "memory");
 }
 
+// The same with an L2 eviction policy.
+__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int row, int kb, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], "
+      "[%2], %6;" ::"r"(smem_addr(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_addr(bar)), "r"(x), "r"(row), "r"(kb), "l"(policy)
+      : "memory");
+}
+
 // Shared-memory matrix descriptor, K-major, 128-byte swizzle: rows are 128 bytes apart, groups of 8 rows 1024 bytes
 // apart (stride byte offset), leading byte offset unused (1), descriptor version 1 for sm_100.
 constexpr uint64_t kDescFixed = (uint64_t(1) << 16)              // leading byte offset (>>4), bits [16,30)
@@ -238,13 +247,18 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       uint32_t stage = 0, phase = 0;
+      // one batch tile: every weight is read once per step, and 530 MB of them would push everything else out of the L2 --
+      // the logits, the activations, the code of the kernels around this one
+      uint64_t policy;
+      if (b_tiles == 1) asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+      else asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
       for (int tile = blockIdx.x; tile < total_tiles && !ab.set(); tile += gridDim.x) {
         const int nt = tile / b_tiles, bt = tile % b_tiles;
         for (int kb = 0; kb < kblocks; kb += group) {
           if (!mbar_wait(&empty[stage], phase ^ 1, ab)) break;
           unsigned char *w_dst = tiles + size_t(stage) * stage_bytes, *a_dst = w_dst + w_bytes;
           mbar_expect_tx(&full[stage], uint32_t(stage_bytes));
-          tma_load_3d(w_dst, &map_w, &full[stage], 0, nt * kTileN, kb);
+          tma_load_3d(w_dst, &map_w, &full[stage], 0, nt * kTileN, kb, policy);
           tma_load_3d(a_dst, &map_a, &full[stage], 0, bt * kRows, kb);
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
