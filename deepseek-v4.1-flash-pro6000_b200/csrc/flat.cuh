@@ -7,8 +7,9 @@
 
 namespace ds41 {
 
-constexpr int kFlatThreads = 512;
-constexpr int kFlatMassThreads = 128;
+constexpr int kFlatThreads = 512;       // statistics and histogram passes
+constexpr int kFlatWindowThreads = 256;
+constexpr int kFlatMassThreads = 128;   // mass pass and resolve
 constexpr int kFlatSub = 1024;      // ids per sub-region: the granularity of the inverse-CDF search
 constexpr int kFlatSubs = 128;      // sub-regions per row (covers the largest vocabulary, 131072)
 constexpr int kFlatBins = 2048;     // histogram bins over the row's logit range
@@ -36,7 +37,7 @@ struct FlatInfo {
   // the mass pass sorts the ids by two thresholds on the logit itself (a quarter of a bin outside the window's edges):
   // y > y_sure: before the window; y < y_tail: beyond it; the rest goes to the list
   float y_sure, y_tail;
-  int pad[2];
+  int pad[2];             // cluster kernel: pad[0] = 1 for a row that it left to its general search
 };
 struct FlatScratch {
   int *pending;                // [4]: rows handed on to the cluster kernel (status -8 / -9); rows replayed   (zeroed every call)
@@ -56,6 +57,13 @@ struct FlatArgs {
   const uint64_t *seeds, *steps;
   uint32_t slot, purpose;
   int32_t *tokens, *status;    // status is required here
+  // Statistics instead of tokens (the verifier): one record per row; rows >= split are rows of logits2; every
+  // draw_every-th of the first `split` rows is also drawn from, at (seeds[row / draw_every], ...)
+  struct RowStats *stats;
+  const float *logits2;
+  int split, draw_every;
+  double log2e_t;              // log2(e) / t and a distance below the maximum at which weights stop falling (set by launch_flat)
+  float floor_gap;
   const HeadRowStats *head_stats;  // optional [rows]: maximum / minimum / finiteness already known (skips the first pass)
   double bound_scale;              // 1; larger values widen the certification bounds (a test hook: more rows get flagged)
   FlatScratch s;
@@ -64,6 +72,12 @@ struct FlatArgs {
 size_t flat_scratch_bytes(int rows);
 // The word (inside `scratch`) that counts the rows launch_flat handed on; valid once its kernels have run.
 const int *flat_pending(const void *scratch);
+// The [rows] records inside `scratch`.
+FlatInfo *flat_info(void *scratch, int rows);
+// Whether rows of this shape can be laid out for it.
+inline bool flat_aligned(const void *logits, long long stride) {
+  return stride != 0 && stride % 4 == 0 && !(reinterpret_cast<uintptr_t>(logits) & 15u);
+}
 // Rows this path decides get their token and status (0 or certification bits); the others get token -1 and status
 // -8 / -9 (to be redone by another path) or -1 (non-finite logits, final).
 cudaError_t launch_flat(FlatArgs a, void *scratch, cudaStream_t stream);

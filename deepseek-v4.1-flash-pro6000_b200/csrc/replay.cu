@@ -16,6 +16,7 @@
 // whole ranges of the key as integer sums and sorts only the few chunks in which it needs the terms one by one.  A
 // full-vocabulary row costs a little under a millisecond; the parallel bound flags a few rows in 10^5.
 #include "replay_core.cuh"
+#include "launch.h"
 #include <atomic>
 
 namespace ds41 {
@@ -30,12 +31,16 @@ __global__ void __launch_bounds__(kRT) replay_sample_kernel(ReplayArgs a) {
   double *p = reinterpret_cast<double *>(mine);
   unsigned long long *key = reinterpret_cast<unsigned long long *>(mine + size_t(kReplayPad) * 8);
   int *idx = reinterpret_cast<int *>(mine + size_t(kReplayPad) * 16);
+  cudaGridDependencySynchronize();
+  int handed_on = 0;
   // Which rows are this CTA's: the status words are read kRT at a time; in the common case (nothing to redo) the
   // kernel is one coalesced read and a vote.
   for (int first = 0; first < a.rows; first += kRT) {
     const int candidate = first + threadIdx.x;
     const int st0 = candidate < a.rows ? a.status[candidate] : 0;
     const bool flagged = st0 > 0 || st0 == -4;
+    if (a.info && blockIdx.x == 0)
+      handed_on += __syncthreads_count(candidate < a.rows && a.info[candidate].pad[0] != 0);
     if (!__syncthreads_or(flagged)) continue;
     for (int row = first + blockIdx.x; row < min(a.rows, first + kRT); row += gridDim.x) {
       const int st = a.status[row];   // the same in every thread
@@ -53,6 +58,7 @@ __global__ void __launch_bounds__(kRT) replay_sample_kernel(ReplayArgs a) {
       __syncthreads();
     }
   }
+  if (a.info && blockIdx.x == 0 && threadIdx.x == 0) a.replayed[-1] = handed_on;
 }
 
 }  // namespace
@@ -68,8 +74,14 @@ cudaError_t launch_replay(const ReplayArgs &a, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     opted.fetch_or(1 << (dev & 31));
   }
-  replay_sample_kernel<<<ctas, kRT, kReplayDynamicBytes, stream>>>(a);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(ctas));
+  cfg.blockDim = dim3(kRT);
+  cfg.dynamicSmemBytes = kReplayDynamicBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1] = {programmatic_launch()};
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, replay_sample_kernel, a);
 }
 
 }  // namespace ds41

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
+#include "flat.cuh"
 
 namespace ds41 {
 
@@ -22,6 +23,8 @@ struct ReplayArgs {
   int32_t *tokens, *status;
   unsigned char *scratch;      // kReplayCtas * kReplayBytesPerCta bytes, 16-byte aligned
   int *replayed;               // optional counter of replayed rows
+  // optional records of the cluster kernel: replayed[-1] is then set to the number of rows left to its general search
+  const FlatInfo *info;
 };
 
 // Verification: transactions whose status carries a certification bit are redone from the logits in the reference's

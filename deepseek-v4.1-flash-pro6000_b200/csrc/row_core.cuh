@@ -72,8 +72,9 @@ struct RowStats {
   int kept;        // number of survivors
   int entered;     // number of ids that entered the softmax
   int status;      // 0, certification bits, or a negative row error
-  int pad;
+  int drawn;       // token drawn from the row with its own uniform (kDrawnClose set: inside the rounding bound); -1: none
 };
+constexpr int kDrawnClose = 1 << 30;
 
 struct Slot {  // one CTA's contribution to a cluster-wide exchange
   double d[4];
@@ -132,6 +133,24 @@ __device__ __forceinline__ double exp_nonpos(double x) {
   return tiny ? 0.0 : scaled;
 }
 
+// Two of them in lockstep, a few ulp each and 0 below -700 (for bounds that allow for 1e-12).
+__device__ __forceinline__ void exp_nonpos2(const double (&x)[2], double (&e)[2]) {
+  constexpr double kMagic = 6755399441055744.0;
+  double t[2], r[2], q[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) { t[i] = fma(fmax(x[i], -700.0), 0x1.71547652b82fep+6, kMagic); r[i] = t[i] - kMagic; }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) r[i] = fma(r[i], -0x1.62e42fefa39efp-7, fmax(x[i], -700.0));
+#pragma unroll
+  for (int i = 0; i < 2; ++i) q[i] = fma(fma(fma(fma(r[i], 1.0 / 24.0, 1.0 / 6.0), r[i], 0.5), r[i], 1.0), r[i], 1.0);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int n = __double2loint(t[i]);
+    const double v = __ldg(&kExp2Table[n & 63]) * q[i];
+    e[i] = __hiloint2double(__double2hiint(v) + (n >> 6) * 1048576, __double2loint(v));
+  }
+}
+
 struct __align__(128) RowSmem {
   float y[kSliceCap];  // staged logits, rewritten in place as effective logits (-inf = excluded)
   union {              // 32 KB: history counters first, cut-search work space afterwards
@@ -144,22 +163,45 @@ struct __align__(128) RowSmem {
       float sorted_y[kListCap];
       int sorted_id[kListCap];
     } w;
-  } u;
+    struct {           // this CTA's candidate keys, those of the whole cluster, and their weights or their order
+      unsigned long long mine[kListCap];
+      unsigned long long all[kListCap];
+      union { double weight[kListCap]; unsigned long long sorted[kListCap]; };
+    } n;
+  } work;
   unsigned long long bin_mass[kBins];  // also holds the sorted candidates' exp values (doubles) while resolving
   int bin_count[kBins];
-  uint32_t mask_words[kSliceCap / 32];
+  union {
+    uint32_t mask_words[kSliceCap / 32];
+    struct { double all[kMaxCluster * kWarps], kept[kMaxCluster * kWarps]; } region;  // masses of the cluster's warp regions
+  };
   Slot exch[2][kMaxCluster];
+  double pow2[64];                     // 2^(-j/64)
   double warp_sum[kWarps];
   double red_d[kWarps];
   float red_f[kWarps];
   int red_i[kWarps];
   int red_j[kWarps];
+  int red_k[kWarps];
   unsigned long long red_q[kWarps];
   Slot outcome;
   unsigned long long mbar;
   unsigned long long bcast_q;
-  int list_count;
+  // one row's facts, worked out by one warp for all of them
+  struct { float max_logit, lowest, cutoff; int best_id, flags, allowed; } facts;
+  struct { float scale; int ok, clipped; double kappa; } map;
+  double u;
+  unsigned long long window[2];        // first bin that may / surely reaches the target << 32 | ids before / through it
+  float edge[2];                       // the logits a quarter of a bin outside the window
+  int counted, late;                   // ids in the cluster's histograms; a slice did not land
+  struct { double z, mass_before, target, lo, hi; } sums;
+  struct { double carry, target, slack; int region, close; } pick;
+  __align__(16) int lists[kMaxCluster];  // candidate keys of every CTA (0 beyond the cluster)
+  int list_count, decided;
   int bcast_i[3];
+};
+static __device__ const double kPow2Neg64[64] = {  // 2^(-j/64), j = 0..63, correctly rounded
+#include "pow2neg64.inc"
 };
 static_assert(kListCap * sizeof(double) <= kBins * sizeof(unsigned long long), "sorted_e aliases bin_mass");
 static_assert(sizeof(RowSmem) <= 113 * 1024, "two CTAs must fit in one SM's shared memory");
@@ -170,8 +212,8 @@ struct RowCtx {
   int rank, nranks, tid, lane, warp;
   int vocab, stride_ids;  // ids per CTA slice (multiple of 32)
   int begin, len;         // this CTA's slice [begin, begin+len)
-  int region;             // ids per warp region (multiple of 32): warp w owns local [w*region, (w+1)*region)
-  int xphase;
+  int region;             // ids per warp region (multiple of 128): warp w owns local [w*region, (w+1)*region)
+  int xphase, copies;     // exchanges and staging copies so far
   int timed_out;          // a staging copy of the row just processed did not land (the same in every CTA of the cluster)
 };
 
@@ -184,8 +226,8 @@ __device__ __forceinline__ RowCtx make_ctx(RowSmem *s, int vocab) {
   c.stride_ids = (((vocab + c.nranks - 1) / c.nranks) + 31) & ~31;
   c.begin = min(vocab, c.rank * c.stride_ids);
   c.len = min(vocab, c.begin + c.stride_ids) - c.begin;
-  c.region = (((c.stride_ids + kWarps - 1) / kWarps) + 31) & ~31;
-  c.xphase = 0;
+  c.region = (((c.stride_ids + kWarps - 1) / kWarps) + 127) & ~127;
+  c.xphase = c.copies = 0;
   c.timed_out = 0;
   return c;
 }
@@ -279,17 +321,23 @@ __device__ __forceinline__ void block_argmax(RowCtx &c, float &v, int &id) {
 // plain coalesced loads.  The wait is bounded: on expiry the row is reported as DS41_B200_ROW_TIMEOUT.
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
+// Once per kernel, before the first row: what does not depend on the kernel in front of this one.
+__device__ __forceinline__ void prepare_smem(RowSmem *s) {
+  if (threadIdx.x == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s->mbar)));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (threadIdx.x < 64) s->pow2[threadIdx.x] = kPow2Neg64[threadIdx.x];
+  if (threadIdx.x < kMaxCluster) s->lists[threadIdx.x] = 0;
+  __syncthreads();
+}
 __device__ __forceinline__ void stage_begin(RowCtx &c, const float *row, bool &used_tma) {
   const float *src = row + c.begin;
   const uint32_t bytes = uint32_t(c.len) * 4u;
   used_tma = c.len > 0 && (bytes & 15u) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
-  if (c.tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&c.s->mbar)));
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
   if (used_tma) {
     if (c.tid == 0) {
+      if (c.copies > 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // (the previous row's writes to the slice)
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&c.s->mbar)), "r"(bytes)
                    : "memory");
       for (uint32_t off = 0; off < bytes; off += 16384u) {
@@ -302,27 +350,28 @@ __device__ __forceinline__ void stage_begin(RowCtx &c, const float *row, bool &u
       }
     }
   } else {
+#pragma unroll 8
     for (int j = c.tid; j < c.len; j += kThreads) c.s->y[j] = __ldg(src + j);
   }
+  // the rest of the last regions reads as excluded ids, so that the passes can take four ids at a time
+  for (int j = c.len + c.tid; j < c.region * kWarps; j += kThreads) c.s->y[j] = -CUDART_INF_F;
 }
-// Returns false if the copy did not land within the bound.
+// Returns false if the copy did not land within the bound (the cluster then takes no further row).
 __device__ __forceinline__ bool stage_wait(RowCtx &c, bool used_tma) {
   bool ok = true;
   if (used_tma) {
     uint32_t done = 0;
     for (int spin = 0; spin < (1 << 22) && !done; ++spin) {
       asm volatile(
-          "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}"
+          "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
           : "=r"(done)
-          : "r"(smem_u32(&c.s->mbar))
+          : "r"(smem_u32(&c.s->mbar)), "r"(uint32_t(c.copies & 1))
           : "memory");
     }
     ok = done != 0;
+    ++c.copies;
   }
   __syncthreads();
-  // the barrier object is initialised again for the cluster's next row (not after a timeout: the copy may still
-  // signal it, and the cluster then takes no further row)
-  if (c.tid == 0 && used_tma && ok) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(&c.s->mbar)) : "memory");
   return ok;
 }
 
@@ -429,8 +478,8 @@ __device__ CutResult find_cut(RowCtx &c, float max_logit, float first_width, int
           if (kMass) tm += *c.cluster.map_shared_rank(&s->bin_mass[b], r);
         }
         for (int r = 0; r < c.nranks; ++r) {
-          *c.cluster.map_shared_rank(&s->u.w.total_count[b], r) = tc;
-          if (kMass) *c.cluster.map_shared_rank(&s->u.w.total_mass[b], r) = tm;
+          *c.cluster.map_shared_rank(&s->work.w.total_count[b], r) = tc;
+          if (kMass) *c.cluster.map_shared_rank(&s->work.w.total_mass[b], r) = tm;
         }
       }
     }
@@ -450,8 +499,8 @@ __device__ CutResult find_cut(RowCtx &c, float max_logit, float first_width, int
       int run_c = count_before_level;
       unsigned long long run_m = mass_before_level;
       for (int base = 0; base < kBins && found < 0; base += 32) {
-        const int vc = s->u.w.total_count[base + c.lane];
-        const unsigned long long vm = kMass ? s->u.w.total_mass[base + c.lane] : 0ull;
+        const int vc = s->work.w.total_count[base + c.lane];
+        const unsigned long long vm = kMass ? s->work.w.total_mass[base + c.lane] : 0ull;
         int sc = vc;
         unsigned long long sm = vm;
 #pragma unroll
@@ -478,7 +527,7 @@ __device__ CutResult find_cut(RowCtx &c, float max_logit, float first_width, int
     const int found = s->bcast_i[0];
     const int before_c = s->bcast_i[1];  // ids before the found bin (or before the overflow bin if none found)
     const unsigned long long before_m = s->bcast_q;
-    const int in_bin = found >= 0 ? s->u.w.total_count[found] : 0;
+    const int in_bin = found >= 0 ? s->work.w.total_count[found] : 0;
     __syncthreads();
     if (found < 0) {  // the crossing is not inside this level's range
       if (L.bounded[L.n - 1] || ovf_total == 0) { chosen = -2; break; }
@@ -539,8 +588,8 @@ __device__ CutResult find_cut(RowCtx &c, float max_logit, float first_width, int
     double before_mass = 0;
     int before_count = 0, after_count = 0;
     int *list_count0 = c.cluster.map_shared_rank(&s->list_count, 0);
-    float *list_y0 = c.cluster.map_shared_rank(s->u.w.list_y, 0);
-    int *list_id0 = c.cluster.map_shared_rank(s->u.w.list_id, 0);
+    float *list_y0 = c.cluster.map_shared_rank(s->work.w.list_y, 0);
+    int *list_id0 = c.cluster.map_shared_rank(s->work.w.list_id, 0);
     for (int it = 0; it < c.region; it += 32) {
       const int j = c.warp * c.region + it + c.lane;
       if (j >= c.len) continue;
@@ -667,16 +716,16 @@ __device__ CutResult find_cut(RowCtx &c, float max_logit, float first_width, int
     if (c.rank == 0) {
       const int n = chosen == -2 ? 0 : min(s->list_count, kListCap);
       for (int i = c.tid; i < n; i += kThreads) {  // exact rank by counting (strict total order)
-        const float yi = s->u.w.list_y[i];
-        const int idi = s->u.w.list_id[i];
+        const float yi = s->work.w.list_y[i];
+        const int idi = s->work.w.list_id[i];
         int r = 0;
         for (int k = 0; k < n; ++k) {
-          const float yk = s->u.w.list_y[k];
-          const int idk = s->u.w.list_id[k];
+          const float yk = s->work.w.list_y[k];
+          const int idk = s->work.w.list_id[k];
           r += (yk > yi || (yk == yi && idk < idi)) ? 1 : 0;
         }
-        s->u.w.sorted_y[r] = yi;
-        s->u.w.sorted_id[r] = idi;
+        s->work.w.sorted_y[r] = yi;
+        s->work.w.sorted_id[r] = idi;
         if (kMass) sorted_e[r] = weight(yi);
       }
       __syncthreads();
@@ -713,8 +762,8 @@ __device__ CutResult find_cut(RowCtx &c, float max_logit, float first_width, int
         outcome.i[1] = amb;
         if (direction == 0) {
           const bool all_kept = chosen == -2 || pos < 0 || (pos == n - 1 && n_after == 0);
-          outcome.f[0] = all_kept ? -CUDART_INF_F : s->u.w.sorted_y[pos];
-          outcome.i[2] = all_kept ? -1 : s->u.w.sorted_id[pos];
+          outcome.f[0] = all_kept ? -CUDART_INF_F : s->work.w.sorted_y[pos];
+          outcome.i[2] = all_kept ? -1 : s->work.w.sorted_id[pos];
           outcome.i[3] = all_kept ? n_before + n : n_before + pos + 1;
           outcome.d[0] = mass;
         }
@@ -730,7 +779,7 @@ __device__ CutResult find_cut(RowCtx &c, float max_logit, float first_width, int
       return out;
     }
     const int next = chosen + v.i[0];  // one bin over at the deepest level; it must fit the list as well
-    if (chosen < 0 || next < 0 || next >= kBins || s->u.w.total_count[next] > kListCap) { out.error = -4; return out; }
+    if (chosen < 0 || next < 0 || next >= kBins || s->work.w.total_count[next] > kListCap) { out.error = -4; return out; }
     chosen = next;
   }
   out.error = -4;

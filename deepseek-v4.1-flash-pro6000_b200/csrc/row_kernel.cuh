@@ -3,7 +3,7 @@
 #pragma once
 #include "row_core.cuh"
 #include "row_fast.cuh"
-#include "row_wide.cuh"
+#include "row_nucleus.cuh"
 
 namespace ds41 {
 
@@ -14,6 +14,8 @@ struct RowArgs {
   long long logits_stride;
   int vocab;
   double temperature;  // already floored; 0 = greedy
+  double log2e_t;         // log2(e) / temperature; the next two: logit distances below the maximum at which the histogram's
+  float reach, floor_gap; // range ends / the weights stop falling (all three set by launch_rows)
   double top_p;
   int top_k;
   float repetition, presence, frequency;
@@ -27,6 +29,16 @@ struct RowArgs {
   int32_t *tokens;
   int32_t *status;
   RowStats *stats;
+  // rows >= split are rows of a second array with the same stride (the verifier's draft rows behind its target rows)
+  const float *logits2;
+  int split;
+  // statistics: every draw_every-th of the first array's rows is also drawn from (the last target row of each sequence,
+  // at (seeds[sequence], steps[sequence], slot, purpose)): the token goes into the record.  0: no draw
+  int draw_every;
+  double bound_scale;          // factor on the certification bounds (1; tests widen them)
+  const HeadRowStats *head_stats;  // optional [rows]: maximum / minimum / finiteness as the head left them (no penalties or mask)
+  FlatInfo *info;              // optional [rows]: what the window search found
+  int *replayed;               // optional counter of the replay behind this kernel, cleared here
   int only_uncovered;  // 1: process only rows the streaming path reported as not covered, leave the others alone
   const int *pending;  // optional, with only_uncovered: number of such rows; 0 = nothing to do, every CTA returns at once
   int rows;            // set by launch_rows: a cluster walks rows cluster, cluster + clusters, ... below this
@@ -168,124 +180,65 @@ __device__ int draw_token(RowCtx &c, double u, double rel_bound, double abs_boun
   return token;
 }
 
-// One row, start to finish, by the whole cluster.  Shared memory needs no particular content on entry.
-template <int kMode>
-__device__ __forceinline__ void row_body(const RowArgs &a, RowCtx &c, RowSmem *s, const int row) {
-  const float *logits = a.logits + size_t(row) * a.logits_stride;
-
-  bool used_tma;
-  stage_begin(c, logits, used_tma);
-  if (a.mask) {
-    const uint32_t *mw = a.mask + size_t(row) * a.mask_stride + (c.begin >> 5);
-    for (int w = c.tid; w < (c.len + 31) / 32; w += kThreads) s->mask_words[w] = __ldg(mw + w);
-  }
-  // ---- history counts (16-bit counters packed in pairs; remote shared-memory atomics route each id to its owner)
-  const bool penalised = a.history != nullptr && (a.repetition != 1.f || a.presence != 0.f || a.frequency != 0.f);
-  int hist_len = penalised ? (a.history_len ? a.history_len[row] : int(a.history_stride)) : 0;
-  const bool bad_history = hist_len < 0 || hist_len > 65535 || (long long)hist_len > a.history_stride;
-  if (bad_history) hist_len = 0;
-  if (hist_len > 0) {
-    for (int j = c.tid; j < kSliceCap / 2; j += kThreads) s->u.count_pairs[j] = 0;
-    c.cluster.sync();
-    const int32_t *h = a.history + size_t(row) * a.history_stride;
-    const int per = (hist_len + c.nranks - 1) / c.nranks;
-    const int h0 = min(hist_len, c.rank * per), h1 = min(hist_len, h0 + per);
-    for (int base = h0 + c.warp * 32; base < h1; base += kThreads) {
-      const int i = base + c.lane;
-      const int id = i < h1 ? __ldg(h + i) : -1;
-      const bool valid = id >= 0 && id < a.vocab;
-      const unsigned peers = __match_any_sync(0xffffffffu, valid ? id : -1);
-      if (valid && c.lane == __ffs(peers) - 1) {
-        const int owner = id / c.stride_ids, local = id - owner * c.stride_ids;
-        atomicAdd(c.cluster.map_shared_rank(&s->u.count_pairs[local >> 1], owner),
-                  uint32_t(__popc(peers)) << ((local & 1) * 16));
-      }
-    }
-    c.cluster.sync();
-  }
-  const bool landed = stage_wait(c, used_tma);
-
-  // ---- effective logits, first maximum, allowed count
-  int flags = (landed ? 0 : 8) | (bad_history ? 4 : 0);
-  float best = -CUDART_INF_F, lowest = CUDART_INF_F;  // lowest: smallest finite effective logit
-  int best_id = 0x7fffffff, allowed = 0;
-  for (int it = 0; it < c.region; it += 32) {
-    const int j = c.warp * c.region + it + c.lane;
-    if (j >= c.len) continue;
-    float x = s->y[j];
-    if ((__float_as_uint(x) & 0x7f800000u) == 0x7f800000u) flags |= 1;
-    if (hist_len > 0) {
-      const uint32_t cnt = (s->u.count_pairs[j >> 1] >> ((j & 1) * 16)) & 0xffffu;
-      if (cnt) {
-        const float v = x > 0.f ? __fdiv_rn(x, a.repetition) : __fmul_rn(x, a.repetition);
-        x = __fsub_rn(v, __fadd_rn(a.presence, __fmul_rn(a.frequency, float(cnt))));
-        if ((__float_as_uint(x) & 0x7f800000u) == 0x7f800000u) flags |= 2;
-      }
-    }
-    const bool ok = !a.mask || ((s->mask_words[j >> 5] >> (j & 31)) & 1u);
-    if (!ok) x = -CUDART_INF_F;
-    s->y[j] = x;
-    if (ok) {
-      ++allowed;
-      if (x > best) { best = x; best_id = c.begin + j; }
-      if (x > -CUDART_INF_F) lowest = fminf(lowest, x);
-    }
-  }
+// Occurrences of this CTA's ids in the row's history, as 16-bit counters packed in pairs.  Every CTA reads the whole
+// history (from L2 after the first of them) and counts the ids of its own slice with shared-memory atomics: eight times
+// the reads, but no cluster barrier and no atomics in another CTA's memory.
+__device__ __forceinline__ void count_history(RowCtx &c, const int32_t *h, int n) {
+  RowSmem *s = c.s;
+  uint4 *zero = reinterpret_cast<uint4 *>(s->work.count_pairs);
+  for (int j = c.tid; j < kSliceCap / 8; j += kThreads) zero[j] = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
-  {
-    Slot mine{};
-    // one fused block reduction: (best, best_id) by "larger value, then lower id", lowest, flags, allowed
+  const unsigned begin = unsigned(c.begin), len = unsigned(c.len);
+  auto count = [&](int id) {
+    const unsigned local = unsigned(id) - begin;   // (padding ids, negative or beyond the vocabulary, are nobody's)
+    if (local < len) atomicAdd(&s->work.count_pairs[local >> 1], 1u << ((local & 1u) * 16u));
+  };
+  int i = 0;
+  if ((reinterpret_cast<uintptr_t>(h) & 15u) == 0) {
+    const int4 *h4 = reinterpret_cast<const int4 *>(h);
+    const int vecs = n >> 2;
+    int v = c.tid;
+    for (; v + 7 * kThreads < vecs; v += 8 * kThreads) {
+      int4 q[8];
 #pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, best_id, o);
-      if (ov > best || (ov == best && oi < best_id)) { best = ov; best_id = oi; }
-      lowest = fminf(lowest, __shfl_xor_sync(0xffffffffu, lowest, o));
-    }
-    flags = int(__reduce_or_sync(0xffffffffu, unsigned(flags)));
-    allowed = __reduce_add_sync(0xffffffffu, allowed);
-    if (c.lane == 0) {
-      s->red_f[c.warp] = best; s->red_j[c.warp] = best_id; s->red_d[c.warp] = double(lowest);
-      s->red_q[c.warp] = (unsigned long long)(unsigned(allowed)) << 32 | unsigned(flags);
-    }
-    __syncthreads();
-    best = s->red_f[0]; best_id = s->red_j[0]; lowest = float(s->red_d[0]);
-    flags = int(unsigned(s->red_q[0])); allowed = int(s->red_q[0] >> 32);
+      for (int k = 0; k < 8; ++k) q[k] = __ldg(h4 + v + k * kThreads);
 #pragma unroll
-    for (int w = 1; w < kWarps; ++w) {
-      const float ov = s->red_f[w];
-      const int oi = s->red_j[w];
-      if (ov > best || (ov == best && oi < best_id)) { best = ov; best_id = oi; }
-      lowest = fminf(lowest, float(s->red_d[w]));
-      flags |= int(unsigned(s->red_q[w]));
-      allowed += int(s->red_q[w] >> 32);
+      for (int k = 0; k < 8; ++k) { count(q[k].x); count(q[k].y); count(q[k].z); count(q[k].w); }
     }
-    __syncthreads();
-    mine.f[0] = best; mine.i[0] = best_id; mine.f[1] = lowest;
-    mine.i[1] = flags;
-    mine.i[2] = allowed;
-    const Slot *all = exchange(c, mine);
-    best = all[0].f[0]; best_id = all[0].i[0]; flags = all[0].i[1]; allowed = all[0].i[2];
-    for (int r = 1; r < c.nranks; ++r) {
-      if (all[r].f[0] > best || (all[r].f[0] == best && all[r].i[0] < best_id)) { best = all[r].f[0]; best_id = all[r].i[0]; }
-      flags |= all[r].i[1];
-      allowed += all[r].i[2];
+    for (; v < vecs; v += kThreads) {
+      const int4 q = __ldg(h4 + v);
+      count(q.x); count(q.y); count(q.z); count(q.w);
     }
-    for (int r = 0; r < c.nranks; ++r) lowest = fminf(lowest, all[r].f[1]);
+    i = vecs << 2;
   }
-  int status = 0;
-  c.timed_out = (flags & 8) ? 1 : 0;
-  if (flags & 8) status = -5;
-  else if (flags & 1) status = -1;
-  else if (flags & 4) status = -7;
-  else if (flags & 2) status = -3;
-  else if (allowed == 0) status = -2;
+#pragma unroll 4
+  for (i += c.tid; i < n; i += kThreads) count(__ldg(h + i));
+}
 
-  const float max_logit = best;
-  const double t = a.temperature;
+// The general search on a valid row in place: top-k and top-p cuts of any kind by multi-level histograms (find_cut), then
+// the draw.  Rows come here when neither of the paths above fits them: plateaus of thousands of equal logits at the cut,
+// top_k in the thousands.  Out of line: its registers are not the other paths'.
+struct SearchArgs {
+  float max_logit;
+  int allowed, top_k;
+  double t, top_p;
+  bool draw;
+  double u, bound_scale;
+};
+struct SearchOut {
+  int status, token, kept, entered;
+  Cut cut;
+  double z, e_kept;
+};
+static __device__ __noinline__ SearchOut general_search(RowCtx &c, SearchArgs a) {
+  RowSmem *s = c.s;
+  const float max_logit = a.max_logit;
+  const double t = a.t;
+  SearchOut o{};
+  o.token = -1; o.kept = o.entered = a.allowed;
   // exp((y - max)/T) with the division replaced by a multiplication: the argument moves by at most one ulp, the
   // value by |argument| * 2^-53 relative (< 100 u), which every comparison made on sums of these weights allows for
-  const double inv_t = t > 0 ? 1.0 / t : 0.0;
+  const double inv_t = 1.0 / t;
   auto weight = [max_logit, inv_t](float y) { return exp_nonpos((double(y) - double(max_logit)) * inv_t); };
   Cut cut{-CUDART_INF_F, -1};
   // value of local id j for the sums and the draw: exp weight of a survivor of the CURRENT cut, else 0
@@ -294,105 +247,326 @@ __device__ __forceinline__ void row_body(const RowArgs &a, RowCtx &c, RowSmem *s
     const double w = weight(y);  // unconditional (0 for an excluded id): independent calls overlap
     return survives(y, c.begin + j, cut) ? w : 0.0;
   };
+  // ---- top-k
+  if (a.top_k > 0 && a.top_k < a.allowed) {
+    CutResult r = find_cut<false>(c, max_logit, 16.f / kBins, a.top_k, 0.0, a.allowed,
+                                  [](float y, int) { return y > -CUDART_INF_F; }, weight);
+    if (r.error) o.status = r.error;
+    else { cut = r.cut; o.entered = o.kept = a.top_k; }
+  }
+  const Cut base = cut;
+  // ---- normaliser and top-p
+  if (o.status == 0 && a.top_p < 1.0) {
+    CutResult r = find_cut<true>(c, max_logit, float(48.0 * t) / kBins, 0, a.top_p, o.entered,
+                                 [base](float y, int id) { return survives(y, id, base); }, weight);
+    if (r.error) o.status = r.error;
+    else {
+      o.z = r.z; o.e_kept = r.e_kept; o.kept = r.kept;
+      if (r.cut.id >= 0) cut = r.cut;
+      if (r.ambiguous) o.status |= 2;
+    }
+    if (o.status >= 0 && a.draw) region_sums(c, value);
+  } else if (o.status == 0) {
+    region_sums(c, value);
+    double block_total = 0;
+    for (int w = 0; w < kWarps; ++w) block_total += s->warp_sum[w];
+    Slot mine{};
+    mine.d[0] = block_total;
+    const Slot *all = exchange(c, mine);
+    for (int r = 0; r < c.nranks; ++r) o.z += all[r].d[0];
+    o.e_kept = o.z;
+  }
+  if (o.status >= 0 && a.draw) {
+    int amb = 0;
+    double total;
+    o.token = draw_token(c, a.u, (2.0 * o.kept + 512.0) * kU * a.bound_scale, 0.0, value, &amb, &total);
+    if (amb) o.status |= 1;
+  }
+  o.cut = cut;
+  return o;
+}
+
+// One row, start to finish, by the whole cluster.  Shared memory needs no particular content on entry.  Returns true if a
+// barrier of the cluster already lies behind the last access to another CTA's shared memory.
+template <int kMode>
+__device__ __forceinline__ bool row_body(const RowArgs &a, RowCtx &c, RowSmem *s, const int row) {
+  const float *logits = row < a.split ? a.logits + size_t(row) * a.logits_stride
+                                      : a.logits2 + size_t(row - a.split) * a.logits_stride;
+
+  bool used_tma;
+  stage_begin(c, logits, used_tma);
+  {  // reset what the paths below count in
+    uint4 *zero = reinterpret_cast<uint4 *>(s->bin_mass);
+    static_assert(sizeof(s->bin_mass) == 16 * kThreads, "one store per thread");
+    zero[c.tid] = make_uint4(0u, 0u, 0u, 0u);
+    if (c.tid < kSampleBins) s->bin_count[c.tid] = 0;
+    if (c.tid == 0) { s->list_count = 0; s->decided = 0; s->window[0] = s->window[1] = ~0ull; }
+  }
+  if (a.mask) {
+    const uint32_t *mw = a.mask + size_t(row) * a.mask_stride + (c.begin >> 5);
+    for (int w = c.tid; w < (c.len + 31) / 32; w += kThreads) s->mask_words[w] = __ldg(mw + w);
+  }
+  const bool penalised = a.history != nullptr && (a.repetition != 1.f || a.presence != 0.f || a.frequency != 0.f);
+  int hist_len = penalised ? (a.history_len ? a.history_len[row] : int(a.history_stride)) : 0;
+  const bool bad_history = hist_len < 0 || hist_len > 65535 || (long long)hist_len > a.history_stride;
+  if (bad_history) hist_len = 0;
+  if (hist_len > 0) count_history(c, a.history + size_t(row) * a.history_stride, hist_len);
+  // the row's uniform, by one lane while the slice is on its way
+  const double t = a.temperature;
+  const bool draw = t != 0 && (kMode == kModeSample ||
+                               (a.draw_every > 0 && row < a.split && row % a.draw_every == a.draw_every - 1));
+  if (draw && c.tid == kThreads - 1) {
+    const int address = kMode == kModeSample ? row : row / a.draw_every;
+    s->u = philox_uniform(a.seeds[address], a.steps[address], a.slot, a.purpose);
+  }
+  // placement of the row's ids on the histogram, by one lane.  A range beyond the exponent limit is cut off there: what lies
+  // further down goes to the last bin, whose lower bracket is then zero
+  auto place_row = [&](float m, float low) {
+    const bool clipped = !(__fsub_rn(m, low) <= a.reach);
+    const FlatMap b = make_map(m, clipped ? __fsub_rn(m, a.reach) : low, a.log2e_t);
+    s->map.scale = b.scale; s->map.kappa = b.kappa; s->map.ok = b.ok ? 1 : 0; s->map.clipped = clipped ? 1 : 0;
+  };
+  const bool known = a.head_stats != nullptr && !penalised && !a.mask && t > 0 && a.top_k == 0 && c.vocab > kListCap;
+  if (known && c.tid == 0) {           // the head left the row's extremes (whether the slices landed comes with the sums)
+    const HeadRowStats h = a.head_stats[row];
+    const float m = unorder_bits(uint32_t(h.max_key >> 32)), low = unorder_bits(~h.min_key);
+    s->facts.max_logit = m; s->facts.lowest = low; s->facts.best_id = int(0xffffffffu - uint32_t(h.max_key));
+    s->facts.flags = int(h.flags & 1u); s->facts.allowed = c.vocab; s->facts.cutoff = -CUDART_INF_F;
+    place_row(m, low);
+  }
+  const bool landed = stage_wait(c, used_tma);
+
+  // ---- effective logits, first maximum, smallest finite logit, allowed count; the threads' own maxima
+  if (!known) {
+    float best = -CUDART_INF_F, low = CUDART_INF_F, poison = 0.f;
+    int id = 0x7fffffff, over = 0, count = 0;
+    float4 *y4 = reinterpret_cast<float4 *>(s->y);
+    const int j0 = c.warp * c.region + 4 * c.lane;
+    auto take = [&](float y, int j) {
+      if (y > best) { best = y; id = j; }
+    };
+    if (hist_len == 0 && !a.mask) {    // every id as it is
+      count = max(0, min(c.len - c.warp * c.region, c.region));   // (per warp; lane 0's counts)
+      if (c.lane) count = 0;
+#pragma unroll 2
+      for (int j = j0; j < j0 + c.region; j += 128) {
+        const int left = c.len - j;
+        const float4 q = y4[j >> 2];
+        if (left >= 4) {
+          poison = fmaf(q.x, 0.f, fmaf(q.y, 0.f, fmaf(q.z, 0.f, fmaf(q.w, 0.f, poison))));  // NaN once a logit is NaN or infinite
+          if (fmaxf(fmaxf(q.x, q.y), fmaxf(q.z, q.w)) > best) { take(q.x, j); take(q.y, j + 1); take(q.z, j + 2); take(q.w, j + 3); }
+          low = fminf(fminf(low, fminf(q.x, q.y)), fminf(q.z, q.w));
+        } else if (left > 0) {         // the last ids of the vocabulary
+          const float y[3] = {q.x, q.y, q.z};
+          for (int k = 0; k < left; ++k) { poison = fmaf(y[k], 0.f, poison); take(y[k], j + k); low = fminf(low, y[k]); }
+        }
+      }
+    } else {
+#pragma unroll 1
+      for (int j = j0; j < j0 + c.region; j += 128) {
+        const int left = c.len - j;
+        if (left <= 0) break;
+        const float4 q = y4[j >> 2];
+        float y[4] = {q.x, q.y, q.z, q.w};
+        unsigned in = left >= 4 ? 15u : (1u << left) - 1u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) poison = fmaf((in >> k) & 1u ? y[k] : 0.f, 0.f, poison);
+        if (a.mask) in &= s->mask_words[j >> 5] >> (j & 31);
+        if (hist_len > 0) {
+          const uint2 w = *reinterpret_cast<const uint2 *>(&s->work.count_pairs[j >> 1]);
+          if (w.x | w.y) {
+#pragma unroll 1
+            for (int k = 0; k < 4; ++k) {
+              const uint32_t cnt = ((k & 2 ? w.y : w.x) >> (16 * (k & 1))) & 0xffffu;
+              if (cnt) {
+                const float x = y[0];  // (rotated below, so that the loop keeps to one copy of the division)
+                const float v = x > 0.f ? __fdiv_rn(x, a.repetition) : __fmul_rn(x, a.repetition);
+                y[0] = __fsub_rn(v, __fadd_rn(a.presence, __fmul_rn(a.frequency, float(cnt))));
+                if ((__float_as_uint(y[0]) & 0x7f800000u) == 0x7f800000u) over = 2;
+              }
+              const float r = y[0];
+              y[0] = y[1]; y[1] = y[2]; y[2] = y[3]; y[3] = r;
+            }
+          }
+        }
+        count += __popc(in);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const bool ok = (in >> k) & 1u;
+          y[k] = ok ? y[k] : -CUDART_INF_F;
+          low = fminf(low, ok ? y[k] : CUDART_INF_F);
+          take(y[k], j + k);
+        }
+        y4[j >> 2] = make_float4(y[0], y[1], y[2], y[3]);
+      }
+    }
+    // one fused reduction: first maximum as (ordered logit, id), smallest, flags, count, least thread maximum
+    int flags = (landed ? 0 : 8) | (bad_history ? 4 : 0) | over | (poison == 0.f ? 0 : 1);
+    const bool sampled = a.top_k > 0 && a.top_k <= kTopkSampled && t > 0;
+    const bool any = best > -CUDART_INF_F;
+    uint32_t top = ordered_bits(best), low_bits = ordered_bits(low), least = any ? top : 0xffffffffu;
+    auto warp_reduce = [&] {
+      const uint32_t m = __reduce_max_sync(0xffffffffu, top);
+      id = int(__reduce_min_sync(0xffffffffu, top == m ? unsigned(id) : 0x7fffffffu));
+      top = m;
+      low_bits = __reduce_min_sync(0xffffffffu, low_bits);
+      flags = int(__reduce_or_sync(0xffffffffu, unsigned(flags)));
+      count = __reduce_add_sync(0xffffffffu, count);
+      if (sampled) least = __reduce_min_sync(0xffffffffu, least);
+    };
+    warp_reduce();
+    if (c.lane == 0) {
+      s->red_q[c.warp] = (unsigned long long)top << 32 | unsigned(id);
+      s->warp_sum[c.warp] = __longlong_as_double((long long)((unsigned long long)low_bits << 32 | least));
+      s->red_j[c.warp] = flags; s->red_k[c.warp] = count;
+    }
+    __syncthreads();
+    uint32_t threshold = 0;
+    if (sampled || c.warp == 0) {
+      const int w = c.lane & (kWarps - 1);
+      const unsigned long long pair = (unsigned long long)__double_as_longlong(s->warp_sum[w]);
+      top = uint32_t(s->red_q[w] >> 32); id = int(uint32_t(s->red_q[w]));
+      low_bits = uint32_t(pair >> 32); least = uint32_t(pair);
+      flags = s->red_j[w]; count = c.lane < kWarps ? s->red_k[w] : 0;
+      warp_reduce();
+      if (sampled) {
+        const float most = unorder_bits(top), fewest = least == 0xffffffffu ? most : unorder_bits(least);
+        const float scale = sample_scale(most, fewest);
+        if (any) atomicAdd(&s->bin_count[sample_bin(best, most, scale)], 1);
+        __syncthreads();
+        if (c.warp == 0)
+          threshold = sampled_threshold(c.lane, s->bin_count, most, fewest, scale,
+                                        (a.top_k + threshold_groups(c) - 1) / threshold_groups(c));
+      }
+    }
+    Slot mine{};                           // (warp 0 has the CTA's values, and is the one that exchange() writes from)
+    mine.q[0] = (unsigned long long)top << 32 | unsigned(c.begin + id);
+    mine.i[0] = int(low_bits); mine.i[1] = flags; mine.i[2] = count; mine.i[3] = int(threshold);
+    const Slot *all = exchange(c, mine);   // (its barrier also separates the reads above from the next use of red_*)
+    if (c.warp == 0) {
+      const int r = c.lane & (kMaxCluster - 1);
+      const bool in = c.lane < c.nranks;
+      top = in ? uint32_t(all[r].q[0] >> 32) : 0u; id = in ? int(uint32_t(all[r].q[0])) : 0x7fffffff;
+      low_bits = in ? uint32_t(all[r].i[0]) : 0xffffffffu;
+      flags = in ? all[r].i[1] : 0; count = in ? all[r].i[2] : 0;
+      threshold = in ? uint32_t(all[r].i[3]) : 0u;
+      warp_reduce();                       // (ids ascend with the rank: the first maximum keeps ties)
+      if (sampled) {                       // the groups-th largest threshold: that many CTAs hold their share above it
+        for (int g = 1; g < threshold_groups(c); ++g) {
+          const uint32_t largest = __reduce_max_sync(0xffffffffu, threshold);
+          const unsigned who = __ballot_sync(0xffffffffu, threshold == largest);
+          if (c.lane == __ffs(who) - 1) threshold = 0u;
+        }
+        threshold = __reduce_max_sync(0xffffffffu, threshold);
+      }
+      if (c.lane == 0) {
+        const float m = unorder_bits(top), lowest_all = unorder_bits(low_bits);
+        s->facts.max_logit = m; s->facts.lowest = lowest_all; s->facts.best_id = id;
+        s->facts.flags = flags; s->facts.allowed = count;
+        s->facts.cutoff = threshold ? unorder_bits(threshold) : -CUDART_INF_F;
+        if (t > 0 && a.top_p < 1.0) place_row(m, lowest_all);
+      }
+    }
+    __syncthreads();
+  }
+  const float max_logit = s->facts.max_logit, lowest = s->facts.lowest, cutoff = s->facts.cutoff;
+  const int best_id = s->facts.best_id, flags = s->facts.flags, allowed = s->facts.allowed;
+  int status = 0;
+  c.timed_out = (flags & 8) ? 1 : 0;
+  if (flags & 8) status = -5;
+  else if (flags & 1) status = -1;
+  else if (flags & 4) status = -7;
+  else if (flags & 2) status = -3;
+  else if (allowed == 0) status = -2;
+
+  Cut cut{-CUDART_INF_F, -1};
   int entered = allowed, kept = allowed;
   double z = 0, e_kept = 0;
   int token = -1;
-
-  bool wide_done = false;
-  if (status == 0 && t != 0 && a.top_p < 1.0 && (a.top_k <= 0 || a.top_k >= allowed) && allowed > 2 * kListCap &&
-      lowest < max_logit) {
-    const WideOutcome w = wide_nucleus(c, max_logit, lowest, t, a.top_p, allowed);
-    if (w.applicable) {
-      wide_done = true;
-      cut = w.cut; kept = w.kept; z = w.z; e_kept = w.e_kept;
-      if (w.ambiguous) status |= 2;
-    }
-  }
-  if (!wide_done) {
-    if (status == 0 && t != 0) {
-      const double u = kMode == kModeSample ? philox_uniform(a.seeds[row], a.steps[row], a.slot, a.purpose) : 0.0;
-      const FastOutcome f = fast_small_support(c, max_logit, t, allowed, a.top_k, a.top_p, u, kMode == kModeSample);
+  bool decided = false, recorded = false, writer = c.rank == 0, closed = false;
+  if (status == 0 && t != 0) {
+    const bool counted = a.top_k > 0 && a.top_k < allowed;
+    if (!counted && allowed > kListCap) {
+      const NucleusArgs na{max_logit, a.floor_gap, a.log2e_t, a.top_p, allowed, landed, draw,
+                           kMode == kModeSample ? a.bound_scale : 1.0, a.bound_scale};
+      const NucleusOut n = nucleus_row(c, na);
+      if (n.timed_out) { c.timed_out = 1; status = -5; decided = true; }
+      else if (n.done) {
+        decided = closed = true;
+        writer = n.mine;       // (the CTA that holds the id at the cut)
+        status = n.status; token = n.token; cut = n.cut; kept = n.kept; z = n.z; e_kept = n.e_kept;
+      }
+      if (a.info && c.rank == 0 && c.tid == 0) {
+        FlatInfo f{};
+        f.max = max_logit; f.min = lowest; f.argmax = best_id;
+        f.applicable = n.done && !n.clipped ? 1 : 0;
+        f.w0 = n.w0; f.w1 = n.w1; f.n_before = n.n_before; f.n_window = n.n_window;
+        f.pad[0] = f.applicable ? 0 : 1;       // left to the general search
+        a.info[row] = f;
+      }
+      recorded = true;
+    } else {
+      const FastOutcome f = fast_small_support(c, max_logit, t, allowed, a.top_k, a.top_p, cutoff, draw ? s->u : 0.0, draw);
       if (f.applicable) {
-        // ranks other than 0 are done after the gather; rank 0 finishes alone and touches only its own shared memory
-        if (c.rank == 0 && c.tid == 0) {
-          if (kMode == kModeSample) {
-            a.tokens[row] = f.token;
-            if (a.status) a.status[row] = f.status;
-          } else {
-            RowStats st;
-            st.z = f.z; st.e_kept = f.e_kept; st.max_logit = max_logit; st.argmax = best_id; st.cut = f.cut;
-            st.kept = f.kept; st.entered = f.entered; st.status = f.status; st.pad = 0;
-            a.stats[row] = st;
-          }
-        }
-        return;
+        decided = true;
+        status = f.status; token = f.token; cut = f.cut; kept = f.kept; entered = f.entered; z = f.z; e_kept = f.e_kept;
       }
     }
   }
-  if (wide_done) {
-    // cut, sums and region sums are in place
-  } else if (status == 0 && t == 0) {
-    token = best_id;
-    kept = 1; z = 1; e_kept = 1;
-    cut.y = max_logit; cut.id = best_id;
-  } else if (status == 0) {
-    // ---- top-k
-    if (a.top_k > 0 && a.top_k < allowed) {
-      CutResult r = find_cut<false>(c, max_logit, 16.f / kBins, a.top_k, 0.0, allowed,
-                                    [](float y, int) { return y > -CUDART_INF_F; }, weight);
-      if (r.error) status = r.error;
-      else { cut = r.cut; entered = kept = a.top_k; }
-    }
-    const Cut base = cut;
-    // ---- normaliser and top-p
-    if (status == 0 && a.top_p < 1.0) {
-      CutResult r = find_cut<true>(c, max_logit, float(48.0 * t) / kBins, 0, a.top_p, entered,
-                                   [base](float y, int id) { return survives(y, id, base); }, weight);
-      if (r.error) status = r.error;
-      else {
-        z = r.z; e_kept = r.e_kept; kept = r.kept;
-        if (r.cut.id >= 0) cut = r.cut;
-        if (r.ambiguous) status |= 2;
-      }
-      if (status >= 0 && kMode == kModeSample) region_sums(c, value);
+  if (a.info && !recorded && c.rank == 0 && c.tid == 0) {
+    FlatInfo f{};
+    f.max = max_logit; f.min = lowest; f.argmax = best_id;
+    f.pad[0] = status == 0 ? 1 : 0;
+    a.info[row] = f;
+  }
+  if (known && !decided) {   // the general search needs every slice in place
+    Slot mine{};
+    mine.i[0] = landed ? 0 : 1;
+    const Slot *all = exchange(c, mine);
+    for (int r = 0; r < c.nranks; ++r)
+      if (all[r].i[0]) { c.timed_out = 1; status = -5; }
+  }
+  if (!decided) {
+    if (status == 0 && t == 0) {
+      token = best_id;
+      kept = 1; z = 1; e_kept = 1;
+      cut.y = max_logit; cut.id = best_id;
     } else if (status == 0) {
-      region_sums(c, value);
-      double block_total = 0;
-      for (int w = 0; w < kWarps; ++w) block_total += s->warp_sum[w];
-      Slot mine{};
-      mine.d[0] = block_total;
-      const Slot *all = exchange(c, mine);
-      for (int r = 0; r < c.nranks; ++r) z += all[r].d[0];
-      e_kept = z;
+      RowCtx copy = c;
+      SearchOut o = general_search(copy, SearchArgs{max_logit, allowed, a.top_k, t, a.top_p, draw, draw ? s->u : 0.0, a.bound_scale});
+      c.xphase = copy.xphase;
+      status = o.status; token = o.token; cut = o.cut; kept = o.kept; entered = o.entered; z = o.z; e_kept = o.e_kept;
     }
   }
-  if (status >= 0 && t != 0 && kMode == kModeSample) {
-    const double u = philox_uniform(a.seeds[row], a.steps[row], a.slot, a.purpose);
-    int amb = 0;
-    double total;
-    token = draw_token(c, u, (2.0 * kept + 512.0) * kU, 0.0, value, &amb, &total);
-    if (amb) status |= 1;
-  }
-  if (c.rank == 0 && c.tid == 0) {
+  if (writer && c.tid == 0) {
     if (kMode == kModeSample) {
       a.tokens[row] = status < 0 ? -1 : token;
       if (a.status) a.status[row] = status;
     } else {
       RowStats st;
       st.z = z; st.e_kept = e_kept; st.max_logit = max_logit; st.argmax = best_id; st.cut = cut;
-      st.kept = kept; st.entered = entered; st.status = status; st.pad = 0;
+      st.kept = kept; st.entered = entered;
+      // a close draw is the drawn token's affair: it only counts if the verifier uses the token
+      st.drawn = draw && status >= 0 && token >= 0 ? token | ((status & 1) ? kDrawnClose : 0) : -1;
+      st.status = status < 0 ? status : status & ~1;
       a.stats[row] = st;
     }
   }
+  return closed;
 }
 
 // A cluster takes rows cluster, cluster + clusters, ...: one row per cluster when the launch has a cluster per row; a
 // small persistent grid when only the rows another path left over (status -8 / -9) are wanted, so that a launch with
 // nothing to do costs a few status reads instead of thousands of cluster launches.
-template <int kMode>
-__global__ void __launch_bounds__(kThreads, 2) row_kernel(RowArgs a) {
+template <int kMode, int kPerSm>
+__global__ void __launch_bounds__(kThreads, kPerSm) row_kernel(const __grid_constant__ RowArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   RowSmem *s = reinterpret_cast<RowSmem *>(smem_raw);
+  prepare_smem(s);
+  // (programmatic launches: what is in front of this kernel in the stream has finished; what follows may be set up)
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+  if (a.replayed && blockIdx.x == 0 && threadIdx.x == 0) *a.replayed = 0;
   if (a.only_uncovered && a.pending && *a.pending == 0) return;  // the same in every CTA of the grid
   RowCtx c = make_ctx(s, a.vocab);
   const int clusters = int(gridDim.x) / c.nranks;
@@ -401,9 +575,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_kernel(RowArgs a) {
       const int st = kMode == kModeSample ? a.status[row] : a.stats[row].status;
       if (st != -8 && st != -9) continue;  // -9: handed on by the batch path for wide nuclei (flat.cuh)
     }
-    row_body<kMode>(a, c, s, row);
     // no CTA may exit, or stage the next row, while a peer can still address its shared memory
-    c.cluster.sync();
+    if (!row_body<kMode>(a, c, s, row)) c.cluster.sync();
     if (c.timed_out) {  // a bounded wait expired: this cluster reports its remaining rows and stops
       if (c.rank == 0 && c.tid == 0) {
         for (int r = row + clusters; r < a.rows; r += clusters) {

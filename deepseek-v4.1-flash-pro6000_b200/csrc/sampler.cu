@@ -4,12 +4,15 @@
 #include "stream_types.cuh"
 #include "flat.cuh"
 #include "replay.cuh"
+#include "launch.h"
 #include "phase_events.h"
 #include "host_error.h"
 #include <cmath>
 #include <cstdlib>
 
 namespace ds41 {
+
+constexpr int kOnePerSm = 96;   // CTAs
 
 int cluster_size_for(int vocab) {
   int n = 1;
@@ -19,32 +22,49 @@ int cluster_size_for(int vocab) {
   return n;
 }
 
-template <int kMode>
-cudaError_t launch_rows(const RowArgs &a, int rows, cudaStream_t stream) {
+template <int kMode, int kPerSm>
+cudaError_t launch_rows(const RowArgs &args, int clusters, int cl, int dev, cudaStream_t stream) {
   static thread_local int configured_device = -1;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
   if (configured_device != dev) {
-    e = cudaFuncSetAttribute(row_kernel<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(RowSmem)));
+    const cudaError_t e = cudaFuncSetAttribute(row_kernel<kMode, kPerSm>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               int(sizeof(RowSmem)));
     if (e != cudaSuccess) return e;
     configured_device = dev;
   }
-  const int cl = cluster_size_for(a.vocab);
-  RowArgs args = a;
-  args.rows = rows;
-  // left-over rows only: a persistent grid of two clusters per 8 SMs walks the status words
-  const int clusters = a.only_uncovered ? (rows < 74 ? rows : 74) : rows;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(unsigned(clusters) * cl);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = sizeof(RowSmem);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = cl; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, row_kernel<kMode>, args);
+  attr[1] = programmatic_launch();
+  cfg.attrs = attr; cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, row_kernel<kMode, kPerSm>, args);
+}
+
+template <int kMode>
+cudaError_t launch_rows(const RowArgs &a, int rows, cudaStream_t stream) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const int cl = cluster_size_for(a.vocab);
+  RowArgs args = a;
+  args.rows = rows;
+  if (!args.logits2) args.split = rows;
+  if (!(args.bound_scale > 0)) args.bound_scale = 1.0;
+  if (a.temperature > 0) {
+    args.log2e_t = kLog2e / a.temperature;
+    args.reach = float(0.999 * kFlatMaxExponent / kLog2e * a.temperature);
+    args.floor_gap = float(650.0 / kLog2e * a.temperature);
+  }
+  // left-over rows only: a persistent grid of two clusters per 8 SMs walks the status words
+  const int clusters = a.only_uncovered ? (rows < 74 ? rows : 74) : rows;
+  // A grid that fits the GPU with one CTA per SM gets 128 registers per thread: no spills, and more of a step's loads and
+  // FP64 chains in flight.  A larger one is better off with two CTAs per SM, which fill each other's waits at the barriers
+  if (clusters * cl <= kOnePerSm) return launch_rows<kMode, 1>(args, clusters, cl, dev, stream);
+  return launch_rows<kMode, 2>(args, clusters, cl, dev, stream);
 }
 template cudaError_t launch_rows<kModeSample>(const RowArgs &, int, cudaStream_t);
 template cudaError_t launch_rows<kModeStats>(const RowArgs &, int, cudaStream_t);
@@ -132,6 +152,27 @@ extern "C" double ds41_spark_uniform_v2(uint64_t seed, uint64_t step, uint32_t s
 }
 extern "C" const char *ds41_spark_error(void) { return last_error(); }
 
+namespace {
+// Up to this many rows the cluster kernel takes a batch cut by top-p alone in one launch.
+constexpr int kClusterRows = 48;
+
+// One launch that decides every row, and the replay of the rows it could not certify.
+int sample_by_clusters(RowArgs a, const ds41_b200_sample_args &p, cudaStream_t stream) {
+  unsigned char *flat_scratch = static_cast<unsigned char *>(p.scratch) + streaming_bytes(p.rows, p.vocab);
+  a.status = p.status ? p.status
+                      : reinterpret_cast<int32_t *>(static_cast<ChunkRecord *>(p.scratch) + size_t(p.rows) * chunks_for(p.vocab));
+  a.head_stats = static_cast<const HeadRowStats *>(p.row_extremes);
+  a.bound_scale = bound_scale();
+  a.info = flat_info(flat_scratch, p.rows);
+  a.replayed = const_cast<int *>(flat_pending(flat_scratch)) + 1;
+  cudaError_t e = launch_rows<kModeSample>(a, p.rows, stream);
+  if (e != cudaSuccess) return int(e);
+  ReplayArgs r{p.logits, p.logits_stride, p.vocab, p.rows, a.temperature, p.top_p, p.seeds, p.steps, p.slot, p.purpose,
+               p.tokens, a.status, flat_scratch + flat_scratch_bytes(p.rows), a.replayed, a.info};
+  return int(launch_replay(r, stream));
+}
+}  // namespace
+
 extern "C" int ds41_b200_sample_logits(const ds41_b200_sample_args *p, cudaStream_t stream) {
   if (!p || p->struct_bytes != sizeof(ds41_b200_sample_args)) return invalid("sample args: struct size / ABI mismatch");
   if (p->rows < 1 || p->vocab < 1 || p->vocab > DS41_B200_MAX_VOCAB) return invalid("sample args: rows/vocab out of range");
@@ -160,7 +201,8 @@ extern "C" int ds41_b200_sample_logits(const ds41_b200_sample_args *p, cudaStrea
   // Batches of rows that are only cut by top-p first go through the batch path; it answers the rows it fits and marks
   // the others -8 / -9, and the paths below then only touch those.
   const bool flat = scratch_ok && flat_shape(p->rows, p->vocab) && p->top_k == 0 && p->temperature > 0 &&
-                    p->logits_stride != 0 && p->logits_stride % 4 == 0 && !(reinterpret_cast<uintptr_t>(p->logits) & 15u);
+                    flat_aligned(p->logits, p->logits_stride);
+  if (flat && p->rows <= kClusterRows) return sample_by_clusters(a, *p, stream);
   // the streaming path covers small nuclei only: a full-vocabulary draw never fits its candidate sets
   const bool streaming = scratch_ok && (p->top_p < 1.0 || p->top_k > 0 || p->temperature == 0);
   if (!flat && !streaming) return int(launch_rows<kModeSample>(a, p->rows, stream));

@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(kCombineThreads) combine_kernel(CombineArgs a)
       else {
         RowStats st{};
         st.z = 1; st.e_kept = 1; st.max_logit = m; st.argmax = arg; st.cut.y = m; st.cut.id = arg; st.kept = 1;
-        st.entered = a.vocab; st.status = status;
+        st.entered = a.vocab; st.status = status; st.drawn = -1;
         a.stats[row] = st;
       }
     }
@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(kCombineThreads) combine_kernel(CombineArgs a)
     if (tid == 0) {
       RowStats st;
       st.z = s.d_out[0]; st.e_kept = s.d_out[1]; st.max_logit = m; st.argmax = arg;
-      st.cut.y = s.sy[kept - 1]; st.cut.id = s.sid[kept - 1]; st.kept = kept; st.entered = s.i_out[2]; st.status = status; st.pad = 0;
+      st.cut.y = s.sy[kept - 1]; st.cut.id = s.sid[kept - 1]; st.kept = kept; st.entered = s.i_out[2]; st.status = status; st.drawn = -1;
       a.stats[row] = st;
     }
     return;

@@ -11,6 +11,7 @@
 //      rows (normally still L2 resident), otherwise the bonus token is drawn from the last target row.
 #include <atomic>
 #include "ds41_b200.h"
+#include "flat.cuh"
 #include "host_error.h"
 #include "replay.cuh"
 #include "row_kernel.cuh"
@@ -23,8 +24,6 @@ template <int kMode>
 cudaError_t launch_rows(const RowArgs &a, int rows, cudaStream_t stream);
 int cluster_size_for(int vocab);
 int chunks_for(int vocab);
-cudaError_t launch_chunks(const ChunkArgs &a, int rows, cudaStream_t stream);
-cudaError_t launch_combine(const CombineArgs &a, bool stats, cudaStream_t stream);
 
 struct VerifyArgs {
   const float *target, *draft;
@@ -46,7 +45,8 @@ struct Measure {  // one row's probability measure: P(id) = survives ? exp((x-ma
     const float y = __ldg(x + id);
     return survives(y, id, st.cut) ? exp_nonpos((double(y) - double(st.max_logit)) * inv_t) * inv_kept : 0.0;
   }
-  __device__ __forceinline__ double bound() const { return 2.0 * (double(st.kept) + 256.0) * kU; }
+  // (a sum of kept weights and one weight: roundings, and the error of a weight of the FP64 passes, kFlatWeightUlps)
+  __device__ __forceinline__ double bound() const { return 2.0 * (double(st.kept) + 1600.0) * kU; }
 };
 
 __global__ void __launch_bounds__(kThreads, 2) verify_kernel(VerifyArgs a) {
@@ -112,6 +112,9 @@ __global__ void __launch_bounds__(kThreads, 2) verify_kernel(VerifyArgs a) {
     Measure P{a.target + (size_t(seq) * (D + 1) + D) * a.vocab, ps, greedy ? 0.0 : 1.0 / a.temperature, 1.0 / ps.e_kept};
     if (greedy) {
       r.tokens[r.emitted++] = P.st.argmax;
+    } else if (ps.drawn >= 0) {   // drawn with the row's statistics
+      if (ps.drawn & kDrawnClose) status |= 1;
+      r.tokens[r.emitted++] = ps.drawn & ~kDrawnClose;
     } else {
       auto value = [&](int j) { return P.at(c.begin + j) * P.st.e_kept; };  // unnormalised weights, as the sampler
       region_sums(c, value);
@@ -136,7 +139,11 @@ __global__ void __launch_bounds__(kThreads, 2) verify_kernel(VerifyArgs a) {
 
 namespace ds41 {
 namespace {
-// [row statistics][chunk records of the streaming path], rounded up to 16 bytes; the replay's rows follow
+// Up to this many rows the cluster kernel takes the statistics in one launch; beyond, the batch path's grid-wide passes do
+// (they need scratch and aligned rows).
+constexpr int kClusterStatRows = 40;
+// [row statistics][room that earlier versions used], rounded up to 16 bytes; the replay's rows follow, then the batch path's
+// scratch
 size_t verify_streaming_bytes(int sequences, int drafts, int vocab) {
   const size_t rows = size_t(sequences) * size_t(2 * drafts + 1);
   return (rows * sizeof(RowStats) + rows * chunks_for(vocab) * sizeof(ChunkRecord) + 15) & ~size_t(15);
@@ -148,7 +155,9 @@ using namespace ds41;
 
 extern "C" size_t ds41_b200_verify_scratch_bytes_for(int sequences, int drafts, int vocab) {
   if (sequences < 1 || drafts < 0 || drafts > 5 || vocab < 1 || vocab > DS41_B200_MAX_VOCAB) return 0;
-  return verify_streaming_bytes(sequences, drafts, vocab) + verify_replay_scratch_bytes();
+  const int rows = sequences * (2 * drafts + 1);
+  return verify_streaming_bytes(sequences, drafts, vocab) + verify_replay_scratch_bytes() +
+         (vocab >= kFlatMinVocab && rows > kClusterStatRows ? flat_scratch_bytes(rows) : 0);
 }
 extern "C" size_t ds41_b200_verify_scratch_bytes(int sequences, int drafts) {
   return ds41_b200_verify_scratch_bytes_for(sequences, drafts, DS41_B200_MAX_VOCAB);
@@ -169,37 +178,41 @@ extern "C" int ds41_b200_verify_logits(const ds41_b200_verify_args *p, cudaStrea
     return invalid("verify scratch too small or misaligned");
   RowStats *pstats = static_cast<RowStats *>(p->scratch);
   RowStats *qstats = pstats + size_t(p->sequences) * (p->drafts + 1);
-  // with room for the chunk records the row statistics come from the streaming path (cluster kernel only for rows
-  // it cannot cover); with statistics-only scratch every row goes through the cluster kernel
+  // one launch over all target and draft rows (the draft rows' records lie right behind the target rows'), which also
+  // draws from every sequence's last target row: the bonus token, should every draft be accepted
   const size_t streaming_need = verify_streaming_bytes(p->sequences, p->drafts, p->vocab);
-  const bool streaming = p->scratch_bytes >= streaming_need;
-  ChunkRecord *records = reinterpret_cast<ChunkRecord *>(pstats + stat_rows);
   RowArgs a{};
   a.vocab = p->vocab; a.logits_stride = p->vocab;
   a.temperature = p->temperature > 0 ? std::fmax(p->temperature, 1e-5) : 0.0;
   a.top_p = p->top_p; a.top_k = 0; a.repetition = 1.f;
-  cudaError_t e = cudaSuccess;
-  auto row_stats = [&](const float *logits, RowStats *stats, int rows, ChunkRecord *rec) -> cudaError_t {
-    a.logits = logits; a.stats = stats; a.only_uncovered = 0;
-    if (streaming) {
-      const int chunks = chunks_for(p->vocab);
-      ChunkArgs c{logits, p->vocab, p->vocab, 0, chunks, a.temperature, rec};
-      cudaError_t err = launch_chunks(c, rows, stream);
-      if (err != cudaSuccess) return err;
-      CombineArgs m{rec, rows, 1, chunks, p->vocab, a.temperature, p->top_p, 0, nullptr, nullptr, 0, 0, nullptr, nullptr, stats};
-      err = launch_combine(m, true, stream);
-      if (err != cudaSuccess) return err;
-      a.only_uncovered = 1;
+  a.stats = pstats;
+  a.logits = p->target_logits;
+  int stat_launch_rows = p->sequences * (p->drafts + 1);
+  if (!greedy) {
+    a.draw_every = p->drafts + 1;
+    a.seeds = p->seeds; a.steps = p->steps; a.slot = uint32_t(p->drafts); a.purpose = 0;
+    a.bound_scale = bound_scale();
+    if (p->drafts) {
+      a.logits2 = p->draft_logits; a.split = stat_launch_rows;
+      stat_launch_rows = int(stat_rows);
     }
-    return launch_rows<kModeStats>(a, rows, stream);
-  };
-  e = row_stats(p->target_logits, pstats, p->sequences * (p->drafts + 1), records);
-  if (e != cudaSuccess) return int(e);
-  if (p->drafts && !greedy) {
-    e = row_stats(p->draft_logits, qstats, p->sequences * p->drafts,
-                  records + size_t(p->sequences) * (p->drafts + 1) * chunks_for(p->vocab));
-    if (e != cudaSuccess) return int(e);
   }
+  cudaError_t e;
+  if (!greedy && stat_launch_rows > kClusterStatRows && p->vocab >= kFlatMinVocab && flat_aligned(p->target_logits, p->vocab) &&
+      (!p->drafts || flat_aligned(p->draft_logits, p->vocab)) &&
+      p->scratch_bytes >= ds41_b200_verify_scratch_bytes_for(p->sequences, p->drafts, p->vocab)) {
+    FlatArgs f{};
+    f.logits = a.logits; f.logits2 = a.logits2; f.split = p->drafts ? a.split : stat_launch_rows;
+    f.stride = p->vocab; f.vocab = p->vocab; f.rows = stat_launch_rows;
+    f.t = a.temperature; f.top_p = p->top_p; f.seeds = p->seeds; f.steps = p->steps; f.slot = a.slot; f.purpose = a.purpose;
+    f.stats = pstats; f.draw_every = a.draw_every; f.bound_scale = a.bound_scale;
+    void *flat_scratch = static_cast<unsigned char *>(p->scratch) + streaming_need + verify_replay_scratch_bytes();
+    if ((e = launch_flat(f, flat_scratch, stream)) != cudaSuccess) return int(e);
+    a.only_uncovered = 1;      // what it could not take
+    a.pending = flat_pending(flat_scratch);
+  }
+  e = launch_rows<kModeStats>(a, stat_launch_rows, stream);
+  if (e != cudaSuccess) return int(e);
   static thread_local int configured_device = -1;
   int dev = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return int(e);
