@@ -49,6 +49,13 @@ __device__ __forceinline__ int flat_sum(FlatRed &r, int v) {
 __device__ __forceinline__ const float *row_logits(const FlatArgs &a, int row) {
   return row < a.split ? a.logits + size_t(row) * a.stride : a.logits2 + size_t(row - a.split) * a.stride;
 }
+// Four consecutive logits.  Rows of an odd vocabulary start at any 4-byte boundary: four coalesced-enough loads then (a warp's
+// four instructions touch the same lines).
+__device__ __forceinline__ float4 load4(const float *p, bool aligned) {
+  if (aligned) return __ldg(reinterpret_cast<const float4 *>(p));
+  return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+__device__ __forceinline__ bool row_aligned(const float *x) { return (reinterpret_cast<uintptr_t>(x) & 15u) == 0; }
 // The row is not decided here: -8 / -9 for the kernels behind (see flat.cuh), -1 for good.
 __device__ __forceinline__ void leave_row(const FlatArgs &a, int row, int status) {
   if (a.stats) {
@@ -110,9 +117,10 @@ __global__ void __launch_bounds__(kFT) flat_stats_kernel(FlatArgs a) {
     if (v > best) { best = v; best_id = id; }
     lowest = fminf(lowest, v);
   };
-  const int vec_end = begin + ((end - begin) & ~3);  // begin is a multiple of 4, rows are 16-byte aligned
+  const bool aligned = row_aligned(x);
+  const int vec_end = begin + ((end - begin) & ~3);  // begin is a multiple of 4
   for (int i = begin + 4 * threadIdx.x; i < vec_end; i += 4 * kFT) {
-    const float4 v = __ldg(reinterpret_cast<const float4 *>(x + i));
+    const float4 v = load4(x + i, aligned);
     take(v.x, i); take(v.y, i + 1); take(v.z, i + 2); take(v.w, i + 3);
   }
   for (int i = vec_end + threadIdx.x; i < end; i += kFT) take(__ldg(x + i), i);
@@ -153,17 +161,18 @@ __global__ void __launch_bounds__(kFT) flat_hist_kernel(FlatArgs a) {
   piece(a, part, &begin, &end);
   const float *x = row_logits(a, row);
   auto take = [&](float y) { bin_add(bins, y, b); };
+  const bool aligned = row_aligned(x);
   const int vec_end = begin + ((end - begin) & ~3);
   int i = begin + 4 * threadIdx.x;
   for (; i + 12 * kFT < vec_end; i += 16 * kFT) {  // four 16-byte loads in flight per thread
     float4 v[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = __ldg(reinterpret_cast<const float4 *>(x + i + 4 * kFT * k));
+    for (int k = 0; k < 4; ++k) v[k] = load4(x + i + 4 * kFT * k, aligned);
 #pragma unroll
     for (int k = 0; k < 4; ++k) { take(v[k].x); take(v[k].y); take(v[k].z); take(v[k].w); }
   }
   for (; i < vec_end; i += 4 * kFT) {
-    const float4 v = __ldg(reinterpret_cast<const float4 *>(x + i));
+    const float4 v = load4(x + i, aligned);
     take(v.x); take(v.y); take(v.z); take(v.w);
   }
   for (int k = vec_end + threadIdx.x; k < end; k += kFT) take(__ldg(x + k));
@@ -301,8 +310,9 @@ __device__ __forceinline__ unsigned mass_sub_region(const float *x, int left, co
   double z = 0, sure = 0;
   unsigned inside = 0;
   const float *mine = x + 4 * lane;
+  const bool aligned = row_aligned(x);   // (sub-regions start at multiples of 1024 ids)
   auto fetch = [&](int i) {
-    if (kWhole) return __ldg(reinterpret_cast<const float4 *>(mine + 128 * i));
+    if (kWhole) return load4(mine + 128 * i, aligned);
     const int id = 128 * i + 4 * lane;
     const float none = -CUDART_INF_F;   // beyond the vocabulary: weighs nothing, before nothing
     return make_float4(id < left ? __ldg(x + id) : none, id + 1 < left ? __ldg(x + id + 1) : none,
@@ -565,7 +575,7 @@ __global__ void __launch_bounds__(kRT4) flat_resolve_kernel(FlatArgs a) {
     const int id0 = sub * kFlatSub + 8 * tid;
     float y[8];
     if (id0 + 8 <= a.vocab) {
-      const float4 p = __ldg(reinterpret_cast<const float4 *>(x + id0)), q = __ldg(reinterpret_cast<const float4 *>(x + id0 + 4));
+      const float4 p = load4(x + id0, row_aligned(x)), q = load4(x + id0 + 4, row_aligned(x));
       y[0] = p.x; y[1] = p.y; y[2] = p.z; y[3] = p.w; y[4] = q.x; y[5] = q.y; y[6] = q.z; y[7] = q.w;
     } else {
 #pragma unroll

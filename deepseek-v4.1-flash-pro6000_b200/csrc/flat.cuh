@@ -49,7 +49,7 @@ struct FlatScratch {
   unsigned long long *lkeys;   // [rows][kFlatList]
 };
 struct FlatArgs {
-  const float *logits;         // rows 16-byte aligned: base and stride
+  const float *logits;         // at any alignment; rows on 16-byte boundaries are read with 16-byte loads
   long long stride;
   int vocab, rows;
   int parts;                   // CTAs per row in the statistics / histogram / mass passes (set by launch_flat)
@@ -74,10 +74,6 @@ size_t flat_scratch_bytes(int rows);
 const int *flat_pending(const void *scratch);
 // The [rows] records inside `scratch`.
 FlatInfo *flat_info(void *scratch, int rows);
-// Whether rows of this shape can be laid out for it.
-inline bool flat_aligned(const void *logits, long long stride) {
-  return stride != 0 && stride % 4 == 0 && !(reinterpret_cast<uintptr_t>(logits) & 15u);
-}
 // Rows this path decides get their token and status (0 or certification bits); the others get token -1 and status
 // -8 / -9 (to be redone by another path) or -1 (non-finite logits, final).
 cudaError_t launch_flat(FlatArgs a, void *scratch, cudaStream_t stream);

@@ -93,11 +93,12 @@ __device__ __forceinline__ void list_ids(RowCtx &c, unsigned inside) {
   __syncwarp();
 }
 
-// All threads of one CTA: the first id of the row in id order whose running kept mass exceeds u * total, from the kept mass
-// of every warp region (s->region.kept) and the one region that holds it.  Ids whose key is at most cut_key are kept.
-// (u = s->u.)  Returns -1 if no id has any mass; *close: the target lies within rel * total of a step on either side.
-__device__ __forceinline__ int draw_region(RowCtx &c, double rel, const RowWeights &w, unsigned long long cut_key,
-                                           bool *close) {
+// All threads of one CTA: the first id of the row in id order whose running mass exceeds u * total (u = s->u), from the mass of
+// every warp region (s->region.kept) and the one region that holds it: value(j, first id, v) gives the masses of two
+// consecutive ids of it, `j` ids into the region of CTA `owner`.  Returns -1 if no id has any mass; *close: the target lies
+// within rel * total + absolute of a step on either side.
+template <class Value>
+__device__ __forceinline__ int draw_region(RowCtx &c, double rel, double absolute, Value value, bool *close) {
   RowSmem *s = c.s;
   if (c.warp == 0) {           // the region: four per lane
     const int r0 = 4 * c.lane;
@@ -126,7 +127,7 @@ __device__ __forceinline__ int draw_region(RowCtx &c, double rel, const RowWeigh
       if (region >= 0) carry = total - s->region.kept[region];
     }
     if (c.lane == 0) {
-      s->pick.region = region; s->pick.carry = carry; s->pick.target = target; s->pick.slack = rel * total;
+      s->pick.region = region; s->pick.carry = carry; s->pick.target = target; s->pick.slack = rel * total + absolute;
       s->pick.close = hit ? 0 : 1;
       s->bcast_i[0] = 0x7fffffff;
     }
@@ -136,15 +137,9 @@ __device__ __forceinline__ int draw_region(RowCtx &c, double rel, const RowWeigh
   const double carry = s->pick.carry, target = s->pick.target, slack = s->pick.slack;
   bool amb = s->pick.close != 0;
   if (region < 0) { *close = true; return -1; }
-  const int owner = region / kWarps, first = (region % kWarps) * c.region, id0 = owner * c.stride_ids + first + 2 * c.tid;
-  const float *yr = c.cluster.map_shared_rank(s->y, owner) + first + 2 * c.tid;
-  float y[2];
-  double v[2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) y[i] = 2 * c.tid + i < c.region ? yr[i] : -CUDART_INF_F;
-  row_weights<2>(y, w, v);
-#pragma unroll
-  for (int i = 0; i < 2; ++i) v[i] = y[i] > -CUDART_INF_F && order_key(y[i], id0 + i) <= cut_key ? v[i] : 0.0;
+  const int owner = region / kWarps, first = (region % kWarps) * c.region;
+  double v[2] = {0, 0};
+  if (2 * c.tid < c.region) value(owner, first + 2 * c.tid, v);
   double c1, c0;
   block_scan(c, s->red_d, v[0] + v[1], &c1, &c0);
   const double before = carry + c0, mid = before + v[0], end = carry + c1;
@@ -426,7 +421,16 @@ __device__ __forceinline__ NucleusOut nucleus_row(RowCtx &c, const NucleusArgs &
       int token = -1;
       if (a.draw) {
         bool close;
-        token = draw_region(c, 2.0 * (double(kept) + kFlatWeightUlps) * kU * a.draw_scale, weights, cut_key, &close);
+        token = draw_region(c, 2.0 * (double(kept) + kFlatWeightUlps) * kU * a.draw_scale, 0.0,
+                            [&](int owner, int j, double (&v)[2]) {   // (the ids whose key is at most the cut's are kept)
+                              const float2 pair = *reinterpret_cast<const float2 *>(c.cluster.map_shared_rank(s->y, owner) + j);
+                              const float y[2] = {pair.x, pair.y};
+                              const int id = owner * c.stride_ids + j;
+                              row_weights<2>(y, weights, v);
+#pragma unroll
+                              for (int i = 0; i < 2; ++i)
+                                v[i] = y[i] > -CUDART_INF_F && order_key(y[i], id + i) <= cut_key ? v[i] : 0.0;
+                            }, &close);
         if (token < 0) mine = false;
         else if (close) status |= 1;
       }

@@ -153,22 +153,29 @@ extern "C" double ds41_spark_uniform_v2(uint64_t seed, uint64_t step, uint32_t s
 extern "C" const char *ds41_spark_error(void) { return last_error(); }
 
 namespace {
-// Up to this many rows the cluster kernel takes a batch cut by top-p alone in one launch.
-constexpr int kClusterRows = 48;
+// Up to this many rows the cluster kernel takes a batch in one launch; larger ones go through the batch path (top-p alone)
+// or the streaming path (top-k, greedy).  Where the two meet, at 129280 ids: top-p 48 rows 65 us against 75, 64 rows 70
+// against 65; top-k 128 rows 64 us against 98, 256 rows 128 against 136; greedy 64 rows 18.5 us against 18.9, 96 rows 27
+// against 23.
+constexpr int kClusterRows = 48, kClusterRowsTopk = 256, kClusterRowsGreedy = 64;
 
-// One launch that decides every row, and the replay of the rows it could not certify.
+// One launch that decides every row, and, for rows cut by top-p alone, the replay of those it could not certify.
 int sample_by_clusters(RowArgs a, const ds41_b200_sample_args &p, cudaStream_t stream) {
-  unsigned char *flat_scratch = static_cast<unsigned char *>(p.scratch) + streaming_bytes(p.rows, p.vocab);
+  unsigned char *behind = static_cast<unsigned char *>(p.scratch) + streaming_bytes(p.rows, p.vocab);
   a.status = p.status ? p.status
                       : reinterpret_cast<int32_t *>(static_cast<ChunkRecord *>(p.scratch) + size_t(p.rows) * chunks_for(p.vocab));
   a.head_stats = static_cast<const HeadRowStats *>(p.row_extremes);
-  a.bound_scale = bound_scale();
-  a.info = flat_info(flat_scratch, p.rows);
-  a.replayed = const_cast<int *>(flat_pending(flat_scratch)) + 1;
+  const bool replay = p.top_k == 0 && a.temperature > 0;
+  if (replay) a.bound_scale = bound_scale();
+  if (flat_shape(p.rows, p.vocab)) {
+    a.info = flat_info(behind, p.rows);
+    a.replayed = const_cast<int *>(flat_pending(behind)) + 1;
+    behind += flat_scratch_bytes(p.rows);
+  }
   cudaError_t e = launch_rows<kModeSample>(a, p.rows, stream);
-  if (e != cudaSuccess) return int(e);
+  if (e != cudaSuccess || !replay) return int(e);
   ReplayArgs r{p.logits, p.logits_stride, p.vocab, p.rows, a.temperature, p.top_p, p.seeds, p.steps, p.slot, p.purpose,
-               p.tokens, a.status, flat_scratch + flat_scratch_bytes(p.rows), a.replayed, a.info};
+               p.tokens, a.status, behind, a.replayed, a.info};
   return int(launch_replay(r, stream));
 }
 }  // namespace
@@ -198,11 +205,12 @@ extern "C" int ds41_b200_sample_logits(const ds41_b200_sample_args *p, cudaStrea
   const size_t need = ds41_b200_sample_scratch_bytes(p->rows, p->vocab);
   const bool scratch_ok = p->scratch && p->scratch_bytes >= need && !(reinterpret_cast<uintptr_t>(p->scratch) & 15u) &&
                           !penalised && !p->mask && p->top_k <= kCand;
-  // Batches of rows that are only cut by top-p first go through the batch path; it answers the rows it fits and marks
-  // the others -8 / -9, and the paths below then only touch those.
-  const bool flat = scratch_ok && flat_shape(p->rows, p->vocab) && p->top_k == 0 && p->temperature > 0 &&
-                    flat_aligned(p->logits, p->logits_stride);
-  if (flat && p->rows <= kClusterRows) return sample_by_clusters(a, *p, stream);
+  // With scratch: small batches by the cluster kernel alone; larger ones of rows that are only cut by top-p first go through
+  // the batch path, which answers the rows it fits and marks the others -8 / -9, and the paths below then only touch those.
+  const bool top_p_only = p->top_k == 0 && p->temperature > 0;
+  const int by_clusters = top_p_only ? kClusterRows : p->temperature > 0 ? kClusterRowsTopk : kClusterRowsGreedy;
+  if (scratch_ok && p->rows <= by_clusters) return sample_by_clusters(a, *p, stream);
+  const bool flat = scratch_ok && flat_shape(p->rows, p->vocab) && top_p_only && p->logits_stride != 0;
   // the streaming path covers small nuclei only: a full-vocabulary draw never fits its candidate sets
   const bool streaming = scratch_ok && (p->top_p < 1.0 || p->top_k > 0 || p->temperature == 0);
   if (!flat && !streaming) return int(launch_rows<kModeSample>(a, p->rows, stream));

@@ -4,15 +4,16 @@
 // sampler's probability rule (engine/src/sampling.cpp:142-219), i.e. the sequence
 //   probabilities_rows(target) ; probabilities(draft_k) ; reject_sample(...)   (engine/src/speculation.cpp:126-182).
 // Two launches:
-//   1. row statistics for every target and draft row (row_kernel<kModeStats>): first maximum, normaliser, top-p cut
-//      and kept mass, written to caller-provided scratch;
-//   2. one cluster per sequence walks the positions: accept test from the two rows' statistics and the two logits at
-//      the draft id; on the first rejection the residual max(0,p-q) is drawn by an inverse CDF streamed from the two
-//      rows (normally still L2 resident), otherwise the bonus token is drawn from the last target row.
+//   1. row statistics for every target and draft row (the cluster kernel, or the batch path's passes for many rows): first
+//      maximum, normaliser, top-p cut and kept mass, written to caller-provided scratch, and the bonus token of every last
+//      target row;
+//   2. one cluster per sequence: accept tests from the two rows' statistics and the two logits at each draft id; on the first
+//      rejection the residual max(0,p-q) is drawn by an inverse CDF streamed from the two rows (normally still L2 resident).
 #include <atomic>
 #include "ds41_b200.h"
 #include "flat.cuh"
 #include "host_error.h"
+#include "launch.h"
 #include "replay.cuh"
 #include "row_kernel.cuh"
 #include "stream_types.cuh"
@@ -49,90 +50,164 @@ struct Measure {  // one row's probability measure: P(id) = survives ? exp((x-ma
   __device__ __forceinline__ double bound() const { return 2.0 * (double(st.kept) + 1600.0) * kU; }
 };
 
-__global__ void __launch_bounds__(kThreads, 2) verify_kernel(VerifyArgs a) {
+// One cluster per sequence.  The accept tests of all positions are taken at once, one lane each (what lies behind the first
+// rejection is not used); only a rejection reads whole rows: the residual's mass per warp region over the cluster, ids that
+// the target row cuts off skipped four at a time, then one CTA draws.  The bonus token came with the statistics.
+struct Walk { int accepted, rejected, status, token; };
+
+__global__ void __launch_bounds__(kThreads, 2) verify_kernel(const __grid_constant__ VerifyArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ Walk walk;
   RowSmem *s = reinterpret_cast<RowSmem *>(smem_raw);
   RowCtx c = make_ctx(s, a.vocab);
-  const int seq = blockIdx.x / c.nranks;
-  const int D = a.drafts;
+  prepare_smem(s);
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+  const int seq = blockIdx.x / c.nranks, D = a.drafts;
   const bool greedy = a.temperature == 0;
-  const uint64_t seed = a.seeds[seq], step = a.steps[seq];
-  ds41_spark_result r{};
-  int status = 0;
-  // any rejected row of this transaction rejects the transaction (the reference computes every p and q row first)
-  for (int k = 0; k <= D; ++k) {
-    const int st = a.pstats[size_t(seq) * (D + 1) + k].status;
-    if (st < 0 && status >= 0) status = st;
-    else if (st > 0 && status >= 0) status |= st;
-  }
-  if (!greedy)
-    for (int k = 0; k < D; ++k) {
-      const int st = a.qstats[size_t(seq) * D + k].status;
-      if (st < 0 && status >= 0) status = st;
-      else if (st > 0 && status >= 0) status |= st;
-    }
-  for (int k = 0; k < D && status >= 0 && !r.rejected; ++k) {
-    const int d = a.ids[size_t(seq) * D + k];
-    if (d < 0 || d >= a.vocab) { status = -6; break; }  // checked only when the position is reached (sampling.cpp:44)
-    const RowStats ps = a.pstats[size_t(seq) * (D + 1) + k];
-    Measure P{a.target + (size_t(seq) * (D + 1) + k) * a.vocab, ps, greedy ? 0.0 : 1.0 / a.temperature, 1.0 / ps.e_kept};
-    bool accept;
-    if (greedy) {
-      accept = d == P.st.argmax;
-      if (!accept) { r.tokens[r.emitted++] = P.st.argmax; r.rejected = 1; }
-    } else {
-      const RowStats qs = a.qstats[size_t(seq) * D + k];
-      Measure Q{a.draft + (size_t(seq) * D + k) * a.vocab, qs, 1.0 / a.temperature, 1.0 / qs.e_kept};
-      const double pd = P.at(d), qd = Q.at(d);
-      if (!(qd > 0)) { status = -6; break; }
-      const double ratio = fmin(1.0, pd / qd);
-      const double u = philox_uniform(seed, step, uint32_t(k), 2);
-      accept = u < ratio;
-      if (ratio < 1.0 && fabs(u - ratio) <= (P.bound() + Q.bound() + 16 * kU) * a.bound_scale * ratio) status |= 4;
-      if (!accept) {
-        // residual draw: inverse CDF over max(0, P - Q) in id order
-        auto value = [&](int j) { const int id = c.begin + j; return fmax(0.0, P.at(id) - Q.at(id)); };
-        region_sums(c, value);
-        int amb = 0;
-        double total = 0;
-        const int support = min(a.vocab, P.st.kept + Q.st.kept);
-        const int token = draw_token(c, philox_uniform(seed, step, uint32_t(k), 3),
-                                     (2.0 * support + 256.0) * kU * a.bound_scale, (P.bound() + Q.bound()) * a.bound_scale,
-                                     value, &amb, &total);
-        if (!(total > 0) || token < 0) { status = -2; break; }
-        if (amb) status |= 8;
-        r.tokens[r.emitted++] = token;
-        r.rejected = 1;
+  const RowStats *ps = a.pstats + size_t(seq) * (D + 1), *qs = a.qstats + size_t(seq) * D;
+  const float *target = a.target + size_t(seq) * (D + 1) * a.vocab, *draft = a.draft + size_t(seq) * D * a.vocab;
+  const double inv_t = greedy ? 0.0 : 1.0 / a.temperature;
+  if (c.warp == 0) {
+    // any rejected row of this transaction rejects the transaction (the reference computes every p and q row first)
+    const bool p_row = c.lane <= D, q_row = !greedy && c.lane >= 8 && c.lane < 8 + D;
+    const int st = p_row ? ps[c.lane].status : q_row ? qs[c.lane - 8].status : 0;
+    const unsigned failed = __ballot_sync(0xffffffffu, st < 0);
+    int status = failed ? __shfl_sync(0xffffffffu, st, __ffs(failed) - 1) : int(__reduce_or_sync(0xffffffffu, unsigned(st)));
+    bool accept = true, wrong = false, close = false;
+    if (status >= 0 && c.lane < D) {
+      const int d = a.ids[size_t(seq) * D + c.lane];
+      wrong = d < 0 || d >= a.vocab;   // (counts only when the position is reached: sampling.cpp:44)
+      if (!wrong && greedy) {
+        accept = d == ps[c.lane].argmax;
+      } else if (!wrong) {
+        const RowStats sp = ps[c.lane], sq = qs[c.lane];
+        const Measure P{target + size_t(c.lane) * a.vocab, sp, inv_t, 1.0 / sp.e_kept};
+        const Measure Q{draft + size_t(c.lane) * a.vocab, sq, inv_t, 1.0 / sq.e_kept};
+        const double pd = P.at(d), qd = Q.at(d);
+        wrong = !(qd > 0);
+        const double ratio = fmin(1.0, pd / qd), u = philox_uniform(a.seeds[seq], a.steps[seq], uint32_t(c.lane), 2);
+        accept = u < ratio;
+        close = ratio < 1.0 && fabs(u - ratio) <= (P.bound() + Q.bound() + 16 * kU) * a.bound_scale * ratio;
       }
     }
-    if (accept) { r.tokens[r.emitted++] = d; ++r.accepted_drafts; }
-  }
-  if (status >= 0 && !r.rejected) {
-    const RowStats ps = a.pstats[size_t(seq) * (D + 1) + D];
-    Measure P{a.target + (size_t(seq) * (D + 1) + D) * a.vocab, ps, greedy ? 0.0 : 1.0 / a.temperature, 1.0 / ps.e_kept};
-    if (greedy) {
-      r.tokens[r.emitted++] = P.st.argmax;
-    } else if (ps.drawn >= 0) {   // drawn with the row's statistics
-      if (ps.drawn & kDrawnClose) status |= 1;
-      r.tokens[r.emitted++] = ps.drawn & ~kDrawnClose;
-    } else {
-      auto value = [&](int j) { return P.at(c.begin + j) * P.st.e_kept; };  // unnormalised weights, as the sampler
-      region_sums(c, value);
-      int amb = 0;
-      double total = 0;
-      const int token = draw_token(c, philox_uniform(seed, step, uint32_t(D), 0),
-                                   (2.0 * P.st.kept + 256.0) * kU * a.bound_scale, 0.0, value, &amb, &total);
-      if (amb) status |= 1;
-      r.tokens[r.emitted++] = token;
+    const unsigned stops = __ballot_sync(0xffffffffu, c.lane < D && (wrong || !accept));
+    const int at = stops ? __ffs(stops) - 1 : D;   // accepted drafts in front of it
+    const unsigned here = __ballot_sync(0xffffffffu, close && c.lane <= at);
+    if (status >= 0 && at < D && __shfl_sync(0xffffffffu, wrong ? 1 : 0, at)) status = -6;
+    if (status >= 0 && here) status |= 4;
+    if (c.lane == 0) {
+      walk.accepted = at; walk.rejected = at < D ? 1 : 0; walk.status = status; walk.token = -1;
+      if (status >= 0) {
+        if (at == D || greedy) {
+          const RowStats &row = ps[at];
+          walk.token = greedy ? row.argmax : row.drawn & ~kDrawnClose;
+          if (!greedy && row.drawn < 0) walk.status = -2;               // (a valid row has always been drawn from)
+          else if (!greedy && (row.drawn & kDrawnClose)) walk.status = status | 1;
+        } else {
+          s->u = philox_uniform(a.seeds[seq], a.steps[seq], uint32_t(at), 3);
+        }
+      }
     }
   }
-  r.accepted_input_rows = r.accepted_drafts + 1;
-  if (status < 0) { r = ds41_spark_result{}; r.emitted = -1; }
-  if (c.rank == 0 && c.tid == 0) {
-    a.results[seq] = r;
-    if (a.status) a.status[seq] = status;
+  __syncthreads();
+  const int at = walk.accepted;
+  if (walk.status >= 0 && walk.rejected && !greedy) {
+    // residual draw: inverse CDF over max(0, P - Q) in id order (sampling.cpp:46-50)
+    const RowStats sp = ps[at], sq = qs[at];
+    const float *xp = target + size_t(at) * a.vocab, *xq = draft + size_t(at) * a.vocab;
+    const double log2e_t = kLog2e * inv_t, inv_p = 1.0 / sp.e_kept, inv_q = 1.0 / sq.e_kept;
+    const float gap = float(650.0 / kLog2e * a.temperature);
+    const RowWeights wp = make_weights(sp.max_logit, log2e_t, gap, s->pow2), wq = make_weights(sq.max_logit, log2e_t, gap, s->pow2);
+    const bool aligned = ((reinterpret_cast<uintptr_t>(xp) | reinterpret_cast<uintptr_t>(xq)) & 15u) == 0;
+    double mass = 0;
+    const int j0 = c.warp * c.region + 4 * c.lane;
+#pragma unroll 1
+    for (int i0 = 0; i0 < c.region / 128; i0 += 4) {   // (four rounds' loads in flight)
+      float yp[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int j = j0 + 128 * (i0 + i);
+        const bool in = i0 + i < c.region / 128;
+        if (aligned && in && j + 4 <= c.len) {
+          const float4 v = __ldg(reinterpret_cast<const float4 *>(xp + c.begin + j));
+          yp[i][0] = v.x; yp[i][1] = v.y; yp[i][2] = v.z; yp[i][3] = v.w;
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) yp[i][k] = in && j + k < c.len ? __ldg(xp + c.begin + j + k) : -CUDART_INF_F;
+        }
+      }
+#pragma unroll 1
+      for (int i = 0; i < 4; ++i) {
+        const int id = c.begin + j0 + 128 * (i0 + i);
+        const float y[4] = {yp[0][0], yp[0][1], yp[0][2], yp[0][3]};
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) yp[r][k] = yp[r + 1][k];
+        bool some = false;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) some = some || (y[k] > -CUDART_INF_F && y[k] >= sp.cut.y);
+        if (!__any_sync(0xffffffffu, some)) continue;   // (a residual mass needs a kept target id)
+        double ep[4], eq[4];
+        float z[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) z[k] = y[k] > -CUDART_INF_F && y[k] >= sp.cut.y ? __ldg(xq + id + k) : -CUDART_INF_F;
+        row_weights<4>(y, wp, ep);
+        row_weights<4>(z, wq, eq);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const double p = y[k] > -CUDART_INF_F && survives(y[k], id + k, sp.cut) ? ep[k] * inv_p : 0.0;
+          const double q = z[k] > -CUDART_INF_F && survives(z[k], id + k, sq.cut) ? eq[k] * inv_q : 0.0;
+          mass += fmax(0.0, p - q);
+        }
+      }
+    }
+    mass = lanes_sum(mass);
+    if (c.lane == 0) c.cluster.map_shared_rank(&s->region, 0)->kept[c.rank * kWarps + c.warp] = mass;
+    c.cluster.sync();
+    if (c.rank == 0) {
+      auto value = [&](int owner, int j, double (&v)[2]) {
+        const int id = owner * c.stride_ids + j, end = min(a.vocab, (owner + 1) * c.stride_ids);
+        float y[2], z[2];
+        double ep[2], eq[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          y[i] = id + i < end ? __ldg(xp + id + i) : -CUDART_INF_F;
+          z[i] = id + i < end ? __ldg(xq + id + i) : -CUDART_INF_F;
+        }
+        row_weights<2>(y, wp, ep);
+        row_weights<2>(z, wq, eq);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const double p = id + i < end && survives(y[i], id + i, sp.cut) ? ep[i] * inv_p : 0.0;
+          const double q = id + i < end && survives(z[i], id + i, sq.cut) ? eq[i] * inv_q : 0.0;
+          v[i] = fmax(0.0, p - q);
+        }
+      };
+      const Measure P{xp, sp, inv_t, inv_p}, Q{xq, sq, inv_t, inv_q};
+      const int support = min(a.vocab, sp.kept + sq.kept);
+      bool close;
+      const int token = draw_region(c, 2.0 * (support + kFlatWeightUlps) * kU * a.bound_scale,
+                                    (P.bound() + Q.bound()) * a.bound_scale, value, &close);
+      if (c.tid == 0) {
+        walk.token = token;
+        walk.status = token < 0 ? -2 : close ? walk.status | 8 : walk.status;
+      }
+    }
   }
-  c.cluster.sync();
+  if (c.rank == 0 && c.tid == 0) {
+    ds41_spark_result r{};
+    if (walk.status < 0) {
+      r.emitted = -1;
+    } else {
+      for (int k = 0; k < at; ++k) r.tokens[r.emitted++] = a.ids[size_t(seq) * D + k];
+      r.tokens[r.emitted++] = walk.token;
+      r.accepted_drafts = at; r.accepted_input_rows = at + 1; r.rejected = walk.rejected;
+    }
+    a.results[seq] = r;
+    if (a.status) a.status[seq] = walk.status;
+  }
 }
 
 }  // namespace ds41
@@ -140,7 +215,7 @@ __global__ void __launch_bounds__(kThreads, 2) verify_kernel(VerifyArgs a) {
 namespace ds41 {
 namespace {
 // Up to this many rows the cluster kernel takes the statistics in one launch; beyond, the batch path's grid-wide passes do
-// (they need scratch and aligned rows).
+// (they need scratch).
 constexpr int kClusterStatRows = 40;
 // [row statistics][room that earlier versions used], rounded up to 16 bytes; the replay's rows follow, then the batch path's
 // scratch
@@ -198,8 +273,7 @@ extern "C" int ds41_b200_verify_logits(const ds41_b200_verify_args *p, cudaStrea
     }
   }
   cudaError_t e;
-  if (!greedy && stat_launch_rows > kClusterStatRows && p->vocab >= kFlatMinVocab && flat_aligned(p->target_logits, p->vocab) &&
-      (!p->drafts || flat_aligned(p->draft_logits, p->vocab)) &&
+  if (!greedy && stat_launch_rows > kClusterStatRows && p->vocab >= kFlatMinVocab &&
       p->scratch_bytes >= ds41_b200_verify_scratch_bytes_for(p->sequences, p->drafts, p->vocab)) {
     FlatArgs f{};
     f.logits = a.logits; f.logits2 = a.logits2; f.split = p->drafts ? a.split : stat_launch_rows;
@@ -229,10 +303,11 @@ extern "C" int ds41_b200_verify_logits(const ds41_b200_verify_args *p, cudaStrea
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = sizeof(RowSmem);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = cl; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  attr[1] = programmatic_launch();
+  cfg.attrs = attr; cfg.numAttrs = 2;
   e = cudaLaunchKernelEx(&cfg, verify_kernel, v);
   if (e != cudaSuccess) return int(e);
   // transactions with a certification bit set: redone in the reference's order of operations, when the caller gave
