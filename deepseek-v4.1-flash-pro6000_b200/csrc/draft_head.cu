@@ -11,6 +11,8 @@
 // the three-kernel prologue.
 #include "ds41_b200.h"
 #include "host_error.h"
+#include "launch.h"
+#include "packed_fma.cuh"
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -37,13 +39,13 @@ __global__ void __launch_bounds__(kHeadThreads) head_compact_kernel(const float 
   const int groups = (N + kRowsPerWarp - 1) / kRowsPerWarp;
   for (int g = blockIdx.x * kHeadWarps + warp; g < groups; g += gridDim.x * kHeadWarps) {
     const int row0 = g * kRowsPerWarp;
-    float acc[kRowsPerWarp][M][4];
+    float2x acc[kRowsPerWarp][M][2];   // accumulators 0 and 1, 2 and 3
 #pragma unroll
     for (int r = 0; r < kRowsPerWarp; ++r)
 #pragma unroll
       for (int m = 0; m < M; ++m)
 #pragma unroll
-        for (int a = 0; a < 4; ++a) acc[r][m][a] = 0.f;
+        for (int a = 0; a < 2; ++a) acc[r][m][a] = 0ull;
     const uint4 *wr[kRowsPerWarp];
 #pragma unroll
     for (int r = 0; r < kRowsPerWarp; ++r)
@@ -60,19 +62,22 @@ __global__ void __launch_bounds__(kHeadThreads) head_compact_kernel(const float 
       const bool more = k + 512 < K;
 #pragma unroll
       for (int r = 0; r < kRowsPerWarp; ++r) far[r] = more ? __ldg(wr[r] + ((k + 512) >> 3)) : nxt[r];
+      float2x wv[kRowsPerWarp][4];
+#pragma unroll
+      for (int r = 0; r < kRowsPerWarp; ++r) {
+        wv[r][0] = promote_bf16x2(cur[r].x); wv[r][1] = promote_bf16x2(cur[r].y);
+        wv[r][2] = promote_bf16x2(cur[r].z); wv[r][3] = promote_bf16x2(cur[r].w);
+      }
 #pragma unroll
       for (int m = 0; m < M; ++m) {
-        const float4 a = *reinterpret_cast<const float4 *>(xs + m * K + k);
-        const float4 b = *reinterpret_cast<const float4 *>(xs + m * K + k + 4);
-        const float xx[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(xs + m * K + k);
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(xs + m * K + k + 4);
 #pragma unroll
         for (int r = 0; r < kRowsPerWarp; ++r) {
-          const uint32_t ww[4] = {cur[r].x, cur[r].y, cur[r].z, cur[r].w};
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float wj = bf16_bits_to_float((j & 1) ? (ww[j >> 1] >> 16) : (ww[j >> 1] & 0xffffu));
-            acc[r][m][j & 3] = __fmaf_rn(wj, xx[j], acc[r][m][j & 3]);
-          }
+          acc[r][m][0] = fma_f32x2(wv[r][0], a.x, acc[r][m][0]);
+          acc[r][m][1] = fma_f32x2(wv[r][1], a.y, acc[r][m][1]);
+          acc[r][m][0] = fma_f32x2(wv[r][2], b.x, acc[r][m][0]);
+          acc[r][m][1] = fma_f32x2(wv[r][3], b.y, acc[r][m][1]);
         }
       }
 #pragma unroll
@@ -82,7 +87,10 @@ __global__ void __launch_bounds__(kHeadThreads) head_compact_kernel(const float 
     for (int r = 0; r < kRowsPerWarp; ++r)
 #pragma unroll
       for (int m = 0; m < M; ++m) {
-        float sum = __fadd_rn(__fadd_rn(acc[r][m][0], acc[r][m][1]), __fadd_rn(acc[r][m][2], acc[r][m][3]));
+        float c[4];
+        unpack_f32x2(acc[r][m][0], c[0], c[1]);
+        unpack_f32x2(acc[r][m][1], c[2], c[3]);
+        float sum = __fadd_rn(__fadd_rn(c[0], c[1]), __fadd_rn(c[2], c[3]));
 #pragma unroll
         for (int d = 16; d; d >>= 1) sum = __fadd_rn(sum, __shfl_down_sync(0xffffffffu, sum, d));
         if (lane == 0 && row0 + r < N) y[size_t(m) * N + row0 + r] = sum;
@@ -90,30 +98,138 @@ __global__ void __launch_bounds__(kHeadThreads) head_compact_kernel(const float 
   }
 }
 
+// The same arithmetic with the weights on their way through shared memory: a lane copies the 16 bytes it will consume itself
+// (cp.async), `stages` steps ahead, so no barrier is needed and what is in flight does not depend on registers.  What bounds
+// the kernel at M = 1 is HBM; a step of two register-held loads ahead left 250-410 us at M = 2..5 (5120 x 129280), because a
+// step's arithmetic is shorter than the memory's latency.
+template <int M, int kRowsPerWarp, int kThreads>
+__global__ void __launch_bounds__(kThreads) head_compact_ring_kernel(const float *__restrict__ x, const __nv_bfloat16 *__restrict__ w,
+                                                                     float *__restrict__ y, int N, int K, int stages) {
+  extern __shared__ __align__(16) float xs[];  // [M][K], then per warp [stages][kRowsPerWarp][512 bytes]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kWarpsHere = kThreads / 32, kStage = kRowsPerWarp * 512;
+  const uint32_t ring = uint32_t(__cvta_generic_to_shared(xs + size_t(M) * K)) + uint32_t(warp * stages * kStage) + lane * 16;
+  const int groups = (N + kRowsPerWarp - 1) / kRowsPerWarp, stride = gridDim.x * kWarpsHere, steps_per_group = K / 256;
+  int next_group = blockIdx.x * kWarpsHere + warp, next_step = 0, next_slot = 0;
+  auto fetch = [&] {   // (an empty group once everything is on its way: the waits count groups)
+    if (next_group < groups) {
+#pragma unroll
+      for (int r = 0; r < kRowsPerWarp; ++r) {
+        const int row = min(next_group * kRowsPerWarp + r, N - 1);   // rows beyond N repeat the last one
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring + uint32_t(next_slot * kStage + r * 512)),
+                     "l"(w + size_t(row) * K + next_step * 256 + lane * 8) : "memory");
+      }
+      if (++next_step == steps_per_group) { next_step = 0; next_group += stride; }
+      if (++next_slot == stages) next_slot = 0;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int i = 0; i + 1 < stages; ++i) fetch();   // (weights only)
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+#pragma unroll 4
+  for (int i = threadIdx.x * 4; i < M * K; i += kThreads * 4)
+    *reinterpret_cast<float4 *>(xs + i) = __ldg(reinterpret_cast<const float4 *>(x + i));
+  __syncthreads();
+  int slot = 0;
+  for (int g = blockIdx.x * kWarpsHere + warp; g < groups; g += stride) {
+    float2x acc[kRowsPerWarp][M][2];   // accumulators 0 and 1, 2 and 3
+#pragma unroll
+    for (int r = 0; r < kRowsPerWarp; ++r)
+#pragma unroll
+      for (int m = 0; m < M; ++m) acc[r][m][0] = acc[r][m][1] = 0ull;
+    for (int step = 0; step < steps_per_group; ++step) {
+      switch (stages) {   // all but the newest stages - 2 groups have landed: this step's has
+        case 2: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
+        case 3: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+        case 4: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+        default: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+      }
+      float2x wv[kRowsPerWarp][4];
+#pragma unroll
+      for (int r = 0; r < kRowsPerWarp; ++r) {
+        uint4 v;
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                     : "r"(ring + uint32_t(slot * kStage + r * 512)) : "memory");
+        wv[r][0] = promote_bf16x2(v.x); wv[r][1] = promote_bf16x2(v.y);
+        wv[r][2] = promote_bf16x2(v.z); wv[r][3] = promote_bf16x2(v.w);
+      }
+      fetch();            // (into the slot that the previous step consumed)
+      if (++slot == stages) slot = 0;
+      const float *xk = xs + step * 256 + lane * 8;
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(xk + m * K);
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(xk + m * K + 4);
+#pragma unroll
+        for (int r = 0; r < kRowsPerWarp; ++r) {
+          acc[r][m][0] = fma_f32x2(wv[r][0], a.x, acc[r][m][0]);
+          acc[r][m][1] = fma_f32x2(wv[r][1], a.y, acc[r][m][1]);
+          acc[r][m][0] = fma_f32x2(wv[r][2], b.x, acc[r][m][0]);
+          acc[r][m][1] = fma_f32x2(wv[r][3], b.y, acc[r][m][1]);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kRowsPerWarp; ++r)
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        float c[4];
+        unpack_f32x2(acc[r][m][0], c[0], c[1]);
+        unpack_f32x2(acc[r][m][1], c[2], c[3]);
+        float sum = __fadd_rn(__fadd_rn(c[0], c[1]), __fadd_rn(c[2], c[3]));
+#pragma unroll
+        for (int d = 16; d; d >>= 1) sum = __fadd_rn(sum, __shfl_down_sync(0xffffffffu, sum, d));
+        const int row = g * kRowsPerWarp + r;
+        if (lane == 0 && row < N) y[size_t(m) * N + row] = sum;
+      }
+  }
+}
+
 // logits[n] = U[n] + bias[n], bias[n] = W[n, 0..256) . e with e = the previous token's Markov embedding promoted to FP32.
 // The reference forms the bias with a library GEMV whose order of summation is not specified; here it is the compact
 // head's order for K = 256 (one step per lane), then the reference's single rounded addition (forward.cu:46).
-__global__ void __launch_bounds__(256) markov_logits_kernel(const float *__restrict__ u,
-                                                            const __nv_bfloat16 *__restrict__ w,
-                                                            const __nv_bfloat16 *__restrict__ emb, float *__restrict__ out,
-                                                            int vocab) {
-  const int lane = threadIdx.x & 31;
-  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (row >= vocab) return;
+// A warp takes eight rows at a time, the next eight on their way while it adds up (one row per warp and 16160 CTAs of eight
+// rows spent more on starting CTAs than on the 66 MB: 19.5 us); the embedding stays in registers.
+constexpr int kMarkovThreads = 256, kMarkovRows = 8;
+__global__ void __launch_bounds__(kMarkovThreads, 3) markov_logits_kernel(const float *__restrict__ u,
+                                                                          const __nv_bfloat16 *__restrict__ w,
+                                                                          const __nv_bfloat16 *__restrict__ emb,
+                                                                          float *__restrict__ out, int vocab) {
+  const int lane = threadIdx.x & 31, stride = (gridDim.x * kMarkovThreads >> 5) * kMarkovRows;
+  int row0 = ((blockIdx.x * kMarkovThreads + threadIdx.x) >> 5) * kMarkovRows;
+  uint4 wv[kMarkovRows];
+  auto fetch = [&](int first) {
+#pragma unroll
+    for (int r = 0; r < kMarkovRows; ++r)
+      wv[r] = __ldg(reinterpret_cast<const uint4 *>(w + size_t(min(first + r, vocab - 1)) * 256) + lane);
+  };
+  if (row0 < vocab) fetch(row0);   // (weights only)
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
   const uint4 ev = __ldg(reinterpret_cast<const uint4 *>(emb) + lane);
-  const uint4 wv = __ldg(reinterpret_cast<const uint4 *>(w + size_t(row) * 256) + lane);
-  const uint32_t ee[4] = {ev.x, ev.y, ev.z, ev.w}, ww[4] = {wv.x, wv.y, wv.z, wv.w};
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  const float2x e[4] = {promote_bf16x2(ev.x), promote_bf16x2(ev.y), promote_bf16x2(ev.z), promote_bf16x2(ev.w)};
+  for (; row0 < vocab; row0 += stride) {
+    float sum[kMarkovRows];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float wj = bf16_bits_to_float((j & 1) ? (ww[j >> 1] >> 16) : (ww[j >> 1] & 0xffffu));
-    const float ej = bf16_bits_to_float((j & 1) ? (ee[j >> 1] >> 16) : (ee[j >> 1] & 0xffffu));
-    acc[j & 3] = __fmaf_rn(wj, ej, acc[j & 3]);
+    for (int r = 0; r < kMarkovRows; ++r) {
+      float2x a01 = fma_f32x2(promote_bf16x2(wv[r].x), e[0], 0ull), a23 = fma_f32x2(promote_bf16x2(wv[r].y), e[1], 0ull);
+      a01 = fma_f32x2(promote_bf16x2(wv[r].z), e[2], a01);
+      a23 = fma_f32x2(promote_bf16x2(wv[r].w), e[3], a23);
+      float c[4];
+      unpack_f32x2(a01, c[0], c[1]);
+      unpack_f32x2(a23, c[2], c[3]);
+      sum[r] = __fadd_rn(__fadd_rn(c[0], c[1]), __fadd_rn(c[2], c[3]));
+    }
+    if (row0 + stride < vocab) fetch(row0 + stride);
+#pragma unroll
+    for (int d = 16; d; d >>= 1)
+#pragma unroll
+      for (int r = 0; r < kMarkovRows; ++r) sum[r] = __fadd_rn(sum[r], __shfl_down_sync(0xffffffffu, sum[r], d));
+#pragma unroll
+    for (int r = 0; r < kMarkovRows; ++r)
+      if (lane == 0 && row0 + r < vocab) out[row0 + r] = __fadd_rn(__ldg(u + row0 + r), sum[r]);
   }
-  float sum = __fadd_rn(__fadd_rn(acc[0], acc[1]), __fadd_rn(acc[2], acc[3]));
-#pragma unroll
-  for (int d = 16; d; d >>= 1) sum = __fadd_rn(sum, __shfl_down_sync(0xffffffffu, sum, d));
-  if (lane == 0) out[row] = __fadd_rn(__ldg(u + row), sum);
 }
 
 // Launch geometry of the reference's RMS norm (ops.cu:16: it follows a PyTorch reduction and depends on the number of
@@ -131,79 +247,128 @@ int rms_geometry(int M, int K, int *width) {
 // reference's accumulation and reduction order (four strided accumulators per thread, ((v0 + v1) + v2) + v3, halving
 // inside segments of `width` threads down to a warp, shuffle-down, then a halving tree over the segments), rsqrtf of
 // mean + eps, x * rstd * weight rounded to BF16, stored as FP32 (the head's input type).
-__global__ void final_norm_kernel(const __nv_bfloat16 *__restrict__ h, const float *__restrict__ pre,
-                                  const __nv_bfloat16 *__restrict__ weight, float *__restrict__ out, int K, float eps,
-                                  int width) {
+// The mix and the output run on all 1024 threads, four columns each; the reduction on the first `threads` of them, as the
+// reference's geometry has it.  (With the reference's 256 threads throughout and 2-byte loads a call took 24 us.)
+constexpr int kNormThreads = 1024;
+__global__ void __launch_bounds__(kNormThreads) final_norm_kernel(const __nv_bfloat16 *__restrict__ h, const float *__restrict__ pre,
+                                                                  const __nv_bfloat16 *__restrict__ weight,
+                                                                  float *__restrict__ out, int K, float eps, int width,
+                                                                  int threads) {
   extern __shared__ __align__(16) unsigned char norm_smem[];
   float *sh = reinterpret_cast<float *>(norm_smem);                        // [512]
   __nv_bfloat16 *xrow = reinterpret_cast<__nv_bfloat16 *>(sh + 512);       // [K]
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
   const int tid = threadIdx.x, row = blockIdx.x;
   float p[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) p[j] = pre[row * 4 + j];
-  for (int k = tid; k < K; k += blockDim.x) {  // HC-pre mix (ops.cu:45-48)
-    float s = 0.f;
+  const bool vectors = ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(weight)) & 7u) == 0 &&
+                       (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  auto load4 = [vectors](const __nv_bfloat16 *from, float (&v)[4]) {
+    if (vectors) {
+      const uint2 raw = __ldg(reinterpret_cast<const uint2 *>(from));
+      v[0] = __uint_as_float(raw.x << 16); v[1] = __uint_as_float(raw.x & 0xffff0000u);
+      v[2] = __uint_as_float(raw.y << 16); v[3] = __uint_as_float(raw.y & 0xffff0000u);
+    } else {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) s = __fadd_rn(s, __fmul_rn(p[j], __bfloat162float(h[(size_t(row) * 4 + j) * K + k])));
-    xrow[k] = __float2bfloat16_rn(s);
-  }
-  __syncthreads();
-  float v[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int i = tid * 4; i < K; i += blockDim.x * 4) {
+      for (int i = 0; i < 4; ++i) v[i] = __bfloat162float(from[i]);
+    }
+  };
+  for (int k = 4 * tid; k < K; k += 4 * kNormThreads) {  // HC-pre mix (ops.cu:45-48); K is a multiple of 4
+    float v[4][4], s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) load4(h + (size_t(row) * 4 + j) * K + k, v[j]);
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      if (i + j < K) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[i] = __fadd_rn(s[i], __fmul_rn(p[j], v[j][i]));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) xrow[k + i] = __float2bfloat16_rn(s[i]);
+  }
+  __syncthreads();
+  const bool in = tid < threads;
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  if (in)
+    for (int i = tid * 4; i < K; i += threads * 4) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
         const float z = __bfloat162float(xrow[i + j]);
         v[j] = __fadd_rn(v[j], __fmul_rn(z, z));
       }
-  }
+    }
   float sum = __fadd_rn(__fadd_rn(__fadd_rn(v[0], v[1]), v[2]), v[3]);
-  sh[tid] = sum;
+  if (in) sh[tid] = sum;
   __syncthreads();
   for (int d = width / 2; d >= 32; d >>= 1) {
-    if (tid % width < d) { sum = __fadd_rn(sum, sh[tid + d]); sh[tid] = sum; }
+    if (in && tid % width < d) { sum = __fadd_rn(sum, sh[tid + d]); sh[tid] = sum; }
     __syncthreads();
   }
   for (int d = 16; d; d >>= 1) sum = __fadd_rn(sum, __shfl_down_sync(0xffffffffu, sum, d));
-  if (tid % width == 0) sh[tid] = sum;
+  if (in && tid % width == 0) sh[tid] = sum;
   __syncthreads();
-  for (int d = (blockDim.x / width) / 2; d; d >>= 1) {
-    if (tid % width == 0 && tid / width < d) { sum = __fadd_rn(sum, sh[tid + d * width]); sh[tid] = sum; }
+  for (int d = (threads / width) / 2; d; d >>= 1) {
+    if (in && tid % width == 0 && tid / width < d) { sum = __fadd_rn(sum, sh[tid + d * width]); sh[tid] = sum; }
     __syncthreads();
   }
-  const float total = sh[0];
-  __syncthreads();
-  if (tid == 0) sh[0] = rsqrtf(__fadd_rn(__fmul_rn(total, 1.f / K), eps));
-  __syncthreads();
-  const float rstd = sh[0];
-  for (int k = tid; k < K; k += blockDim.x) {
-    const __nv_bfloat16 yb =
-        __float2bfloat16_rn(__fmul_rn(__fmul_rn(__bfloat162float(xrow[k]), rstd), __bfloat162float(weight[k])));
-    out[size_t(row) * K + k] = __bfloat162float(yb);
+  const float rstd = rsqrtf(__fadd_rn(__fmul_rn(sh[0], 1.f / K), eps));
+  for (int k = 4 * tid; k < K; k += 4 * kNormThreads) {
+    float g[4], y[4];
+    load4(weight + k, g);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      y[i] = __bfloat162float(__float2bfloat16_rn(__fmul_rn(__fmul_rn(__bfloat162float(xrow[k + i]), rstd), g[i])));
+    float *to = out + size_t(row) * K + k;
+    if (vectors) {
+      *reinterpret_cast<float4 *>(to) = make_float4(y[0], y[1], y[2], y[3]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) to[i] = y[i];
+    }
   }
+}
+
+template <int M, int kRowsPerWarp, int kThreads>
+cudaError_t launch_compact_ring(const float *x, const void *w, float *y, int N, int K, int stages, int dev, int sms,
+                                cudaStream_t stream) {
+  static thread_local int configured = -1;
+  if (configured != dev) {
+    const cudaError_t e = cudaFuncSetAttribute(head_compact_ring_kernel<M, kRowsPerWarp, kThreads>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return e;
+    configured = dev;
+  }
+  const int groups = (N + kRowsPerWarp - 1) / kRowsPerWarp, warps = kThreads / 32, most = (groups + warps - 1) / warps;
+  const size_t smem = size_t(M) * K * sizeof(float) + size_t(warps) * stages * kRowsPerWarp * 512;
+  return launch_early(head_compact_ring_kernel<M, kRowsPerWarp, kThreads>, sms < most ? sms : most, kThreads, smem, stream,
+                      x, static_cast<const __nv_bfloat16 *>(w), y, N, K, stages);
 }
 
 template <int M>
 cudaError_t launch_compact(const float *x, const void *w, float *y, int N, int K, cudaStream_t stream) {
-  // weight rows that share one read of an activation fragment; at one or two batch rows the kernel only streams
-  // weights and more resident CTAs (fewer registers each) keep more loads in flight
-  constexpr int kRowsPerWarp = M <= 2 ? 2 : M <= 6 ? 4 : 2;
-  const size_t smem = size_t(M) * K * sizeof(float);
-  static thread_local int configured = -1;
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
+  // One CTA of sixteen warps per SM (twelve, with 168 registers per thread, from M = 5 on).  Weight rows that share one read of an activation fragment: per 512 bytes of weights and
+  // row M * 8 / rows cycles of shared memory, against the 22 cycles they take to arrive: four rows, or what the registers
+  // hold (three at M = 8).  A ring of 2, 3, 4 or 6 steps, what the activations leave room for.
+  constexpr int kRing = M <= 7 ? 4 : 3, kRingThreads = M <= 4 ? 512 : 384;
+  const size_t activations = size_t(M) * K * sizeof(float), step = size_t(kRingThreads / 32) * kRing * 512;
+  const int room = int((227 * 1024 - activations) / step);
+  const int stages = room >= 6 ? 6 : room > 4 ? 4 : room;
+  if (stages >= 2) return launch_compact_ring<M, kRing, kRingThreads>(x, w, y, N, K, stages, dev, sms, stream);
+  // activations that fill the shared memory: two steps of weights ahead in registers
+  constexpr int kRowsPerWarp = 2;
+  static thread_local int configured = -1;
   if (configured != dev) {
     e = cudaFuncSetAttribute(head_compact_kernel<M, kRowsPerWarp>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
     configured = dev;
   }
-  const int per_sm = smem <= 48 * 1024 ? 4 : smem <= 100 * 1024 ? 2 : 1;
-  const int groups = (N + kRowsPerWarp - 1) / kRowsPerWarp;
-  int grid = sms * per_sm;
-  if (grid > (groups + kHeadWarps - 1) / kHeadWarps) grid = (groups + kHeadWarps - 1) / kHeadWarps;
-  head_compact_kernel<M, kRowsPerWarp><<<grid, kHeadThreads, smem, stream>>>(x, static_cast<const __nv_bfloat16 *>(w), y, N, K);
+  const int groups = (N + kRowsPerWarp - 1) / kRowsPerWarp, most = (groups + kHeadWarps - 1) / kHeadWarps;
+  head_compact_kernel<M, kRowsPerWarp><<<sms < most ? sms : most, kHeadThreads, activations, stream>>>(
+      x, static_cast<const __nv_bfloat16 *>(w), y, N, K);
   return cudaGetLastError();
 }
 
@@ -236,11 +401,14 @@ extern "C" int ds41_b200_markov_logits(const float *draft_row, const void *marko
   if (!draft_row || !markov_weight_bf16 || !embedding_bf16 || !logits || vocab < 1 ||
       (reinterpret_cast<uintptr_t>(markov_weight_bf16) & 15u) || (reinterpret_cast<uintptr_t>(embedding_bf16) & 15u))
     return invalid("Markov logits arguments");
-  const long long threads = (long long)vocab * 32;
-  markov_logits_kernel<<<unsigned((threads + 255) / 256), 256, 0, stream>>>(
-      draft_row, static_cast<const __nv_bfloat16 *>(markov_weight_bf16), static_cast<const __nv_bfloat16 *>(embedding_bf16),
-      logits, vocab);
-  return int(cudaGetLastError());
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return int(e);
+  const int most = (vocab + kMarkovThreads / 32 * kMarkovRows - 1) / (kMarkovThreads / 32 * kMarkovRows);
+  return int(launch_early(markov_logits_kernel, 3 * sms < most ? 3 * sms : most, kMarkovThreads, 0, stream, draft_row,
+                          static_cast<const __nv_bfloat16 *>(markov_weight_bf16),
+                          static_cast<const __nv_bfloat16 *>(embedding_bf16), logits, vocab));
 }
 
 extern "C" int ds41_b200_final_norm(const void *h_bf16, const float *pre, const void *norm_weight_bf16, float *x_f32, int M,
@@ -250,8 +418,7 @@ extern "C" int ds41_b200_final_norm(const void *h_bf16, const float *pre, const 
     return invalid("final norm arguments");
   int width = 0;
   const int threads = rms_geometry(M, K, &width);
-  final_norm_kernel<<<M, threads, 512 * sizeof(float) + size_t(K) * 2, stream>>>(
-      static_cast<const __nv_bfloat16 *>(h_bf16), pre, static_cast<const __nv_bfloat16 *>(norm_weight_bf16), x_f32, K, eps,
-      width);
-  return int(cudaGetLastError());
+  return int(launch_early(final_norm_kernel, M, kNormThreads, 512 * sizeof(float) + size_t(K) * 2, stream,
+                          static_cast<const __nv_bfloat16 *>(h_bf16), pre, static_cast<const __nv_bfloat16 *>(norm_weight_bf16),
+                          x_f32, K, eps, width, threads));
 }

@@ -676,19 +676,6 @@ FlatInfo *flat_info(void *scratch, int rows) {
   return reinterpret_cast<FlatInfo *>(static_cast<unsigned char *>(scratch) + 4 * sizeof(int) + size_t(rows) * before);
 }
 
-namespace {
-template <class Kernel>
-cudaError_t launch_pass(Kernel kernel, int ctas, int threads, const FlatArgs &a, cudaStream_t stream) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(unsigned(ctas));
-  cfg.blockDim = dim3(unsigned(threads));
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1] = {programmatic_launch()};
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, a);
-}
-}  // namespace
-
 cudaError_t launch_flat(FlatArgs a, void *scratch, cudaStream_t stream) {
   if (!a.logits2) a.split = a.rows;
   a.log2e_t = kLog2e / a.t;
@@ -715,11 +702,11 @@ cudaError_t launch_flat(FlatArgs a, void *scratch, cudaStream_t stream) {
   if (e != cudaSuccess) return e;
   phase_restart();
   phase_mark(stream);
-  if (!a.head_stats && (e = launch_pass(flat_stats_kernel, a.rows * parts, kFT, a, stream)) != cudaSuccess) return e;
+  if (!a.head_stats && (e = launch_early(flat_stats_kernel, a.rows * parts, kFT, 0, stream, a)) != cudaSuccess) return e;
   phase_mark(stream);
-  if (!full && (e = launch_pass(flat_hist_kernel, a.rows * parts, kFT, a, stream)) != cudaSuccess) return e;
+  if (!full && (e = launch_early(flat_hist_kernel, a.rows * parts, kFT, 0, stream, a)) != cudaSuccess) return e;
   phase_mark(stream);
-  if ((e = launch_pass(flat_window_kernel, a.rows, kFlatWindowThreads, a, stream)) != cudaSuccess) return e;
+  if ((e = launch_early(flat_window_kernel, a.rows, kFlatWindowThreads, 0, stream, a)) != cudaSuccess) return e;
   phase_mark(stream);
   // the mass pass: four warps per CTA, one 1024-id sub-region per warp and round.  Six CTAs fit an SM (888 at a time on
   // the GPU), so the rows are cut into as many pieces as give about four waves or more: a grid of 1.4 waves (256 rows x
@@ -728,9 +715,9 @@ cudaError_t launch_flat(FlatArgs a, void *scratch, cudaStream_t stream) {
   while (mass_parts < 16 && a.rows * mass_parts < 2960) mass_parts <<= 1;
   FlatArgs m = a;
   m.parts = mass_parts;
-  if ((e = launch_pass(flat_mass_kernel, a.rows * mass_parts, kFlatMassThreads, m, stream)) != cudaSuccess) return e;
+  if ((e = launch_early(flat_mass_kernel, a.rows * mass_parts, kFlatMassThreads, 0, stream, m)) != cudaSuccess) return e;
   phase_mark(stream);
-  if ((e = launch_pass(flat_resolve_kernel, a.rows, kRT4, a, stream)) != cudaSuccess) return e;
+  if ((e = launch_early(flat_resolve_kernel, a.rows, kRT4, 0, stream, a)) != cudaSuccess) return e;
   phase_mark(stream);
   return cudaGetLastError();
 }

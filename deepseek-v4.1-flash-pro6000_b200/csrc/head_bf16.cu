@@ -2,14 +2,18 @@
 // bit.  The reference kernels (components/fuse-head/src/head_half_tree.cu:7-21, head_half_tune.cu:7-22) fix the FP32
 // arithmetic of out[m,n] = sum_k W[n,k] * x[m,k]: sixteen chains per output, chain l takes k = l, l+16, l+32, ... in
 // ascending order with one fused multiply-add per term, then the chains are added by a four-level tree (distance 8, 4,
-// 2, 1 over the chain index) and +0.f canonicalises a negative zero.  This kernel keeps exactly that order — every
-// intermediate is the same FP32 number — and changes only how the bytes move: a persistent CTA keeps the M activation
-// rows in shared memory, streams 64 weight rows x 256 K at a time through a double buffer with 16-byte cp.async copies
-// (512 bytes contiguous per weight row and copy, against 32 bytes per half-warp step in the reference), and each thread runs
-// the chains of two weight rows so that every activation load feeds two fused multiply-adds.
-// HBM-bound: the BF16 weights, 2*N*K bytes (1.32 GB at N=129280, K=5120), are read exactly once.
+// 2, 1 over the chain index) and +0.f canonicalises a negative zero.  This kernel keeps exactly that order -- every
+// intermediate is the same FP32 number -- and changes only how the bytes and the chains move: persistent CTAs keep the M
+// activation rows in shared memory, and every warp streams 32 weight rows x 64 K at a time through a ring of its own
+// (16-byte cp.async copies, no barrier of the CTA).  Four lanes share a weight row, each with four neighbouring chains (k .. k +
+// 3), so that one 8-byte load feeds four chains and the chains advance two at a time by packed FMAs; a lane has four rows, so
+// that an activation read from shared memory is used four times: per 512 bytes of weights that is 2 M cycles of shared
+// memory plus 8 for the weights, against the 22 they take to arrive (with one row per lane, M = 3 took 377 us, with two
+// 276).  HBM-bound: the BF16 weights, 2*N*K bytes (1.32 GB at N=129280, K=5120), are read exactly once.
 #include "ds41_b200.h"
 #include "host_error.h"
+#include "launch.h"
+#include "packed_fma.cuh"
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -17,108 +21,127 @@
 namespace ds41 {
 namespace {
 
-constexpr int kRowsPerCta = 64, kChunkK = 256, kHeadBf16Threads = 16 * kRowsPerCta / 2;  // 512: two rows per thread
-constexpr int kRowPitch = kChunkK * 2 + 32;  // bytes; the 32-byte skew keeps the two rows of a warp on different banks
+constexpr int kLaneRows = 4, kWarpRows = 8 * kLaneRows;                  // weight rows per lane; per warp (four lanes each)
+constexpr int kChunkK = 64, kRowPitch = kChunkK * 2 + 32;                // bytes; the skew keeps eight rows on different banks
+constexpr int kStageBytes = kWarpRows * kRowPitch;                       // 5 KB
+constexpr int kMostWarps = 7;   // 129280 rows are 3.9 rounds of 148 x 7 warps x 32 rows (eight warps: 3.4, the fourth half empty)
+constexpr size_t kSmemBudget = 227 * 1024;
 
 template <int M>
-__global__ void __launch_bounds__(kHeadBf16Threads) head_bf16_kernel(const float *x, const __nv_bfloat16 *w, float *y,
-                                                                     int N, int K) {
+__global__ void __launch_bounds__(32 * kMostWarps, 1) head_bf16_kernel(const float *x, const __nv_bfloat16 *w, float *y,
+                                                                       int N, int K, int stages) {
   extern __shared__ __align__(16) unsigned char smem[];
-  // activations chain-major: x[m][l + 16 j] at sx[(m * 16 + l) * pitch + j], so that a chain reads four consecutive
-  // terms with one 16-byte load (the pitch of K/16 + 4 floats spreads the sixteen chains over the banks)
-  float *sx = reinterpret_cast<float *>(smem);
-  const int pitch = K / 16 + 4;
-  unsigned char *sw = smem + size_t(M) * 16 * pitch * sizeof(float);             // [2][kRowsPerCta][kRowPitch]
-  const int tid = threadIdx.x, lane = tid & 15, pair = tid >> 4;                 // rows pair and pair + 32 of the block
-  for (int i = tid; i < M * K; i += kHeadBf16Threads) {
-    const int m = i / K, k = i - m * K;
-    sx[(m * 16 + (k & 15)) * pitch + (k >> 4)] = __ldg(x + i);
-  }
-  const int blocks = (N + kRowsPerCta - 1) / kRowsPerCta, chunks = K / kChunkK;
-  auto stage = [&](int block, int chunk, int buf) {  // 64 rows x 512 bytes, 16 bytes per copy
-    unsigned char *dst = sw + size_t(buf) * kRowsPerCta * kRowPitch;
-    for (int i = tid; i < kRowsPerCta * (kChunkK * 2 / 16); i += kHeadBf16Threads) {
-      const int r = i / (kChunkK * 2 / 16), c = i % (kChunkK * 2 / 16);
-      const int row = block * kRowsPerCta + r;
-      const uint32_t d = uint32_t(__cvta_generic_to_shared(dst + r * kRowPitch + c * 16));
-      if (row < N) {
-        const void *src = reinterpret_cast<const unsigned char *>(w + size_t(row) * K + size_t(chunk) * kChunkK) + c * 16;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-      } else {
-        *reinterpret_cast<uint4 *>(dst + r * kRowPitch + c * 16) = make_uint4(0u, 0u, 0u, 0u);  // the reference uses weight 0
+  float *sx = reinterpret_cast<float *>(smem);                                   // [M][K], then per warp [stages][32][kRowPitch]
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int quarter = lane & 3, row_in = lane >> 2;                              // chains 4 quarter .. + 3 of rows row_in + 8 r
+  unsigned char *ring = smem + size_t(M) * K * sizeof(float) + size_t(warp) * stages * kStageBytes;
+  const int groups = (N + kWarpRows - 1) / kWarpRows, chunks = K / kChunkK, stride = gridDim.x * warps;
+  // copies: lane l takes the 16-byte piece l % 8 of rows l / 8, l / 8 + 4, ...
+  const uint32_t copy_to = uint32_t(__cvta_generic_to_shared(ring)) + uint32_t((lane >> 3) * kRowPitch + (lane & 7) * 16);
+  int next_group = blockIdx.x * warps + warp, next_chunk = 0, next_slot = 0;
+  auto fetch = [&] {   // (an empty group once everything is on its way: the waits count groups)
+    if (next_group < groups) {
+      const int row0 = next_group * kWarpRows + (lane >> 3);
+#pragma unroll
+      for (int i = 0; i < kWarpRows / 4; ++i) {
+        const uint32_t d = copy_to + uint32_t(next_slot * kStageBytes + 4 * i * kRowPitch);
+        const int row = row0 + 4 * i;
+        const bool in = row < N;   // (beyond N: zeros; the reference uses weight 0)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d),
+                     "l"(w + size_t(in ? row : 0) * K + next_chunk * kChunkK + (lane & 7) * 8), "r"(in ? 16 : 0) : "memory");
       }
+      if (++next_chunk == chunks) { next_chunk = 0; next_group += stride; }
+      if (++next_slot == stages) next_slot = 0;
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  int buf = 0;
-  if (int(blockIdx.x) < blocks) stage(blockIdx.x, 0, 0);
-  for (int block = blockIdx.x; block < blocks; block += gridDim.x) {
-    float acc0[M], acc1[M];
+  for (int i = 0; i + 1 < stages; ++i) fetch();   // (weights only)
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+  if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < M * K / 4; i += blockDim.x)
+      reinterpret_cast<float4 *>(sx)[i] = __ldg(reinterpret_cast<const float4 *>(x) + i);
+  } else {
+    for (int i = threadIdx.x; i < M * K; i += blockDim.x) sx[i] = __ldg(x + i);
+  }
+  __syncthreads();
+  int slot = 0;
+  for (int g = blockIdx.x * warps + warp; g < groups; g += stride) {
+    float2x acc[kLaneRows][M][2];   // chains 4 quarter and + 1, + 2 and + 3
 #pragma unroll
-    for (int m = 0; m < M; ++m) { acc0[m] = 0.f; acc1[m] = 0.f; }
+    for (int r = 0; r < kLaneRows; ++r)
+#pragma unroll
+      for (int m = 0; m < M; ++m) acc[r][m][0] = acc[r][m][1] = 0ull;
     for (int chunk = 0; chunk < chunks; ++chunk) {
-      // next copy in flight while this chunk is consumed
-      int nb = block, nc = chunk + 1;
-      if (nc == chunks) { nb = block + gridDim.x; nc = 0; }
-      if (nb < blocks) stage(nb, nc, buf ^ 1); else asm volatile("cp.async.commit_group;" ::: "memory");
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-      __syncthreads();
-      const unsigned char *rows = sw + size_t(buf) * kRowsPerCta * kRowPitch;
-      const __nv_bfloat16 *w0 = reinterpret_cast<const __nv_bfloat16 *>(rows + pair * kRowPitch);
-      const __nv_bfloat16 *w1 = reinterpret_cast<const __nv_bfloat16 *>(rows + (pair + kRowsPerCta / 2) * kRowPitch);
-      const float *xs = sx + lane * pitch + chunk * (kChunkK / 16);  // this chain's terms of the chunk, row m at + m*16*pitch
+      if (stages == 4) asm volatile("cp.async.wait_group 2;" ::: "memory");
+      else if (stages == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
+      else asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();        // this chunk has landed for every lane, and every lane is done with the slot that is filled next
+      fetch();
+      const unsigned char *rows = ring + slot * kStageBytes + row_in * kRowPitch + quarter * 8;
+      if (++slot == stages) slot = 0;
+      const float *xs = sx + chunk * kChunkK + quarter * 4;
 #pragma unroll
-      for (int q = 0; q < kChunkK / 64; ++q) {  // four terms of the chain per round, in ascending k
-        float4 xv[M];
+      for (int j = 0; j < kChunkK / 16; ++j) {   // the chains' next terms, in ascending k
+        float2x wv[kLaneRows][2];
 #pragma unroll
-        for (int m = 0; m < M; ++m) xv[m] = *reinterpret_cast<const float4 *>(xs + size_t(m) * 16 * pitch + 4 * q);
+        for (int r = 0; r < kLaneRows; ++r) {
+          const uint2 v = *reinterpret_cast<const uint2 *>(rows + r * 8 * kRowPitch + j * 32);
+          wv[r][0] = promote_bf16x2(v.x); wv[r][1] = promote_bf16x2(v.y);
+        }
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const int k = lane + 16 * (4 * q + t);
-          const float a0 = __bfloat162float(w0[k]), a1 = __bfloat162float(w1[k]);
+        for (int m = 0; m < M; ++m) {
+          const ulonglong2 xv = *reinterpret_cast<const ulonglong2 *>(xs + size_t(m) * K + j * 16);
 #pragma unroll
-          for (int m = 0; m < M; ++m) {
-            const float xt = t == 0 ? xv[m].x : t == 1 ? xv[m].y : t == 2 ? xv[m].z : xv[m].w;
-            acc0[m] = __fmaf_rn(a0, xt, acc0[m]);
-            acc1[m] = __fmaf_rn(a1, xt, acc1[m]);
+          for (int r = 0; r < kLaneRows; ++r) {
+            acc[r][m][0] = fma_f32x2(wv[r][0], xv.x, acc[r][m][0]);
+            acc[r][m][1] = fma_f32x2(wv[r][1], xv.y, acc[r][m][1]);
           }
         }
       }
-      __syncthreads();
-      buf ^= 1;
     }
-    const int row0 = block * kRowsPerCta + pair, row1 = row0 + kRowsPerCta / 2;
 #pragma unroll
-    for (int m = 0; m < M; ++m) {
-      for (int d = 8; d; d >>= 1) {
-        acc0[m] = __fadd_rn(acc0[m], __shfl_down_sync(0xffffffffu, acc0[m], d, 16));
-        acc1[m] = __fadd_rn(acc1[m], __shfl_down_sync(0xffffffffu, acc1[m], d, 16));
+    for (int r = 0; r < kLaneRows; ++r) {
+      const int row = g * kWarpRows + row_in + 8 * r;
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        float c[4];   // the tree over the chains: distance 8, 4 across the four lanes, 2, 1 inside the lane
+        unpack_f32x2(acc[r][m][0], c[0], c[1]);
+        unpack_f32x2(acc[r][m][1], c[2], c[3]);
+#pragma unroll
+        for (int d = 2; d; d >>= 1)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) c[i] = __fadd_rn(c[i], __shfl_down_sync(0xffffffffu, c[i], d, 4));
+        c[0] = __fadd_rn(c[0], c[2]); c[1] = __fadd_rn(c[1], c[3]);
+        const float sum = __fadd_rn(c[0], c[1]);
+        if (quarter == 0 && row < N) y[size_t(m) * N + row] = __fadd_rn(sum, 0.f);
       }
-      if (lane == 0 && row0 < N) y[size_t(m) * N + row0] = __fadd_rn(acc0[m], 0.f);
-      if (lane == 0 && row1 < N) y[size_t(m) * N + row1] = __fadd_rn(acc1[m], 0.f);
     }
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 template <int M>
 cudaError_t launch_head_bf16(const float *x, const void *w, float *y, int N, int K, cudaStream_t stream) {
-  const size_t smem = size_t(M) * (K + 64) * sizeof(float) + 2 * size_t(kRowsPerCta) * kRowPitch;
+  const size_t activations = size_t(M) * K * sizeof(float);
+  int warps = kMostWarps;   // fewer where the activations leave no room for a ring of two stages per warp
+  while (warps > 1 && activations + size_t(warps) * 2 * kStageBytes > kSmemBudget) --warps;
+  int stages = 4;
+  while (stages > 1 && activations + size_t(warps) * stages * kStageBytes > kSmemBudget) --stages;
+  if (stages < 2) return cudaErrorInvalidValue;
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   static thread_local int configured = -1;
   if (configured != dev) {
-    e = cudaFuncSetAttribute(head_bf16_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    e = cudaFuncSetAttribute(head_bf16_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBudget));
     if (e != cudaSuccess) return e;
     configured = dev;
   }
-  if (smem > 227 * 1024) return cudaErrorInvalidValue;
-  const int blocks = (N + kRowsPerCta - 1) / kRowsPerCta;
-  head_bf16_kernel<M><<<blocks < sms ? blocks : sms, kHeadBf16Threads, smem, stream>>>(
-      x, static_cast<const __nv_bfloat16 *>(w), y, N, K);
-  return cudaGetLastError();
+  const int groups = (N + kWarpRows - 1) / kWarpRows, most = (groups + warps - 1) / warps;
+  return launch_early(head_bf16_kernel<M>, most < sms ? most : sms, 32 * warps, activations + size_t(warps) * stages * kStageBytes,
+                      stream, x, static_cast<const __nv_bfloat16 *>(w), y, N, K, stages);
 }
 
 }  // namespace
@@ -129,8 +152,8 @@ using namespace ds41;
 // General shapes (the tests use small N); ds41_fuse_head_decode below is the reference's restricted entry point.
 extern "C" int ds41_b200_head_bf16(const float *x, const void *weights_bf16, float *out, int M, int N, int K,
                                    cudaStream_t stream) {
-  if (!x || !weights_bf16 || !out || M < 1 || M > 6 || N < 1 || K < kChunkK || K % kChunkK ||
-      size_t(M) * (K + 64) * sizeof(float) + 2 * size_t(kRowsPerCta) * kRowPitch > 227 * 1024)
+  if (!x || !weights_bf16 || !out || M < 1 || M > 6 || N < 1 || K < 256 || K % 256 ||
+      size_t(M) * (K + 64) * sizeof(float) + 69632 > 227 * 1024)
     return invalid("BF16 head arguments (1 <= M <= 6, K a multiple of 256, M*K*4 bytes of activations + 68 KB within 227 KB)");
   if ((reinterpret_cast<uintptr_t>(weights_bf16) & 15u)) return invalid("BF16 head: weights must be 16-byte aligned");
   cudaError_t e;

@@ -20,6 +20,7 @@
 #include "ds41_b200.h"
 #include "flat.cuh"
 #include "host_error.h"
+#include "launch.h"
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
@@ -252,13 +253,26 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       uint64_t policy;
       if (b_tiles == 1) asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
       else asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
+      // the ring's first weights do not depend on the kernel in front of this one (the quantiser): they are on their way
+      // while it finishes
+      int early = kblocks / group < kStages ? kblocks / group : kStages;
+      for (int s = 0; s < early; ++s) {
+        mbar_expect_tx(&full[s], uint32_t(stage_bytes));
+        tma_load_3d(tiles + size_t(s) * stage_bytes, &map_w, &full[s], 0, int(blockIdx.x) / b_tiles * kTileN, s * group, policy);
+      }
+      cudaGridDependencySynchronize();
+      cudaTriggerProgrammaticLaunchCompletion();
       for (int tile = blockIdx.x; tile < total_tiles && !ab.set(); tile += gridDim.x) {
         const int nt = tile / b_tiles, bt = tile % b_tiles;
         for (int kb = 0; kb < kblocks; kb += group) {
           if (!mbar_wait(&empty[stage], phase ^ 1, ab)) break;
           unsigned char *w_dst = tiles + size_t(stage) * stage_bytes, *a_dst = w_dst + w_bytes;
-          mbar_expect_tx(&full[stage], uint32_t(stage_bytes));
-          tma_load_3d(w_dst, &map_w, &full[stage], 0, nt * kTileN, kb, policy);
+          if (early > 0) {
+            --early;
+          } else {
+            mbar_expect_tx(&full[stage], uint32_t(stage_bytes));
+            tma_load_3d(w_dst, &map_w, &full[stage], 0, nt * kTileN, kb, policy);
+          }
           tma_load_3d(a_dst, &map_a, &full[stage], 0, bt * kRows, kb);
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
@@ -266,6 +280,7 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (one lane)
+    cudaGridDependencySynchronize();
     if (lane == 0) {
       constexpr uint32_t idesc = umma_idesc(kTileN);
       const uint32_t tiles16 = smem_addr(tiles) >> 4, stage16 = uint32_t(stage_bytes) >> 4;
@@ -295,6 +310,7 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     }
   } else if ((warp & 3) < kQuads) {
     // ------------------------------------------------------------------ epilogue: warp = (lane quadrant, column group)
+    cudaGridDependencySynchronize();
     const int quad = warp & 3;          // TMEM lanes [32*quad, 32*quad+32) are readable by this warp: batch rows
     const int group = (warp - 2) >> 2;  // vocabulary ids [32*group, 32*group+32) of the tile
     const int row = quad * 32 + lane;   // batch row inside the tile
@@ -479,6 +495,8 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 // Activation quantisation: per (row, 128-wide K group) scale = 2^ceil(log2(max(amax,1e-4)/448)), e4m3 round to
 // nearest even with saturation (components/dense/src/dense.cu:8-16 with the group widened from 32 to 128).
 __global__ void quantize_kernel(const __nv_bfloat16 *x, uint8_t *a, float *scale, int groups) {
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
   const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (g >= groups) return;
   const uint2 raw = *reinterpret_cast<const uint2 *>(x + size_t(g) * 128 + lane * 4);
@@ -498,6 +516,15 @@ __global__ void quantize_kernel(const __nv_bfloat16 *x, uint8_t *a, float *scale
   }
   *reinterpret_cast<uint32_t *>(a + size_t(g) * 128 + lane * 4) = packed;
   if (lane == 0) scale[g] = s;
+}
+
+// Clears the row records before the head raises them.  (A memset would stand between two programmatic launches and wait for
+// the first; this kernel lets the head start at once -- the kernel in front of it has itself waited for everything
+// earlier -- and only finishes after that kernel.)
+__global__ void clear_stats_kernel(HeadRowStats *stats, int rows) {
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+  for (int i = threadIdx.x; i < rows; i += blockDim.x) stats[i] = HeadRowStats{0ull, 0u, 0u};
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -552,8 +579,7 @@ cudaError_t launch_head(const CUtensorMap &mw, const CUtensorMap &ma, const Head
   const int tiles = ((p.N + kVocab - 1) / kVocab) * b_tiles;
   int grid = tiles < sms ? tiles : sms;
   if (b_tiles <= grid) grid -= grid % b_tiles;  // every CTA then keeps one batch tile (and its scale table) for good
-  head_fp8_kernel<kRows, kVocab><<<grid, kHeadThreads, smem, stream>>>(mw, ma, q);
-  return cudaGetLastError();
+  return launch_early(head_fp8_kernel<kRows, kVocab>, grid, kHeadThreads, smem, stream, mw, ma, q);
 }
 
 }  // namespace
@@ -565,9 +591,8 @@ extern "C" int ds41_b200_quantize_activations(const void *x_bf16, void *a_e4m3, 
                                               cudaStream_t stream) {
   if (!x_bf16 || !a_e4m3 || !a_scale || M < 1 || K < 128 || K % 128) return invalid("quantize arguments");
   const int groups = M * (K / 128);
-  quantize_kernel<<<(groups * 32 + 255) / 256, 256, 0, stream>>>(static_cast<const __nv_bfloat16 *>(x_bf16),
-                                                                 static_cast<uint8_t *>(a_e4m3), a_scale, groups);
-  return int(cudaGetLastError());
+  return int(launch_early(quantize_kernel, (groups * 32 + 255) / 256, 256, 0, stream, static_cast<const __nv_bfloat16 *>(x_bf16),
+                          static_cast<uint8_t *>(a_e4m3), a_scale, groups));
 }
 
 namespace {
@@ -594,7 +619,7 @@ extern "C" int ds41_b200_head_fp8_stats(const void *a_e4m3, const float *a_scale
       logits_stride < N || !row_extremes || (reinterpret_cast<uintptr_t>(row_extremes) & 15u))
     return invalid("head arguments");
   static_assert(sizeof(HeadRowStats) == DS41_B200_ROW_EXTREMES_BYTES, "row record size");
-  cudaError_t e = cudaMemsetAsync(row_extremes, 0, size_t(M) * sizeof(HeadRowStats), stream);
+  const cudaError_t e = launch_early(clear_stats_kernel, 1, 512, 0, stream, static_cast<HeadRowStats *>(row_extremes), M);
   if (e != cudaSuccess) return int(e);
   HeadArgs p{};
   p.a_scale = a_scale; p.w_scale = w_scale; p.logits = logits; p.ldl = logits_stride;

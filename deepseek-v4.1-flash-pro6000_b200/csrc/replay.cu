@@ -74,14 +74,7 @@ cudaError_t launch_replay(const ReplayArgs &a, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     opted.fetch_or(1 << (dev & 31));
   }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(unsigned(ctas));
-  cfg.blockDim = dim3(kRT);
-  cfg.dynamicSmemBytes = kReplayDynamicBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1] = {programmatic_launch()};
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, replay_sample_kernel, a);
+  return launch_early(replay_sample_kernel, ctas, kRT, kReplayDynamicBytes, stream, a);
 }
 
 }  // namespace ds41
