@@ -5,17 +5,41 @@
 //   ds41_b200_verify_probabilities   ds41_spark_verify_v2       (:39-56)
 //   ds41_spark_sample_gpu_v2 / ds41_spark_verify_gpu_v2          (third_party/spark/src/sampling.cu:24-39,71-72;
 //                                                                 spark.h:133-134: FP32 measures normalised in FP64)
-// Every sum runs on one thread in index order, as the reference's host loops do, so that for the same probability rows
-// the results are the reference's bit for bit (no exponential is involved once the rows exist; ds41_b200_probabilities
-// itself can differ from the host's rows in the last place of exp()).  One CTA per row / per transaction: these are
-// compatibility and reporting paths (milliseconds per full-vocabulary row), not the decode-rate path.
+// Every sum has the roundings of the reference's host loops, so that for the same probability rows the results are the
+// reference's bit for bit (no exponential is involved once the rows exist; ds41_b200_probabilities itself can differ from the
+// host's rows in the last place of exp()).  Probability rows (prob_rows.cuh) and the verification take a cluster per row or
+// transaction; the other calls, and what the verification cannot certify from parallel sums, one CTA that follows the chains
+// (replay_core.cuh).  2 drafts + 3 target rows of 129280 to their verification record: 1475 us with one CTA for everything,
+// 882 with the certified verification, 213 with the clusters for the rows.
 #include "ds41_b200.h"
 #include "host_error.h"
-#include "replay_core.cuh"
+#include "launch.h"
+#include "prob_rows.cuh"
+#include "row_nucleus.cuh"
 #include <cmath>
 
 namespace ds41 {
+int cluster_size_for(int vocab);
 namespace {
+
+// One launch of `clusters` clusters of cl CTAs, with the kernel's shared memory allowed on the current device.
+template <class Args>
+cudaError_t launch_clusters(void (*kernel)(Args), int clusters, int cl, int threads, size_t smem, cudaStream_t stream,
+                            const Args &args) {
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(clusters) * unsigned(cl));
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(cl); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1] = programmatic_launch();
+  cfg.attrs = attr; cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, kernel, args);
+}
 
 constexpr int kRowNotNormalized = DS41_B200_ROW_NOT_NORMALIZED;
 
@@ -55,46 +79,6 @@ __device__ int first_max(ReplaySmem &s, const T *p, int n) {
     if (s.stage[w] > best || (s.stage[w] == best && s.red_i[w] < best_id)) { best = s.stage[w]; best_id = s.red_i[w]; }
   __syncthreads();
   return best_id == 0x7fffffff ? 0 : best_id;
-}
-
-struct ProbArgs {
-  const float *logits;
-  long long stride;
-  int rows, vocab;
-  double t, top_p;
-  double *out;
-  int32_t *status;
-  unsigned char *scratch;
-};
-
-__global__ void __launch_bounds__(kRT) probabilities_kernel(ProbArgs a) {
-  __shared__ ReplaySmem s;
-  extern __shared__ __align__(16) unsigned char dynamic[];
-  unsigned char *mine = a.scratch + size_t(blockIdx.x) * size_t(kReplayPad) * 12;
-  unsigned long long *key = reinterpret_cast<unsigned long long *>(mine);
-  int *idx = reinterpret_cast<int *>(mine + size_t(kReplayPad) * 8);
-  for (int row = blockIdx.x; row < a.rows; row += gridDim.x) {
-    const float *x = a.logits + size_t(row) * a.stride;
-    double *p = a.out + size_t(row) * a.vocab;
-    int bad = 0;
-    for (int i = threadIdx.x; i < a.vocab; i += kRT)
-      if ((__float_as_uint(x[i]) & 0x7f800000u) == 0x7f800000u) bad = 1;
-    bad = __syncthreads_or(bad);
-    if (bad) {  // "nonfinite logits" (sampling.cpp:32)
-      for (int i = threadIdx.x; i < a.vocab; i += kRT) p[i] = CUDART_NAN;
-      if (threadIdx.x == 0) a.status[row] = DS41_B200_ROW_NONFINITE;
-      __syncthreads();
-      continue;
-    }
-    if (a.t == 0) {  // one-hot at the first maximum
-      const int b = first_max(s, x, a.vocab);
-      for (int i = threadIdx.x; i < a.vocab; i += kRT) p[i] = i == b ? 1.0 : 0.0;
-    } else {
-      replay_probabilities(s, x, a.vocab, a.t, a.top_p, p, key, idx, dynamic);
-    }
-    if (threadIdx.x == 0) a.status[row] = 0;
-    __syncthreads();
-  }
 }
 
 template <class T>
@@ -150,13 +134,144 @@ struct VerifyRowsArgs {
   uint64_t seed, step;
   ds41_spark_result *results;
   int32_t *status;
+  int only_pending;      // 1: only the transactions that verify_rows_fast_kernel marked
 };
+
+// ---- the certified form of the same on probability rows: one cluster per transaction.  The accept tests are plain
+// arithmetic on single entries; what the reference's chains decide -- whether a row sums to one within 1e-8, and where a draw
+// falls -- is decided from parallel sums unless it lies within twice the difference that the two ways of summing can make
+// (vocab * 2^-53 relative per chain).  Such a transaction is marked and left to the literal kernel below.
+constexpr int kPending = -99, kMaxRowsChecked = 11;
+struct FastVerify {
+  double sum[kMaxCluster][kMaxRowsChecked];
+  int bad[kMaxCluster][kMaxRowsChecked];
+  double warp[kWarps];
+  int at, code, checks;   // first position that is not accepted; 0 rejected, else its status; q rows to check
+};
+
+__global__ void __launch_bounds__(kThreads, 2) verify_rows_fast_kernel(VerifyRowsArgs<double> a) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ FastVerify f;
+  RowSmem *s = reinterpret_cast<RowSmem *>(smem_raw);
+  RowCtx c = make_ctx(s, a.vocab);
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+  const int seq = blockIdx.x / c.nranks, n = a.vocab, D = a.drafts;
+  const double *p = a.p + size_t(seq) * (D + 1) * n, *q = a.q ? a.q + size_t(seq) * D * n : nullptr;
+  const int32_t *ids = a.draft_ids ? a.draft_ids + size_t(seq) * D : nullptr;
+  if (c.warp == 0) {
+    bool stop = false;
+    int code = 0;
+    if (c.lane < D) {
+      const int d = ids[c.lane];
+      if (d < 0 || d >= n) {
+        stop = true; code = DS41_B200_ROW_DRAFT;
+      } else {
+        const double pd = p[size_t(c.lane) * n + d], qd = q[size_t(c.lane) * n + d];
+        if (!(qd > 0)) { stop = true; code = DS41_B200_ROW_DRAFT; }
+        else stop = !(philox_uniform(a.seeds[seq], a.steps[seq], uint32_t(c.lane), 2u) < fmin(1.0, pd / qd));
+      }
+    }
+    const unsigned stops = __ballot_sync(0xffffffffu, stop);
+    const int at = stops ? __ffs(stops) - 1 : D;
+    code = __shfl_sync(0xffffffffu, code, at);
+    // the q row of every position that is reached is checked, except where the id already ends the walk
+    const bool id_wrong = at < D && (ids[at] < 0 || ids[at] >= n);
+    if (c.lane == 0) {
+      f.at = at; f.code = at < D ? code : 0; f.checks = at < D && !id_wrong ? at + 1 : at;
+      s->u = philox_uniform(a.seeds[seq], a.steps[seq], uint32_t(at), at < D ? 3u : 0u);
+    }
+  }
+  __syncthreads();
+  const int at = f.at, rows = D + 1 + f.checks;
+  const int j0 = c.warp * c.region, j1 = min(j0 + c.region, c.len);   // this warp's region of the slice
+  FastVerify *f0 = c.cluster.map_shared_rank(&f, 0);
+  for (int r = 0; r < rows; ++r) {
+    const double *row = (r <= D ? p + size_t(r) * n : q + size_t(r - D - 1) * n) + c.begin;
+    double sum = 0;
+    int bad = 0;
+#pragma unroll 8
+    for (int j = j0 + c.lane; j < j1; j += 32) {
+      const double v = __ldcg(row + j);
+      bad |= !(v >= 0.0 && v < CUDART_INF);
+      sum += v;
+    }
+    const double w = lanes_sum(sum);
+    if (c.lane == 0) f.warp[c.warp] = w;
+    bad = __syncthreads_or(bad);
+    if (c.tid == 0) {
+      double total = 0;
+      for (int v = 0; v < kWarps; ++v) total += f.warp[v];
+      f0->sum[c.rank][r] = total;
+      f0->bad[c.rank][r] = bad;
+    }
+    __syncthreads();
+  }
+  // the row (or residual) that is drawn from: its mass per warp region
+  const double *pk = p + size_t(at) * n, *qk = at < D ? q + size_t(at) * n : nullptr;
+  const bool draws = f.code == 0;
+  if (draws) {
+    double mass = 0;
+#pragma unroll 8
+    for (int j = j0 + c.lane; j < j1; j += 32) {
+      const double v = __ldcg(pk + c.begin + j);
+      mass += qk ? fmax(0.0, v - __ldcg(qk + c.begin + j)) : v;
+    }
+    mass = lanes_sum(mass);
+    if (c.lane == 0) c.cluster.map_shared_rank(&s->region, 0)->kept[c.rank * kWarps + c.warp] = mass;
+  }
+  c.cluster.sync();
+  if (c.rank != 0) return;
+  // the rows in the order in which the reference checks them: every target row, then the draft rows as they are reached
+  int status = 0;
+  bool pending = false;
+  for (int r = 0; r < rows && status == 0; ++r) {
+    double z = 0;
+    int bad = 0;
+    for (int k = 0; k < c.nranks; ++k) { z += f.sum[k][r]; bad |= f.bad[k][r]; }
+    const double off = fabs(z - 1.0);
+    if (bad) status = DS41_B200_ROW_NONFINITE;
+    else if (off > 1e-8 + 1e-10) status = kRowNotNormalized;
+    else if (off > 1e-8 - 1e-10) pending = true;
+  }
+  if (status == 0) status = f.code;
+  int token = -1;
+  if (status == 0 && !pending) {
+    bool close;
+    const double rel = 2.0 * (2.0 * double(n) + 1024.0) * kU;
+    token = draw_region(c, rel, 0.0, [&](int owner, int j, double (&v)[2]) {
+      const int id = owner * c.stride_ids + j, end = min(n, (owner + 1) * c.stride_ids);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        v[i] = id + i < end ? __ldcg(pk + id + i) : 0.0;
+        if (qk && id + i < end) v[i] = fmax(0.0, v[i] - __ldcg(qk + id + i));
+      }
+    }, &close);
+    if (token < 0 || close) pending = true;
+  }
+  if (c.tid == 0) {
+    ds41_spark_result r{};
+    if (pending) {
+      r.emitted = kPending;
+    } else if (status) {
+      r.emitted = -1;
+    } else {
+      for (int k = 0; k < at; ++k) r.tokens[r.emitted++] = ids[k];
+      r.tokens[r.emitted++] = token;
+      r.accepted_drafts = at; r.accepted_input_rows = at + 1; r.rejected = at < D ? 1 : 0;
+    }
+    a.results[seq] = r;
+    if (a.status && !pending) a.status[seq] = status;
+  }
+}
 
 // verify_impl of the reference (sampling.cpp:39-53) for one transaction per CTA.
 template <class T, bool kMeasure>
 __global__ void __launch_bounds__(kRT) verify_rows_kernel(VerifyRowsArgs<T> a) {
   __shared__ ReplaySmem s;
+  cudaGridDependencySynchronize();
   for (int seq = blockIdx.x; seq < a.sequences; seq += gridDim.x) {
+    if (a.only_pending && a.results[seq].emitted != kPending) continue;   // the same in every thread
     const int n = a.vocab, count = a.drafts;
     const T *p = a.p + size_t(seq) * (count + 1) * n;
     const T *q = a.q ? a.q + size_t(seq) * count * n : nullptr;
@@ -353,12 +468,8 @@ extern "C" int ds41_b200_probabilities(const ds41_b200_prob_args *p, cudaStream_
   ProbArgs a{p->logits, p->logits_stride, p->rows, p->vocab,
              p->temperature > 0 ? std::fmax(p->temperature, 1e-5) : 0.0,  // engine/src/sampling.cpp:209-210
              p->top_p, p->probabilities, p->status, static_cast<unsigned char *>(p->scratch)};
-  const int ctas = int(need / (size_t(kReplayPad) * 12));
-  const cudaError_t e = cudaFuncSetAttribute(probabilities_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             int(kReplayDynamicBytes));
-  if (e != cudaSuccess) return int(e);
-  probabilities_kernel<<<ctas, kRT, kReplayDynamicBytes, stream>>>(a);
-  return int(cudaGetLastError());
+  const int cl = cluster_size_for(p->vocab), clusters = int(need / (size_t(kReplayPad) * 12));
+  return int(launch_clusters(probability_rows_kernel, clusters, cl, kRT, sizeof(ProbSmem), stream, a));
 }
 
 extern "C" int ds41_b200_sample_probabilities(const double *p, int rows, int vocab, int64_t stride, const uint64_t *seeds,
@@ -378,9 +489,14 @@ extern "C" int ds41_b200_verify_probabilities(const int32_t *draft_ids, const do
   if (!results || !p || sequences < 1 || drafts < 0 || drafts > 5 || vocab < 1 || !seeds || !steps ||
       (drafts && (!draft_ids || (!q && !greedy))))
     return invalid("verify arguments");
-  VerifyRowsArgs<double> a{draft_ids, q, p, sequences, drafts, vocab, greedy ? 1 : 0, seeds, steps, 0, 0, results, status};
-  verify_rows_kernel<double, false><<<grid_for(sequences), kRT, 0, stream>>>(a);
-  return int(cudaGetLastError());
+  VerifyRowsArgs<double> a{draft_ids, q, p, sequences, drafts, vocab, greedy ? 1 : 0, seeds, steps, 0, 0, results, status, 0};
+  if (!greedy && vocab <= DS41_B200_MAX_VOCAB) {
+    const cudaError_t e = launch_clusters(verify_rows_fast_kernel, sequences, cluster_size_for(vocab), kThreads, sizeof(RowSmem),
+                                          stream, a);
+    if (e != cudaSuccess) return int(e);
+    a.only_pending = 1;   // what it could not certify
+  }
+  return int(launch_early(verify_rows_kernel<double, false>, grid_for(sequences), kRT, 0, stream, a));
 }
 
 // The reference's device sampler ABI (spark.h:133-134): FP32 measures on the device, one row / one transaction, the
@@ -397,7 +513,7 @@ extern "C" int ds41_spark_verify_gpu_v2(const int32_t *d, const float *q, const 
                                         uint64_t seed, uint64_t step, ds41_spark_result *out, void *stream) {
   if (!out || !p || drafts < 0 || drafts > 5 || vocab < 1 || (drafts && (!d || (!q && !greedy))))
     return int(cudaErrorInvalidValue);
-  VerifyRowsArgs<float> a{d, q, p, 1, drafts, vocab, greedy ? 1 : 0, nullptr, nullptr, seed, step, out, nullptr};
+  VerifyRowsArgs<float> a{d, q, p, 1, drafts, vocab, greedy ? 1 : 0, nullptr, nullptr, seed, step, out, nullptr, 0};
   verify_rows_kernel<float, true><<<1, kRT, 0, static_cast<cudaStream_t>(stream)>>>(a);
   return int(cudaGetLastError());
 }

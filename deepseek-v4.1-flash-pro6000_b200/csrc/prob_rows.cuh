@@ -1,0 +1,435 @@
+// Probability rows (probabilities(), sampling.cpp:30-38) by one cluster per row.  A row's values depend on two chains of the
+// reference: z = the sum of the exponentials in id order, and the top-p mass, summed over the stable order until it reaches
+// top_p.  Both have to keep every rounding, and both split: inside one binade of the accumulator a chain is an integer sum
+// (replay_core.cuh), so the terms are cut into tiles; parallel sums of the tiles tell each tile in which binade the chain will
+// reach it; every tile's integer sum at that spacing is taken at the same time; and one warp walks the tile sums (32 at a step)
+// and goes through the terms only of those tiles in which the chain leaves its binade, meets a tie or stops, or which guessed
+// wrong: about one per binade, a dozen for a row.  What a tile adds is exact in each of these cases.
+// The order is put together only as far as it can matter: ids go to buckets of their key, lower bounds of the buckets' masses
+// give a bucket by whose end the chain has surely stopped, and of the buckets before it only the tile that holds the cut is sorted.
+#pragma once
+#include "replay_core.cuh"
+#include "window.cuh"
+
+namespace ds41 {
+namespace {
+
+constexpr int kTileIds = 512;                                 // terms of z per warp: 16 a lane, the row's slice in one round
+constexpr int kRowWarps = kRT / 32;
+constexpr int kOrderChunk = 256, kOrderChunks = 512;          // positions of the order per tile of the mass; most tiles
+constexpr int kLiteral = 32;                                  // first terms of a chain from zero, added one by one
+constexpr int kMassBits = 44, kCountBits = 18;                // a bucket's lower bound of mass over its count, in one word
+static_assert(kRowWarps * kTileIds == kSliceCap, "one tile per warp");
+static_assert(kOrderChunks * kOrderChunk >= DS41_B200_MAX_VOCAB, "tiles of the order");
+
+struct ProbArgs {
+  const float *logits;
+  long long stride;
+  int rows, vocab;
+  double t, top_p;
+  double *out;
+  int32_t *status;
+  unsigned char *scratch;   // per cluster: kReplayPad keys and ids of the order
+};
+
+struct ProbFact { float best, low; int best_id, bad; };
+struct ProbCut { double mass; unsigned long long key; int id, sorted; };   // sorted = 0: the order has to be sorted as a whole
+
+struct ProbSmem {
+  double p[kSliceCap];
+  ReplaySmem r;
+  int count[kBuckets];           // ids of this slice in each bucket; then this slice's next place in the bucket
+  int starts[kBuckets + 1];      // ids of the row in each bucket; then its first position
+  double part[kOrderChunks];     // parallel sums of the tiles, in every CTA
+  unsigned long long units[kOrderChunks];   // rank 0: integer sums of the tiles
+  int binade[kOrderChunks];      // rank 0: at which binade; -1 if a term ties
+  ProbFact fact[2][kMaxCluster];
+  ProbCut cut;
+  double z;
+  int limit, at, found;
+};
+
+// Where the walk stands after the tiles from `c` on that are plain integer sums: the first tile that is not (or `tiles`).
+template <class Stop>
+__device__ int walk_plain(const ProbSmem &s, int c, int tiles, double &acc, Stop stop) {
+  const int lane = threadIdx.x & 31;
+  for (;;) {
+    int be;
+    unsigned long long s0;
+    split_double(acc, be, s0);
+    const int i = c + lane;
+    const bool ok = i < tiles && s.binade[i] == be && s.units[i] < kTwo53;
+    const unsigned long long through = s0 + lanes_scan(lane, ok ? s.units[i] : 0ull);
+    const bool plain = ok && through < kTwo53 && !stop(join_double(through, be));
+    const unsigned ends = __ballot_sync(0xffffffffu, !plain);
+    const int f = ends ? __ffs(ends) - 1 : 32;
+    if (f > 0) acc = join_double(__shfl_sync(0xffffffffu, through, f - 1), be);
+    c += f;
+    if (f < 32) return min(c, tiles);
+  }
+}
+
+// exact_sequential of a short run of non-negative terms by one warp: value(0) .. value(m - 1) on top of acc, the first
+// `literal` of them one by one (a chain that starts from zero leaves a binade with almost every one of its first terms).
+template <class Value, class Stop>
+__device__ SeqResult warp_sequential(int m, Value value, Stop stop, double acc, int literal) {
+  const int lane = threadIdx.x & 31;
+  literal = min(literal, m);
+#pragma unroll 8
+  for (int i = 0; i < literal; ++i) {
+    const double before = acc;
+    acc = __dadd_rn(acc, value(i));
+    if (stop(acc)) return SeqResult{i, acc, before};
+  }
+  for (int base = literal; base < m; base += 128) {
+    double v[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) v[r] = base + 4 * lane + r < m ? value(base + 4 * lane + r) : 0.0;
+    int pos = base;
+    for (;;) {   // uniform: one pass per stretch inside one binade
+      int be;
+      unsigned long long s0, t[4], sum = 0;
+      split_double(acc, be, s0);
+      unsigned ties = 0;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        bool tie = false;
+        t[r] = base + 4 * lane + r >= pos ? to_units(v[r], be, &tie) : 0ull;
+        ties |= tie ? 1u << r : 0u;
+        sum += t[r];
+      }
+      const unsigned long long through = s0 + lanes_scan(lane, sum);
+      const unsigned looks = __ballot_sync(0xffffffffu, ties != 0 || through >= kTwo53 || stop(join_double(through, be)));
+      if (!looks) {
+        acc = join_double(__shfl_sync(0xffffffffu, through, 31), be);
+        break;
+      }
+      const int who = __ffs(looks) - 1;
+      int at = -1;
+      double next = 0.0, before = 0.0;
+      unsigned long long running = through - sum;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        if (at >= 0 || base + 4 * lane + r < pos) continue;
+        const unsigned long long through_r = running + t[r];
+        if (((ties >> r) & 1u) || through_r >= kTwo53) {   // the reference's own addition
+          at = r; before = join_double(running, be); next = __dadd_rn(before, v[r]);
+        } else if (stop(join_double(through_r, be))) {
+          at = r; before = join_double(running, be); next = join_double(through_r, be);
+        }
+        running = through_r;
+      }
+      at = __shfl_sync(0xffffffffu, at, who);
+      acc = __shfl_sync(0xffffffffu, next, who);
+      before = __shfl_sync(0xffffffffu, before, who);
+      at += base + 4 * who;
+      if (stop(acc)) return SeqResult{at, acc, before};
+      pos = at + 1;
+      if (pos >= base + 128) break;
+    }
+  }
+  return SeqResult{-1, acc, acc};
+}
+
+// What the tiles' parallel sums say of the accumulator in front of tile c.
+__device__ __forceinline__ int guess_binade(const ProbSmem &s, int c) {
+  const int lane = threadIdx.x & 31;
+  double before = 0;
+  for (int i = lane; i < c; i += 32) before += s.part[i];
+  int be;
+  unsigned long long units;
+  split_double(lanes_sum(before), be, units);
+  return be;
+}
+__device__ __forceinline__ unsigned long long lanes_sum_u64(unsigned long long v) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Positions of the order's tile c: the buckets that begin within its kOrderChunk positions, up to `end`.
+__device__ __forceinline__ void order_chunk(const BucketOrder &b, int c, int end, int *st, int *m) {
+  *st = min(end, b.starts[b.bucket_from(c * kOrderChunk)]);
+  *m = min(end, b.starts[b.bucket_from((c + 1) * kOrderChunk)]) - *st;
+}
+
+// key[0..m) / idx[0..m) of the order into s.r.key / s.r.idx, sorted; m <= kTile.  All threads of the CTA.
+__device__ void sort_chunk(ReplaySmem &s, const unsigned long long *key, const int *idx, int m) {
+  const int tid = threadIdx.x;
+  int padded = 2;
+  while (padded < m) padded <<= 1;
+  for (int i = tid; i < padded; i += kRT) {
+    s.key[i] = i < m ? __ldcg(key + i) : ~0ull;
+    s.idx[i] = i < m ? __ldcg(idx + i) : 0x7fffffff;
+  }
+  __syncthreads();
+  for (int k = 2; k <= padded; k <<= 1)
+    for (int jj = k >> 1; jj > 0; jj >>= 1) {
+      for (int i = tid; i < padded / 2; i += kRT) {
+        const int lo = ((i & ~(jj - 1)) << 1) | (i & (jj - 1)), hi = lo + jj;   // jj is a power of two
+        const bool up = (lo & k) == 0;
+        const unsigned long long ka = s.key[lo], kb = s.key[hi];
+        const int ia = s.idx[lo], ib = s.idx[hi];
+        if (key_less(kb, ib, ka, ia) == up) { s.key[lo] = kb; s.key[hi] = ka; s.idx[lo] = ib; s.idx[hi] = ia; }
+      }
+      __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  ProbSmem &s = *reinterpret_cast<ProbSmem *>(smem_raw);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = int(cluster.block_rank()), ranks = int(cluster.num_blocks());
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = a.vocab;
+  const int stride = (((n + ranks - 1) / ranks) + 31) & ~31, begin = min(n, rank * stride), len = min(n, begin + stride) - begin;
+  const int slot = blockIdx.x / ranks, first = warp * kTileIds + lane;   // the thread's ids: first + 32 r
+  const double top = a.top_p;
+  unsigned long long *key = reinterpret_cast<unsigned long long *>(a.scratch + size_t(slot) * size_t(kReplayPad) * 12);
+  int *idx = reinterpret_cast<int *>(key + kReplayPad);
+  ProbSmem *s0 = cluster.map_shared_rank(&s, 0);
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+  int parity = 0;
+  for (int row = slot; row < a.rows; row += gridDim.x / ranks, parity ^= 1) {
+    const float *x = a.logits + size_t(row) * a.stride + begin;
+    double *out = a.out + size_t(row) * n + begin;
+    // the slice, read once; first maximum, minimum (where the order's bucket grid ends), non-finite entries
+    float v[kTileIds / 32];
+#pragma unroll
+    for (int r = 0; r < kTileIds / 32; ++r) v[r] = first + 32 * r < len ? __ldg(x + first + 32 * r) : -CUDART_INF_F;
+    ProbFact f{-CUDART_INF_F, CUDART_INF_F, 0x7fffffff, 0};
+#pragma unroll
+    for (int r = 0; r < kTileIds / 32; ++r) {
+      if (first + 32 * r >= len) break;
+      if ((__float_as_uint(v[r]) & 0x7f800000u) == 0x7f800000u) f.bad = 1;
+      if (v[r] > f.best) { f.best = v[r]; f.best_id = begin + first + 32 * r; }
+      f.low = fminf(f.low, v[r]);
+    }
+    auto join = [](ProbFact &m, const ProbFact &o) {
+      if (o.best > m.best || (o.best == m.best && o.best_id < m.best_id)) { m.best = o.best; m.best_id = o.best_id; }
+      m.low = fminf(m.low, o.low);
+      m.bad |= o.bad;
+    };
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      ProbFact g;
+      g.best = __shfl_xor_sync(0xffffffffu, f.best, o);
+      g.low = __shfl_xor_sync(0xffffffffu, f.low, o);
+      g.best_id = __shfl_xor_sync(0xffffffffu, f.best_id, o);
+      g.bad = __shfl_xor_sync(0xffffffffu, f.bad, o);
+      join(f, g);
+    }
+    ProbFact *warps = reinterpret_cast<ProbFact *>(s.r.stage);
+    if (lane == 0) warps[warp] = f;
+    for (int i = tid; i < kBuckets; i += kRT) s.count[i] = 0;
+    __syncthreads();
+    if (tid < ranks) {
+      f = warps[0];
+      for (int w = 1; w < kRowWarps; ++w) join(f, warps[w]);
+      cluster.map_shared_rank(&s, tid)->fact[parity][rank] = f;
+    }
+    cluster.sync();
+    f = s.fact[parity][0];
+    for (int k = 1; k < ranks; ++k) join(f, s.fact[parity][k]);
+    if (rank == 0 && tid == 0) a.status[row] = f.bad ? DS41_B200_ROW_NONFINITE : 0;
+    if (f.bad || a.t == 0) {   // "nonfinite logits" (sampling.cpp:32); one-hot at the first maximum
+      for (int j = tid; j < len; j += kRT) out[j] = f.bad ? CUDART_NAN : begin + j == f.best_id ? 1.0 : 0.0;
+      continue;
+    }
+
+    // exponentials and z
+    const double xb = double(f.best);
+    double sum = 0;
+#pragma unroll 4
+    for (int r = 0; r < kTileIds / 32; ++r) {
+      if (first + 32 * r >= len) break;
+      const double e = exp_nonpos((double(v[r]) - xb) / a.t);
+      s.p[first + 32 * r] = e;
+      sum += e;
+    }
+    sum = lanes_sum(sum);
+    if (lane < ranks) cluster.map_shared_rank(&s, lane)->part[rank * kRowWarps + warp] = sum;
+    cluster.sync();
+    {
+      const int be = guess_binade(s, rank * kRowWarps + warp);
+      unsigned long long units = 0;
+      int ties = 0;
+#pragma unroll 4
+      for (int r = 0; r < kTileIds / 32; ++r) {
+        if (first + 32 * r >= len) break;
+        bool tie;
+        units += to_units(s.p[first + 32 * r], be, &tie);
+        ties |= tie ? 1 : 0;
+      }
+      units = lanes_sum_u64(units);
+      ties = __any_sync(0xffffffffu, ties);
+      if (lane == 0) { s0->units[rank * kRowWarps + warp] = units; s0->binade[rank * kRowWarps + warp] = ties ? -1 : be; }
+    }
+    cluster.sync();
+    if (rank == 0 && warp == 0) {
+      auto never = [](double) { return false; };
+      const int tiles = ranks * kRowWarps;
+      double acc = 0.0;
+      for (int c = 0; (c = walk_plain(s, c, tiles, acc, never)) < tiles; ++c) {
+        const int owner = c / kRowWarps, at = (c % kRowWarps) * kTileIds, have = min(n - owner * stride, stride) - at;
+        const double *terms = cluster.map_shared_rank(s.p, owner) + at;
+        acc = warp_sequential(max(0, min(kTileIds, have)), [terms](int i) { return terms[i]; }, never, acc, c == 0 ? kLiteral : 0).acc;
+      }
+      if (lane < ranks) cluster.map_shared_rank(&s, lane)->z = acc;
+    }
+    cluster.sync();
+    const double z = s.z;
+    if (!(top < 1.0)) {
+#pragma unroll 4
+      for (int r = 0; r < kTileIds / 32; ++r)
+        if (first + 32 * r < len) out[first + 32 * r] = s.p[first + 32 * r] / z;
+      continue;
+    }
+
+    // the order, as far as it matters: ids per bucket of every slice, the slices' places in the buckets, first positions
+    BucketOrder b;
+    b.starts = s.starts;
+    b.n = n;
+    bucket_grid(b, 1.0 / z, exp_nonpos((double(f.low) - xb) / a.t) / z);
+#pragma unroll 4
+    for (int r = 0; r < kTileIds / 32; ++r) {
+      if (first + 32 * r >= len) break;
+      const double p = s.p[first + 32 * r] / z;
+      s.p[first + 32 * r] = p;
+      atomicAdd(&s.count[b.bucket_of(order_key(p))], 1);
+    }
+    cluster.sync();
+    const int per = kBuckets / ranks;
+    for (int i = rank * per + tid; i < (rank + 1) * per; i += kRT) {
+      int c[kMaxCluster], run = 0;
+#pragma unroll
+      for (int k = 0; k < kMaxCluster; ++k) c[k] = k < ranks ? cluster.map_shared_rank(&s, k)->count[i] : 0;
+#pragma unroll
+      for (int k = 0; k < kMaxCluster; ++k) {
+        if (k < ranks) cluster.map_shared_rank(&s, k)->count[i] = run;
+        run += c[k];
+      }
+#pragma unroll
+      for (int k = 0; k < kMaxCluster; ++k)
+        if (k < ranks) cluster.map_shared_rank(&s, k)->starts[i] = run;
+    }
+    if (tid == 0) s.limit = kBuckets - 1;
+    cluster.sync();
+    {
+      // The first bucket by whose end the mass is surely past top_p: every entry of a bucket is at least its last key's p.
+      // (1e-9 of room over what the chain's own rounding can take away, vocab * 2^-53.)
+      constexpr int kPer = kBuckets / kRT;
+      unsigned long long mine[kPer], all = 0, total;
+#pragma unroll
+      for (int r = 0; r < kPer; ++r) {
+        const int i = tid * kPer + r, c = s.starts[i];
+        mine[r] = ((unsigned long long)(double(c) * b.least(i) * double(1ull << kMassBits)) << kCountBits) | unsigned(c);
+        all += mine[r];
+      }
+      unsigned long long run = block_exclusive_u64(s.r, all, &total);
+      const unsigned long long want = (unsigned long long)(top * (1.0 + 1e-9) * double(1ull << kMassBits)) + 1;
+#pragma unroll
+      for (int r = 0; r < kPer; ++r) {
+        s.starts[tid * kPer + r] = int(run & ((1u << kCountBits) - 1));
+        const unsigned long long next = run + mine[r];
+        if ((run >> kCountBits) < want && (next >> kCountBits) >= want) s.limit = tid * kPer + r;   // at most one thread
+        run = next;
+      }
+      if (tid == 0) s.starts[kBuckets] = n;
+    }
+    __syncthreads();
+    const int limit = s.limit, end = s.starts[limit + 1];
+#pragma unroll 4
+    for (int r = 0; r < kTileIds / 32; ++r) {
+      if (first + 32 * r >= len) break;
+      const unsigned long long k = order_key(s.p[first + 32 * r]);
+      const int q = b.bucket_of(k);
+      if (q > limit) continue;
+      const int pos = s.starts[q] + atomicAdd(&s.count[q], 1);
+      key[pos] = k; idx[pos] = begin + first + 32 * r;
+    }
+    cluster.sync();
+    const int chunks = (end + kOrderChunk - 1) / kOrderChunk;
+    if (chunks > 1) {   // (the first tile's terms are gone through in any case)
+      for (int c = rank + ranks * warp; c < chunks; c += ranks * kRowWarps) {
+        int st, m;
+        order_chunk(b, c, end, &st, &m);
+        double part = 0;
+        for (int j = lane; j < m; j += 32) part += key_mass(__ldcg(key + st + j));
+        part = lanes_sum(part);
+        if (lane < ranks) cluster.map_shared_rank(&s, lane)->part[c] = part;
+      }
+      cluster.sync();
+      for (int c = rank + ranks * warp; c < chunks; c += ranks * kRowWarps) {
+        int st, m, ties = 0;
+        order_chunk(b, c, end, &st, &m);
+        const int be = guess_binade(s, c);
+        unsigned long long units = 0;
+        for (int j = lane; j < m; j += 32) {
+          bool tie;
+          units += to_units(key_mass(__ldcg(key + st + j)), be, &tie);
+          ties |= tie ? 1 : 0;
+        }
+        units = lanes_sum_u64(units);
+        ties = __any_sync(0xffffffffu, ties);
+        if (lane == 0) { s0->units[c] = units; s0->binade[c] = ties ? -1 : be; }
+      }
+      cluster.sync();
+    }
+    auto past = [top](double mass) { return !(mass < top); };   // the reference's loop: mass += p[idx[k++]] while k < n && mass < top
+    auto publish = [&](const ProbCut &cut) { if (lane < ranks) cluster.map_shared_rank(&s, lane)->cut = cut; };   // one warp
+    if (rank == 0) {
+      double acc = 0.0;   // of warp 0
+      ProbCut cut{0.0, ~0ull, 0x7fffffff, 1};
+      for (int c = 0;; ++c) {
+        if (warp == 0) {
+          if (c > 0) c = walk_plain(s, c, chunks, acc, past);
+          if (lane == 0) s.at = c;
+        }
+        __syncthreads();
+        c = s.at;
+        if (c >= chunks) { cut.mass = acc; cut.sorted = end == n; break; }   // ran through: everything is kept
+        int st, m;
+        order_chunk(b, c, end, &st, &m);
+        if (m > kTile) { cut.sorted = 0; break; }                          // a long run of (nearly) equal entries
+        sort_chunk(s.r, key + st, idx + st, m);
+        if (warp == 0) {
+          const SeqResult r = warp_sequential(m, [&s](int i) { return key_mass(s.r.key[i]); }, past, acc, c == 0 ? kLiteral : 0);
+          acc = r.acc;
+          if (lane == 0) s.found = r.found;
+        }
+        __syncthreads();
+        if (s.found >= 0) { cut.mass = acc; cut.key = s.r.key[s.found]; cut.id = s.r.idx[s.found]; break; }
+      }
+      if (warp == 0) publish(cut);
+    }
+    cluster.sync();
+    if (!s.cut.sorted) {   // (the same in every CTA)
+      for (int j = tid; j < len; j += kRT) { key[begin + j] = order_key(s.p[j]); idx[begin + j] = begin + j; }
+      for (int j = n + rank * kRT + tid; j < kReplayPad; j += ranks * kRT) { key[j] = ~0ull; idx[j] = 0x7fffffff; }
+      cluster.sync();
+      if (rank == 0) {
+        sort_pairs(s.r, key, idx);
+        const SeqResult r = exact_sequential(s.r, n, [key](int i) { return key_mass(key[i]); }, past);
+        ProbCut cut{r.acc, ~0ull, 0x7fffffff, 1};
+        if (r.found >= 0) { cut.key = key[r.found]; cut.id = idx[r.found]; }
+        if (warp == 0) publish(cut);
+      }
+      cluster.sync();
+    }
+    // the rest is zeroed and every p divided by the kept mass
+    const ProbCut cut = s.cut;
+#pragma unroll 4
+    for (int r = 0; r < kTileIds / 32; ++r) {
+      const int j = first + 32 * r;
+      if (j >= len) break;
+      const double p = s.p[j];
+      const unsigned long long k = order_key(p);
+      out[j] = k < cut.key || (k == cut.key && begin + j <= cut.id) ? p / cut.mass : 0.0;
+    }
+  }
+}
+
+}  // namespace
+}  // namespace ds41

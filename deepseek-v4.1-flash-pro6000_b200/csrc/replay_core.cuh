@@ -181,11 +181,19 @@ __device__ SeqResult exact_sequential(ReplaySmem &s, int n, Value value, Stop st
     start = head;
   }
   int parity = 0;
+  // every thread keeps kSumPer consecutive terms in registers, and the next tile's are on their way while it works on one
+  double v[kSumPer], next[kSumPer];
+#pragma unroll
+  for (int r = 0; r < kSumPer; ++r) next[r] = start + tid * kSumPer + r < n ? value(start + tid * kSumPer + r) : 0.0;
   for (int base = start; base < n; base += kSumTile) {
     const int m = min(kSumTile, n - base);
-    // every thread keeps kSumPer consecutive terms in registers
-    double v[kSumPer];
     int bad = 0;
+#pragma unroll
+    for (int r = 0; r < kSumPer; ++r) {
+      v[r] = next[r];
+      const int i = base + kSumTile + tid * kSumPer + r;
+      next[r] = i < n ? value(i) : 0.0;
+    }
     {
       // A first look at the tile as a whole: if no term is invalid or ties, and the chain neither leaves its binade nor
       // stops by the tile's end, the tile is one integer sum (one barrier).
@@ -195,8 +203,6 @@ __device__ SeqResult exact_sequential(ReplaySmem &s, int n, Value value, Stop st
       int tied = 0;
 #pragma unroll
       for (int r = 0; r < kSumPer; ++r) {
-        const int i = tid * kSumPer + r;
-        v[r] = i < m ? value(base + i) : 0.0;
         bad |= !(v[r] >= 0.0 && v[r] < CUDART_INF);
         bool tie;
         quick += to_units(v[r], be0, &tie);
@@ -346,23 +352,32 @@ struct BucketOrder {
     }
     return lo;
   }
+  // no p of bucket i is less
+  __device__ __forceinline__ double least(int i) const {
+    const double hi = double(hi_min) + ceil(double(i + 1) / double(scale) * (1.0 + 1e-6)) + 2.0;
+    return i == kBuckets - 1 || hi > 4294967295.0 ? 0.0 : __hiloint2double(int(~uint32_t(hi)), 0);
+  }
 };
 
 __device__ __forceinline__ unsigned long long order_key(double p) { return ~(unsigned long long)__double_as_longlong(p); }
+__device__ __forceinline__ double key_mass(unsigned long long key) { return __longlong_as_double((long long)~key); }
 
-// The bucket grid for probabilities between p_max and p_low (or kSpanCap below p_max; the rest shares the last bucket);
-// clears the counters.  Every thread gets the same record.
+// The bucket grid for probabilities between p_max and p_low (or kSpanCap below p_max; the rest shares the last bucket).
+__device__ __forceinline__ void bucket_grid(BucketOrder &b, double p_max, double p_low) {
+  b.hi_min = uint32_t(order_key(p_max) >> 32);
+  const uint32_t hi_low = uint32_t(order_key(p_low) >> 32);
+  uint32_t span = p_low > 0 ? (hi_low >= b.hi_min ? hi_low - b.hi_min + 1 : 1) : uint32_t(kSpanCap);
+  if (span > uint32_t(kSpanCap)) span = kSpanCap;
+  b.scale = float(kBuckets - 1) / float(span);
+}
+// The grid with cleared counters.  Every thread gets the same record.
 __device__ BucketOrder bucket_begin(unsigned char *dynamic, int n, double p_max, double p_low) {
   BucketOrder b;
   b.wkey = reinterpret_cast<unsigned long long *>(dynamic);
   b.widx = reinterpret_cast<int *>(dynamic + size_t(kRT / 32) * kWarpSort * 8);
   b.starts = reinterpret_cast<int *>(dynamic + size_t(kRT / 32) * kWarpSort * 12);
   b.n = n;
-  b.hi_min = uint32_t(order_key(p_max) >> 32);
-  const uint32_t hi_low = uint32_t(order_key(p_low) >> 32);
-  uint32_t span = p_low > 0 ? (hi_low >= b.hi_min ? hi_low - b.hi_min + 1 : 1) : uint32_t(kSpanCap);
-  if (span > uint32_t(kSpanCap)) span = kSpanCap;
-  b.scale = float(kBuckets - 1) / float(span);
+  bucket_grid(b, p_max, p_low);
   for (int i = threadIdx.x; i <= kBuckets; i += kRT) b.starts[i] = 0;
   __syncthreads();
   return b;

@@ -1,6 +1,6 @@
 """The sizes at which a sampling or verification call changes its path (csrc/sampler.cu, csrc/verify.cu): the last batch of the
 cluster kernel and the first of the grid-wide passes, rows at odd addresses, vocabularies around the cluster sizes.  Tokens
-and records against the CPU oracle."""
+and records against the CPU oracle; likewise the operators on probability rows (csrc/prob.cu)."""
 import numpy as np
 import pytest
 import torch
@@ -59,3 +59,54 @@ def test_verification(pkg, oracle, seqs, drafts, vocab, t, top, sigma):
     got = pkg.results_to_numpy(res)
     assert (st.cpu().numpy() == 0).all()
     assert all((got[f] == want[f]).all() for f in ("tokens", "emitted", "accepted_drafts", "rejected")), (got, want)
+
+
+@pytest.mark.parametrize("rows,vocab", [(34, 700), (3, 16384), (3, 16385), (3, 32769), (3, 131072), (2, 1)])
+@pytest.mark.parametrize("t,top", [(0.7, 0.95), (1.0, 1.0)])
+def test_probability_rows(pkg, oracle, rows, vocab, t, top):
+    x = oracle.gen_logits(17 + vocab, rows, vocab)
+    x[1] = oracle.gen_normal(18, vocab, (1, vocab), 1.28)[0]
+    if rows > 2:
+        x[2, : (vocab + 1) // 2] = x[2].max()                     # thousands tied at the cut: the order is sorted as a whole
+    got, st = pkg.probabilities(cu(x), t, top)
+    got = got.cpu().numpy()
+    assert (st.cpu().numpy() == 0).all()
+    for r in range(rows):
+        want = oracle.probabilities(x[r], t, top)
+        assert np.array_equal(got[r] > 0, want > 0), (r, int((got[r] > 0).sum()), int((want > 0).sum()))
+        assert (np.abs(got[r] - want) <= 8 * 2.0 ** -52 * want).all()
+
+
+@pytest.mark.parametrize("vocab", [129280, 16385, 700])
+def test_verified_rows_and_their_faults(pkg, oracle, vocab):
+    """Every transaction has its own fault; the status and, without one, the record are the reference's."""
+    cases, drafts = 9, 3
+    target = oracle.gen_logits(27, cases * (drafts + 1), vocab)
+    draft = oracle.gen_perturbed(27, target.reshape(cases, drafts + 1, vocab)[:, :drafts].reshape(-1, vocab), 0.2)
+    p = np.stack([oracle.probabilities(r, 0.7, 0.95) for r in target]).reshape(cases, drafts + 1, vocab)
+    q = np.stack([oracle.probabilities(r, 0.7, 0.95) for r in draft]).reshape(cases, drafts, vocab)
+    seeds, steps = np.arange(cases) + 5, np.arange(cases) + 70
+    ids = np.array([[oracle.sample(q[s, k], int(seeds[s]), int(steps[s]), k, 1) for k in range(drafts)] for s in range(cases)],
+                   np.int32)
+    p[1, drafts] *= 1.001                       # the last target row counts although it may not be reached
+    p[2, 0, 3] = np.nan
+    q[3, 0, 5] = -1e-3
+    ids[4, 0] = vocab
+    q[5, 0, ids[5, 0]] = 0.0                     # not normalised either: that comes first
+    p[6, 1] *= 1.0 + 1.00005e-8 / p[6, 1].sum()  # too close to the limit for the parallel sums
+    q[7, drafts - 1, 0] = np.inf                 # counts only if that position is reached
+    p[8, 0, :] = 0.0                            # rejected or accepted, from a row with one entry
+    p[8, 0, 1] = 1.0
+    res, st = pkg.verify_probabilities(cu(ids.reshape(-1)), cu(q.reshape(-1, vocab)), cu(p.reshape(-1, vocab)), drafts,
+                                       u64(seeds), u64(steps))
+    got, st = pkg.results_to_numpy(res), st.cpu().numpy()
+    for s in range(cases):
+        try:
+            want = oracle.verify(ids[s], q[s], p[s], False, int(seeds[s]), int(steps[s]))
+        except ValueError:
+            assert st[s] < 0 and got["emitted"][s] == -1, s
+            continue
+        assert st[s] == 0 and got["emitted"][s] == want.emitted and got["rejected"][s] == want.rejected, s
+        assert got["accepted_drafts"][s] == want.accepted_drafts
+        assert list(got["tokens"][s][:want.emitted]) == list(want.tokens[:want.emitted]), s
+    assert st[1] == -10 and st[4] < 0 and (st[[2, 3]] < 0).all()
