@@ -10,7 +10,7 @@
 // host's rows in the last place of exp()).  Probability rows (prob_rows.cuh) and the verification take a cluster per row or
 // transaction; the other calls, and what the verification cannot certify from parallel sums, one CTA that follows the chains
 // (replay_core.cuh).  2 drafts + 3 target rows of 129280 to their verification record: 1475 us with one CTA for everything,
-// 882 with the certified verification, 213 with the clusters for the rows.
+// 882 with the certified verification, 164 with the clusters for the rows.
 #include "ds41_b200.h"
 #include "host_error.h"
 #include "launch.h"
@@ -145,7 +145,8 @@ constexpr int kPending = -99, kMaxRowsChecked = 11;
 struct FastVerify {
   double sum[kMaxCluster][kMaxRowsChecked];
   int bad[kMaxCluster][kMaxRowsChecked];
-  double warp[kWarps];
+  double warp_sum[kWarps][kMaxRowsChecked];
+  unsigned warp_bad[kWarps];
   int at, code, checks;   // first position that is not accepted; 0 rejected, else its status; q rows to check
 };
 
@@ -186,37 +187,53 @@ __global__ void __launch_bounds__(kThreads, 2) verify_rows_fast_kernel(VerifyRow
   const int at = f.at, rows = D + 1 + f.checks;
   const int j0 = c.warp * c.region, j1 = min(j0 + c.region, c.len);   // this warp's region of the slice
   FastVerify *f0 = c.cluster.map_shared_rank(&f, 0);
+  // every row's region, 16 bytes a lane where all rows allow it; nothing waits for a row's end
+  const bool wide = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(q)) & 15u) == 0 && n % 2 == 0;
+  auto region = [&](auto &&one) {
+    if (wide) {
+#pragma unroll 8
+      for (int j = j0 + 2 * c.lane; j < j1; j += 64) { one(j, true); }
+    } else {
+#pragma unroll 8
+      for (int j = j0 + c.lane; j < j1; j += 32) { one(j, false); }
+    }
+  };
+  unsigned bad = 0;
   for (int r = 0; r < rows; ++r) {
     const double *row = (r <= D ? p + size_t(r) * n : q + size_t(r - D - 1) * n) + c.begin;
     double sum = 0;
-    int bad = 0;
-#pragma unroll 8
-    for (int j = j0 + c.lane; j < j1; j += 32) {
-      const double v = __ldcg(row + j);
-      bad |= !(v >= 0.0 && v < CUDART_INF);
-      sum += v;
-    }
-    const double w = lanes_sum(sum);
-    if (c.lane == 0) f.warp[c.warp] = w;
-    bad = __syncthreads_or(bad);
-    if (c.tid == 0) {
-      double total = 0;
-      for (int v = 0; v < kWarps; ++v) total += f.warp[v];
-      f0->sum[c.rank][r] = total;
-      f0->bad[c.rank][r] = bad;
-    }
-    __syncthreads();
+    int out = 0;
+    region([&](int j, bool two) {
+      const double2 v = two ? __ldcg(reinterpret_cast<const double2 *>(row + j)) : make_double2(__ldcg(row + j), 0.0);
+      out |= !(v.x >= 0.0 && v.x < CUDART_INF) || !(v.y >= 0.0 && v.y < CUDART_INF);
+      sum += v.x + v.y;
+    });
+    bad |= out ? 1u << r : 0u;
+    sum = lanes_sum(sum);
+    if (c.lane == 0) f.warp_sum[c.warp][r] = sum;
+  }
+  bad = __reduce_or_sync(0xffffffffu, bad);
+  if (c.lane == 0) f.warp_bad[c.warp] = bad;
+  __syncthreads();
+  if (c.tid < rows) {
+    double total = 0;
+    unsigned any = 0;
+    for (int w = 0; w < kWarps; ++w) { total += f.warp_sum[w][c.tid]; any |= f.warp_bad[w]; }
+    f0->sum[c.rank][c.tid] = total;
+    f0->bad[c.rank][c.tid] = (any >> c.tid) & 1u;
   }
   // the row (or residual) that is drawn from: its mass per warp region
   const double *pk = p + size_t(at) * n, *qk = at < D ? q + size_t(at) * n : nullptr;
   const bool draws = f.code == 0;
   if (draws) {
     double mass = 0;
-#pragma unroll 8
-    for (int j = j0 + c.lane; j < j1; j += 32) {
-      const double v = __ldcg(pk + c.begin + j);
-      mass += qk ? fmax(0.0, v - __ldcg(qk + c.begin + j)) : v;
-    }
+    const double *pr = pk + c.begin, *qr = qk ? qk + c.begin : nullptr;
+    region([&](int j, bool two) {
+      const double2 v = two ? __ldcg(reinterpret_cast<const double2 *>(pr + j)) : make_double2(__ldcg(pr + j), 0.0);
+      if (!qr) { mass += v.x + v.y; return; }
+      const double2 w = two ? __ldcg(reinterpret_cast<const double2 *>(qr + j)) : make_double2(__ldcg(qr + j), 0.0);
+      mass += fmax(0.0, v.x - w.x) + fmax(0.0, v.y - w.y);
+    });
     mass = lanes_sum(mass);
     if (c.lane == 0) c.cluster.map_shared_rank(&s->region, 0)->kept[c.rank * kWarps + c.warp] = mass;
   }

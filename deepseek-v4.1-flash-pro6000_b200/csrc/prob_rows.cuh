@@ -16,8 +16,9 @@ namespace {
 
 constexpr int kTileIds = 512;                                 // terms of z per warp: 16 a lane, the row's slice in one round
 constexpr int kRowWarps = kRT / 32;
-constexpr int kOrderChunk = 256, kOrderChunks = 512;          // positions of the order per tile of the mass; most tiles
-constexpr int kLiteral = 32;                                  // first terms of a chain from zero, added one by one
+constexpr int kOrderChunk = 128, kOrderChunks = 1024;         // positions of the order per tile of the mass; most tiles
+constexpr int kLiteralSum = 128, kLiteralMass = 32;           // first terms of a chain from zero, added one by one
+constexpr int kRecords = 30, kRun = kTileIds / 32;            // tiles of z with a record; consecutive terms per lane of it
 constexpr int kMassBits = 44, kCountBits = 18;                // a bucket's lower bound of mass over its count, in one word
 static_assert(kRowWarps * kTileIds == kSliceCap, "one tile per warp");
 static_assert(kOrderChunks * kOrderChunk >= DS41_B200_MAX_VOCAB, "tiles of the order");
@@ -35,19 +36,36 @@ struct ProbArgs {
 struct ProbFact { float best, low; int best_id, bad; };
 struct ProbCut { double mass; unsigned long long key; int id, sorted; };   // sorted = 0: the order has to be sorted as a whole
 
+// A tile of z in which the chain is expected to leave its binade, as its 32 runs of consecutive terms: what the runs up to
+// each lane's add in that binade and what the runs after it add in the next one.  With the accumulator in front of the tile
+// known, the run in which it crosses follows, and only that one's 16 terms have to be added.
+struct Crossing {
+  unsigned long long through[32], after[32];
+  unsigned ties, ties_next;      // runs with a tie at either spacing
+  int binade;
+};
+
 struct ProbSmem {
   double p[kSliceCap];
-  ReplaySmem r;
+  union {
+    ReplaySmem r;                // sorting and the literal chains
+    struct {                     // rank 0, while z is summed
+      Crossing crossing[kRecords];
+    };
+    ProbFact warps[kRowWarps];
+  };
   int count[kBuckets];           // ids of this slice in each bucket; then this slice's next place in the bucket
   int starts[kBuckets + 1];      // ids of the row in each bucket; then its first position
   double part[kOrderChunks];     // parallel sums of the tiles, in every CTA
   unsigned long long units[kOrderChunks];   // rank 0: integer sums of the tiles
-  int binade[kOrderChunks];      // rank 0: at which binade; -1 if a term ties
+  int binade[kOrderChunks];      // rank 0: at which binade; -1 if a term ties; -2 - i: crossing[i]
   ProbFact fact[2][kMaxCluster];
   ProbCut cut;
   double z;
-  int limit, at, found;
+  int limit, at, found, crossings;
 };
+
+static_assert(sizeof(ProbSmem) <= 227 * 1024, "shared memory of one CTA");
 
 // Where the walk stands after the tiles from `c` on that are plain integer sums: the first tile that is not (or `tiles`).
 template <class Stop>
@@ -74,12 +92,22 @@ __device__ int walk_plain(const ProbSmem &s, int c, int tiles, double &acc, Stop
 template <class Value, class Stop>
 __device__ SeqResult warp_sequential(int m, Value value, Stop stop, double acc, int literal) {
   const int lane = threadIdx.x & 31;
-  literal = min(literal, m);
-#pragma unroll 8
-  for (int i = 0; i < literal; ++i) {
-    const double before = acc;
-    acc = __dadd_rn(acc, value(i));
-    if (stop(acc)) return SeqResult{i, acc, before};
+#pragma unroll 1
+  for (int i = 0; i < min(literal, m); i += 8) {   // (literal is a multiple of 8)
+    double v[8], sum[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) v[r] = i + r < m ? value(i + r) : 0.0;
+    sum[0] = __dadd_rn(acc, v[0]);
+#pragma unroll
+    for (int r = 1; r < 8; ++r) sum[r] = __dadd_rn(sum[r - 1], v[r]);
+    if (stop(sum[7])) {   // (monotone)
+      SeqResult out{-1, 0.0, 0.0};
+#pragma unroll
+      for (int r = 7; r >= 0; --r)
+        if (stop(sum[r])) out = SeqResult{i + r, sum[r], r ? sum[r - 1] : acc};
+      return out;
+    }
+    acc = sum[7];
   }
   for (int base = literal; base < m; base += 128) {
     double v[4];
@@ -131,16 +159,50 @@ __device__ SeqResult warp_sequential(int m, Value value, Stop stop, double acc, 
   return SeqResult{-1, acc, acc};
 }
 
+__device__ __forceinline__ int binade_of(double x) {
+  int be;
+  unsigned long long units;
+  split_double(x, be, units);
+  return be;
+}
 // What the tiles' parallel sums say of the accumulator in front of tile c.
-__device__ __forceinline__ int guess_binade(const ProbSmem &s, int c) {
+__device__ __forceinline__ double guess_before(const ProbSmem &s, int c) {
   const int lane = threadIdx.x & 31;
   double before = 0;
   for (int i = lane; i < c; i += 32) before += s.part[i];
-  int be;
-  unsigned long long units;
-  split_double(lanes_sum(before), be, units);
-  return be;
+  return lanes_sum(before);
 }
+
+// Sums rn(x / U), U = 2^(be - 1075), with three additions a term: x + M for M = 1.5 * 2^52 U is rounded to a multiple of U, and
+// what it lost shows a tie.  Terms of 2^51 U and more, and spacings without room below them, count as a tie: such a tile is
+// gone through.
+struct UnitSum {
+  double magic, half, large;
+  unsigned long long units = 0;
+  bool tie;
+  __device__ __forceinline__ explicit UnitSum(int be) {
+    tie = be < 64 || be > 2040;
+    const double u = tie ? 1.0 : __hiloint2double(max(be - 52, 1) << 20, 0);
+    magic = 1.5 * 0x1p52 * u; half = 0.5 * u; large = 0x1p51 * u;
+  }
+  __device__ __forceinline__ void add(double x) {
+    const double t = x + magic, lost = x - (t - magic);
+    units += (unsigned long long)(__double_as_longlong(t) - __double_as_longlong(magic));
+    tie |= fabs(lost) == half || x >= large;
+  }
+};
+
+// a / b rounded, from y = 1 / b rounded: two remainder steps (P. Markstein, IBM J. Res. Dev. 34(1), 1990: with the first result
+// within an ulp the second is the rounded quotient), for quotients and remainders in the normal range.
+__device__ __forceinline__ double divide_by(double a, double b, double y) {
+  double q = a * y;
+  q = fma(fma(-q, b, a), y, q);
+  return fma(fma(-q, b, a), y, q);
+}
+__device__ __forceinline__ double share_of(double a, double b, double y) {   // a in [0, 1], b in about [2^-60, 2^20]
+  return a >= 0x1p-900 ? divide_by(a, b, y) : a / b;
+}
+
 __device__ __forceinline__ unsigned long long lanes_sum_u64(unsigned long long v) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -153,8 +215,10 @@ __device__ __forceinline__ void order_chunk(const BucketOrder &b, int c, int end
   *m = min(end, b.starts[b.bucket_from((c + 1) * kOrderChunk)]) - *st;
 }
 
-// key[0..m) / idx[0..m) of the order into s.r.key / s.r.idx, sorted; m <= kTile.  All threads of the CTA.
-__device__ void sort_chunk(ReplaySmem &s, const unsigned long long *key, const int *idx, int m) {
+// key[0..m) / idx[0..m) of the order, sorted: into s.key / s.idx from the returned position on.  m <= kTile; all threads of
+// the CTA.  Up to kTile / 2 every entry counts the entries before it, four, two or one threads per entry (the usual 130 to 200:
+// 50 steps without a barrier); more take a bitonic sort.
+__device__ int sort_chunk(ReplaySmem &s, const unsigned long long *key, const int *idx, int m) {
   const int tid = threadIdx.x;
   int padded = 2;
   while (padded < m) padded <<= 1;
@@ -163,6 +227,21 @@ __device__ void sort_chunk(ReplaySmem &s, const unsigned long long *key, const i
     s.idx[i] = i < m ? __ldcg(idx + i) : 0x7fffffff;
   }
   __syncthreads();
+  if (m <= kTile / 2) {
+    const int shift = m <= kRT / 4 ? 2 : m <= kRT / 2 ? 1 : 0, i = tid >> shift, per = 1 << shift;
+    const unsigned long long k = i < m ? s.key[i] : 0ull;
+    const int id = i < m ? s.idx[i] : 0;
+    int before = 0;
+    if (i < m) {
+#pragma unroll 4
+      for (int j = tid & (per - 1); j < m; j += per) before += key_less(s.key[j], s.idx[j], k, id) ? 1 : 0;
+    }
+    if (shift >= 1) before += __shfl_xor_sync(0xffffffffu, before, 1);
+    if (shift >= 2) before += __shfl_xor_sync(0xffffffffu, before, 2);
+    if (i < m && (tid & (per - 1)) == 0) { s.key[kTile / 2 + before] = k; s.idx[kTile / 2 + before] = id; }
+    __syncthreads();
+    return kTile / 2;
+  }
   for (int k = 2; k <= padded; k <<= 1)
     for (int jj = k >> 1; jj > 0; jj >>= 1) {
       for (int i = tid; i < padded / 2; i += kRT) {
@@ -174,6 +253,69 @@ __device__ void sort_chunk(ReplaySmem &s, const unsigned long long *key, const i
       }
       __syncthreads();
     }
+  return 0;
+}
+
+// Tile c of z by the warp that holds it: its plain integer sum, or a record of where it may cross.
+__device__ __forceinline__ void sum_tile(const ProbSmem &s, ProbSmem *s0, int c, const double *terms, int have) {
+  const int lane = threadIdx.x & 31;
+  const double before = guess_before(s, c);
+  const int be = binade_of(before);
+  UnitSum sum(be);
+#pragma unroll 4
+  for (int r = 0; r < kRun; ++r)
+    if (lane + 32 * r < have) sum.add(terms[lane + 32 * r]);
+  const unsigned long long units = lanes_sum_u64(sum.units);
+  const int ties = __any_sync(0xffffffffu, sum.tie);
+  int slot = kRecords;
+  if (c > 0 && (ties || binade_of(before + s.part[c]) != be)) {
+    if (lane == 0) slot = atomicAdd(&s0->crossings, 1);
+    slot = __shfl_sync(0xffffffffu, slot, 0);
+    if (slot < kRecords) {
+      unsigned long long now = 0, next = 0;
+      int tie_now = 0, tie_next = 0;
+#pragma unroll 2
+      for (int r = 0; r < kRun; ++r) {
+        if (lane * kRun + r >= have) break;
+        const double x = terms[lane * kRun + r];
+        bool t0, t1;
+        now += to_units(x, be, &t0);
+        next += to_units(x, be + 1, &t1);
+        tie_now |= t0 ? 1 : 0; tie_next |= t1 ? 1 : 0;
+      }
+      const unsigned long long through = lanes_scan(lane, now), upto = lanes_scan(lane, next);
+      Crossing *rec = &s0->crossing[slot];
+      rec->through[lane] = through;
+      rec->after[lane] = __shfl_sync(0xffffffffu, upto, 31) - upto;
+      const unsigned tn = __ballot_sync(0xffffffffu, tie_now), tx = __ballot_sync(0xffffffffu, tie_next);
+      if (lane == 0) { rec->ties = tn; rec->ties_next = tx; rec->binade = be; }
+    }
+  }
+  if (lane == 0) { s0->units[c] = units; s0->binade[c] = slot < kRecords ? -2 - slot : ties ? -1 : be; }
+}
+
+// The accumulator after a tile of z that has a record, on top of acc; *at: the first term it does not include (kTileIds: none).
+__device__ double cross_tile(const Crossing &rec, const double *terms, int have, double acc, int *at) {
+  const int lane = threadIdx.x & 31;
+  int be;
+  unsigned long long s0;
+  split_double(acc, be, s0);
+  *at = 0;
+  if (be != rec.binade) return acc;
+  const unsigned long long through = s0 + rec.through[lane];
+  const unsigned looks = __ballot_sync(0xffffffffu, through >= kTwo53 || ((rec.ties >> lane) & 1u));
+  *at = kTileIds;
+  if (!looks) return join_double(__shfl_sync(0xffffffffu, through, 31), be);
+  const int run = __ffs(looks) - 1, i = run * kRun + lane;
+  const double v = lane < kRun && i < have ? terms[i] : 0.0;
+  if (run > 0) acc = join_double(__shfl_sync(0xffffffffu, through, run - 1), be);
+#pragma unroll
+  for (int r = 0; r < kRun; ++r) acc = __dadd_rn(acc, __shfl_sync(0xffffffffu, v, r));
+  split_double(acc, be, s0);
+  const unsigned long long end = s0 + rec.after[run];
+  if (be == rec.binade + 1 && (rec.ties_next >> run) <= 1u && end < kTwo53) return join_double(end, be);
+  *at = (run + 1) * kRun;
+  return acc;
 }
 
 __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
@@ -211,23 +353,26 @@ __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
       m.low = fminf(m.low, o.low);
       m.bad |= o.bad;
     };
+    auto join_lanes = [&join](ProbFact &m) {
 #pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      ProbFact g;
-      g.best = __shfl_xor_sync(0xffffffffu, f.best, o);
-      g.low = __shfl_xor_sync(0xffffffffu, f.low, o);
-      g.best_id = __shfl_xor_sync(0xffffffffu, f.best_id, o);
-      g.bad = __shfl_xor_sync(0xffffffffu, f.bad, o);
-      join(f, g);
-    }
-    ProbFact *warps = reinterpret_cast<ProbFact *>(s.r.stage);
-    if (lane == 0) warps[warp] = f;
+      for (int o = 16; o; o >>= 1) {
+        ProbFact g;
+        g.best = __shfl_xor_sync(0xffffffffu, m.best, o);
+        g.low = __shfl_xor_sync(0xffffffffu, m.low, o);
+        g.best_id = __shfl_xor_sync(0xffffffffu, m.best_id, o);
+        g.bad = __shfl_xor_sync(0xffffffffu, m.bad, o);
+        join(m, g);
+      }
+    };
+    join_lanes(f);
+    if (lane == 0) s.warps[warp] = f;
     for (int i = tid; i < kBuckets; i += kRT) s.count[i] = 0;
+    if (tid == 0) s.crossings = 0;
     __syncthreads();
-    if (tid < ranks) {
-      f = warps[0];
-      for (int w = 1; w < kRowWarps; ++w) join(f, warps[w]);
-      cluster.map_shared_rank(&s, tid)->fact[parity][rank] = f;
+    if (warp == 0) {
+      f = s.warps[lane];
+      join_lanes(f);
+      if (lane < ranks) cluster.map_shared_rank(&s, lane)->fact[parity][rank] = f;
     }
     cluster.sync();
     f = s.fact[parity][0];
@@ -239,33 +384,19 @@ __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
     }
 
     // exponentials and z
-    const double xb = double(f.best);
+    const double xb = double(f.best), inv_t = 1.0 / a.t;
     double sum = 0;
 #pragma unroll 4
     for (int r = 0; r < kTileIds / 32; ++r) {
       if (first + 32 * r >= len) break;
-      const double e = exp_nonpos((double(v[r]) - xb) / a.t);
+      const double e = exp_nonpos(divide_by(double(v[r]) - xb, a.t, inv_t));
       s.p[first + 32 * r] = e;
       sum += e;
     }
     sum = lanes_sum(sum);
     if (lane < ranks) cluster.map_shared_rank(&s, lane)->part[rank * kRowWarps + warp] = sum;
     cluster.sync();
-    {
-      const int be = guess_binade(s, rank * kRowWarps + warp);
-      unsigned long long units = 0;
-      int ties = 0;
-#pragma unroll 4
-      for (int r = 0; r < kTileIds / 32; ++r) {
-        if (first + 32 * r >= len) break;
-        bool tie;
-        units += to_units(s.p[first + 32 * r], be, &tie);
-        ties |= tie ? 1 : 0;
-      }
-      units = lanes_sum_u64(units);
-      ties = __any_sync(0xffffffffu, ties);
-      if (lane == 0) { s0->units[rank * kRowWarps + warp] = units; s0->binade[rank * kRowWarps + warp] = ties ? -1 : be; }
-    }
+    sum_tile(s, s0, rank * kRowWarps + warp, s.p + warp * kTileIds, len - warp * kTileIds);
     cluster.sync();
     if (rank == 0 && warp == 0) {
       auto never = [](double) { return false; };
@@ -274,16 +405,20 @@ __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
       for (int c = 0; (c = walk_plain(s, c, tiles, acc, never)) < tiles; ++c) {
         const int owner = c / kRowWarps, at = (c % kRowWarps) * kTileIds, have = min(n - owner * stride, stride) - at;
         const double *terms = cluster.map_shared_rank(s.p, owner) + at;
-        acc = warp_sequential(max(0, min(kTileIds, have)), [terms](int i) { return terms[i]; }, never, acc, c == 0 ? kLiteral : 0).acc;
+        int done = 0;
+        if (s.binade[c] <= -2) acc = cross_tile(s.crossing[-2 - s.binade[c]], terms, have, acc, &done);
+        if (done < min(kTileIds, have))
+          acc = warp_sequential(min(kTileIds, have) - done, [terms, done](int i) { return terms[done + i]; }, never, acc,
+                                c == 0 ? kLiteralSum : 0).acc;
       }
       if (lane < ranks) cluster.map_shared_rank(&s, lane)->z = acc;
     }
     cluster.sync();
-    const double z = s.z;
+    const double z = s.z, inv_z = 1.0 / z;
     if (!(top < 1.0)) {
 #pragma unroll 4
       for (int r = 0; r < kTileIds / 32; ++r)
-        if (first + 32 * r < len) out[first + 32 * r] = s.p[first + 32 * r] / z;
+        if (first + 32 * r < len) out[first + 32 * r] = share_of(s.p[first + 32 * r], z, inv_z);
       continue;
     }
 
@@ -291,11 +426,11 @@ __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
     BucketOrder b;
     b.starts = s.starts;
     b.n = n;
-    bucket_grid(b, 1.0 / z, exp_nonpos((double(f.low) - xb) / a.t) / z);
+    const double step = bucket_grid(b, inv_z, exp_nonpos((double(f.low) - xb) / a.t) / z);
 #pragma unroll 4
     for (int r = 0; r < kTileIds / 32; ++r) {
       if (first + 32 * r >= len) break;
-      const double p = s.p[first + 32 * r] / z;
+      const double p = share_of(s.p[first + 32 * r], z, inv_z);
       s.p[first + 32 * r] = p;
       atomicAdd(&s.count[b.bucket_of(order_key(p))], 1);
     }
@@ -324,7 +459,7 @@ __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
 #pragma unroll
       for (int r = 0; r < kPer; ++r) {
         const int i = tid * kPer + r, c = s.starts[i];
-        mine[r] = ((unsigned long long)(double(c) * b.least(i) * double(1ull << kMassBits)) << kCountBits) | unsigned(c);
+        mine[r] = ((unsigned long long)(double(c) * b.least(i, step) * double(1ull << kMassBits)) << kCountBits) | unsigned(c);
         all += mine[r];
       }
       unsigned long long run = block_exclusive_u64(s.r, all, &total);
@@ -362,17 +497,13 @@ __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
       }
       cluster.sync();
       for (int c = rank + ranks * warp; c < chunks; c += ranks * kRowWarps) {
-        int st, m, ties = 0;
+        int st, m;
         order_chunk(b, c, end, &st, &m);
-        const int be = guess_binade(s, c);
-        unsigned long long units = 0;
-        for (int j = lane; j < m; j += 32) {
-          bool tie;
-          units += to_units(key_mass(__ldcg(key + st + j)), be, &tie);
-          ties |= tie ? 1 : 0;
-        }
-        units = lanes_sum_u64(units);
-        ties = __any_sync(0xffffffffu, ties);
+        const int be = binade_of(guess_before(s, c));
+        UnitSum sum(be);
+        for (int j = lane; j < m; j += 32) sum.add(key_mass(__ldcg(key + st + j)));
+        const unsigned long long units = lanes_sum_u64(sum.units);
+        const int ties = __any_sync(0xffffffffu, sum.tie);
         if (lane == 0) { s0->units[c] = units; s0->binade[c] = ties ? -1 : be; }
       }
       cluster.sync();
@@ -393,14 +524,15 @@ __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
         int st, m;
         order_chunk(b, c, end, &st, &m);
         if (m > kTile) { cut.sorted = 0; break; }                          // a long run of (nearly) equal entries
-        sort_chunk(s.r, key + st, idx + st, m);
+        const int at = sort_chunk(s.r, key + st, idx + st, m);
         if (warp == 0) {
-          const SeqResult r = warp_sequential(m, [&s](int i) { return key_mass(s.r.key[i]); }, past, acc, c == 0 ? kLiteral : 0);
+          const SeqResult r = warp_sequential(m, [&s, at](int i) { return key_mass(s.r.key[at + i]); }, past, acc,
+                                                c == 0 ? kLiteralMass : 0);
           acc = r.acc;
           if (lane == 0) s.found = r.found;
         }
         __syncthreads();
-        if (s.found >= 0) { cut.mass = acc; cut.key = s.r.key[s.found]; cut.id = s.r.idx[s.found]; break; }
+        if (s.found >= 0) { cut.mass = acc; cut.key = s.r.key[at + s.found]; cut.id = s.r.idx[at + s.found]; break; }
       }
       if (warp == 0) publish(cut);
     }
@@ -420,13 +552,14 @@ __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
     }
     // the rest is zeroed and every p divided by the kept mass
     const ProbCut cut = s.cut;
+    const double inv_mass = 1.0 / cut.mass;
 #pragma unroll 4
     for (int r = 0; r < kTileIds / 32; ++r) {
       const int j = first + 32 * r;
       if (j >= len) break;
       const double p = s.p[j];
       const unsigned long long k = order_key(p);
-      out[j] = k < cut.key || (k == cut.key && begin + j <= cut.id) ? p / cut.mass : 0.0;
+      out[j] = k < cut.key || (k == cut.key && begin + j <= cut.id) ? share_of(p, cut.mass, inv_mass) : 0.0;
     }
   }
 }

@@ -353,8 +353,8 @@ struct BucketOrder {
     return lo;
   }
   // no p of bucket i is less
-  __device__ __forceinline__ double least(int i) const {
-    const double hi = double(hi_min) + ceil(double(i + 1) / double(scale) * (1.0 + 1e-6)) + 2.0;
+  __device__ __forceinline__ double least(int i, double step) const {   // step: what bucket_grid returned
+    const double hi = double(hi_min) + double(i + 1) * step + 3.0;
     return i == kBuckets - 1 || hi > 4294967295.0 ? 0.0 : __hiloint2double(int(~uint32_t(hi)), 0);
   }
 };
@@ -363,12 +363,14 @@ __device__ __forceinline__ unsigned long long order_key(double p) { return ~(uns
 __device__ __forceinline__ double key_mass(unsigned long long key) { return __longlong_as_double((long long)~key); }
 
 // The bucket grid for probabilities between p_max and p_low (or kSpanCap below p_max; the rest shares the last bucket).
-__device__ __forceinline__ void bucket_grid(BucketOrder &b, double p_max, double p_low) {
+// Returns upper-word steps per bucket, rounded up.
+__device__ __forceinline__ double bucket_grid(BucketOrder &b, double p_max, double p_low) {
   b.hi_min = uint32_t(order_key(p_max) >> 32);
   const uint32_t hi_low = uint32_t(order_key(p_low) >> 32);
   uint32_t span = p_low > 0 ? (hi_low >= b.hi_min ? hi_low - b.hi_min + 1 : 1) : uint32_t(kSpanCap);
   if (span > uint32_t(kSpanCap)) span = kSpanCap;
   b.scale = float(kBuckets - 1) / float(span);
+  return double(span) * ((1.0 + 1e-6) / double(kBuckets - 1));
 }
 // The grid with cleared counters.  Every thread gets the same record.
 __device__ BucketOrder bucket_begin(unsigned char *dynamic, int n, double p_max, double p_low) {
