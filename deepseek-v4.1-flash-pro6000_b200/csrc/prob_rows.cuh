@@ -17,7 +17,6 @@ namespace {
 constexpr int kTileIds = 512;                                 // terms of z per warp: 16 a lane, the row's slice in one round
 constexpr int kRowWarps = kRT / 32;
 constexpr int kOrderChunk = 128, kOrderChunks = 1024;         // positions of the order per tile of the mass; most tiles
-constexpr int kLiteralSum = 128, kLiteralMass = 32;           // first terms of a chain from zero, added one by one
 constexpr int kRecords = 30, kRun = kTileIds / 32;            // tiles of z with a record; consecutive terms per lane of it
 constexpr int kMassBits = 44, kCountBits = 18;                // a bucket's lower bound of mass over its count, in one word
 static_assert(kRowWarps * kTileIds == kSliceCap, "one tile per warp");
@@ -62,7 +61,7 @@ struct ProbSmem {
   ProbFact fact[2][kMaxCluster];
   ProbCut cut;
   double z;
-  int limit, at, found, crossings;
+  int limit, at, at_first, at_count, found, crossings;
 };
 
 static_assert(sizeof(ProbSmem) <= 227 * 1024, "shared memory of one CTA");
@@ -87,74 +86,30 @@ __device__ int walk_plain(const ProbSmem &s, int c, int tiles, double &acc, Stop
   }
 }
 
-// exact_sequential of a short run of non-negative terms by one warp: value(0) .. value(m - 1) on top of acc, the first
-// `literal` of them one by one (a chain that starts from zero leaves a binade with almost every one of its first terms).
+// A short run of a chain as the reference runs it: value(0) .. value(m - 1) on top of acc, one warp.  Every lane loads a term of
+// the next 32 while all add those before (9 cycles a term), which for the few hundred terms of a tile is less than integer sums
+// cost that start again at every tie: terms 2^k below the accumulator tie once in 2^k.
 template <class Value, class Stop>
-__device__ SeqResult warp_sequential(int m, Value value, Stop stop, double acc, int literal) {
+__device__ SeqResult warp_sequential(int m, Value value, Stop stop, double acc) {
   const int lane = threadIdx.x & 31;
+  double next = lane < m ? value(lane) : 0.0, after = lane + 32 < m ? value(lane + 32) : 0.0;
+  __syncwarp();
 #pragma unroll 1
-  for (int i = 0; i < min(literal, m); i += 8) {   // (literal is a multiple of 8)
-    double v[8], sum[8];
+  for (int i = 0; i < m; i += 32) {
+    const double v = next;
+    next = after;
+    after = i + 64 + lane < m ? value(i + 64 + lane) : 0.0;
+    double sum = acc;
 #pragma unroll
-    for (int r = 0; r < 8; ++r) v[r] = i + r < m ? value(i + r) : 0.0;
-    sum[0] = __dadd_rn(acc, v[0]);
-#pragma unroll
-    for (int r = 1; r < 8; ++r) sum[r] = __dadd_rn(sum[r - 1], v[r]);
-    if (stop(sum[7])) {   // (monotone)
-      SeqResult out{-1, 0.0, 0.0};
-#pragma unroll
-      for (int r = 7; r >= 0; --r)
-        if (stop(sum[r])) out = SeqResult{i + r, sum[r], r ? sum[r - 1] : acc};
-      return out;
+    for (int r = 0; r < 32; ++r) sum = __dadd_rn(sum, __shfl_sync(0xffffffffu, v, r));
+    if (__any_sync(0xffffffffu, stop(sum))) {   // (the same in every lane; monotone) the first term it stops at
+      for (int r = 0; r < 32; ++r) {
+        const double before = acc;
+        acc = __dadd_rn(acc, __shfl_sync(0xffffffffu, v, r));
+        if (stop(acc)) return SeqResult{i + r, acc, before};
+      }
     }
-    acc = sum[7];
-  }
-  for (int base = literal; base < m; base += 128) {
-    double v[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) v[r] = base + 4 * lane + r < m ? value(base + 4 * lane + r) : 0.0;
-    int pos = base;
-    for (;;) {   // uniform: one pass per stretch inside one binade
-      int be;
-      unsigned long long s0, t[4], sum = 0;
-      split_double(acc, be, s0);
-      unsigned ties = 0;
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        bool tie = false;
-        t[r] = base + 4 * lane + r >= pos ? to_units(v[r], be, &tie) : 0ull;
-        ties |= tie ? 1u << r : 0u;
-        sum += t[r];
-      }
-      const unsigned long long through = s0 + lanes_scan(lane, sum);
-      const unsigned looks = __ballot_sync(0xffffffffu, ties != 0 || through >= kTwo53 || stop(join_double(through, be)));
-      if (!looks) {
-        acc = join_double(__shfl_sync(0xffffffffu, through, 31), be);
-        break;
-      }
-      const int who = __ffs(looks) - 1;
-      int at = -1;
-      double next = 0.0, before = 0.0;
-      unsigned long long running = through - sum;
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        if (at >= 0 || base + 4 * lane + r < pos) continue;
-        const unsigned long long through_r = running + t[r];
-        if (((ties >> r) & 1u) || through_r >= kTwo53) {   // the reference's own addition
-          at = r; before = join_double(running, be); next = __dadd_rn(before, v[r]);
-        } else if (stop(join_double(through_r, be))) {
-          at = r; before = join_double(running, be); next = join_double(through_r, be);
-        }
-        running = through_r;
-      }
-      at = __shfl_sync(0xffffffffu, at, who);
-      acc = __shfl_sync(0xffffffffu, next, who);
-      before = __shfl_sync(0xffffffffu, before, who);
-      at += base + 4 * who;
-      if (stop(acc)) return SeqResult{at, acc, before};
-      pos = at + 1;
-      if (pos >= base + 128) break;
-    }
+    acc = sum;
   }
   return SeqResult{-1, acc, acc};
 }
@@ -209,10 +164,19 @@ __device__ __forceinline__ unsigned long long lanes_sum_u64(unsigned long long v
   return v;
 }
 
-// Positions of the order's tile c: the buckets that begin within its kOrderChunk positions, up to `end`.
-__device__ __forceinline__ void order_chunk(const BucketOrder &b, int c, int end, int *st, int *m) {
-  *st = min(end, b.starts[b.bucket_from(c * kOrderChunk)]);
-  *m = min(end, b.starts[b.bucket_from((c + 1) * kOrderChunk)]) - *st;
+// Positions of the order's tile c: the buckets that begin within its kOrderChunk positions, up to `end`.  One warp: each lane
+// looks at one of 32 places, three times.
+__device__ __forceinline__ int first_from(const int *starts, int v) {   // the first bucket that begins at v or later
+  const int lane = threadIdx.x & 31;
+  static_assert(kBuckets == 32 * 32 * 4, "three steps");
+  int lo = 128 * __popc(__ballot_sync(0xffffffffu, starts[128 * lane + 127] < v));
+  if (lo == kBuckets) return lo;
+  lo += 4 * __popc(__ballot_sync(0xffffffffu, starts[lo + 4 * lane + 3] < v));
+  return lo + __popc(__ballot_sync(0xffffffffu, lane < 4 && starts[lo + (lane & 3)] < v));
+}
+__device__ __forceinline__ void order_chunk(const int *starts, int c, int end, int *st, int *m) {
+  *st = min(end, starts[first_from(starts, c * kOrderChunk)]);
+  *m = min(end, starts[first_from(starts, (c + 1) * kOrderChunk)]) - *st;
 }
 
 // key[0..m) / idx[0..m) of the order, sorted: into s.key / s.idx from the returned position on.  m <= kTile; all threads of
@@ -272,22 +236,18 @@ __device__ __forceinline__ void sum_tile(const ProbSmem &s, ProbSmem *s0, int c,
     if (lane == 0) slot = atomicAdd(&s0->crossings, 1);
     slot = __shfl_sync(0xffffffffu, slot, 0);
     if (slot < kRecords) {
-      unsigned long long now = 0, next = 0;
-      int tie_now = 0, tie_next = 0;
-#pragma unroll 2
+      UnitSum now(be), next(be + 1);
+#pragma unroll 4
       for (int r = 0; r < kRun; ++r) {
         if (lane * kRun + r >= have) break;
         const double x = terms[lane * kRun + r];
-        bool t0, t1;
-        now += to_units(x, be, &t0);
-        next += to_units(x, be + 1, &t1);
-        tie_now |= t0 ? 1 : 0; tie_next |= t1 ? 1 : 0;
+        now.add(x); next.add(x);
       }
-      const unsigned long long through = lanes_scan(lane, now), upto = lanes_scan(lane, next);
+      const unsigned long long through = lanes_scan(lane, now.units), upto = lanes_scan(lane, next.units);
       Crossing *rec = &s0->crossing[slot];
       rec->through[lane] = through;
       rec->after[lane] = __shfl_sync(0xffffffffu, upto, 31) - upto;
-      const unsigned tn = __ballot_sync(0xffffffffu, tie_now), tx = __ballot_sync(0xffffffffu, tie_next);
+      const unsigned tn = __ballot_sync(0xffffffffu, now.tie), tx = __ballot_sync(0xffffffffu, next.tie);
       if (lane == 0) { rec->ties = tn; rec->ties_next = tx; rec->binade = be; }
     }
   }
@@ -312,8 +272,9 @@ __device__ double cross_tile(const Crossing &rec, const double *terms, int have,
 #pragma unroll
   for (int r = 0; r < kRun; ++r) acc = __dadd_rn(acc, __shfl_sync(0xffffffffu, v, r));
   split_double(acc, be, s0);
-  const unsigned long long end = s0 + rec.after[run];
-  if (be == rec.binade + 1 && (rec.ties_next >> run) <= 1u && end < kTwo53) return join_double(end, be);
+  const bool next = be == rec.binade + 1;
+  const unsigned long long end = s0 + (next ? rec.after[run] : rec.through[31] - rec.through[run]);
+  if ((next || be == rec.binade) && ((next ? rec.ties_next : rec.ties) >> run) <= 1u && end < kTwo53) return join_double(end, be);
   *at = (run + 1) * kRun;
   return acc;
 }
@@ -408,8 +369,7 @@ __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
         int done = 0;
         if (s.binade[c] <= -2) acc = cross_tile(s.crossing[-2 - s.binade[c]], terms, have, acc, &done);
         if (done < min(kTileIds, have))
-          acc = warp_sequential(min(kTileIds, have) - done, [terms, done](int i) { return terms[done + i]; }, never, acc,
-                                c == 0 ? kLiteralSum : 0).acc;
+          acc = warp_sequential(min(kTileIds, have) - done, [terms, done](int i) { return terms[done + i]; }, never, acc).acc;
       }
       if (lane < ranks) cluster.map_shared_rank(&s, lane)->z = acc;
     }
@@ -489,7 +449,7 @@ __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
     if (chunks > 1) {   // (the first tile's terms are gone through in any case)
       for (int c = rank + ranks * warp; c < chunks; c += ranks * kRowWarps) {
         int st, m;
-        order_chunk(b, c, end, &st, &m);
+        order_chunk(s.starts, c, end, &st, &m);
         double part = 0;
         for (int j = lane; j < m; j += 32) part += key_mass(__ldcg(key + st + j));
         part = lanes_sum(part);
@@ -498,7 +458,7 @@ __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
       cluster.sync();
       for (int c = rank + ranks * warp; c < chunks; c += ranks * kRowWarps) {
         int st, m;
-        order_chunk(b, c, end, &st, &m);
+        order_chunk(s.starts, c, end, &st, &m);
         const int be = binade_of(guess_before(s, c));
         UnitSum sum(be);
         for (int j = lane; j < m; j += 32) sum.add(key_mass(__ldcg(key + st + j)));
@@ -516,18 +476,18 @@ __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
       for (int c = 0;; ++c) {
         if (warp == 0) {
           if (c > 0) c = walk_plain(s, c, chunks, acc, past);
-          if (lane == 0) s.at = c;
+          int st = 0, m = 0;
+          if (c < chunks) order_chunk(s.starts, c, end, &st, &m);
+          if (lane == 0) { s.at = c; s.at_first = st; s.at_count = m; }
         }
         __syncthreads();
         c = s.at;
         if (c >= chunks) { cut.mass = acc; cut.sorted = end == n; break; }   // ran through: everything is kept
-        int st, m;
-        order_chunk(b, c, end, &st, &m);
+        const int st = s.at_first, m = s.at_count;
         if (m > kTile) { cut.sorted = 0; break; }                          // a long run of (nearly) equal entries
         const int at = sort_chunk(s.r, key + st, idx + st, m);
         if (warp == 0) {
-          const SeqResult r = warp_sequential(m, [&s, at](int i) { return key_mass(s.r.key[at + i]); }, past, acc,
-                                                c == 0 ? kLiteralMass : 0);
+          const SeqResult r = warp_sequential(m, [&s, at](int i) { return key_mass(s.r.key[at + i]); }, past, acc);
           acc = r.acc;
           if (lane == 0) s.found = r.found;
         }
