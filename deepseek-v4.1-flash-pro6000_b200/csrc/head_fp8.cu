@@ -16,6 +16,11 @@
 // a ring of shared-memory stages, warp 1 issues four K=32 tcgen05.mma per 128-wide K block into one of four TMEM
 // accumulators, sixteen epilogue warps (lane quadrant x 32-column group) pull each finished K block out of TMEM
 // (tcgen05.ld), hand the accumulator back at once, scale and add in fp32 registers.
+// What bounds it (129280 x 4096, us with quantisation and launch): up to 32 rows the weights' 530 MB (88 and 96 against 77 to 81
+// for the copies alone); from 64 rows on the epilogue, whose hand-over of every K block and output of every tile the tensor
+// pipe waits for: 102 at 64, 119 at 128, 198 at 256, 690 at 1024 rows, where the copies alone take 81, 90, 121 and 404.  The
+// issuing warp waits as a whole and elects the lane that issues (108 to 104 at 64 rows against one lane on its own path), the
+// epilogue has the weight scales in shared memory and spends half the instructions on statistics and stores (735 to 690).
 // Every wait is bounded; on expiry the kernel raises *error_flag, frees its TMEM and returns.
 #include "ds41_b200.h"
 #include "flat.cuh"
@@ -34,6 +39,7 @@ namespace {
 
 constexpr int kTmemColumns = 512;  // all of an SM's tensor memory: 4 accumulators of 128 columns or 2 of 256
 constexpr int kTileK = 128;   // K elements per block = one 128-byte swizzle row of e4m3
+constexpr int kEpiWarps = 16, kHeadThreads = 64 + 32 * kEpiWarps;
 constexpr uint32_t kSpinLimit = 1u << 22;
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return uint32_t(__cvta_generic_to_shared(p)); }
@@ -115,6 +121,12 @@ __device__ __forceinline__ void umma_f8(uint32_t tmem_d, uint64_t a_desc, uint64
       "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(kAccumulate ? 1 : 0)
       : "memory");
 }
+// true in one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(one));
+  return one != 0;
+}
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
@@ -164,9 +176,9 @@ struct HeadSmem {
   // stage (or to the pad after the last one) and only feed TMEM lanes nobody reads
   static constexpr int kPadBytes = (128 - kRows) * kTileK;
   static constexpr int kMaxStages = 12;
-  // bytes beside the stages: alignment slack, pad, scale table [K/128][kRows], barriers and flags
+  // bytes beside the stages: alignment slack, pad, scale tables [K/128][kRows] and [warps][K/128], barriers and flags
   static constexpr size_t fixed_bytes(int kblocks) {
-    return 1024 + kPadBytes + size_t(kblocks) * kRows * 4 + (2 * kMaxStages + 2 * kAccBufs) * 8 + 16;
+    return 1024 + kPadBytes + size_t(kblocks) * (kRows + kEpiWarps) * 4 + (2 * kMaxStages + 2 * kAccBufs) * 8 + 16;
   }
   // a stage holds `group` consecutive K blocks (one TMA box per operand)
   static constexpr int stages(int kblocks, int group) {
@@ -177,7 +189,6 @@ struct HeadSmem {
 };
 
 constexpr int kMaxOwners = 8;
-constexpr int kEpiWarps = 16, kHeadThreads = 64 + 32 * kEpiWarps;
 struct HeadArgs {
   const float *a_scale;  // [M, K/128]
   const float *w_scale;  // [ceil(N/128), K/128]
@@ -219,7 +230,8 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~uintptr_t(1023));
   float *sa = reinterpret_cast<float *>(tiles + size_t(kStages) * stage_bytes + Smem::kPadBytes);  // [K/128][kRows]
   const int kblocks = p.K / kTileK;
-  uint64_t *bars = reinterpret_cast<uint64_t *>(sa + size_t(kblocks) * kRows);
+  float *sw = sa + size_t(kblocks) * kRows;                                                              // [epilogue warp][K/128]
+  uint64_t *bars = reinterpret_cast<uint64_t *>(sw + size_t(kblocks) * kEpiWarps);
   uint64_t *full = bars, *empty = bars + kMaxStages, *acc_full = bars + 2 * kMaxStages, *acc_empty = acc_full + kAccBufs;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + kAccBufs);
   int *abort_word = reinterpret_cast<int *>(tmem_slot + 1);
@@ -279,33 +291,36 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer (one lane)
+    // ------------------------------------------------------------------ MMA issuer: the warp waits together, one lane issues
     cudaGridDependencySynchronize();
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(kTileN);
-      const uint32_t tiles16 = smem_addr(tiles) >> 4, stage16 = uint32_t(stage_bytes) >> 4;
-      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
-      for (int tile = blockIdx.x; tile < total_tiles && !ab.set(); tile += gridDim.x) {
-        bool ok = true;
-        for (int kb = 0; kb < kblocks && ok; kb += group) {
-          if (!mbar_wait(&full[stage], phase, ab)) break;
-          uint32_t w16 = tiles16 + stage * stage16, a16 = w16 + (w_bytes >> 4);  // addresses >> 4
-          for (int g = 0; g < group; ++g) {
-            if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, ab)) { ok = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t d_addr = tmem_base + acc * kTileN;
+    constexpr uint32_t idesc = umma_idesc(kTileN);
+    const uint32_t tiles16 = smem_addr(tiles) >> 4, stage16 = uint32_t(stage_bytes) >> 4;
+    const bool leader = elect_one();
+    uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+    for (int tile = blockIdx.x; tile < total_tiles && !__any_sync(0xffffffffu, ab.set()); tile += gridDim.x) {
+      bool ok = true;
+      for (int kb = 0; kb < kblocks && ok; kb += group) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], phase, ab))) break;
+        uint32_t w16 = tiles16 + stage * stage16, a16 = w16 + (w_bytes >> 4);  // addresses >> 4
+        for (int g = 0; g < group; ++g) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[acc], acc_phase ^ 1, ab));
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t d_addr = tmem_base + acc * kTileN;
+          if (leader) {
             // D[batch row, vocabulary id] (+)= A[batch row, k] * W[vocabulary id, k], K = 32 bytes per instruction
             umma_f8<false>(d_addr, umma_desc16(a16), umma_desc16(w16), idesc);
             umma_f8<true>(d_addr, umma_desc16(a16 + 2), umma_desc16(w16 + 2), idesc);
             umma_f8<true>(d_addr, umma_desc16(a16 + 4), umma_desc16(w16 + 4), idesc);
             umma_f8<true>(d_addr, umma_desc16(a16 + 6), umma_desc16(w16 + 6), idesc);
             umma_commit(&acc_full[acc]);   // accumulator of this K block is complete
-            if (++acc == kAccBufs) { acc = 0; acc_phase ^= 1; }
-            w16 += (kTileN * kTileK) >> 4; a16 += (kRows * kTileK) >> 4;
+            if (g + 1 == group) umma_commit(&empty[stage]);  // the stage may be refilled once these MMAs have read it
           }
-          if (ok) umma_commit(&empty[stage]);  // the stage may be refilled once these MMAs have read it
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
+          __syncwarp();
+          if (++acc == kAccBufs) { acc = 0; acc_phase ^= 1; }
+          w16 += (kTileN * kTileK) >> 4; a16 += (kRows * kTileK) >> 4;
         }
+        if (++stage == kStages) { stage = 0; phase ^= 1; }
       }
     }
   } else if ((warp & 3) < kQuads) {
@@ -316,18 +331,32 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const int row = quad * 32 + lane;   // batch row inside the tile
     const int et = (group * kQuads + quad) * 32 + lane;  // 0..kEpiActive-1
     const uint32_t lane_base = tmem_base + group * kMyCols + (uint32_t(quad * 32) << 16);
+    float *my_sw = sw + size_t(warp - 2) * kblocks;
     uint32_t acc = 0, acc_phase = 0;
     int table_bt = -1;
     bool alive = true;  // warp-uniform; once false the remaining tiles are walked without waiting or computing,
                         // so that all epilogue threads still meet at every named barrier
-    // running statistics of this thread's batch row over the tiles of one batch tile (vocabulary tiles come in
-    // ascending order, so a strict comparison keeps the first maximum)
-    float st_best = -CUDART_INF_F, st_low = CUDART_INF_F, st_bad = 0.f;
-    int st_id = 0x7fffffff;
+    // running statistics of this thread's batch row over the tiles of one batch tile (vocabulary tiles come in ascending
+    // order, so a strict comparison keeps the first tile with the maximum; which of its columns it was is looked up in the
+    // logits when the row is left)
+    float st_best = -CUDART_INF_F, st_low = CUDART_INF_F, st_bad = 0.f, st_bad1 = 0.f;
+    int st_at = -1;
     const bool stats_on = p.row_stats != nullptr || p.owner_stats_offset != 0;
+    auto row_of = [&](int m) {   // batch row m of the output
+      if (p.rows_per_owner == 0) return p.logits + size_t(m) * p.ldl;
+      const int owner = m / p.rows_per_owner;
+      return p.owner_base[owner] + size_t(m - owner * p.rows_per_owner) * p.ldl + p.col_offset;
+    };
     auto flush_stats = [&](int bt_of) {
       const int m = bt_of * kRows + row;
-      if (stats_on && st_id != 0x7fffffff && row < kRows && m < p.M) {
+      __syncwarp();   // (the row's logits were written by other lanes)
+      if (stats_on && st_at >= 0 && row < kRows && m < p.M) {
+        const float *x = row_of(m);
+        int st_id = st_at;
+        const int end = min(p.N, st_at + kMyCols);
+#pragma unroll 16
+        for (int n = end - 1; n >= st_at; --n)
+          if (x[n] == st_best) st_id = n;
         auto ordered = [](float v) {
           const uint32_t bits = __float_as_uint(v == 0.f ? 0.f : v);  // -0 and +0 are the same logit
           return bits ^ ((bits >> 31) ? 0xffffffffu : 0x80000000u);
@@ -340,15 +369,15 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                                                               p.owner_stats_offset) + (m - owner * p.rows_per_owner);
           atomicMax_system(&rs->max_key, key);
           atomicMax_system(&rs->min_key, ~ordered(st_low));
-          if (st_bad != st_bad) atomicOr_system(&rs->flags, 1u);
+          if (st_bad + st_bad1 != 0.f) atomicOr_system(&rs->flags, 1u);
         } else {
           HeadRowStats *rs = p.row_stats + m;
           atomicMax(&rs->max_key, key);
           atomicMax(&rs->min_key, ~ordered(st_low));
-          if (st_bad != st_bad) atomicOr(&rs->flags, 1u);
+          if (st_bad + st_bad1 != 0.f) atomicOr(&rs->flags, 1u);
         }
       }
-      st_best = -CUDART_INF_F; st_low = CUDART_INF_F; st_bad = 0.f; st_id = 0x7fffffff;
+      st_best = -CUDART_INF_F; st_low = CUDART_INF_F; st_bad = st_bad1 = 0.f; st_at = -1;
     };
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
       const int nt = tile / b_tiles, bt = tile % b_tiles;
@@ -366,17 +395,18 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       // fp32 scale of the 128-row weight block this warp's columns belong to (a 256-wide tile spans two blocks)
       const int w_block = min((nt * kTileN + group * kMyCols) / 128, (p.N + 127) / 128 - 1);
       const float *wsc = p.w_scale + size_t(w_block) * kblocks;
+      // copied once per tile: a global load in the loop below, even one that hits, delays the hand-over of each accumulator
+      for (int i = lane; i < kblocks; i += 32) my_sw[i] = __ldg(wsc + i);
+      __syncwarp();
       float sum[kMyCols];
 #pragma unroll
       for (int c = 0; c < kMyCols; ++c) sum[c] = 0.f;
-      float w_next = __ldg(wsc);
       for (int kb = 0; kb < kblocks && alive; ++kb) {
         alive = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], acc_phase, ab));
         if (!alive) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const float scale = sa[kb * kRows + (row < kRows ? row : 0)] * w_next;
+        const float scale = sa[kb * kRows + (row < kRows ? row : 0)] * my_sw[kb];
         const unsigned long long scale2 = pack2(scale, scale);
-        if (kb + 1 < kblocks) w_next = __ldg(wsc + kb + 1);
         if constexpr (kMyCols == 32) {
           uint32_t r[32];
           tmem_ld32(lane_base + acc * kTileN, r);
@@ -405,79 +435,91 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         }
         if (++acc == kAccBufs) { acc = 0; acc_phase ^= 1; }
       }
-      // Output.  Lane l holds row l of the warp's 32 x 32 block.  Written as it is, one store instruction would touch
-      // 32 rows with 16 bytes each; an 8 x 8 transpose of the 16-byte column groups across the lanes that share
-      // l % 4 (butterflies at lane distances 4, 8, 16) turns that into 4 rows with 128 contiguous bytes each, which is
-      // what a peer GPU's memory wants to be written with (and the local L2 as well).
+      // Output, while the tensor cores wait: as few instructions as it takes.
+      const int n0 = nt * kTileN + group * kMyCols;
+      const bool whole = n0 + kMyCols <= p.N;
       if (alive && stats_on) {
-        const int n0 = nt * kTileN + group * kMyCols;
-        if (n0 + kMyCols <= p.N) {
+        if (whole) {
+          float hi = sum[0], low = sum[0];
+          const unsigned long long zero2 = pack2(0.f, 0.f);
 #pragma unroll
-          for (int c = 0; c < kMyCols; ++c) {
-            const float v = sum[c];
-            st_bad = fmaf(v, 0.f, st_bad);  // NaN once any logit is NaN or infinite
-            if (v > st_best) { st_best = v; st_id = n0 + c; }
-            st_low = fminf(st_low, v);
-          }
+          for (int c = 1; c < kMyCols; ++c) { hi = fmaxf(hi, sum[c]); low = fminf(low, sum[c]); }
+#pragma unroll
+          for (int c = 0; c < kMyCols; c += 2)   // NaN once any logit is NaN or infinite
+            fma2_acc(st_bad, st_bad1, __float_as_uint(sum[c]), __float_as_uint(sum[c + 1]), zero2);
+          if (hi > st_best) { st_best = hi; st_at = n0; }
+          st_low = fminf(st_low, low);
         } else {
 #pragma unroll
           for (int c = 0; c < kMyCols; ++c) {
             const float v = sum[c];
             if (n0 + c < p.N) {
               st_bad = fmaf(v, 0.f, st_bad);
-              if (v > st_best) { st_best = v; st_id = n0 + c; }
+              if (v > st_best) { st_best = v; st_at = n0; }
               st_low = fminf(st_low, v);
             }
           }
         }
       }
+      // Lane l holds row l of the warp's 32 x 32 block.  Written as it is, one store instruction would touch 32 rows with 16
+      // bytes each; butterflies of the 16-byte column groups at lane distances 8 and 16 turn that into 8 rows with 64
+      // contiguous bytes, which the local L2 takes at its full rate, and one more at distance 4 into 4 rows with 128 bytes,
+      // which is what a peer GPU's memory wants to be written with.
       if (alive) {
+        const bool scattered = p.rows_per_owner != 0;
+        const bool plain = !scattered && whole && p.ldl % 4 == 0 && (reinterpret_cast<uintptr_t>(p.logits) & 15u) == 0;
 #pragma unroll
-       for (int half = 0; half < kMyCols / 32; ++half) {
-        float4 x[8];
+        for (int half = 0; half < kMyCols / 32; ++half) {
+          float4 x[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
-          x[c] = make_float4(sum[32 * half + 4 * c], sum[32 * half + 4 * c + 1], sum[32 * half + 4 * c + 2], sum[32 * half + 4 * c + 3]);
+          for (int c = 0; c < 8; ++c)
+            x[c] = make_float4(sum[32 * half + 4 * c], sum[32 * half + 4 * c + 1], sum[32 * half + 4 * c + 2], sum[32 * half + 4 * c + 3]);
+          auto exchange = [&](int bit, int dist) {   // column group bit of the index <-> the lane bit of that distance
+            const bool upper = (lane & dist) != 0;
 #pragma unroll
-        for (int s3 = 0; s3 < 3; ++s3) {
-          const int dist = 4 << s3;
-          const bool upper = (lane >> (2 + s3)) & 1;
+            for (int c = 0; c < 8; ++c) {
+              if ((c >> bit) & 1) continue;
+              const int c2 = c | (1 << bit);
+              const float4 give = upper ? x[c] : x[c2];
+              float4 take;
+              take.x = __shfl_xor_sync(0xffffffffu, give.x, dist);
+              take.y = __shfl_xor_sync(0xffffffffu, give.y, dist);
+              take.z = __shfl_xor_sync(0xffffffffu, give.z, dist);
+              take.w = __shfl_xor_sync(0xffffffffu, give.w, dist);
+              if (upper) x[c] = take; else x[c2] = take;
+            }
+          };
+          exchange(0, 8);
+          exchange(1, 16);
+          exchange(2, 4);
+          // x[c] = columns [4 * (lane / 8) + 16 * (lane / 4 % 2), +4) of block row 8 * (c % 4) + 4 * (c / 4) + lane % 4
+          if (plain) {
+            const int r = quad * 32 + (lane & 3), rows = min(kRows, p.M - bt * kRows) - r;
+            float *dst = p.logits + size_t(bt * kRows + r) * p.ldl + n0 + 32 * half + 4 * (lane >> 3) + 16 * ((lane >> 2) & 1);
+            const long long step = 4 * p.ldl;
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            if ((c >> s3) & 1) continue;
-            const int c2 = c | (1 << s3);
-            const float4 give = upper ? x[c] : x[c2];
-            float4 take;
-            take.x = __shfl_xor_sync(0xffffffffu, give.x, dist);
-            take.y = __shfl_xor_sync(0xffffffffu, give.y, dist);
-            take.z = __shfl_xor_sync(0xffffffffu, give.z, dist);
-            take.w = __shfl_xor_sync(0xffffffffu, give.w, dist);
-            if (upper) x[c] = take; else x[c2] = take;
+            for (int c = 0; c < 8; ++c) {
+              if (4 * c < rows) *reinterpret_cast<float4 *>(dst) = x[(c >> 1) | ((c & 1) << 2)];
+              dst += step;
+            }
+          } else {
+            const int n = n0 + 32 * half + 4 * (lane >> 3) + 16 * ((lane >> 2) & 1);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+              const int r = quad * 32 + 8 * (c & 3) + 4 * (c >> 2) + (lane & 3), m = bt * kRows + r;
+              if (r >= kRows || m >= p.M || n >= p.N) continue;
+              float *dst = row_of(m) + n;
+              if (n + 4 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
+                *reinterpret_cast<float4 *>(dst) = x[c];
+              } else {
+                const float v[4] = {x[c].x, x[c].y, x[c].z, x[c].w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                  if (n + k < p.N) dst[k] = v[k];
+              }
+            }
           }
         }
-        // now x[a] = columns [4*(lane/4), +4) of block row 4*a + lane%4
-        const int n = nt * kTileN + group * kMyCols + 32 * half + 4 * (lane >> 2);
-#pragma unroll
-        for (int a8 = 0; a8 < 8; ++a8) {
-          const int r = quad * 32 + 4 * a8 + (lane & 3), m = bt * kRows + r;
-          if (r >= kRows || m >= p.M || n >= p.N) continue;
-          float *dst;
-          if (p.rows_per_owner == 0) {
-            dst = p.logits + size_t(m) * p.ldl + n;
-          } else {
-            const int owner = m / p.rows_per_owner;
-            dst = p.owner_base[owner] + size_t(m - owner * p.rows_per_owner) * p.ldl + p.col_offset + n;
-          }
-          if (n + 4 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
-            *reinterpret_cast<float4 *>(dst) = x[a8];
-          } else {
-            const float v[4] = {x[a8].x, x[a8].y, x[a8].z, x[a8].w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              if (n + k < p.N) dst[k] = v[k];
-          }
-        }
-       }
       }
     }
     if (alive && table_bt >= 0) flush_stats(table_bt);
