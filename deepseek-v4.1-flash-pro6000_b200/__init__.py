@@ -60,6 +60,13 @@ class ScoreArgs(C.Structure):
                 ("top_n", _i32), ("logsumexp", _P), ("top1", _P), ("top_ids", _P), ("top_logprob", _P), ("status", _P)]
 
 
+class ProbArgs(C.Structure):
+    _fields_ = [("struct_bytes", C.c_uint32), ("rows", C.c_int32), ("vocab", C.c_int32), ("logits", C.c_void_p),
+                ("logits_stride", C.c_int64), ("temperature", C.c_double), ("top_p", C.c_double),
+                ("probabilities", C.c_void_p), ("status", C.c_void_p), ("scratch", C.c_void_p),
+                ("scratch_bytes", C.c_size_t)]
+
+
 _lib = None
 
 
@@ -98,6 +105,12 @@ def lib():
         L.ds41_dense_head_compact.argtypes = [_P, _P, _P, C.c_int, C.c_int, C.c_int, _P]
         L.ds41_b200_markov_logits.argtypes = [_P, _P, _P, _P, C.c_int, _P]
         L.ds41_b200_final_norm.argtypes = [_P, _P, _P, _P, C.c_int, C.c_int, _f32, _P]
+        L.ds41_b200_head_f32.argtypes = [_P, _P, _P, C.c_int, C.c_int, C.c_int, _P]
+        L.ds41_b200_probabilities_scratch_bytes.restype = C.c_size_t
+        L.ds41_b200_probabilities_scratch_bytes.argtypes = [C.c_int]
+        L.ds41_b200_sample_probabilities.argtypes = [_P, C.c_int, C.c_int, _i64, _P, _P, C.c_uint32, C.c_uint32, _P, _P, _P]
+        L.ds41_b200_verify_probabilities.argtypes = [_P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, _P, _P, _P, _P, _P]
+        L.ds41_b200_probabilities.argtypes = [C.POINTER(ProbArgs), _P]
         _lib = L
     return _lib
 
@@ -113,6 +126,21 @@ def _check(rc, what):
 
 def _stream():
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+_current_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+
+
+def _launch(device, what, fn, *args):
+    """fn(*args, the device's current stream) with `device` current.  The stream is asked for as a bare handle and the device is
+    switched only when it has to be: the guard and the stream object cost 5 of the 17 to 23 us that a small call takes here."""
+    index = device.index
+    if _current_device() != index:
+        with torch.cuda.device(index):
+            return _launch(device, what, fn, *args)
+    rc = fn(*args, _raw_stream(index))
+    if rc:
+        _check(rc, what)
 
 
 def _dev(t, dtype, name):
@@ -203,8 +231,7 @@ def sample_logits(logits, temperature, top_p, seeds, steps, slot=0, purpose=Purp
     a.scratch = scratch.data_ptr() if scratch is not None else None
     a.scratch_bytes = scratch.numel() if scratch is not None else 0
     a.row_extremes = row_extremes.data_ptr() if row_extremes is not None else None
-    with torch.cuda.device(logits.device):
-        _check(lib().ds41_b200_sample_logits(C.byref(a), _stream()), "ds41_b200_sample_logits")
+    _launch(logits.device, "ds41_b200_sample_logits", lib().ds41_b200_sample_logits, C.byref(a))
     return tokens, status
 
 
@@ -229,9 +256,8 @@ def verify_logits(target_logits, draft_logits, draft_ids, drafts, temperature, t
         raise ValueError("speculative row count")
     sequences = rows // (drafts + 1)
     device = target_logits.device
-    need = verify_scratch_bytes(sequences, drafts, vocab)
     if scratch is None:
-        scratch = torch.empty(need, dtype=torch.uint8, device=device)
+        scratch = torch.empty(verify_scratch_bytes(sequences, drafts, vocab), dtype=torch.uint8, device=device)
     if results is None:
         results = torch.empty(sequences * C.sizeof(SparkResult), dtype=torch.uint8, device=device)
     if status is None:
@@ -246,8 +272,7 @@ def verify_logits(target_logits, draft_logits, draft_ids, drafts, temperature, t
     a.seeds, a.steps = seeds.data_ptr(), steps.data_ptr()
     a.results, a.status = results.data_ptr(), status.data_ptr()
     a.scratch, a.scratch_bytes = scratch.data_ptr(), scratch.numel()
-    with torch.cuda.device(device):
-        _check(lib().ds41_b200_verify_logits(C.byref(a), _stream()), "ds41_b200_verify_logits")
+    _launch(device, "ds41_b200_verify_logits", lib().ds41_b200_verify_logits, C.byref(a))
     return results, status
 
 
@@ -264,9 +289,8 @@ def quantize_activations(x_bf16, a=None, a_scale=None):
         a = torch.empty((M, K), dtype=torch.uint8, device=x_bf16.device)
     if a_scale is None:
         a_scale = torch.empty((M, K // 128), dtype=torch.float32, device=x_bf16.device)
-    with torch.cuda.device(x_bf16.device):
-        _check(lib().ds41_b200_quantize_activations(x_bf16.data_ptr(), a.data_ptr(), a_scale.data_ptr(), M, K, _stream()),
-               "ds41_b200_quantize_activations")
+    _launch(x_bf16.device, "ds41_b200_quantize_activations", lib().ds41_b200_quantize_activations, x_bf16.data_ptr(),
+            a.data_ptr(), a_scale.data_ptr(), M, K)
     return a, a_scale
 
 
@@ -281,19 +305,15 @@ def head_fp8(a, a_scale, w, w_scale, logits=None, error_flag=None, row_extremes=
     if logits is None:
         logits = torch.empty((M, N), dtype=torch.float32, device=a.device)
     flag = error_flag.data_ptr() if error_flag is not None else None
-    with torch.cuda.device(a.device):
-        if row_extremes is None:
-            _check(lib().ds41_b200_head_fp8(a.data_ptr(), a_scale.data_ptr(), w.data_ptr(), w_scale.data_ptr(),
-                                            logits.data_ptr(), logits.stride(0), M, N, K, flag, _stream()),
-                   "ds41_b200_head_fp8")
-        else:
-            row_extremes = _dev(row_extremes, torch.uint8, "row_extremes")
-            if row_extremes.numel() < 16 * M:
-                raise ValueError("row_extremes must hold 16 bytes per row")
-            _check(lib().ds41_b200_head_fp8_stats(a.data_ptr(), a_scale.data_ptr(), w.data_ptr(), w_scale.data_ptr(),
-                                                  logits.data_ptr(), logits.stride(0), M, N, K,
-                                                  row_extremes.data_ptr(), flag, _stream()),
-                   "ds41_b200_head_fp8_stats")
+    if row_extremes is None:
+        _launch(a.device, "ds41_b200_head_fp8", lib().ds41_b200_head_fp8, a.data_ptr(), a_scale.data_ptr(), w.data_ptr(),
+                w_scale.data_ptr(), logits.data_ptr(), logits.stride(0), M, N, K, flag)
+    else:
+        row_extremes = _dev(row_extremes, torch.uint8, "row_extremes")
+        if row_extremes.numel() < 16 * M:
+            raise ValueError("row_extremes must hold 16 bytes per row")
+        _launch(a.device, "ds41_b200_head_fp8_stats", lib().ds41_b200_head_fp8_stats, a.data_ptr(), a_scale.data_ptr(),
+                w.data_ptr(), w_scale.data_ptr(), logits.data_ptr(), logits.stride(0), M, N, K, row_extremes.data_ptr(), flag)
     return logits
 
 
@@ -308,8 +328,7 @@ def head_bf16(x, w_bf16, out=None, decode_symbol=False):
     if out is None:
         out = torch.empty((M, N), dtype=torch.float32, device=x.device)
     fn = lib().ds41_fuse_head_decode if decode_symbol else lib().ds41_b200_head_bf16
-    with torch.cuda.device(x.device):
-        _check(fn(x.data_ptr(), w_bf16.data_ptr(), out.data_ptr(), M, N, K, _stream()), "BF16 head")
+    _launch(x.device, "BF16 head", fn, x.data_ptr(), w_bf16.data_ptr(), out.data_ptr(), M, N, K)
     return out
 
 
@@ -321,10 +340,8 @@ def head_f32(x, w_f32, out=None):
     N = w_f32.shape[0]
     if out is None:
         out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    L = lib()
-    L.ds41_b200_head_f32.argtypes = [_P, _P, _P, C.c_int, C.c_int, C.c_int, _P]
-    with torch.cuda.device(x.device):
-        _check(L.ds41_b200_head_f32(x.data_ptr(), w_f32.data_ptr(), out.data_ptr(), M, N, K, _stream()), "ds41_b200_head_f32")
+    _launch(x.device, "ds41_b200_head_f32", lib().ds41_b200_head_f32, x.data_ptr(), w_f32.data_ptr(), out.data_ptr(), M,
+            N, K)
     return out
 
 
@@ -337,9 +354,8 @@ def head_compact(x, w_bf16, out=None):
     N = w_bf16.shape[0]
     if out is None:
         out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
-        _check(lib().ds41_dense_head_compact(x.data_ptr(), w_bf16.data_ptr(), out.data_ptr(), M, N, K, _stream()),
-               "ds41_dense_head_compact")
+    _launch(x.device, "ds41_dense_head_compact", lib().ds41_dense_head_compact, x.data_ptr(), w_bf16.data_ptr(),
+            out.data_ptr(), M, N, K)
     return out
 
 
@@ -353,9 +369,8 @@ def markov_logits(draft_row, markov_weight, embedding, out=None):
         raise ValueError("markov_weight must be [V,256] and embedding [256]")
     if out is None:
         out = torch.empty_like(draft_row)
-    with torch.cuda.device(draft_row.device):
-        _check(lib().ds41_b200_markov_logits(draft_row.data_ptr(), markov_weight.data_ptr(), embedding.data_ptr(),
-                                             out.data_ptr(), draft_row.numel(), _stream()), "ds41_b200_markov_logits")
+    _launch(draft_row.device, "ds41_b200_markov_logits", lib().ds41_b200_markov_logits, draft_row.data_ptr(),
+            markov_weight.data_ptr(), embedding.data_ptr(), out.data_ptr(), draft_row.numel())
     return out
 
 
@@ -370,9 +385,8 @@ def final_norm(h, pre, norm_weight, eps=1e-20, out=None):
         raise ValueError("h must be [M,4,K], pre [M,4], norm_weight [K]")
     if out is None:
         out = torch.empty((M, K), dtype=torch.float32, device=h.device)
-    with torch.cuda.device(h.device):
-        _check(lib().ds41_b200_final_norm(h.data_ptr(), pre.data_ptr(), norm_weight.data_ptr(), out.data_ptr(), M, K,
-                                          eps, _stream()), "ds41_b200_final_norm")
+    _launch(h.device, "ds41_b200_final_norm", lib().ds41_b200_final_norm, h.data_ptr(), pre.data_ptr(),
+            norm_weight.data_ptr(), out.data_ptr(), M, K, eps)
     return out
 
 
@@ -391,16 +405,8 @@ def score_logits(logits, top_n=0):
     status = torch.empty(rows, dtype=torch.int32, device=dev)
     a = ScoreArgs(C.sizeof(ScoreArgs), rows, vocab, logits.data_ptr(), logits.stride(0), top_n, lse.data_ptr(),
                   top1.data_ptr(), ids.data_ptr() if top_n else None, lp.data_ptr() if top_n else None, status.data_ptr())
-    with torch.cuda.device(dev):
-        _check(lib().ds41_b200_score_logits(C.byref(a), _stream()), "ds41_b200_score_logits")
+    _launch(dev, "ds41_b200_score_logits", lib().ds41_b200_score_logits, C.byref(a))
     return lse, top1, ids, lp, status
-
-
-class ProbArgs(C.Structure):
-    _fields_ = [("struct_bytes", C.c_uint32), ("rows", C.c_int32), ("vocab", C.c_int32), ("logits", C.c_void_p),
-                ("logits_stride", C.c_int64), ("temperature", C.c_double), ("top_p", C.c_double),
-                ("probabilities", C.c_void_p), ("status", C.c_void_p), ("scratch", C.c_void_p),
-                ("scratch_bytes", C.c_size_t)]
 
 
 def probabilities(logits, temperature, top_p):
@@ -410,17 +416,13 @@ def probabilities(logits, temperature, top_p):
     logits = _dev(logits, torch.float32, "logits")
     rows, vocab = logits.shape
     L = lib()
-    L.ds41_b200_probabilities_scratch_bytes.restype = C.c_size_t
-    L.ds41_b200_probabilities_scratch_bytes.argtypes = [C.c_int]
-    L.ds41_b200_probabilities.argtypes = [C.POINTER(ProbArgs), _P]
     need = L.ds41_b200_probabilities_scratch_bytes(rows)
     out = torch.empty((rows, vocab), dtype=torch.float64, device=logits.device)
     status = torch.empty(rows, dtype=torch.int32, device=logits.device)
     scratch = torch.empty(need, dtype=torch.uint8, device=logits.device)
     a = ProbArgs(C.sizeof(ProbArgs), rows, vocab, logits.data_ptr(), logits.stride(0), float(temperature), float(top_p),
                  out.data_ptr(), status.data_ptr(), scratch.data_ptr(), need)
-    with torch.cuda.device(logits.device):
-        _check(L.ds41_b200_probabilities(C.byref(a), _stream()), "ds41_b200_probabilities")
+    _launch(logits.device, "ds41_b200_probabilities", L.ds41_b200_probabilities, C.byref(a))
     return out, status
 
 
@@ -433,11 +435,9 @@ def sample_probabilities(p, seeds, steps, slot=0, purpose=Purpose.Target):
     tokens = torch.empty(rows, dtype=torch.int32, device=p.device)
     status = torch.empty(rows, dtype=torch.int32, device=p.device)
     L = lib()
-    L.ds41_b200_sample_probabilities.argtypes = [_P, C.c_int, C.c_int, _i64, _P, _P, C.c_uint32, C.c_uint32, _P, _P, _P]
-    with torch.cuda.device(p.device):
-        _check(L.ds41_b200_sample_probabilities(p.data_ptr(), rows, vocab, p.stride(0), seeds.data_ptr(), steps.data_ptr(),
-                                                int(slot), int(purpose), tokens.data_ptr(), status.data_ptr(), _stream()),
-               "ds41_b200_sample_probabilities")
+    _launch(p.device, "ds41_b200_sample_probabilities", L.ds41_b200_sample_probabilities, p.data_ptr(), rows, vocab,
+            p.stride(0), seeds.data_ptr(), steps.data_ptr(), int(slot), int(purpose), tokens.data_ptr(),
+            status.data_ptr())
     return tokens, status
 
 
@@ -453,13 +453,10 @@ def verify_probabilities(draft_ids, q, p, drafts, seeds, steps, greedy=False):
     results = torch.empty(sequences * C.sizeof(SparkResult), dtype=torch.uint8, device=p.device)
     status = torch.empty(sequences, dtype=torch.int32, device=p.device)
     L = lib()
-    L.ds41_b200_verify_probabilities.argtypes = [_P, _P, _P, C.c_int, C.c_int, C.c_int, C.c_int, _P, _P, _P, _P, _P]
-    with torch.cuda.device(p.device):
-        _check(L.ds41_b200_verify_probabilities(draft_ids.data_ptr() if draft_ids is not None else None,
-                                                q.data_ptr() if q is not None else None, p.data_ptr(), sequences,
-                                                drafts, vocab, 1 if greedy else 0, seeds.data_ptr(), steps.data_ptr(),
-                                                results.data_ptr(), status.data_ptr(), _stream()),
-               "ds41_b200_verify_probabilities")
+    _launch(p.device, "ds41_b200_verify_probabilities", L.ds41_b200_verify_probabilities,
+            draft_ids.data_ptr() if draft_ids is not None else None, q.data_ptr() if q is not None else None,
+            p.data_ptr(), sequences, drafts, vocab, 1 if greedy else 0, seeds.data_ptr(), steps.data_ptr(),
+            results.data_ptr(), status.data_ptr())
     return results, status
 
 
@@ -470,9 +467,8 @@ def spark_sample_gpu_v2(p_f32, seed, step, slot=0, purpose=Purpose.Target):
     token = torch.empty(1, dtype=torch.int32, device=p_f32.device)
     L = lib()
     L.ds41_spark_sample_gpu_v2.argtypes = [_P, C.c_int, C.c_uint64, C.c_uint64, C.c_uint32, C.c_uint32, _P, _P]
-    with torch.cuda.device(p_f32.device):
-        _check(L.ds41_spark_sample_gpu_v2(p_f32.data_ptr(), p_f32.numel(), int(seed), int(step), int(slot), int(purpose),
-                                          token.data_ptr(), _stream()), "ds41_spark_sample_gpu_v2")
+    _launch(p_f32.device, "ds41_spark_sample_gpu_v2", L.ds41_spark_sample_gpu_v2, p_f32.data_ptr(), p_f32.numel(),
+            int(seed), int(step), int(slot), int(purpose), token.data_ptr())
     return int(token.item())
 
 
@@ -505,9 +501,8 @@ def logits_sha256(logits):
         raise ValueError("logits must be a CUDA fp32 [rows, vocab] tensor with unit inner stride")
     rows, vocab = logits.shape
     out = torch.empty((rows, 32), dtype=torch.uint8, device=logits.device)
-    with torch.cuda.device(logits.device):
-        _check(lib().ds41_b200_logits_sha256(logits.data_ptr(), rows, vocab, logits.stride(0), out.data_ptr(), _stream()),
-               "ds41_b200_logits_sha256")
+    _launch(logits.device, "ds41_b200_logits_sha256", lib().ds41_b200_logits_sha256, logits.data_ptr(), rows, vocab,
+            logits.stride(0), out.data_ptr())
     return [bytes(r).hex() for r in out.cpu().numpy()]
 
 
@@ -525,9 +520,7 @@ def fuse_head_fp8(x_bf16, w, w_scale, logits=None, workspace=None, error_flag=No
         logits = torch.empty((M, N), dtype=torch.float32, device=x_bf16.device)
     if workspace is None:
         workspace = torch.empty(fuse_head_fp8_workspace_bytes(M, K), dtype=torch.uint8, device=x_bf16.device)
-    with torch.cuda.device(x_bf16.device):
-        _check(lib().ds41_fuse_head_fp8(x_bf16.data_ptr(), w.data_ptr(), w_scale.data_ptr(), logits.data_ptr(), M, N, K,
-                                        workspace.data_ptr(), workspace.numel(),
-                                        error_flag.data_ptr() if error_flag is not None else None, _stream()),
-               "ds41_fuse_head_fp8")
+    _launch(x_bf16.device, "ds41_fuse_head_fp8", lib().ds41_fuse_head_fp8, x_bf16.data_ptr(), w.data_ptr(),
+            w_scale.data_ptr(), logits.data_ptr(), M, N, K, workspace.data_ptr(), workspace.numel(),
+            error_flag.data_ptr() if error_flag is not None else None)
     return logits

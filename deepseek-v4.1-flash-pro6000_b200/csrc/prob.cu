@@ -23,10 +23,15 @@ int cluster_size_for(int vocab);
 namespace {
 
 // One launch of `clusters` clusters of cl CTAs, with the kernel's shared memory allowed on the current device.
-template <class Args>
-cudaError_t launch_clusters(void (*kernel)(Args), int clusters, int cl, int threads, size_t smem, cudaStream_t stream,
-                            const Args &args) {
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+template <auto kernel, class Args>
+cudaError_t launch_clusters(int clusters, int cl, int threads, size_t smem, cudaStream_t stream, const Args &args) {
+  static thread_local int configured = -1;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && configured != dev) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e == cudaSuccess) configured = dev;
+  }
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(unsigned(clusters) * unsigned(cl));
@@ -486,7 +491,7 @@ extern "C" int ds41_b200_probabilities(const ds41_b200_prob_args *p, cudaStream_
              p->temperature > 0 ? std::fmax(p->temperature, 1e-5) : 0.0,  // engine/src/sampling.cpp:209-210
              p->top_p, p->probabilities, p->status, static_cast<unsigned char *>(p->scratch)};
   const int cl = cluster_size_for(p->vocab), clusters = int(need / (size_t(kReplayPad) * 12));
-  return int(launch_clusters(probability_rows_kernel, clusters, cl, kRT, sizeof(ProbSmem), stream, a));
+  return int(launch_clusters<probability_rows_kernel>(clusters, cl, kRT, sizeof(ProbSmem), stream, a));
 }
 
 extern "C" int ds41_b200_sample_probabilities(const double *p, int rows, int vocab, int64_t stride, const uint64_t *seeds,
@@ -508,7 +513,7 @@ extern "C" int ds41_b200_verify_probabilities(const int32_t *draft_ids, const do
     return invalid("verify arguments");
   VerifyRowsArgs<double> a{draft_ids, q, p, sequences, drafts, vocab, greedy ? 1 : 0, seeds, steps, 0, 0, results, status, 0};
   if (!greedy && vocab <= DS41_B200_MAX_VOCAB) {
-    const cudaError_t e = launch_clusters(verify_rows_fast_kernel, sequences, cluster_size_for(vocab), kThreads, sizeof(RowSmem),
+    const cudaError_t e = launch_clusters<verify_rows_fast_kernel>(sequences, cluster_size_for(vocab), kThreads, sizeof(RowSmem),
                                           stream, a);
     if (e != cudaSuccess) return int(e);
     a.only_pending = 1;   // what it could not certify
