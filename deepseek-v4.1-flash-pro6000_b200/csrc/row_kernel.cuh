@@ -215,6 +215,38 @@ __device__ __forceinline__ void count_history(RowCtx &c, const int32_t *h, int n
   for (i += c.tid; i < n; i += kThreads) count(__ldg(h + i));
 }
 
+// The penalties of the ids that occur in the history, on the staged logits; 2 if one is no longer finite (its logit then stays).
+// A thread looks through 32 counters and goes through those that are not zero: few ids occur, and in the pass over the logits
+// nearly every group of 128 has one of them, for which the whole warp took four rounds (constrained 256 rows, 32768 tokens:
+// 13 of 51 thousand cycles a slice).
+__device__ __forceinline__ int apply_penalties(RowCtx &c, float repetition, float presence, float frequency) {
+  RowSmem *s = c.s;
+  const uint4 *quads = reinterpret_cast<const uint4 *>(s->work.count_pairs);   // eight ids each, zero beyond the slice
+  const uint16_t *counts = reinterpret_cast<const uint16_t *>(s->work.count_pairs);
+  static_assert(kSliceCap / 8 == 4 * kThreads, "four per thread");
+  unsigned bits = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint4 q = quads[c.tid + k * kThreads];
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      bits |= (w[i] & 0xffffu) ? 1u << (8 * k + 2 * i) : 0u;
+      bits |= (w[i] >> 16) ? 2u << (8 * k + 2 * i) : 0u;
+    }
+  }
+  int over = 0;
+  for (; bits; bits &= bits - 1u) {
+    const int bit = __ffs(bits) - 1, j = 8 * (c.tid + (bit >> 3) * kThreads) + (bit & 7);
+    const float x = s->y[j];
+    const float v = x > 0.f ? __fdiv_rn(x, repetition) : __fmul_rn(x, repetition);
+    const float y = __fsub_rn(v, __fadd_rn(presence, __fmul_rn(frequency, float(counts[j]))));
+    if ((__float_as_uint(y) & 0x7f800000u) == 0x7f800000u) over = 2;
+    else s->y[j] = y;
+  }
+  return over;
+}
+
 // The general search on a valid row in place: top-k and top-p cuts of any kind by multi-level histograms (find_cut), then
 // the draw.  Rows come here when neither of the paths above fits them: plateaus of thousands of equal logits at the cut,
 // top_k in the thousands.  Out of line: its registers are not the other paths'.
@@ -345,7 +377,11 @@ __device__ __forceinline__ bool row_body(const RowArgs &a, RowCtx &c, RowSmem *s
     auto take = [&](float y, int j) {
       if (y > best) { best = y; id = j; }
     };
-    if (hist_len == 0 && !a.mask) {    // every id as it is
+    if (hist_len > 0) {
+      over = apply_penalties(c, a.repetition, a.presence, a.frequency);
+      __syncthreads();
+    }
+    if (!a.mask) {
       count = max(0, min(c.len - c.warp * c.region, c.region));   // (per warp; lane 0's counts)
       if (c.lane) count = 0;
 #pragma unroll 2
@@ -362,7 +398,7 @@ __device__ __forceinline__ bool row_body(const RowArgs &a, RowCtx &c, RowSmem *s
         }
       }
     } else {
-#pragma unroll 1
+#pragma unroll 2
       for (int j = j0; j < j0 + c.region; j += 128) {
         const int left = c.len - j;
         if (left <= 0) break;
@@ -371,31 +407,18 @@ __device__ __forceinline__ bool row_body(const RowArgs &a, RowCtx &c, RowSmem *s
         unsigned in = left >= 4 ? 15u : (1u << left) - 1u;
 #pragma unroll
         for (int k = 0; k < 4; ++k) poison = fmaf((in >> k) & 1u ? y[k] : 0.f, 0.f, poison);
-        if (a.mask) in &= s->mask_words[j >> 5] >> (j & 31);
-        if (hist_len > 0) {
-          const uint2 w = *reinterpret_cast<const uint2 *>(&s->work.count_pairs[j >> 1]);
-          if (w.x | w.y) {
-#pragma unroll 1
-            for (int k = 0; k < 4; ++k) {
-              const uint32_t cnt = ((k & 2 ? w.y : w.x) >> (16 * (k & 1))) & 0xffffu;
-              if (cnt) {
-                const float x = y[0];  // (rotated below, so that the loop keeps to one copy of the division)
-                const float v = x > 0.f ? __fdiv_rn(x, a.repetition) : __fmul_rn(x, a.repetition);
-                y[0] = __fsub_rn(v, __fadd_rn(a.presence, __fmul_rn(a.frequency, float(cnt))));
-                if ((__float_as_uint(y[0]) & 0x7f800000u) == 0x7f800000u) over = 2;
-              }
-              const float r = y[0];
-              y[0] = y[1]; y[1] = y[2]; y[2] = y[3]; y[3] = r;
-            }
-          }
-        }
-        count += __popc(in);
+        in &= s->mask_words[j >> 5] >> (j & 31);
+        if (in) {                        // (a grammar allows a few per cent: most groups of 128 hold none)
+          count += __popc(in);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const bool ok = (in >> k) & 1u;
-          y[k] = ok ? y[k] : -CUDART_INF_F;
-          low = fminf(low, ok ? y[k] : CUDART_INF_F);
-          take(y[k], j + k);
+          for (int k = 0; k < 4; ++k) {
+            const bool ok = (in >> k) & 1u;
+            y[k] = ok ? y[k] : -CUDART_INF_F;
+            low = fminf(low, ok ? y[k] : CUDART_INF_F);
+            take(y[k], j + k);
+          }
+        } else {
+          y[0] = y[1] = y[2] = y[3] = -CUDART_INF_F;
         }
         y4[j >> 2] = make_float4(y[0], y[1], y[2], y[3]);
       }
