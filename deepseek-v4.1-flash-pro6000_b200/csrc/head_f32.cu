@@ -8,62 +8,83 @@
 // 16-byte loads, activations in shared memory, all rows of the (small) batch per pass over the weights.
 #include "ds41_b200.h"
 #include "host_error.h"
+#include "launch.h"
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 namespace ds41 {
 namespace {
 
-constexpr int kF32Threads = 256, kF32Warps = kF32Threads / 32, kF32RowsPerWarp = 2;
+// Every thread has two 16-byte loads per row in flight ahead of the one it works on, 64 KB per SM.  Where an SM has one CTA they
+// run on across the ends of the rows, and the first ones do not wait for the kernel in front of this one: weights are nobody's
+// output.  The shape follows what an SM can hold beside the activations: one row of them leaves room for four small CTAs; up
+// to six rows take one CTA of 32 warps with two weight rows each; more rows, where the shared-memory reads of the activations
+// weigh in, sixteen warps with four weight rows, so that each is used four times.  HBM-bound; 129280 x 5120, us at M = 1 to 8
+// (405 at the rate of a plain copy): 411 432 434 439 422 429 455 491; sixteen warps of four rows throughout 440 443 434 442
+// 449 450 448 459; CTAs of eight warps with two rows, as many as the activations allow, 405 621 684 688 731 1219 1240 1241.
+template <int M>
+struct F32Shape {
+  static constexpr int kRows = M <= 6 ? 2 : 4, kThreads = M == 1 ? 256 : M <= 6 ? 1024 : 512, kPerSm = M == 1 ? 4 : 1;
+  static constexpr int kWarps = kThreads / 32, kAhead = 2;
+};
 
 template <int M>
-__global__ void __launch_bounds__(kF32Threads) head_f32_kernel(const float *__restrict__ x, const float *__restrict__ w,
-                                                               float *__restrict__ y, int N, int K) {
+__global__ void __launch_bounds__(F32Shape<M>::kThreads, F32Shape<M>::kPerSm)
+head_f32_kernel(const float *x, const float *__restrict__ w, float *y, int N, int K) {
+  constexpr int kRows = F32Shape<M>::kRows, kThreads = F32Shape<M>::kThreads, kWarps = F32Shape<M>::kWarps;
+  constexpr int kAhead = F32Shape<M>::kAhead;
+  constexpr bool kAcross = F32Shape<M>::kPerSm == 1;   // (other CTAs cover a row's end)
   extern __shared__ __align__(16) float xs[];  // [M][K]
-  for (int i = threadIdx.x * 4; i < M * K; i += kF32Threads * 4)
-    *reinterpret_cast<float4 *>(xs + i) = __ldg(reinterpret_cast<const float4 *>(x + i));
-  __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int groups = (N + kF32RowsPerWarp - 1) / kF32RowsPerWarp;
-  for (int g = blockIdx.x * kF32Warps + warp; g < groups; g += gridDim.x * kF32Warps) {
-    const int row0 = g * kF32RowsPerWarp;
-    float acc[kF32RowsPerWarp][M];
+  const int groups = (N + kRows - 1) / kRows, stride = gridDim.x * kWarps;
+  int fetch_group = blockIdx.x * kWarps + warp, fetch_k = lane * 4;
+  auto fetch = [&](float4 (&to)[kRows]) {
+    if (kAcross ? fetch_group >= groups : fetch_k >= K) return;
 #pragma unroll
-    for (int r = 0; r < kF32RowsPerWarp; ++r)
+    for (int r = 0; r < kRows; ++r)   // rows beyond N repeat the last one
+      to[r] = __ldcs(reinterpret_cast<const float4 *>(w + size_t(min(fetch_group * kRows + r, N - 1)) * K + fetch_k));
+    if ((fetch_k += 128) >= K && kAcross) { fetch_k = lane * 4; fetch_group += stride; }
+  };
+  float4 buf[kAhead + 1][kRows];
+#pragma unroll
+  for (int i = 0; i < kAhead; ++i) fetch(buf[i]);
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+  for (int i = threadIdx.x * 4; i < M * K; i += kThreads * 4)
+    *reinterpret_cast<float4 *>(xs + i) = *reinterpret_cast<const float4 *>(x + i);
+  __syncthreads();
+  for (int g = blockIdx.x * kWarps + warp; g < groups; g += stride) {
+    const int row0 = g * kRows;
+    if (!kAcross && g != blockIdx.x * kWarps + warp) {
+      fetch_group = g; fetch_k = lane * 4;
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) fetch(buf[i]);
+    }
+    float acc[kRows][M];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
 #pragma unroll
       for (int m = 0; m < M; ++m) acc[r][m] = 0.f;
-    const float4 *wr[kF32RowsPerWarp];
-#pragma unroll
-    for (int r = 0; r < kF32RowsPerWarp; ++r)
-      wr[r] = reinterpret_cast<const float4 *>(w + size_t(min(row0 + r, N - 1)) * K);  // rows beyond N repeat the last one
-    // two 16-byte loads per row in flight ahead of the one being consumed
-    float4 cur[kF32RowsPerWarp], nxt[kF32RowsPerWarp];
-#pragma unroll
-    for (int r = 0; r < kF32RowsPerWarp; ++r) {
-      cur[r] = __ldg(wr[r] + lane);
-      nxt[r] = 128 < K ? __ldg(wr[r] + lane + 32) : cur[r];
-    }
     for (int k = lane * 4; k < K; k += 128) {
-      float4 far[kF32RowsPerWarp];
-      const bool more = k + 256 < K;
-#pragma unroll
-      for (int r = 0; r < kF32RowsPerWarp; ++r) far[r] = more ? __ldg(wr[r] + ((k + 256) >> 2)) : nxt[r];
+      fetch(buf[kAhead]);
 #pragma unroll
       for (int m = 0; m < M; ++m) {
         const float4 a = *reinterpret_cast<const float4 *>(xs + m * K + k);
 #pragma unroll
-        for (int r = 0; r < kF32RowsPerWarp; ++r) {
-          acc[r][m] = __fmaf_rn(cur[r].x, a.x, acc[r][m]);
-          acc[r][m] = __fmaf_rn(cur[r].y, a.y, acc[r][m]);
-          acc[r][m] = __fmaf_rn(cur[r].z, a.z, acc[r][m]);
-          acc[r][m] = __fmaf_rn(cur[r].w, a.w, acc[r][m]);
+        for (int r = 0; r < kRows; ++r) {
+          acc[r][m] = __fmaf_rn(buf[0][r].x, a.x, acc[r][m]);
+          acc[r][m] = __fmaf_rn(buf[0][r].y, a.y, acc[r][m]);
+          acc[r][m] = __fmaf_rn(buf[0][r].z, a.z, acc[r][m]);
+          acc[r][m] = __fmaf_rn(buf[0][r].w, a.w, acc[r][m]);
         }
       }
 #pragma unroll
-      for (int r = 0; r < kF32RowsPerWarp; ++r) { cur[r] = nxt[r]; nxt[r] = far[r]; }
+      for (int i = 0; i < kAhead; ++i)
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) buf[i][r] = buf[i + 1][r];
     }
 #pragma unroll
-    for (int r = 0; r < kF32RowsPerWarp; ++r)
+    for (int r = 0; r < kRows; ++r)
 #pragma unroll
       for (int m = 0; m < M; ++m) {
         float sum = acc[r][m];
@@ -77,22 +98,20 @@ __global__ void __launch_bounds__(kF32Threads) head_f32_kernel(const float *__re
 template <int M>
 cudaError_t launch_f32(const float *x, const float *w, float *y, int N, int K, cudaStream_t stream) {
   const size_t smem = size_t(M) * K * sizeof(float);
-  static thread_local int configured = -1;
-  int dev = 0, sms = 0;
+  static thread_local int configured = -1, sms = 0;
+  int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return e;
-  if (configured != dev) {
-    e = cudaFuncSetAttribute(head_f32_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e != cudaSuccess) return e;
-    configured = dev;
+  if (e == cudaSuccess && configured != dev) {
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(head_f32_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e == cudaSuccess) configured = dev;
   }
-  const int per_sm = smem <= 56 * 1024 ? 4 : smem <= 100 * 1024 ? 2 : 1;
-  const int groups = (N + kF32RowsPerWarp - 1) / kF32RowsPerWarp;
-  int grid = sms * per_sm;
-  if (grid > (groups + kF32Warps - 1) / kF32Warps) grid = (groups + kF32Warps - 1) / kF32Warps;
-  head_f32_kernel<M><<<grid, kF32Threads, smem, stream>>>(x, w, y, N, K);
-  return cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  using Shape = F32Shape<M>;
+  // (a long K leaves one activation row less room than four CTAs need)
+  const int per_sm = Shape::kPerSm > 1 && smem > 54 * 1024 ? (smem > 110 * 1024 ? 1 : 2) : Shape::kPerSm;
+  const int groups = (N + Shape::kRows - 1) / Shape::kRows, ctas = (groups + Shape::kWarps - 1) / Shape::kWarps;
+  return launch_early(head_f32_kernel<M>, sms * per_sm < ctas ? sms * per_sm : ctas, Shape::kThreads, smem, stream, x, w, y, N, K);
 }
 
 }  // namespace
