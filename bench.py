@@ -214,10 +214,11 @@ class HeadSample:
         self.sharded = None
         self.exchange_note = None
         self.sampler_rows = batch
-        # own kernels per step: quantise, head, then the sampler call = flat_hist / flat_window / flat_mass / flat_resolve,
-        # the cluster kernel's persistent grid for rows handed on and the replay kernel for uncertified rows (both
-        # return at once when there is nothing for them); flat_stats is not launched: the head's epilogue left its records
-        self.launches_per_step = 8
+        # own kernels per step: quantise, clearing of the row records, head, then the sampler call: the cluster kernel and the
+        # replay kernel up to 48 rows, else flat_hist / flat_window / flat_mass / flat_resolve, the cluster kernel's
+        # persistent grid for rows handed on and the replay kernel for uncertified rows (both return at once when there is
+        # nothing for them); flat_stats is not launched: the head's epilogue left its records
+        self.launches_per_step = 5 if batch <= 48 else 9
         if world > 1:
             self.sharded = import_module("ds41_b200.sharded").ShardedDecodeTail(pkg, device, batch, self.v0, self.vn,
                                                                               VOCAB, temperature, top_p, strategy,

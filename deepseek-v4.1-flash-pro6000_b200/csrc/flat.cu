@@ -10,10 +10,10 @@
 //                                    exact id counts before and inside it.  Rows this path does not fit get status -8
 //                                    (the caller sends them to the other paths), non-finite rows -1.
 //   flat_mass_kernel    (row, part)  the FP64 pass, dense and branch free: every id's weight 2^-((max-y)*log2(e)/T) from a
-//                                    256-entry table and a degree-4 polynomial (12 FP64 instructions per id); per 1024-id
+//                                    64-entry table and a degree-4 polynomial (11 FP64 instructions per id); per 1024-id
 //                                    sub-region the sum over all ids and over the ids before the window; the window's
-//                                    ids go to a per-row list.
-//   flat_resolve_kernel (row)        sorts the list exactly, FP64 prefix sums -> certified cut; kept mass per sub-region
+//                                    ids go to a per-row list by way of a buffer of each warp.
+//   flat_resolve_kernel (row)        orders the list by buckets, FP64 prefix sums -> certified cut; kept mass per sub-region
 //                                    -> the sub-region that holds u * total -> walks its 1024 ids.
 // Rule, error bounds and status words are those of the cluster kernel (row_kernel.cuh); the reference rule is
 // engine/third_party/spark/src/sampling.cpp:18-38.
@@ -30,7 +30,6 @@ constexpr int kFT = kFlatThreads;
 constexpr int kFW = kFT / 32;
 
 struct FlatRed {  // per-CTA scratch for block reductions / prefix sums
-  double d[kFW], e[kFW];
   float f[kFW], g[kFW];
   int i[kFW], j[kFW];
 };

@@ -71,7 +71,7 @@ template cudaError_t launch_rows<kModeStats>(const RowArgs &, int, cudaStream_t)
 
 int chunks_for(int vocab);
 cudaError_t launch_chunks(const ChunkArgs &a, int rows, cudaStream_t stream);
-cudaError_t launch_combine(const CombineArgs &a, bool stats, cudaStream_t stream);
+cudaError_t launch_combine(const CombineArgs &a, cudaStream_t stream);
 
 }  // namespace ds41
 
@@ -247,12 +247,12 @@ extern "C" int ds41_b200_sample_logits(const ds41_b200_sample_args *p, cudaStrea
   }
   if (streaming) {
     // streaming path: chunk records -> combine -> cluster kernel only for the rows the combine could not cover
-    ChunkArgs c{p->logits, p->logits_stride, p->vocab, 0, chunks, a.temperature, records, nullptr};
+    ChunkArgs c{p->logits, p->logits_stride, p->vocab, 0, chunks, a.temperature, records};
     e = launch_chunks(c, p->rows, stream);
     if (e != cudaSuccess) return int(e);
     CombineArgs m{records, p->rows, 1, chunks, p->vocab, a.temperature, p->top_p, p->top_k, p->seeds, p->steps, p->slot,
-                  p->purpose, p->tokens, status, nullptr, 0};
-    e = launch_combine(m, false, stream);
+                  p->purpose, p->tokens, status};
+    e = launch_combine(m, stream);
     if (e != cudaSuccess) return int(e);
   }
   a.status = status;

@@ -1,4 +1,4 @@
-// Host side of the streaming sampler (stream.cuh): launch helpers shared by the sampler and the verifier, and the
+// Host side of the streaming sampler (stream.cuh): launch helpers, and the
 // C-ABI entry points of the vocabulary-sharded path (a shard publishes the records of its chunks, the caller
 // all-gathers them, every rank combines).
 #include "ds41_b200.h"
@@ -17,20 +17,16 @@ cudaError_t launch_chunks(const ChunkArgs &a, int rows, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_combine(const CombineArgs &a, bool stats, cudaStream_t stream) {
+cudaError_t launch_combine(const CombineArgs &a, cudaStream_t stream) {
   static thread_local int configured = -1;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (configured != dev) {  // the combine needs more than the default 48 KB of dynamic shared memory
-    e = cudaFuncSetAttribute(combine_kernel<kCombineStats>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(CombineSmem)));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(combine_kernel<kCombineDraw>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(CombineSmem)));
-    if (e != cudaSuccess) return e;
-    configured = dev;
+  if (e == cudaSuccess && configured != dev) {  // the combine needs more than the default 48 KB of dynamic shared memory
+    e = cudaFuncSetAttribute(combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(CombineSmem)));
+    if (e == cudaSuccess) configured = dev;
   }
-  if (stats) combine_kernel<kCombineStats><<<a.rows, kCombineThreads, sizeof(CombineSmem), stream>>>(a);
-  else combine_kernel<kCombineDraw><<<a.rows, kCombineThreads, sizeof(CombineSmem), stream>>>(a);
+  if (e != cudaSuccess) return e;
+  combine_kernel<<<a.rows, kCombineThreads, sizeof(CombineSmem), stream>>>(a);
   return cudaGetLastError();
 }
 
@@ -62,6 +58,6 @@ extern "C" int ds41_b200_shard_combine(const ds41_b200_shard_combine_args *p, cu
   if (p->slot > 5 || p->purpose > 3) return invalid("Philox v2 address out of range");
   CombineArgs a{reinterpret_cast<const ChunkRecord *>(p->gathered), p->rows, p->ranks, p->chunks, p->vocab,
                 p->temperature > 0 ? std::fmax(p->temperature, 1e-5) : 0.0, p->top_p, p->top_k, p->seeds, p->steps, p->slot,
-                p->purpose, p->tokens, p->status, nullptr};
-  return int(launch_combine(a, false, stream));
+                p->purpose, p->tokens, p->status};
+  return int(launch_combine(a, stream));
 }

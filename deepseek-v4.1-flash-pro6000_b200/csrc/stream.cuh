@@ -40,7 +40,6 @@ __global__ void __launch_bounds__(kChunkThreads, 4) chunk_kernel(ChunkArgs a) {
   __shared__ ChunkSmem s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int row = blockIdx.x / a.chunks, chunk = blockIdx.x % a.chunks;
-  if (a.only_uncovered && a.only_uncovered[row] != kNotCovered) return;  // the same in every thread
   const int begin = min(a.vocab_local, chunk * kChunkIds);
   const int len = min(a.vocab_local, begin + kChunkIds) - begin;
   ChunkRecord *out = a.out + size_t(row) * a.chunks + chunk;
@@ -282,12 +281,10 @@ struct CombineSmem {
   int n_filtered;
 };
 
-template <int kMode>
 __global__ void __launch_bounds__(kCombineThreads) combine_kernel(CombineArgs a) {
   extern __shared__ __align__(16) unsigned char combine_raw[];
   CombineSmem &s = *reinterpret_cast<CombineSmem *>(combine_raw);
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (a.only_uncovered && a.status[row] != kNotCovered) return;  // the same in every thread
   const int nrec = a.groups * a.per_group;
   const double t = a.temperature;
   auto rec = [&](int r) -> const ChunkRecord & {
@@ -315,15 +312,7 @@ __global__ void __launch_bounds__(kCombineThreads) combine_kernel(CombineArgs a)
     status = error ? error : (escalate ? kNotCovered : 0);
   }
   if (status < 0 || t == 0) {
-    if (tid == 0) {
-      if (kMode == kCombineDraw) { a.tokens[row] = status < 0 ? -1 : arg; if (a.status) a.status[row] = status; }
-      else {
-        RowStats st{};
-        st.z = 1; st.e_kept = 1; st.max_logit = m; st.argmax = arg; st.cut.y = m; st.cut.id = arg; st.kept = 1;
-        st.entered = a.vocab; st.status = status; st.drawn = -1;
-        a.stats[row] = st;
-      }
-    }
+    if (tid == 0) { a.tokens[row] = status < 0 ? -1 : arg; if (a.status) a.status[row] = status; }
     return;
   }
   if (tid < nrec) s.hw[tid] = s.hz[tid] > 0 ? exp((double(s.hmax[tid]) - double(m)) / t) : 0.0;
@@ -476,19 +465,7 @@ __global__ void __launch_bounds__(kCombineThreads) combine_kernel(CombineArgs a)
   status = s.i_out[0];
   const int kept = s.i_out[1];
   if (status == kNotCovered) {
-    if (tid == 0) {
-      if (kMode == kCombineDraw) { a.tokens[row] = -1; if (a.status) a.status[row] = kNotCovered; }
-      else { RowStats st{}; st.status = kNotCovered; st.max_logit = m; st.argmax = arg; a.stats[row] = st; }
-    }
-    return;
-  }
-  if (kMode == kCombineStats) {
-    if (tid == 0) {
-      RowStats st;
-      st.z = s.d_out[0]; st.e_kept = s.d_out[1]; st.max_logit = m; st.argmax = arg;
-      st.cut.y = s.sy[kept - 1]; st.cut.id = s.sid[kept - 1]; st.kept = kept; st.entered = s.i_out[2]; st.status = status; st.drawn = -1;
-      a.stats[row] = st;
-    }
+    if (tid == 0) { a.tokens[row] = -1; if (a.status) a.status[row] = kNotCovered; }
     return;
   }
   // ---- survivors in id order, then the reference's draw

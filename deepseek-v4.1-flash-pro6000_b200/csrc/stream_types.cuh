@@ -10,7 +10,7 @@
 //                    that sent 64 ids but not all of its ids must have its last candidate outside the kept set,
 //                    otherwise ids that were not sent might survive and the row is reported NOT_COVERED (the caller
 //                    then runs the cluster kernel, which handles any support size, on that row).
-// The same two kernels serve the single-GPU sampler, the verifier's row statistics and the vocabulary-sharded path
+// The same two kernels serve the single-GPU sampler and the vocabulary-sharded path
 // (a shard is just a set of chunks).
 #pragma once
 #include "row_core.cuh"
@@ -46,10 +46,7 @@ struct ChunkArgs {
   int vocab_local, id_offset, chunks;  // chunks per row (>= ceil(vocab_local/kChunkIds); extra chunks are empty)
   double temperature;
   ChunkRecord *out;  // [rows][chunks]
-  const int32_t *only_uncovered;  // if set: only rows whose status word there is -8 are processed
 };
-
-enum CombineMode { kCombineDraw = 0, kCombineStats = 1 };
 
 struct CombineArgs {
   const ChunkRecord *records;  // [groups][rows][per_group]: groups = ranks (all-gathered) or 1
@@ -59,8 +56,6 @@ struct CombineArgs {
   const uint64_t *seeds, *steps;
   uint32_t slot, purpose;
   int32_t *tokens, *status;
-  RowStats *stats;
-  int only_uncovered;  // only rows whose status word is -8 are processed (the others already have their answer)
 };
 
 

@@ -154,12 +154,12 @@ typedef struct ds41_b200_sample_args {
   int32_t *tokens;            /* [rows] out */
   int32_t *status;            /* [rows] out, see above; may be NULL */
   void *scratch;              /* optional device scratch of ds41_b200_sample_scratch_bytes(rows, vocab) bytes, 16-byte
-                                 aligned.  With it, rows without penalties / bitmask and with top_k <= 64 are tried,
-                                 per row, by two batch-parallel paths before the cluster kernel: without top_k (rows
-                                 16-byte aligned, vocab >= 16384) the batch path (grid-wide kernels: histogram,
-                                 window, FP64 masses, resolve), then the streaming path for small nuclei (chunk
-                                 records + a per-row combine).  Rows neither can take, and calls without scratch,
-                                 use the cluster kernel.  Same results on every path.  With scratch, rows whose
+                                 aligned.  With it, larger batches of rows without penalties / bitmask and with
+                                 top_k <= 64 (more than 48 rows cut by top-p, 256 by top-k, 64 greedy) take a
+                                 batch-parallel path before the cluster kernel: without top_k (vocab >= 16384)
+                                 grid-wide kernels (histogram, window, FP64 masses, resolve), otherwise the streaming
+                                 path (chunk records + a per-row combine).  Rows these cannot take, smaller batches and
+                                 calls without scratch use the cluster kernel.  Same results on every path.  With scratch, rows whose
                                  decision fell inside the rounding bound of the parallel sums (status bits 1 / 2) are
                                  redone in the same call in the reference's order of operations and leave with
                                  status 0 (the scratch holds the replay's rows too: about 10 MB). */
@@ -178,8 +178,8 @@ int ds41_b200_sample_logits(const ds41_b200_sample_args *args, cudaStream_t stre
  * from (spark.h:101-105).  Sequence s uses the address (seeds[s], steps[s], slot = position, purpose =
  * ACCEPT / RESIDUAL / TARGET) exactly as the reference.  temperature 0 selects the greedy rule (draft_logits
  * may then be NULL).  `scratch` is caller-owned device memory of ds41_b200_verify_scratch_bytes() bytes (16-byte
- * aligned): 48 bytes of statistics per logits row, the streaming path's chunk records, and 7.3 MB for the replay of
- * transactions whose decisions fell inside the rounding bound (status bits 1 / 2 / 4 / 8: redone in the same call in
+ * aligned): 56 bytes of statistics per logits row, the streaming path's chunk records, the batch path's work space (for
+ * more than 40 logits rows), and 7.3 MB for the replay of transactions whose decisions fell inside the rounding bound (status bits 1 / 2 / 4 / 8: redone in the same call in
  * the reference's order, they leave with status 0).  With less the call still works: without the replay's share the
  * bits stay in the status words; with the statistics alone every row goes through the cluster kernel. */
 typedef struct ds41_b200_verify_args {
