@@ -27,13 +27,18 @@ __device__ __forceinline__ float bf16_bits_to_float(uint32_t bits16) { return __
 // Arithmetic of the reference kernel head<M, 8, 4> for one output: lane l of 32 takes k = 8 l + 256 i, i = 0, 1, ...;
 // element j of its eight goes to accumulator j % 4 by fused multiply-add (so accumulator a sees k + a, k + a + 4 of every
 // i, in that order); at the end (a0 + a1) + (a2 + a3), then the five-level shuffle-down tree over the lanes.
+// Where the four activations 4 i .. 4 i + 3 lie in shared memory, in units of four: a lane uses eight neighbouring ones of a
+// block of 256; the first four of all lanes come first, then the others, so that a warp's 16-byte reads touch every bank once
+// (32 bytes a lane in place took two passes, which from M = 4 on cost more than the weights).
+__device__ __forceinline__ int activation_slot(int i) { return (i & ~63) | ((i & 1) << 5) | ((i & 63) >> 1); }
+
 template <int M, int kRowsPerWarp>
 __global__ void __launch_bounds__(kHeadThreads) head_compact_kernel(const float *__restrict__ x,
                                                                     const __nv_bfloat16 *__restrict__ w,
                                                                     float *__restrict__ y, int N, int K) {
   extern __shared__ __align__(16) float xs[];  // [M][K]
-  for (int i = threadIdx.x * 4; i < M * K; i += kHeadThreads * 4)
-    *reinterpret_cast<float4 *>(xs + i) = __ldg(reinterpret_cast<const float4 *>(x + i));
+  for (int i = threadIdx.x; i < M * K / 4; i += kHeadThreads)
+    reinterpret_cast<float4 *>(xs)[activation_slot(i)] = __ldg(reinterpret_cast<const float4 *>(x) + i);
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int groups = (N + kRowsPerWarp - 1) / kRowsPerWarp;
@@ -70,8 +75,8 @@ __global__ void __launch_bounds__(kHeadThreads) head_compact_kernel(const float 
       }
 #pragma unroll
       for (int m = 0; m < M; ++m) {
-        const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(xs + m * K + k);
-        const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(xs + m * K + k + 4);
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(xs + m * K + k - lane * 4);
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(xs + m * K + k - lane * 4 + 128);
 #pragma unroll
         for (int r = 0; r < kRowsPerWarp; ++r) {
           acc[r][m][0] = fma_f32x2(wv[r][0], a.x, acc[r][m][0]);
@@ -128,8 +133,8 @@ __global__ void __launch_bounds__(kThreads) head_compact_ring_kernel(const float
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();
 #pragma unroll 4
-  for (int i = threadIdx.x * 4; i < M * K; i += kThreads * 4)
-    *reinterpret_cast<float4 *>(xs + i) = __ldg(reinterpret_cast<const float4 *>(x + i));
+  for (int i = threadIdx.x; i < M * K / 4; i += kThreads)
+    reinterpret_cast<float4 *>(xs)[activation_slot(i)] = __ldg(reinterpret_cast<const float4 *>(x) + i);
   __syncthreads();
   int slot = 0;
   for (int g = blockIdx.x * kWarpsHere + warp; g < groups; g += stride) {
@@ -156,11 +161,11 @@ __global__ void __launch_bounds__(kThreads) head_compact_ring_kernel(const float
       }
       fetch();            // (into the slot that the previous step consumed)
       if (++slot == stages) slot = 0;
-      const float *xk = xs + step * 256 + lane * 8;
+      const float *xk = xs + step * 256 + lane * 4;
 #pragma unroll
       for (int m = 0; m < M; ++m) {
         const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(xk + m * K);
-        const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(xk + m * K + 4);
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(xk + m * K + 128);
 #pragma unroll
         for (int r = 0; r < kRowsPerWarp; ++r) {
           acc[r][m][0] = fma_f32x2(wv[r][0], a.x, acc[r][m][0]);
@@ -350,10 +355,12 @@ cudaError_t launch_compact(const float *x, const void *w, float *y, int N, int K
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
-  // One CTA of sixteen warps per SM (twelve, with 168 registers per thread, from M = 5 on).  Weight rows that share one read of an activation fragment: per 512 bytes of weights and
-  // row M * 8 / rows cycles of shared memory, against the 22 cycles they take to arrive: four rows, or what the registers
-  // hold (three at M = 8).  A ring of 2, 3, 4 or 6 steps, what the activations leave room for.
-  constexpr int kRing = M <= 7 ? 4 : 3, kRingThreads = M <= 4 ? 512 : 384;
+  // One CTA of sixteen warps per SM (twelve, with 168 registers per thread, from M = 5 on).  Weight rows that share one read of
+  // an activation fragment: per 512 bytes of weights and row M * 8 / rows cycles of shared memory, against the 22 cycles they
+  // take to arrive: four rows (five at M = 5: 227 to 220 us), or what the registers hold (three at M = 8; five at M = 6 spill:
+  // 392 us).  A ring of 2, 3, 4 or 6 steps, what the activations leave room for.  129280 x 5120, us at M = 1 to 8: 194 190 193
+  // 194 220 257 375 355 (195 190 195 215 286 328 423 515 with the activations' fragments in place, 32 bytes a lane).
+  constexpr int kRing = M == 5 ? 5 : M <= 7 ? 4 : 3, kRingThreads = M <= 4 ? 512 : 384;
   const size_t activations = size_t(M) * K * sizeof(float), step = size_t(kRingThreads / 32) * kRing * 512;
   const int room = int((227 * 1024 - activations) / step);
   const int stages = room >= 6 ? 6 : room > 4 ? 4 : room;
