@@ -4,12 +4,12 @@
 // ascending order with one fused multiply-add per term, then the chains are added by a four-level tree (distance 8, 4,
 // 2, 1 over the chain index) and +0.f canonicalises a negative zero.  This kernel keeps exactly that order -- every
 // intermediate is the same FP32 number -- and changes only how the bytes and the chains move: persistent CTAs keep the M
-// activation rows in shared memory, and every warp streams 32 weight rows x 64 K at a time through a ring of its own
+// activation rows in shared memory, and every warp streams 16 or 32 weight rows x 64 K at a time through a ring of its own
 // (16-byte cp.async copies, no barrier of the CTA).  Four lanes share a weight row, each with four neighbouring chains (k .. k +
-// 3), so that one 8-byte load feeds four chains and the chains advance two at a time by packed FMAs; a lane has four rows, so
-// that an activation read from shared memory is used four times: per 512 bytes of weights that is 2 M cycles of shared
-// memory plus 8 for the weights, against the 22 they take to arrive (with one row per lane, M = 3 took 377 us, with two
-// 276).  HBM-bound: the BF16 weights, 2*N*K bytes (1.32 GB at N=129280, K=5120), are read exactly once.
+// 3), so that one 8-byte load feeds four chains and the chains advance two at a time by packed FMAs; a lane has two or four
+// rows, so that an activation read from shared memory is used as often: with four, per 512 bytes of weights that is 2 M cycles
+// of shared memory plus 8 for the weights, against the 22 they take to arrive.  HBM-bound: the BF16 weights, 2*N*K bytes
+// (1.32 GB at N=129280, K=5120), are read exactly once.
 #include "ds41_b200.h"
 #include "host_error.h"
 #include "launch.h"
@@ -21,15 +21,22 @@
 namespace ds41 {
 namespace {
 
-constexpr int kLaneRows = 4, kWarpRows = 8 * kLaneRows;                  // weight rows per lane; per warp (four lanes each)
-constexpr int kChunkK = 64, kRowPitch = kChunkK * 2 + 32;                // bytes; the skew keeps eight rows on different banks
-constexpr int kStageBytes = kWarpRows * kRowPitch;                       // 5 KB
-constexpr int kMostWarps = 7;   // 129280 rows are 3.9 rounds of 148 x 7 warps x 32 rows (eight warps: 3.4, the fourth half empty)
+constexpr int kChunkK = 64, kRowPitch = kChunkK * 2 + 32;   // bytes; the skew keeps eight rows on different banks
+// Weight rows per lane, per warp (four lanes each), bytes of a stage (2.5 or 5 KB) and the most warps.  Up to three activation
+// rows twice the warps hide more latency than the second use of an activation saves (M = 1 to 6: 194 197 202 235 261 321 us with
+// two rows per lane, 196 200 208 232 255 252 with four); 129280 rows are 3.9 rounds of 148 SMs x 7 warps x 32 rows, or 14 x 16
+// (eight or sixteen warps: 3.4, the fourth half empty).
+template <int M>
+struct Shape {
+  static constexpr int kLaneRows = M <= 3 ? 2 : 4, kWarpRows = 8 * kLaneRows, kStageBytes = kWarpRows * kRowPitch;
+  static constexpr int kMostWarps = M <= 3 ? 14 : 7;
+};
 constexpr size_t kSmemBudget = 227 * 1024;
 
 template <int M>
-__global__ void __launch_bounds__(32 * kMostWarps, 1) head_bf16_kernel(const float *x, const __nv_bfloat16 *w, float *y,
+__global__ void __launch_bounds__(32 * Shape<M>::kMostWarps, 1) head_bf16_kernel(const float *x, const __nv_bfloat16 *w, float *y,
                                                                        int N, int K, int stages) {
+  constexpr int kLaneRows = Shape<M>::kLaneRows, kWarpRows = Shape<M>::kWarpRows, kStageBytes = Shape<M>::kStageBytes;
   extern __shared__ __align__(16) unsigned char smem[];
   float *sx = reinterpret_cast<float *>(smem);                                   // [M][K], then per warp [stages][32][kRowPitch]
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -126,7 +133,8 @@ __global__ void __launch_bounds__(32 * kMostWarps, 1) head_bf16_kernel(const flo
 template <int M>
 cudaError_t launch_head_bf16(const float *x, const void *w, float *y, int N, int K, cudaStream_t stream) {
   const size_t activations = size_t(M) * K * sizeof(float);
-  int warps = kMostWarps;   // fewer where the activations leave no room for a ring of two stages per warp
+  constexpr int kStageBytes = Shape<M>::kStageBytes, kWarpRows = Shape<M>::kWarpRows;
+  int warps = Shape<M>::kMostWarps;   // fewer where the activations leave no room for a ring of two stages per warp
   while (warps > 1 && activations + size_t(warps) * 2 * kStageBytes > kSmemBudget) --warps;
   int stages = 4;
   while (stages > 1 && activations + size_t(warps) * stages * kStageBytes > kSmemBudget) --stages;
