@@ -337,10 +337,11 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     bool alive = true;  // warp-uniform; once false the remaining tiles are walked without waiting or computing,
                         // so that all epilogue threads still meet at every named barrier
     // running statistics of this thread's batch row over the tiles of one batch tile (vocabulary tiles come in ascending
-    // order, so a strict comparison keeps the first tile with the maximum; which of its columns it was is looked up in the
-    // logits when the row is left)
+    // order, so a strict comparison keeps the first maximum).  With 32 columns a thread the column is looked for only in a tile
+    // that raises the maximum of one of the warp's rows.  (Looking it up in the logits when the row is left took 10 us at 128
+    // rows and 28 at 256: the reads stand behind everything that the GPU has just written.)
     float st_best = -CUDART_INF_F, st_low = CUDART_INF_F, st_bad = 0.f, st_bad1 = 0.f;
-    int st_at = -1;
+    int st_id = 0x7fffffff;
     const bool stats_on = p.row_stats != nullptr || p.owner_stats_offset != 0;
     auto row_of = [&](int m) {   // batch row m of the output
       if (p.rows_per_owner == 0) return p.logits + size_t(m) * p.ldl;
@@ -349,14 +350,7 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     };
     auto flush_stats = [&](int bt_of) {
       const int m = bt_of * kRows + row;
-      __syncwarp();   // (the row's logits were written by other lanes)
-      if (stats_on && st_at >= 0 && row < kRows && m < p.M) {
-        const float *x = row_of(m);
-        int st_id = st_at;
-        const int end = min(p.N, st_at + kMyCols);
-#pragma unroll 16
-        for (int n = end - 1; n >= st_at; --n)
-          if (x[n] == st_best) st_id = n;
+      if (stats_on && st_id != 0x7fffffff && row < kRows && m < p.M) {
         auto ordered = [](float v) {
           const uint32_t bits = __float_as_uint(v == 0.f ? 0.f : v);  // -0 and +0 are the same logit
           return bits ^ ((bits >> 31) ? 0xffffffffu : 0x80000000u);
@@ -377,7 +371,7 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
           if (st_bad + st_bad1 != 0.f) atomicOr(&rs->flags, 1u);
         }
       }
-      st_best = -CUDART_INF_F; st_low = CUDART_INF_F; st_bad = st_bad1 = 0.f; st_at = -1;
+      st_best = -CUDART_INF_F; st_low = CUDART_INF_F; st_bad = st_bad1 = 0.f; st_id = 0x7fffffff;
     };
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
       const int nt = tile / b_tiles, bt = tile % b_tiles;
@@ -440,22 +434,36 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       const bool whole = n0 + kMyCols <= p.N;
       if (alive && stats_on) {
         if (whole) {
-          float hi = sum[0], low = sum[0];
           const unsigned long long zero2 = pack2(0.f, 0.f);
-#pragma unroll
-          for (int c = 1; c < kMyCols; ++c) { hi = fmaxf(hi, sum[c]); low = fminf(low, sum[c]); }
 #pragma unroll
           for (int c = 0; c < kMyCols; c += 2)   // NaN once any logit is NaN or infinite
             fma2_acc(st_bad, st_bad1, __float_as_uint(sum[c]), __float_as_uint(sum[c + 1]), zero2);
-          if (hi > st_best) { st_best = hi; st_at = n0; }
-          st_low = fminf(st_low, low);
+          if constexpr (kMyCols == 32) {
+            float hi = sum[0], low = sum[0];
+#pragma unroll
+            for (int c = 1; c < kMyCols; ++c) { hi = fmaxf(hi, sum[c]); low = fminf(low, sum[c]); }
+            if (__any_sync(0xffffffffu, hi > st_best)) {
+              int at = 0;
+#pragma unroll
+              for (int c = kMyCols - 1; c > 0; --c) at = sum[c] == hi ? c : at;
+              if (sum[0] == hi) at = 0;
+              if (hi > st_best) { st_best = hi; st_id = n0 + at; }
+            }
+            st_low = fminf(st_low, low);
+          } else {                               // (no registers to spare)
+#pragma unroll
+            for (int c = 0; c < kMyCols; ++c) {
+              if (sum[c] > st_best) { st_best = sum[c]; st_id = n0 + c; }
+              st_low = fminf(st_low, sum[c]);
+            }
+          }
         } else {
 #pragma unroll
           for (int c = 0; c < kMyCols; ++c) {
             const float v = sum[c];
             if (n0 + c < p.N) {
               st_bad = fmaf(v, 0.f, st_bad);
-              if (v > st_best) { st_best = v; st_at = n0; }
+              if (v > st_best) { st_best = v; st_id = n0 + c; }
               st_low = fminf(st_low, v);
             }
           }
