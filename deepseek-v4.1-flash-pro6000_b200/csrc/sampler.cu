@@ -155,9 +155,11 @@ extern "C" const char *ds41_spark_error(void) { return last_error(); }
 namespace {
 // Up to this many rows the cluster kernel takes a batch in one launch; larger ones go through the batch path (top-p alone)
 // or the streaming path (top-k, greedy).  Where the two meet, at 129280 ids: top-p 48 rows 65 us against 75, 64 rows 70
-// against 65; top-k 128 rows 64 us against 98, 256 rows 128 against 136; greedy 64 rows 18.5 us against 18.9, 96 rows 27
-// against 23.
-constexpr int kClusterRows = 48, kClusterRowsTopk = 256, kClusterRowsGreedy = 64;
+// against 65; greedy 64 rows 18.5 us against 18.9, 96 rows 27 against 23.  Rows cut by top-k cost the cluster kernel the same at
+// any vocabulary of eight slices, and the streaming path what their ids take to read: 129280 ids 140 rows 71 us against 76, 200
+// rows 100 against 95; 40000 ids 65 rows 31 against 41, 100 rows 50 against 45.
+constexpr int kClusterRows = 48, kClusterRowsGreedy = 64;
+int cluster_rows_topk(int vocab) { return vocab > 32768 ? 44 + vocab / 1114 : 256; }
 
 // One launch that decides every row, and, for rows cut by top-p alone, the replay of those it could not certify.
 int sample_by_clusters(RowArgs a, const ds41_b200_sample_args &p, cudaStream_t stream) {
@@ -208,7 +210,7 @@ extern "C" int ds41_b200_sample_logits(const ds41_b200_sample_args *p, cudaStrea
   // With scratch: small batches by the cluster kernel alone; larger ones of rows that are only cut by top-p first go through
   // the batch path, which answers the rows it fits and marks the others -8 / -9, and the paths below then only touch those.
   const bool top_p_only = p->top_k == 0 && p->temperature > 0;
-  const int by_clusters = top_p_only ? kClusterRows : p->temperature > 0 ? kClusterRowsTopk : kClusterRowsGreedy;
+  const int by_clusters = top_p_only ? kClusterRows : p->temperature > 0 ? cluster_rows_topk(p->vocab) : kClusterRowsGreedy;
   if (scratch_ok && p->rows <= by_clusters) return sample_by_clusters(a, *p, stream);
   const bool flat = scratch_ok && flat_shape(p->rows, p->vocab) && top_p_only && p->logits_stride != 0;
   // the streaming path covers small nuclei only: a full-vocabulary draw never fits its candidate sets

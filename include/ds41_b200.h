@@ -155,7 +155,7 @@ typedef struct ds41_b200_sample_args {
   int32_t *status;            /* [rows] out, see above; may be NULL */
   void *scratch;              /* optional device scratch of ds41_b200_sample_scratch_bytes(rows, vocab) bytes, 16-byte
                                  aligned.  With it, larger batches of rows without penalties / bitmask and with
-                                 top_k <= 64 (more than 48 rows cut by top-p, 256 by top-k, 64 greedy) take a
+                                 top_k <= 64 (more than 48 rows cut by top-p, 80 to 256 by top-k, 64 greedy) take a
                                  batch-parallel path before the cluster kernel: without top_k (vocab >= 16384)
                                  grid-wide kernels (histogram, window, FP64 masses, resolve), otherwise the streaming
                                  path (chunk records + a per-row combine).  Rows these cannot take, smaller batches and
