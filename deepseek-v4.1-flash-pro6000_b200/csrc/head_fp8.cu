@@ -350,25 +350,30 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     };
     auto flush_stats = [&](int bt_of) {
       const int m = bt_of * kRows + row;
-      if (stats_on && st_id != 0x7fffffff && row < kRows && m < p.M) {
+      if (stats_on && row < kRows && m < p.M) {
         auto ordered = [](float v) {
           const uint32_t bits = __float_as_uint(v == 0.f ? 0.f : v);  // -0 and +0 are the same logit
           return bits ^ ((bits >> 31) ? 0xffffffffu : 0x80000000u);
         };
         const unsigned long long key = (unsigned long long)(ordered(st_best)) << 32 |
                                        (0xffffffffu - uint32_t(st_id + p.col_offset));
+        const bool any = st_id != 0x7fffffff, bad = st_bad + st_bad1 != 0.f;   // (only NaN and -inf: no maximum, but the flag)
         if (p.owner_stats_offset) {
           const int owner = m / p.rows_per_owner;
           HeadRowStats *rs = reinterpret_cast<HeadRowStats *>(reinterpret_cast<unsigned char *>(p.owner_base[owner]) +
                                                               p.owner_stats_offset) + (m - owner * p.rows_per_owner);
-          atomicMax_system(&rs->max_key, key);
-          atomicMax_system(&rs->min_key, ~ordered(st_low));
-          if (st_bad + st_bad1 != 0.f) atomicOr_system(&rs->flags, 1u);
+          if (any) {
+            atomicMax_system(&rs->max_key, key);
+            atomicMax_system(&rs->min_key, ~ordered(st_low));
+          }
+          if (bad) atomicOr_system(&rs->flags, 1u);
         } else {
           HeadRowStats *rs = p.row_stats + m;
-          atomicMax(&rs->max_key, key);
-          atomicMax(&rs->min_key, ~ordered(st_low));
-          if (st_bad + st_bad1 != 0.f) atomicOr(&rs->flags, 1u);
+          if (any) {
+            atomicMax(&rs->max_key, key);
+            atomicMax(&rs->min_key, ~ordered(st_low));
+          }
+          if (bad) atomicOr(&rs->flags, 1u);
         }
       }
       st_best = -CUDART_INF_F; st_low = CUDART_INF_F; st_bad = st_bad1 = 0.f; st_id = 0x7fffffff;

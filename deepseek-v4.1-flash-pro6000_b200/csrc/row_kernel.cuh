@@ -358,9 +358,13 @@ __device__ __forceinline__ bool row_body(const RowArgs &a, RowCtx &c, RowSmem *s
     const FlatMap b = make_map(m, clipped ? __fsub_rn(m, a.reach) : low, a.log2e_t);
     s->map.scale = b.scale; s->map.kappa = b.kappa; s->map.ok = b.ok ? 1 : 0; s->map.clipped = clipped ? 1 : 0;
   };
-  const bool known = a.head_stats != nullptr && !penalised && !a.mask && t > 0 && a.top_k == 0 && c.vocab > kListCap;
+  bool known = a.head_stats != nullptr && !penalised && !a.mask && t > 0 && a.top_k == 0 && c.vocab > kListCap;
+  HeadRowStats h{};
+  if (known) {                         // the same in every thread of the cluster
+    h = a.head_stats[row];
+    known = (__float_as_uint(unorder_bits(uint32_t(h.max_key >> 32))) & 0x7f800000u) != 0x7f800000u;   // else the logits decide
+  }
   if (known && c.tid == 0) {           // the head left the row's extremes (whether the slices landed comes with the sums)
-    const HeadRowStats h = a.head_stats[row];
     const float m = unorder_bits(uint32_t(h.max_key >> 32)), low = unorder_bits(~h.min_key);
     s->facts.max_logit = m; s->facts.lowest = low; s->facts.best_id = int(0xffffffffu - uint32_t(h.max_key));
     s->facts.flags = int(h.flags & 1u); s->facts.allowed = c.vocab; s->facts.cutoff = -CUDART_INF_F;

@@ -212,6 +212,37 @@ def test_row_extremes_from_the_head(pkg, oracle, M):
     assert st2[M // 2] == -1 and tok2[M // 2] == -1 and (np.delete(st2, M // 2) == 0).all()
 
 
+@pytest.mark.parametrize("kind", ["nan", "-inf"])
+@pytest.mark.parametrize("M", [1, 8, 48, 49, 130])   # the last two: the batch path, and the head's 256-column tiles
+def test_row_without_any_usable_logit(pkg, M, kind):
+    """A row of nothing but NaN, or nothing but -inf, leaves no maximum in the head's record; its flag still says that it is
+    not finite, and the sampler rejects it as it does without the records."""
+    N, K = 129280, 128
+    g = torch.Generator(device="cuda").manual_seed(5 + M)
+    code = torch.randint(0x30, 0x50, (N, K), device="cuda", generator=g, dtype=torch.int32).to(torch.uint8)   # positive e4m3
+    ws = torch.full((N // 128, 1), 0.01, device="cuda")
+    a = torch.randint(0xB0, 0xD0, (M, K), device="cuda", generator=g, dtype=torch.int32).to(torch.uint8)      # negative: every dot is
+    a_scale = torch.full((M, 1), 0.05, device="cuda")
+    bad = M // 2
+    a_scale[bad] = float("nan") if kind == "nan" else float("inf")
+    ext = torch.full((M, 16), 0xAB, dtype=torch.uint8, device="cuda")
+    logits = pkg.head_fp8(a, a_scale, code, ws, row_extremes=ext)
+    torch.cuda.synchronize()
+    row = logits[bad]
+    assert bool(torch.isnan(row).all() if kind == "nan" else (row == -float("inf")).all())
+    flags = ext.cpu().numpy().view(np.uint32).reshape(M, 4)[:, 3]
+    seeds, steps = np.arange(M) + 3, np.arange(M) + 9
+    tok, st, _ = sample(pkg, logits, 0.7, 0.95, seeds, steps, row_extremes=ext)
+    ref, rst, _ = sample(pkg, logits, 0.7, 0.95, seeds, steps)
+    assert st[bad] == -1 and tok[bad] == -1 and rst[bad] == -1
+    assert (tok == ref).all() and (st == rst).all() and (np.delete(st, bad) == 0).all()
+    assert flags[bad] == 1 and (np.delete(flags, bad) == 0).all()
+    # a record without a maximum is not trusted, whatever its flag says
+    ext[bad] = 0
+    tok, st, _ = sample(pkg, logits, 0.7, 0.95, seeds, steps, row_extremes=ext)
+    assert (tok == ref).all() and (st == rst).all()
+
+
 @pytest.mark.parametrize("case", range(8))
 def test_random_shapes_agree_with_cluster_kernel(pkg, case):
     """Randomised distributions (scale, offset, tails), temperatures and top-p: the batch path and the cluster kernel are
