@@ -55,7 +55,7 @@ __device__ __forceinline__ float4 load4(const float *p, bool aligned) {
   return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
 }
 __device__ __forceinline__ bool row_aligned(const float *x) { return (reinterpret_cast<uintptr_t>(x) & 15u) == 0; }
-// The row is not decided here: -8 / -9 for the kernels behind (see flat.cuh), -1 for good.
+// The row is not decided here: kNotCovered / kNeedsCluster for the kernels behind, -1 for good.
 __device__ __forceinline__ void leave_row(const FlatArgs &a, int row, int status) {
   if (a.stats) {
     RowStats st{};
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kFlatWindowThreads) flat_window_kernel(FlatArg
       info.w0 = kFlatBins; info.w1 = kFlatBins - 1; info.n_before = a.vocab; info.n_window = 0;
       info.y_sure = -CUDART_INF_F; info.y_tail = CUDART_INF_F;  // every (finite) logit is before the window
       a.s.info[row] = info;
-      if (!usable) { leave_row(a, row, -8); atomicAdd(a.s.pending, 1); }
+      if (!usable) { leave_row(a, row, kNotCovered); atomicAdd(a.s.pending, 1); }
     }
     return;
   }
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kFlatWindowThreads) flat_window_kernel(FlatArg
       info.y_tail = float(double(b.m) - (double(kFlatFrac) * (w1 + 1) + quarter) / double(b.scale));
     }
     a.s.info[row] = info;
-    if (!ok) { leave_row(a, row, -8); atomicAdd(a.s.pending, 1); }
+    if (!ok) { leave_row(a, row, kNotCovered); atomicAdd(a.s.pending, 1); }
   }
 }
 

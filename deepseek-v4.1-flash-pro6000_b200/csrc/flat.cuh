@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
+#include "row_status.h"
 
 namespace ds41 {
 
@@ -20,9 +21,6 @@ constexpr int kFlatMaxParts = 32;   // CTAs per row of the streaming passes: 1, 
 constexpr int kFlatMinRows = 1;
 constexpr int kFlatMinVocab = 16384;
 constexpr double kFlatMaxExponent = 600.0;  // rows whose range * log2(e)/T exceeds this go to the other paths
-// internal status word: this path could not certify the row and its nucleus may be wide; only the cluster kernel may
-// take it (the streaming path's candidate sets never cover such a row).  Never returned to the caller.
-constexpr int kNeedsCluster = -9;
 
 struct FlatPartial { float max, min; int argmax, flags; };
 // Row statistics as the FP8 head's epilogue leaves them (ds41_b200_head_fp8_stats): zero-initialised, then raised with

@@ -4,6 +4,7 @@
 #include "row_core.cuh"
 #include "row_fast.cuh"
 #include "row_nucleus.cuh"
+#include "row_status.h"
 
 namespace ds41 {
 
@@ -583,7 +584,7 @@ __device__ __forceinline__ bool row_body(const RowArgs &a, RowCtx &c, RowSmem *s
 }
 
 // A cluster takes rows cluster, cluster + clusters, ...: one row per cluster when the launch has a cluster per row; a
-// small persistent grid when only the rows another path left over (status -8 / -9) are wanted, so that a launch with
+// small persistent grid when only the rows another path left over (handed_on) are wanted, so that a launch with
 // nothing to do costs a few status reads instead of thousands of cluster launches.
 template <int kMode, int kPerSm>
 __global__ void __launch_bounds__(kThreads, kPerSm) row_kernel(const __grid_constant__ RowArgs a) {
@@ -600,20 +601,19 @@ __global__ void __launch_bounds__(kThreads, kPerSm) row_kernel(const __grid_cons
   for (int row = int(blockIdx.x) / c.nranks; row < a.rows; row += clusters) {
     if (a.only_uncovered) {  // same answer in every CTA of the cluster
       const int st = kMode == kModeSample ? a.status[row] : a.stats[row].status;
-      if (st != -8 && st != -9) continue;  // -9: handed on by the batch path for wide nuclei (flat.cuh)
+      if (!handed_on(st)) continue;
     }
     // no CTA may exit, or stage the next row, while a peer can still address its shared memory
     if (!row_body<kMode>(a, c, s, row)) c.cluster.sync();
     if (c.timed_out) {  // a bounded wait expired: this cluster reports its remaining rows and stops
       if (c.rank == 0 && c.tid == 0) {
         for (int r = row + clusters; r < a.rows; r += clusters) {
-          if (kMode == kModeSample) {
-            if (a.only_uncovered && a.status[r] != -8 && a.status[r] != -9) continue;
-            a.tokens[r] = -1;
-            if (a.status) a.status[r] = -5;
-          } else if (!a.only_uncovered || a.stats[r].status == -8) {
-            a.stats[r].status = -5;
-          }
+          const int before = !a.only_uncovered ? 0 : kMode == kModeSample ? a.status[r] : a.stats[r].status;
+          const int status = after_timeout(before, a.only_uncovered != 0);
+          if (status == before) continue;      // decided in front of this launch
+          if (kMode == kModeStats) a.stats[r].status = status;
+          else a.tokens[r] = -1;
+          if (kMode == kModeSample && a.status) a.status[r] = status;
         }
       }
       break;

@@ -15,6 +15,7 @@
 #pragma once
 #include "row_core.cuh"
 #include "row_fast.cuh"
+#include "row_status.h"
 
 namespace ds41 {
 
@@ -26,7 +27,6 @@ constexpr int kChunkBins = 512;                        // count histogram over d
 constexpr int kChunkList = 256;
 constexpr int kCand = 64;
 constexpr int kMaxRecords = 17;                        // ceil(131072 / 8192) + 1 for uneven shards
-constexpr int kNotCovered = -8;
 
 struct ChunkRecord {  // layout = ds41_b200_shard_row
   double z;           // sum over the chunk's ids of exp((y - max_logit)/T)
