@@ -159,6 +159,7 @@ __global__ void __launch_bounds__(kThreads, 2) verify_rows_fast_kernel(VerifyRow
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ FastVerify f;
   RowSmem *s = reinterpret_cast<RowSmem *>(smem_raw);
+  cluster_announce();
   RowCtx c = make_ctx(s, a.vocab);
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();
@@ -191,7 +192,6 @@ __global__ void __launch_bounds__(kThreads, 2) verify_rows_fast_kernel(VerifyRow
   __syncthreads();
   const int at = f.at, rows = D + 1 + f.checks;
   const int j0 = c.warp * c.region, j1 = min(j0 + c.region, c.len);   // this warp's region of the slice
-  FastVerify *f0 = c.cluster.map_shared_rank(&f, 0);
   // every row's region, 16 bytes a lane where all rows allow it; nothing waits for a row's end
   const bool wide = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(q)) & 15u) == 0 && n % 2 == 0;
   auto region = [&](auto &&one) {
@@ -220,6 +220,8 @@ __global__ void __launch_bounds__(kThreads, 2) verify_rows_fast_kernel(VerifyRow
   bad = __reduce_or_sync(0xffffffffu, bad);
   if (c.lane == 0) f.warp_bad[c.warp] = bad;
   __syncthreads();
+  cluster_await();
+  FastVerify *f0 = c.cluster.map_shared_rank(&f, 0);
   if (c.tid < rows) {
     double total = 0;
     unsigned any = 0;

@@ -282,6 +282,7 @@ __device__ double cross_tile(const Crossing &rec, const double *terms, int have,
 __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   ProbSmem &s = *reinterpret_cast<ProbSmem *>(smem_raw);
+  cluster_announce();
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = int(cluster.block_rank()), ranks = int(cluster.num_blocks());
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = a.vocab;
@@ -290,9 +291,10 @@ __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
   const double top = a.top_p;
   unsigned long long *key = reinterpret_cast<unsigned long long *>(a.scratch + size_t(slot) * size_t(kReplayPad) * 12);
   int *idx = reinterpret_cast<int *>(key + kReplayPad);
-  ProbSmem *s0 = cluster.map_shared_rank(&s, 0);
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();
+  cluster_await();
+  ProbSmem *s0 = cluster.map_shared_rank(&s, 0);
   int parity = 0;
   for (int row = slot; row < a.rows; row += gridDim.x / ranks, parity ^= 1) {
     const float *x = a.logits + size_t(row) * a.stride + begin;

@@ -232,6 +232,13 @@ __device__ __forceinline__ RowCtx make_ctx(RowSmem *s, int vocab) {
   return c;
 }
 
+// A CTA's shared memory may be touched by another CTA only once that CTA has started, that is behind some barrier of the whole
+// cluster.  Kernels whose first access has none in front of it anyway announce their CTAs and await the others (all threads; the
+// arrival orders no memory, and a wait costs about 0.7 us even where everybody has long arrived: 256 constrained rows 207 -> 212
+// us with one in row_kernel, which therefore starts with an exchange that reads).
+__device__ __forceinline__ void cluster_announce() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_await() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+
 // All-gather of one Slot per CTA.  Every thread of the CTA must pass the same `mine`.  Two buffers alternate, so a
 // fast CTA's next exchange cannot overwrite values a slower CTA is still reading (a third exchange can only start
 // after the second one's cluster barrier, which every CTA reaches after it has finished reading the first).
@@ -241,6 +248,17 @@ __device__ __forceinline__ const Slot *exchange(RowCtx &c, const Slot &mine) {
   if (c.tid < c.nranks) *c.cluster.map_shared_rank(&buf[c.rank], c.tid) = mine;
   c.cluster.sync();
   return buf;
+}
+// The same for the first exchange of a row, which no barrier of the cluster may lie in front of: every CTA leaves its slot (of
+// thread 0) in its own shared memory, and lane r of warp 0 receives CTA r's by reading it behind the barrier.
+__device__ __forceinline__ Slot exchange_by_reading(RowCtx &c, const Slot &mine) {
+  Slot *at = &c.s->exch[c.xphase & 1][0];
+  ++c.xphase;
+  if (c.tid == 0) *at = mine;
+  c.cluster.sync();
+  Slot got{};
+  if (c.tid < c.nranks) got = *c.cluster.map_shared_rank(at, c.tid);
+  return got;
 }
 
 // Block-wide reductions in a fixed order (bitwise reproducible run to run).  Result returned to every thread.

@@ -470,14 +470,13 @@ __device__ __forceinline__ bool row_body(const RowArgs &a, RowCtx &c, RowSmem *s
     Slot mine{};                           // (warp 0 has the CTA's values, and is the one that exchange() writes from)
     mine.q[0] = (unsigned long long)top << 32 | unsigned(c.begin + id);
     mine.i[0] = int(low_bits); mine.i[1] = flags; mine.i[2] = count; mine.i[3] = int(threshold);
-    const Slot *all = exchange(c, mine);   // (its barrier also separates the reads above from the next use of red_*)
+    const Slot its = exchange_by_reading(c, mine);   // (its barrier also separates the reads above from the next use of red_*)
     if (c.warp == 0) {
-      const int r = c.lane & (kMaxCluster - 1);
       const bool in = c.lane < c.nranks;
-      top = in ? uint32_t(all[r].q[0] >> 32) : 0u; id = in ? int(uint32_t(all[r].q[0])) : 0x7fffffff;
-      low_bits = in ? uint32_t(all[r].i[0]) : 0xffffffffu;
-      flags = in ? all[r].i[1] : 0; count = in ? all[r].i[2] : 0;
-      threshold = in ? uint32_t(all[r].i[3]) : 0u;
+      top = uint32_t(its.q[0] >> 32); id = in ? int(uint32_t(its.q[0])) : 0x7fffffff;
+      low_bits = in ? uint32_t(its.i[0]) : 0xffffffffu;
+      flags = its.i[1]; count = its.i[2];
+      threshold = uint32_t(its.i[3]);
       warp_reduce();                       // (ids ascend with the rank: the first maximum keeps ties)
       if (sampled) {                       // the groups-th largest threshold: that many CTAs hold their share above it
         for (int g = 1; g < threshold_groups(c); ++g) {
@@ -506,6 +505,8 @@ __device__ __forceinline__ bool row_body(const RowArgs &a, RowCtx &c, RowSmem *s
   else if (flags & 4) status = -7;
   else if (flags & 2) status = -3;
   else if (allowed == 0) status = -2;
+  // With the head's record nothing has been exchanged yet: where the histogram's barrier will not come first either, one here.
+  if (known && (status != 0 || a.top_p >= 1.0 || !s->map.ok)) c.cluster.sync();
 
   Cut cut{-CUDART_INF_F, -1};
   int entered = allowed, kept = allowed;

@@ -86,6 +86,7 @@ __device__ __forceinline__ void score_slice(const float *x, int begin, int end, 
 
 __global__ void __launch_bounds__(kScoreThreads) score_kernel(ds41_b200_score_args a) {
   __shared__ ScoreSmem s;
+  cluster_announce();
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = int(cluster.block_rank()), nranks = int(cluster.num_blocks());
   const int row = int(blockIdx.x) / nranks, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -119,6 +120,7 @@ __global__ void __launch_bounds__(kScoreThreads) score_kernel(ds41_b200_score_ar
     }
     threshold = lo;
   }
+  cluster_await();
   if (tid < nranks) *cluster.map_shared_rank(&s.slots[rank], tid) = ScoreSlot{first, 0.0, threshold, bad_here ? 1 : 0};
   cluster.sync();
   unsigned long long best = ~0ull;

@@ -113,7 +113,9 @@ __global__ void __launch_bounds__(kThreads, 2) verify_kernel(const __grid_consta
   __syncthreads();
   const int at = walk.accepted;
   if (walk.status >= 0 && walk.rejected && !greedy) {
-    // residual draw: inverse CDF over max(0, P - Q) in id order (sampling.cpp:46-50)
+    // residual draw: inverse CDF over max(0, P - Q) in id order (sampling.cpp:46-50).  (Every CTA of the cluster has worked
+    // out the same walk, so all of them come here.)
+    cluster_announce();
     const RowStats sp = ps[at], sq = qs[at];
     const float *xp = target + size_t(at) * a.vocab, *xq = draft + size_t(at) * a.vocab;
     const double log2e_t = kLog2e * inv_t, inv_p = 1.0 / sp.e_kept, inv_q = 1.0 / sq.e_kept;
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(kThreads, 2) verify_kernel(const __grid_consta
       }
     }
     mass = lanes_sum(mass);
+    cluster_await();
     if (c.lane == 0) c.cluster.map_shared_rank(&s->region, 0)->kept[c.rank * kWarps + c.warp] = mass;
     c.cluster.sync();
     if (c.rank == 0) {

@@ -225,6 +225,8 @@ def test_row_without_any_usable_logit(pkg, M, kind):
     a_scale = torch.full((M, 1), 0.05, device="cuda")
     bad = M // 2
     a_scale[bad] = float("nan") if kind == "nan" else float("inf")
+    if M > 1:
+        a[0] = 0   # a row of equal logits: a record, but no range to place the ids on
     ext = torch.full((M, 16), 0xAB, dtype=torch.uint8, device="cuda")
     logits = pkg.head_fp8(a, a_scale, code, ws, row_extremes=ext)
     torch.cuda.synchronize()
@@ -232,9 +234,11 @@ def test_row_without_any_usable_logit(pkg, M, kind):
     assert bool(torch.isnan(row).all() if kind == "nan" else (row == -float("inf")).all())
     flags = ext.cpu().numpy().view(np.uint32).reshape(M, 4)[:, 3]
     seeds, steps = np.arange(M) + 3, np.arange(M) + 9
-    tok, st, _ = sample(pkg, logits, 0.7, 0.95, seeds, steps, row_extremes=ext)
-    ref, rst, _ = sample(pkg, logits, 0.7, 0.95, seeds, steps)
-    assert st[bad] == -1 and tok[bad] == -1 and rst[bad] == -1
+    for top in (1.0, 0.95):
+        tok, st, _ = sample(pkg, logits, 0.7, top, seeds, steps, row_extremes=ext)
+        ref, rst, _ = sample(pkg, logits, 0.7, top, seeds, steps)
+        assert st[bad] == -1 and tok[bad] == -1 and rst[bad] == -1
+        assert (tok == ref).all() and (st == rst).all()
     assert (tok == ref).all() and (st == rst).all() and (np.delete(st, bad) == 0).all()
     assert flags[bad] == 1 and (np.delete(flags, bad) == 0).all()
     # a record without a maximum is not trusted, whatever its flag says

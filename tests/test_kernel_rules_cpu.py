@@ -1,0 +1,88 @@
+"""Rules of the CUDA sources that no run can show to be broken (what they guard against is a race), checked on the text."""
+import os
+import re
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "deepseek-v4.1-flash-pro6000_b200", "csrc")
+
+
+def source(name):
+    return re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+
+
+def braced(text, start):
+    """What stands between the first brace from `start` on and the brace that closes it."""
+    at = begin = text.index("{", start) + 1
+    depth = 1
+    while depth:
+        depth += {"{": 1, "}": -1}.get(text[at], 0)
+        at += 1
+    return text[begin:at - 1]
+
+
+def kernels():
+    """(file, kernel, parameters, body) of every __global__ function."""
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith((".cu", ".cuh")):
+            continue
+        text = source(name)
+        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\s*\(", text):
+            at, depth = m.end(), 1
+            while depth:
+                depth += {"(": 1, ")": -1}.get(text[at], 0)
+                at += 1
+            parameters = text[m.end():at - 1]
+            yield name, m.group(1), parameters, braced(text, at)
+
+
+def test_every_kernel_is_found():
+    found = {k for _, k, _, _ in kernels()}
+    assert len(found) >= 22 and {"row_kernel", "head_fp8_kernel", "verify_rows_fast_kernel", "flat_mass_kernel"} <= found
+    assert sum(source(n).count("__global__") for n in os.listdir(CSRC) if n.endswith((".cu", ".cuh"))) == len(list(kernels()))
+
+
+REMOTE = re.compile(r"map_shared_rank|\bexchange\(c,|\bexchange_by_reading\(|\brow_body\s*<|cluster\.sync\(|\bdraw_region\(|"
+                    r"\bnucleus_row\(|\bfast_small_support\(|\bgeneral_search\(")
+
+
+def test_cluster_kernels_wait_until_every_cta_has_started():
+    """Another CTA's shared memory is touched only behind a barrier of the whole cluster, without which that CTA need not have
+    started: announced, then awaited, in the same block and without a way around it, before the first access."""
+    seen = set()
+    for name, kernel, _, body in kernels():
+        if not re.search(r"make_ctx\(|this_cluster\(", body):
+            assert not REMOTE.search(body), (name, kernel)
+            continue
+        seen.add(kernel)
+        if kernel == "row_kernel":
+            continue                     # the next test
+        assert body.count("cluster_announce();") == 1 and body.count("cluster_await();") == 1, (name, kernel)
+        announced, awaited = body.index("cluster_announce();"), body.index("cluster_await();")
+        assert announced < awaited < REMOTE.search(body).start(), (name, kernel)
+        between = body[announced:awaited]
+        assert "return" not in between and between.count("{") == between.count("}"), (name, kernel)
+        if kernel == "verify_kernel":    # inside the branch that a rejection takes, which holds every access
+            branch = body.index("if (walk.status >= 0 && walk.rejected && !greedy)")
+            assert branch < announced and not REMOTE.search(body.replace(braced(body, branch), "")), kernel
+        else:
+            assert "{" not in body[:announced] and "return" not in body[:announced], (name, kernel)
+    assert seen == {"row_kernel", "verify_kernel", "verify_rows_fast_kernel", "probability_rows_kernel", "score_kernel"}
+
+
+def test_first_exchange_of_a_row_reads():
+    """row_kernel has no barrier of the cluster in front of its rows: a row begins with an exchange in which every CTA writes to
+    its own memory and reads the others' behind the barrier, or, with the head's record, with a plain barrier."""
+    text = source("row_kernel.cuh")
+    body = braced(text, text.index("bool row_body("))
+    calls = [m.group(0) for m in REMOTE.finditer(body)]
+    assert calls[:2] == ["exchange_by_reading(", "cluster.sync("], calls
+    barrier = "if (known && (status != 0 || a.top_p >= 1.0 || !s->map.ok)) c.cluster.sync();"
+    assert body.index("exchange_by_reading(") < body.index(barrier) < body.index("nucleus_row(")
+    assert body.rindex("if (!known) {", 0, body.index("exchange_by_reading(")) > 0
+    text = source("row_nucleus.cuh")     # with a cut, the row's range usable: the histogram's barrier comes first
+    body = braced(text, text.index("NucleusOut nucleus_row("))
+    first = REMOTE.search(body)
+    assert first.group(0) == "cluster.sync(" and "return" not in body[:first.start()].replace("if (!s->map.ok) return out;", "")
+    text = source("row_core.cuh")
+    body = braced(text, text.index("Slot exchange_by_reading("))
+    assert body.index("*at = mine") < body.index("cluster.sync(") < body.index("map_shared_rank")
