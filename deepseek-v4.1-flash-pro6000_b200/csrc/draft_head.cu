@@ -129,9 +129,12 @@ __global__ void __launch_bounds__(kThreads) head_compact_ring_kernel(const float
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  for (int i = 0; i + 1 < stages; ++i) fetch();   // (weights only)
+  if (lane < 4 * kRowsPerWarp && next_group * kRowsPerWarp + (lane >> 2) < N)   // the ring's first weights, 128 bytes per lane and step
+    for (int i = 0; i + 1 < stages && i < steps_per_group; ++i)
+      prefetch_l2(w + size_t(next_group * kRowsPerWarp + (lane >> 2)) * K + i * 256 + (lane & 3) * 64);
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();
+  for (int i = 0; i + 1 < stages; ++i) fetch();
 #pragma unroll 4
   for (int i = threadIdx.x; i < M * K / 4; i += kThreads)
     reinterpret_cast<float4 *>(xs)[activation_slot(i)] = __ldg(reinterpret_cast<const float4 *>(x) + i);
@@ -209,9 +212,10 @@ __global__ void __launch_bounds__(kMarkovThreads, 3) markov_logits_kernel(const 
     for (int r = 0; r < kMarkovRows; ++r)
       wv[r] = __ldg(reinterpret_cast<const uint4 *>(w + size_t(min(first + r, vocab - 1)) * 256) + lane);
   };
-  if (row0 < vocab) fetch(row0);   // (weights only)
+  if (row0 + (lane >> 2) < vocab) prefetch_l2(w + size_t(row0) * 256 + lane * 64);   // the first eight rows, 128 bytes per lane
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();
+  if (row0 < vocab) fetch(row0);
   const uint4 ev = __ldg(reinterpret_cast<const uint4 *>(emb) + lane);
   const float2x e[4] = {promote_bf16x2(ev.x), promote_bf16x2(ev.y), promote_bf16x2(ev.z), promote_bf16x2(ev.w)};
   for (; row0 < vocab; row0 += stride) {

@@ -64,9 +64,11 @@ __global__ void __launch_bounds__(32 * Shape<M>::kMostWarps, 1) head_bf16_kernel
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  for (int i = 0; i + 1 < stages; ++i) fetch();   // (weights only)
+  if (lane < kWarpRows && next_group * kWarpRows + lane < N)   // the ring's first weights, a line of a row per lane and chunk
+    for (int i = 0; i + 1 < stages; ++i) prefetch_l2(w + size_t(next_group * kWarpRows + lane) * K + i * kChunkK);
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();
+  for (int i = 0; i + 1 < stages; ++i) fetch();
   if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
 #pragma unroll 4
     for (int i = threadIdx.x; i < M * K / 4; i += blockDim.x)

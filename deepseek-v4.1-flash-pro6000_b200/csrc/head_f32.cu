@@ -16,8 +16,8 @@ namespace ds41 {
 namespace {
 
 // Every thread has two 16-byte loads per row in flight ahead of the one it works on, 64 KB per SM.  Where an SM has one CTA they
-// run on across the ends of the rows, and the first ones do not wait for the kernel in front of this one: weights are nobody's
-// output.  The shape follows what an SM can hold beside the activations: one row of them leaves room for four small CTAs; up
+// run on across the ends of the rows, and the first ones are on their way to the L2 before the kernel in front of this one has
+// finished.  The shape follows what an SM can hold beside the activations: one row of them leaves room for four small CTAs; up
 // to six rows take one CTA of 32 warps with two weight rows each; more rows, where the shared-memory reads of the activations
 // weigh in, sixteen warps with four weight rows, so that each is used four times.  HBM-bound; 129280 x 5120, us at M = 1 to 8
 // (405 at the rate of a plain copy): 411 432 434 439 422 429 455 491; sixteen warps of four rows throughout 440 443 434 442
@@ -46,10 +46,13 @@ head_f32_kernel(const float *x, const float *__restrict__ w, float *y, int N, in
     if ((fetch_k += 128) >= K && kAcross) { fetch_k = lane * 4; fetch_group += stride; }
   };
   float4 buf[kAhead + 1][kRows];
-#pragma unroll
-  for (int i = 0; i < kAhead; ++i) fetch(buf[i]);
+  if (lane < 4 * kRows && fetch_group * kRows + (lane >> 2) < N)   // the first weights, 128 bytes per lane and step
+    for (int i = 0; i < kAhead && 128 * i < K; ++i)
+      prefetch_l2(w + size_t(fetch_group * kRows + (lane >> 2)) * K + 128 * i + 32 * (lane & 3));
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();
+#pragma unroll
+  for (int i = 0; i < kAhead; ++i) fetch(buf[i]);
   for (int i = threadIdx.x * 4; i < M * K; i += kThreads * 4)
     *reinterpret_cast<float4 *>(xs + i) = *reinterpret_cast<const float4 *>(x + i);
   __syncthreads();

@@ -101,6 +101,13 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, u
       : "memory");
 }
 
+// The same box into the L2 only.
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap *map, int x, int row, int kb, uint64_t policy) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile.L2::cache_hint [%0, {%1, %2, %3}], %4;" ::
+                   "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(row), "r"(kb), "l"(policy)
+               : "memory");
+}
+
 // Shared-memory matrix descriptor, K-major, 128-byte swizzle: rows are 128 bytes apart, groups of 8 rows 1024 bytes
 // apart (stride byte offset), leading byte offset unused (1), descriptor version 1 for sm_100.
 constexpr uint64_t kDescFixed = (uint64_t(1) << 16)              // leading byte offset (>>4), bits [16,30)
@@ -265,13 +272,9 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       uint64_t policy;
       if (b_tiles == 1) asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
       else asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
-      // the ring's first weights do not depend on the kernel in front of this one (the quantiser): they are on their way
-      // while it finishes
-      int early = kblocks / group < kStages ? kblocks / group : kStages;
-      for (int s = 0; s < early; ++s) {
-        mbar_expect_tx(&full[s], uint32_t(stage_bytes));
-        tma_load_3d(tiles + size_t(s) * stage_bytes, &map_w, &full[s], 0, int(blockIdx.x) / b_tiles * kTileN, s * group, policy);
-      }
+      // the ring's first weights are on their way to the L2 while the kernel in front of this one (the quantiser) finishes
+      const int early = kblocks / group < kStages ? kblocks / group : kStages;
+      for (int s = 0; s < early; ++s) tma_prefetch_3d(&map_w, 0, int(blockIdx.x) / b_tiles * kTileN, s * group, policy);
       cudaGridDependencySynchronize();
       cudaTriggerProgrammaticLaunchCompletion();
       for (int tile = blockIdx.x; tile < total_tiles && !ab.set(); tile += gridDim.x) {
@@ -279,12 +282,8 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         for (int kb = 0; kb < kblocks; kb += group) {
           if (!mbar_wait(&empty[stage], phase ^ 1, ab)) break;
           unsigned char *w_dst = tiles + size_t(stage) * stage_bytes, *a_dst = w_dst + w_bytes;
-          if (early > 0) {
-            --early;
-          } else {
-            mbar_expect_tx(&full[stage], uint32_t(stage_bytes));
-            tma_load_3d(w_dst, &map_w, &full[stage], 0, nt * kTileN, kb, policy);
-          }
+          mbar_expect_tx(&full[stage], uint32_t(stage_bytes));
+          tma_load_3d(w_dst, &map_w, &full[stage], 0, nt * kTileN, kb, policy);
           tma_load_3d(a_dst, &map_a, &full[stage], 0, bt * kRows, kb);
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }

@@ -1,8 +1,9 @@
 // Programmatic dependent launch: the kernel's launch and prologue overlap the end of the kernel in front of it in the
-// stream.  Every kernel launched this way calls cudaGridDependencySynchronize() in every CTA, on every path, before it touches
-// what an earlier kernel may have written, and lets the kernel behind it start only after that call; so when a kernel
-// starts early, everything in front of its predecessor has finished, and weights, which no kernel of this library writes,
-// may be read before the call.
+// stream.  Every kernel launched this way calls cudaGridDependencySynchronize() in every CTA, on every path, before it reads or
+// writes anything that another kernel may write or read.  That includes the weights: the kernel in front may be the one that
+// writes them, and may let its successor start long before it has finished.  What comes earlier is set-up on chip and, for the
+// weights, prefetch_l2: a line on its way into the L2 is a copy that later writes replace there, so it hides the memory's
+// latency without fixing what will be read.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -25,6 +26,10 @@ cudaError_t launch_early(void (*kernel)(Params...), int ctas, int threads, size_
   cudaLaunchAttribute attr[1] = {programmatic_launch()};
   cfg.attrs = attr; cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
+__device__ __forceinline__ void prefetch_l2(const void *p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(p)));
 }
 
 }  // namespace ds41

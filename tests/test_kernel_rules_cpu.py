@@ -86,3 +86,41 @@ def test_first_exchange_of_a_row_reads():
     text = source("row_core.cuh")
     body = braced(text, text.index("Slot exchange_by_reading("))
     assert body.index("*at = mine") < body.index("cluster.sync(") < body.index("map_shared_rank")
+
+
+WAIT = "cudaGridDependencySynchronize();"
+
+
+def early_kernels():
+    """The kernels that are launched before the one in front of them has finished (csrc/launch.h)."""
+    names = set()
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh")):
+            names |= set(re.findall(r"\blaunch_early\(\s*(\w+)|\blaunch_clusters<(\w+)>|cudaLaunchKernelEx\(&cfg, (\w+)", source(name)))
+    return {n for group in names for n in group if n} - {"kernel", "score_kernel"}   # (a template's parameter; launched plainly)
+
+
+def without_lambdas(text):
+    """What a text runs by itself: definitions `auto name = [...](...) {...};` are taken out, whose calls stay."""
+    while (m := re.search(r"auto \w+ = \[", text)):
+        text = text[:m.start()] + text[text.index("{", m.start()) + len(braced(text, m.start())) + 2:]
+    return text
+
+
+def test_early_kernels_wait_before_they_touch_global_memory():
+    early = early_kernels()
+    assert {"row_kernel", "head_fp8_kernel", "flat_mass_kernel", "verify_rows_fast_kernel", "replay_sample_kernel"} <= early
+    seen = {}
+    for name, kernel, parameters, body in kernels():
+        if kernel not in early:
+            continue
+        seen[kernel] = name
+        text = without_lambdas(body)
+        assert WAIT in text, (name, kernel)
+        pointers = re.findall(r"\*\s*(?:__restrict__\s*)?(\w+)\s*(?:,|$)", parameters)
+        touch = r"__ldg\(|__ldc|load_input\(|tma_load|cp\.async\.c|\bfetch\(|stage_begin\(|\brow_body|\b[ap]\.\w+\["
+        touch += "".join(rf"|\b{p}\[|(?<!prefetch_l2\()\b{p} \+" for p in pointers)
+        for part in re.split(r"\} else if \(", text) if kernel == "head_fp8_kernel" else [text]:   # (its warps go separate ways)
+            before = part[:part.index(WAIT)] if WAIT in part else ""
+            assert not re.search(touch, before), (name, kernel, re.search(touch, before))
+    assert set(seen) == early, early - set(seen)
