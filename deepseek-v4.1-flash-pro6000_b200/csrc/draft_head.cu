@@ -108,8 +108,8 @@ __global__ void __launch_bounds__(kHeadThreads) head_compact_kernel(const float 
 // the kernel at M = 1 is HBM; a step of two register-held loads ahead left 250-410 us at M = 2..5 (5120 x 129280), because a
 // step's arithmetic is shorter than the memory's latency.
 template <int M, int kRowsPerWarp, int kThreads>
-__global__ void __launch_bounds__(kThreads) head_compact_ring_kernel(const float *__restrict__ x, const __nv_bfloat16 *__restrict__ w,
-                                                                     float *__restrict__ y, int N, int K, int stages) {
+__global__ void __launch_bounds__(kThreads) head_compact_ring_kernel(const float *x, const __nv_bfloat16 *w,
+                                                                     float *y, int N, int K, int stages) {
   extern __shared__ __align__(16) float xs[];  // [M][K], then per warp [stages][kRowsPerWarp][512 bytes]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int kWarpsHere = kThreads / 32, kStage = kRowsPerWarp * 512;
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kThreads) head_compact_ring_kernel(const float
   for (int i = 0; i + 1 < stages; ++i) fetch();
 #pragma unroll 4
   for (int i = threadIdx.x; i < M * K / 4; i += kThreads)
-    reinterpret_cast<float4 *>(xs)[activation_slot(i)] = __ldg(reinterpret_cast<const float4 *>(x) + i);
+    reinterpret_cast<float4 *>(xs)[activation_slot(i)] = load_input(reinterpret_cast<const float4 *>(x) + i);
   __syncthreads();
   int slot = 0;
   for (int g = blockIdx.x * kWarpsHere + warp; g < groups; g += stride) {
@@ -200,23 +200,23 @@ __global__ void __launch_bounds__(kThreads) head_compact_ring_kernel(const float
 // A warp takes eight rows at a time, the next eight on their way while it adds up (one row per warp and 16160 CTAs of eight
 // rows spent more on starting CTAs than on the 66 MB: 19.5 us); the embedding stays in registers.
 constexpr int kMarkovThreads = 256, kMarkovRows = 8;
-__global__ void __launch_bounds__(kMarkovThreads, 3) markov_logits_kernel(const float *__restrict__ u,
-                                                                          const __nv_bfloat16 *__restrict__ w,
-                                                                          const __nv_bfloat16 *__restrict__ emb,
-                                                                          float *__restrict__ out, int vocab) {
+__global__ void __launch_bounds__(kMarkovThreads, 3) markov_logits_kernel(const float *u,
+                                                                          const __nv_bfloat16 *w,
+                                                                          const __nv_bfloat16 *emb,
+                                                                          float *out, int vocab) {
   const int lane = threadIdx.x & 31, stride = (gridDim.x * kMarkovThreads >> 5) * kMarkovRows;
   int row0 = ((blockIdx.x * kMarkovThreads + threadIdx.x) >> 5) * kMarkovRows;
   uint4 wv[kMarkovRows];
   auto fetch = [&](int first) {
 #pragma unroll
     for (int r = 0; r < kMarkovRows; ++r)
-      wv[r] = __ldg(reinterpret_cast<const uint4 *>(w + size_t(min(first + r, vocab - 1)) * 256) + lane);
+      wv[r] = load_input(reinterpret_cast<const uint4 *>(w + size_t(min(first + r, vocab - 1)) * 256) + lane);
   };
   if (row0 + (lane >> 2) < vocab) prefetch_l2(w + size_t(row0) * 256 + lane * 64);   // the first eight rows, 128 bytes per lane
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();
   if (row0 < vocab) fetch(row0);
-  const uint4 ev = __ldg(reinterpret_cast<const uint4 *>(emb) + lane);
+  const uint4 ev = load_input(reinterpret_cast<const uint4 *>(emb) + lane);
   const float2x e[4] = {promote_bf16x2(ev.x), promote_bf16x2(ev.y), promote_bf16x2(ev.z), promote_bf16x2(ev.w)};
   for (; row0 < vocab; row0 += stride) {
     float sum[kMarkovRows];
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(kMarkovThreads, 3) markov_logits_kernel(const 
       for (int r = 0; r < kMarkovRows; ++r) sum[r] = __fadd_rn(sum[r], __shfl_down_sync(0xffffffffu, sum[r], d));
 #pragma unroll
     for (int r = 0; r < kMarkovRows; ++r)
-      if (lane == 0 && row0 + r < vocab) out[row0 + r] = __fadd_rn(__ldg(u + row0 + r), sum[r]);
+      if (lane == 0 && row0 + r < vocab) out[row0 + r] = __fadd_rn(load_input(u + row0 + r), sum[r]);
   }
 }
 
@@ -259,9 +259,9 @@ int rms_geometry(int M, int K, int *width) {
 // The mix and the output run on all 1024 threads, four columns each; the reduction on the first `threads` of them, as the
 // reference's geometry has it.  (With the reference's 256 threads throughout and 2-byte loads a call took 24 us.)
 constexpr int kNormThreads = 1024;
-__global__ void __launch_bounds__(kNormThreads) final_norm_kernel(const __nv_bfloat16 *__restrict__ h, const float *__restrict__ pre,
-                                                                  const __nv_bfloat16 *__restrict__ weight,
-                                                                  float *__restrict__ out, int K, float eps, int width,
+__global__ void __launch_bounds__(kNormThreads) final_norm_kernel(const __nv_bfloat16 *h, const float *pre,
+                                                                  const __nv_bfloat16 *weight,
+                                                                  float *out, int K, float eps, int width,
                                                                   int threads) {
   extern __shared__ __align__(16) unsigned char norm_smem[];
   float *sh = reinterpret_cast<float *>(norm_smem);                        // [512]
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(kNormThreads) final_norm_kernel(const __nv_bfl
                        (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
   auto load4 = [vectors](const __nv_bfloat16 *from, float (&v)[4]) {
     if (vectors) {
-      const uint2 raw = __ldg(reinterpret_cast<const uint2 *>(from));
+      const uint2 raw = load_input(reinterpret_cast<const uint2 *>(from));
       v[0] = __uint_as_float(raw.x << 16); v[1] = __uint_as_float(raw.x & 0xffff0000u);
       v[2] = __uint_as_float(raw.y << 16); v[3] = __uint_as_float(raw.y & 0xffff0000u);
     } else {

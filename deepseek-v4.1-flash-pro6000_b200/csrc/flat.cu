@@ -51,8 +51,8 @@ __device__ __forceinline__ const float *row_logits(const FlatArgs &a, int row) {
 // Four consecutive logits.  Rows of an odd vocabulary start at any 4-byte boundary: four coalesced-enough loads then (a warp's
 // four instructions touch the same lines).
 __device__ __forceinline__ float4 load4(const float *p, bool aligned) {
-  if (aligned) return __ldg(reinterpret_cast<const float4 *>(p));
-  return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+  if (aligned) return load_input(reinterpret_cast<const float4 *>(p));
+  return make_float4(load_input(p), load_input(p + 1), load_input(p + 2), load_input(p + 3));
 }
 __device__ __forceinline__ bool row_aligned(const float *x) { return (reinterpret_cast<uintptr_t>(x) & 15u) == 0; }
 // The row is not decided here: kNotCovered / kNeedsCluster for the kernels behind, -1 for good.
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kFT) flat_stats_kernel(FlatArgs a) {
     const float4 v = load4(x + i, aligned);
     take(v.x, i); take(v.y, i + 1); take(v.z, i + 2); take(v.w, i + 3);
   }
-  for (int i = vec_end + threadIdx.x; i < end; i += kFT) take(__ldg(x + i), i);
+  for (int i = vec_end + threadIdx.x; i < end; i += kFT) take(load_input(x + i), i);
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, o);
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kFT) flat_hist_kernel(FlatArgs a) {
     const float4 v = load4(x + i, aligned);
     take(v.x); take(v.y); take(v.z); take(v.w);
   }
-  for (int k = vec_end + threadIdx.x; k < end; k += kFT) take(__ldg(x + k));
+  for (int k = vec_end + threadIdx.x; k < end; k += kFT) take(load_input(x + k));
   __syncthreads();
   int seen = 0;
   unsigned long long *out = a.s.hist + size_t(row) * kFlatBins;
@@ -314,8 +314,8 @@ __device__ __forceinline__ unsigned mass_sub_region(const float *x, int left, co
     if (kWhole) return load4(mine + 128 * i, aligned);
     const int id = 128 * i + 4 * lane;
     const float none = -CUDART_INF_F;   // beyond the vocabulary: weighs nothing, before nothing
-    return make_float4(id < left ? __ldg(x + id) : none, id + 1 < left ? __ldg(x + id + 1) : none,
-                       id + 2 < left ? __ldg(x + id + 2) : none, id + 3 < left ? __ldg(x + id + 3) : none);
+    return make_float4(id < left ? load_input(x + id) : none, id + 1 < left ? load_input(x + id + 1) : none,
+                       id + 2 < left ? load_input(x + id + 2) : none, id + 3 < left ? load_input(x + id + 3) : none);
   };
   auto consume = [&](const float4 &v, int i) {
     const float y[4] = {v.x, v.y, v.z, v.w};
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(kFlatMassThreads, 6) flat_mass_kernel(FlatArgs
           int slot = buffered + through - count;
           for (; inside; inside &= inside - 1u, ++slot) {
             const int bit = __ffs(inside) - 1, id = base + ((bit >> 2) * 32 + lane) * 4 + (bit & 3);
-            mine.key[slot] = order_key(__ldg(x + id), id);
+            mine.key[slot] = order_key(load_input(x + id), id);
           }
           __syncwarp();
           buffered += total;
@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(kRT4) flat_resolve_kernel(FlatArgs a) {
       y[0] = p.x; y[1] = p.y; y[2] = p.z; y[3] = p.w; y[4] = q.x; y[5] = q.y; y[6] = q.z; y[7] = q.w;
     } else {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) y[i] = id0 + i < a.vocab ? __ldg(x + id0 + i) : -CUDART_INF_F;
+      for (int i = 0; i < 8; ++i) y[i] = id0 + i < a.vocab ? load_input(x + id0 + i) : -CUDART_INF_F;
     }
     double v[8], mine = 0;
     row_weights<8>(y, w, v);

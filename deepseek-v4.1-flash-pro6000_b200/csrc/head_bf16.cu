@@ -72,9 +72,9 @@ __global__ void __launch_bounds__(32 * Shape<M>::kMostWarps, 1) head_bf16_kernel
   if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
 #pragma unroll 4
     for (int i = threadIdx.x; i < M * K / 4; i += blockDim.x)
-      reinterpret_cast<float4 *>(sx)[i] = __ldg(reinterpret_cast<const float4 *>(x) + i);
+      reinterpret_cast<float4 *>(sx)[i] = load_input(reinterpret_cast<const float4 *>(x) + i);
   } else {
-    for (int i = threadIdx.x; i < M * K; i += blockDim.x) sx[i] = __ldg(x + i);
+    for (int i = threadIdx.x; i < M * K; i += blockDim.x) sx[i] = load_input(x + i);
   }
   __syncthreads();
   int slot = 0;

@@ -30,7 +30,7 @@ struct F32Shape {
 
 template <int M>
 __global__ void __launch_bounds__(F32Shape<M>::kThreads, F32Shape<M>::kPerSm)
-head_f32_kernel(const float *x, const float *__restrict__ w, float *y, int N, int K) {
+head_f32_kernel(const float *x, const float *w, float *y, int N, int K) {
   constexpr int kRows = F32Shape<M>::kRows, kThreads = F32Shape<M>::kThreads, kWarps = F32Shape<M>::kWarps;
   constexpr int kAhead = F32Shape<M>::kAhead;
   constexpr bool kAcross = F32Shape<M>::kPerSm == 1;   // (other CTAs cover a row's end)

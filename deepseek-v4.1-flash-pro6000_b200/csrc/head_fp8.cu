@@ -385,7 +385,7 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         asm volatile("bar.sync 1, %0;" ::"n"(kEpiActive) : "memory");  // readers of the previous table are done
         for (int i = et; i < kblocks * kRows; i += kEpiActive) {
           const int r = i / kblocks, kb = i % kblocks, m = bt * kRows + r;
-          sa[kb * kRows + r] = m < p.M ? __ldg(p.a_scale + size_t(m) * kblocks + kb) : 0.f;
+          sa[kb * kRows + r] = m < p.M ? load_input(p.a_scale + size_t(m) * kblocks + kb) : 0.f;
         }
         asm volatile("bar.sync 1, %0;" ::"n"(kEpiActive) : "memory");
         table_bt = bt;
@@ -394,7 +394,7 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       const int w_block = min((nt * kTileN + group * kMyCols) / 128, (p.N + 127) / 128 - 1);
       const float *wsc = p.w_scale + size_t(w_block) * kblocks;
       // copied once per tile: a global load in the loop below, even one that hits, delays the hand-over of each accumulator
-      for (int i = lane; i < kblocks; i += 32) my_sw[i] = __ldg(wsc + i);
+      for (int i = lane; i < kblocks; i += 32) my_sw[i] = load_input(wsc + i);
       __syncwarp();
       float sum[kMyCols];
 #pragma unroll

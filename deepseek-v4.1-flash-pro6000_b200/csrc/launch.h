@@ -28,6 +28,11 @@ cudaError_t launch_early(void (*kernel)(Params...), int ctas, int threads, size_
   return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
 
+// Loads of such data go this way (or are plain): the read-only path (__ldg, const __restrict__ parameters) is only for what nobody
+// writes while the kernel runs, and an early kernel runs while the one in front still writes.
+template <class T>
+__device__ __forceinline__ T load_input(const T *p) { return __ldca(p); }
+
 __device__ __forceinline__ void prefetch_l2(const void *p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(p)));
 }

@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kRT, 1) probability_rows_kernel(ProbArgs a) {
     // the slice, read once; first maximum, minimum (where the order's bucket grid ends), non-finite entries
     float v[kTileIds / 32];
 #pragma unroll
-    for (int r = 0; r < kTileIds / 32; ++r) v[r] = first + 32 * r < len ? __ldg(x + first + 32 * r) : -CUDART_INF_F;
+    for (int r = 0; r < kTileIds / 32; ++r) v[r] = first + 32 * r < len ? load_input(x + first + 32 * r) : -CUDART_INF_F;
     ProbFact f{-CUDART_INF_F, CUDART_INF_F, 0x7fffffff, 0};
 #pragma unroll
     for (int r = 0; r < kTileIds / 32; ++r) {

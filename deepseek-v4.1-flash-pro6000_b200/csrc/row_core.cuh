@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
+#include "launch.h"
 
 namespace ds41 {
 
@@ -369,7 +370,7 @@ __device__ __forceinline__ void stage_begin(RowCtx &c, const float *row, bool &u
     }
   } else {
 #pragma unroll 8
-    for (int j = c.tid; j < c.len; j += kThreads) c.s->y[j] = __ldg(src + j);
+    for (int j = c.tid; j < c.len; j += kThreads) c.s->y[j] = load_input(src + j);
   }
   // the rest of the last regions reads as excluded ids, so that the passes can take four ids at a time
   for (int j = c.len + c.tid; j < c.region * kWarps; j += kThreads) c.s->y[j] = -CUDART_INF_F;

@@ -202,18 +202,18 @@ __device__ __forceinline__ void count_history(RowCtx &c, const int32_t *h, int n
     for (; v + 7 * kThreads < vecs; v += 8 * kThreads) {
       int4 q[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) q[k] = __ldg(h4 + v + k * kThreads);
+      for (int k = 0; k < 8; ++k) q[k] = load_input(h4 + v + k * kThreads);
 #pragma unroll
       for (int k = 0; k < 8; ++k) { count(q[k].x); count(q[k].y); count(q[k].z); count(q[k].w); }
     }
     for (; v < vecs; v += kThreads) {
-      const int4 q = __ldg(h4 + v);
+      const int4 q = load_input(h4 + v);
       count(q.x); count(q.y); count(q.z); count(q.w);
     }
     i = vecs << 2;
   }
 #pragma unroll 4
-  for (i += c.tid; i < n; i += kThreads) count(__ldg(h + i));
+  for (i += c.tid; i < n; i += kThreads) count(load_input(h + i));
 }
 
 // The penalties of the ids that occur in the history, on the staged logits; 2 if one is no longer finite (its logit then stays).
@@ -337,7 +337,7 @@ __device__ __forceinline__ bool row_body(const RowArgs &a, RowCtx &c, RowSmem *s
   }
   if (a.mask) {
     const uint32_t *mw = a.mask + size_t(row) * a.mask_stride + (c.begin >> 5);
-    for (int w = c.tid; w < (c.len + 31) / 32; w += kThreads) s->mask_words[w] = __ldg(mw + w);
+    for (int w = c.tid; w < (c.len + 31) / 32; w += kThreads) s->mask_words[w] = load_input(mw + w);
   }
   const bool penalised = a.history != nullptr && (a.repetition != 1.f || a.presence != 0.f || a.frequency != 0.f);
   int hist_len = penalised ? (a.history_len ? a.history_len[row] : int(a.history_stride)) : 0;

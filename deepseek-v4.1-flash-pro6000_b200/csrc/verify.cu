@@ -43,7 +43,7 @@ struct Measure {  // one row's probability measure: P(id) = survives ? exp((x-ma
   RowStats st;
   double inv_t, inv_kept;  // 1/T and 1/e_kept: multiplications instead of divisions (a few ulp, inside bound())
   __device__ __forceinline__ double at(int id) const {
-    const float y = __ldg(x + id);
+    const float y = load_input(x + id);
     return survives(y, id, st.cut) ? exp_nonpos((double(y) - double(st.max_logit)) * inv_t) * inv_kept : 0.0;
   }
   // (a sum of kept weights and one weight: roundings, and the error of a weight of the FP64 passes, kFlatWeightUlps)
@@ -132,11 +132,11 @@ __global__ void __launch_bounds__(kThreads, 2) verify_kernel(const __grid_consta
         const int j = j0 + 128 * (i0 + i);
         const bool in = i0 + i < c.region / 128;
         if (aligned && in && j + 4 <= c.len) {
-          const float4 v = __ldg(reinterpret_cast<const float4 *>(xp + c.begin + j));
+          const float4 v = load_input(reinterpret_cast<const float4 *>(xp + c.begin + j));
           yp[i][0] = v.x; yp[i][1] = v.y; yp[i][2] = v.z; yp[i][3] = v.w;
         } else {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) yp[i][k] = in && j + k < c.len ? __ldg(xp + c.begin + j + k) : -CUDART_INF_F;
+          for (int k = 0; k < 4; ++k) yp[i][k] = in && j + k < c.len ? load_input(xp + c.begin + j + k) : -CUDART_INF_F;
         }
       }
 #pragma unroll 1
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kThreads, 2) verify_kernel(const __grid_consta
         double ep[4], eq[4];
         float z[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) z[k] = y[k] > -CUDART_INF_F && y[k] >= sp.cut.y ? __ldg(xq + id + k) : -CUDART_INF_F;
+        for (int k = 0; k < 4; ++k) z[k] = y[k] > -CUDART_INF_F && y[k] >= sp.cut.y ? load_input(xq + id + k) : -CUDART_INF_F;
         row_weights<4>(y, wp, ep);
         row_weights<4>(z, wq, eq);
 #pragma unroll
@@ -176,8 +176,8 @@ __global__ void __launch_bounds__(kThreads, 2) verify_kernel(const __grid_consta
         double ep[2], eq[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          y[i] = id + i < end ? __ldg(xp + id + i) : -CUDART_INF_F;
-          z[i] = id + i < end ? __ldg(xq + id + i) : -CUDART_INF_F;
+          y[i] = id + i < end ? load_input(xp + id + i) : -CUDART_INF_F;
+          z[i] = id + i < end ? load_input(xq + id + i) : -CUDART_INF_F;
         }
         row_weights<2>(y, wp, ep);
         row_weights<2>(z, wq, eq);

@@ -124,3 +124,21 @@ def test_early_kernels_wait_before_they_touch_global_memory():
             before = part[:part.index(WAIT)] if WAIT in part else ""
             assert not re.search(touch, before), (name, kernel, re.search(touch, before))
     assert set(seen) == early, early - set(seen)
+
+
+def test_no_read_only_loads_of_what_the_kernel_in_front_may_write():
+    """The read-only path is for data that nobody writes while the kernel runs: constants, and the inputs of kernels that are not
+    launched early (the score, the streaming path, the compact head whose activations fill the shared memory)."""
+    early = early_kernels()
+    plain_files = {"score.cu", "stream.cuh"}
+    for name, kernel, parameters, _ in kernels():
+        if kernel in early:
+            assert name not in plain_files and "__restrict__" not in parameters, (name, kernel)
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith((".cu", ".cuh", ".h")) or name in plain_files:
+            continue
+        text = source(name)
+        for _, kernel, _, body in (k for k in kernels() if k[0] == name and k[1] not in early):
+            text = text.replace(body, "")
+        assert set(re.findall(r"__ldg\(([^)]*)\)", text)) <= {"&kExp2Table[n & 63]"}, name
+        assert "ld.global.nc" not in text, name
