@@ -573,8 +573,9 @@ __global__ void quantize_kernel(const __nv_bfloat16 *x, uint8_t *a, float *scale
 }
 
 // Clears the row records before the head raises them.  (A memset would stand between two programmatic launches and wait for
-// the first; this kernel lets the head start at once -- the kernel in front of it has itself waited for everything
-// earlier -- and only finishes after that kernel.)
+// the first.  This kernel lets the head be set up at once, ahead of its own wait: the head touches nothing before this kernel
+// has finished, which it only does after the kernel in front of it.  With the wait first a decode step takes 126.6 us instead
+// of 126.0 at 8 rows, 170.9 instead of 169.9 at 64.)
 __global__ void clear_stats_kernel(HeadRowStats *stats, int rows) {
   cudaTriggerProgrammaticLaunchCompletion();
   cudaGridDependencySynchronize();

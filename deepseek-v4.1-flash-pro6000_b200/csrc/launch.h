@@ -4,6 +4,9 @@
 // writes them, and may let its successor start long before it has finished.  What comes earlier is set-up on chip and, for the
 // weights, prefetch_l2: a line on its way into the L2 is a copy that later writes replace there, so it hides the memory's
 // latency without fixing what will be read.
+// Since every kernel waits for the one in front of it to have finished, which waited likewise, everything in front of a kernel has
+// finished once its own wait returns, whenever each of them let its successor start: most do so right after their wait, the
+// kernel that clears the head's records before it, the last of a call not at all (its end does).
 #pragma once
 #include <cuda_runtime.h>
 

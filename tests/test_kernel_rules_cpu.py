@@ -142,3 +142,13 @@ def test_no_read_only_loads_of_what_the_kernel_in_front_may_write():
             text = text.replace(body, "")
         assert set(re.findall(r"__ldg\(([^)]*)\)", text)) <= {"&kExp2Table[n & 63]"}, name
         assert "ld.global.nc" not in text, name
+
+
+def test_only_the_clearing_kernel_signals_before_its_wait():
+    """csrc/launch.h says which kernels let their successor start when: after their own wait, but for one."""
+    before = set()
+    for _, kernel, _, body in kernels():
+        signal = "cudaTriggerProgrammaticLaunchCompletion();"
+        if signal in body and body.index(signal) < body.index(WAIT):
+            before.add(kernel)
+    assert before == {"clear_stats_kernel"}
