@@ -16,7 +16,6 @@
 #include "launch.h"
 #include "replay.cuh"
 #include "row_kernel.cuh"
-#include "stream_types.cuh"
 #include <cmath>
 
 namespace ds41 {
@@ -24,7 +23,6 @@ namespace ds41 {
 template <int kMode>
 cudaError_t launch_rows(const RowArgs &a, int rows, cudaStream_t stream);
 int cluster_size_for(int vocab);
-int chunks_for(int vocab);
 
 struct VerifyArgs {
   const float *target, *draft;
@@ -220,11 +218,10 @@ namespace {
 // Up to this many rows the cluster kernel takes the statistics in one launch; beyond, the batch path's grid-wide passes do
 // (they need scratch).
 constexpr int kClusterStatRows = 40;
-// [row statistics][room that earlier versions used], rounded up to 16 bytes; the replay's rows follow, then the batch path's
-// scratch
-size_t verify_streaming_bytes(int sequences, int drafts, int vocab) {
-  const size_t rows = size_t(sequences) * size_t(2 * drafts + 1);
-  return (rows * sizeof(RowStats) + rows * chunks_for(vocab) * sizeof(ChunkRecord) + 15) & ~size_t(15);
+// The scratch begins with the row statistics; the replay's rows follow, then the batch path's scratch.
+size_t verify_stats_bytes(int sequences, int drafts) {
+  static_assert(sizeof(RowStats) % 16 == 0, "what follows is aligned");
+  return size_t(sequences) * size_t(2 * drafts + 1) * sizeof(RowStats);
 }
 }  // namespace
 }  // namespace ds41
@@ -234,7 +231,7 @@ using namespace ds41;
 extern "C" size_t ds41_b200_verify_scratch_bytes_for(int sequences, int drafts, int vocab) {
   if (sequences < 1 || drafts < 0 || drafts > 5 || vocab < 1 || vocab > DS41_B200_MAX_VOCAB) return 0;
   const int rows = sequences * (2 * drafts + 1);
-  return verify_streaming_bytes(sequences, drafts, vocab) + verify_replay_scratch_bytes() +
+  return verify_stats_bytes(sequences, drafts) + verify_replay_scratch_bytes() +
          (vocab >= kFlatMinVocab && rows > kClusterStatRows ? flat_scratch_bytes(rows) : 0);
 }
 extern "C" size_t ds41_b200_verify_scratch_bytes(int sequences, int drafts) {
@@ -252,13 +249,13 @@ extern "C" int ds41_b200_verify_logits(const ds41_b200_verify_args *p, cudaStrea
       (p->drafts && (!p->draft_ids || (!p->draft_logits && !greedy))))
     return invalid("verify arguments");
   const size_t stat_rows = size_t(p->sequences) * size_t(2 * p->drafts + 1);
-  if (!p->scratch || p->scratch_bytes < stat_rows * sizeof(RowStats) || (reinterpret_cast<uintptr_t>(p->scratch) & 15u))
+  const size_t stats_bytes = verify_stats_bytes(p->sequences, p->drafts);
+  if (!p->scratch || p->scratch_bytes < stats_bytes || (reinterpret_cast<uintptr_t>(p->scratch) & 15u))
     return invalid("verify scratch too small or misaligned");
   RowStats *pstats = static_cast<RowStats *>(p->scratch);
   RowStats *qstats = pstats + size_t(p->sequences) * (p->drafts + 1);
   // one launch over all target and draft rows (the draft rows' records lie right behind the target rows'), which also
   // draws from every sequence's last target row: the bonus token, should every draft be accepted
-  const size_t streaming_need = verify_streaming_bytes(p->sequences, p->drafts, p->vocab);
   RowArgs a{};
   a.vocab = p->vocab; a.logits_stride = p->vocab;
   a.temperature = p->temperature > 0 ? std::fmax(p->temperature, 1e-5) : 0.0;
@@ -283,7 +280,7 @@ extern "C" int ds41_b200_verify_logits(const ds41_b200_verify_args *p, cudaStrea
     f.stride = p->vocab; f.vocab = p->vocab; f.rows = stat_launch_rows;
     f.t = a.temperature; f.top_p = p->top_p; f.seeds = p->seeds; f.steps = p->steps; f.slot = a.slot; f.purpose = a.purpose;
     f.stats = pstats; f.draw_every = a.draw_every; f.bound_scale = a.bound_scale;
-    void *flat_scratch = static_cast<unsigned char *>(p->scratch) + streaming_need + verify_replay_scratch_bytes();
+    void *flat_scratch = static_cast<unsigned char *>(p->scratch) + stats_bytes + verify_replay_scratch_bytes();
     if ((e = launch_flat(f, flat_scratch, stream)) != cudaSuccess) return int(e);
     a.only_uncovered = 1;      // what it could not take
     a.pending = flat_pending(flat_scratch);
@@ -315,10 +312,10 @@ extern "C" int ds41_b200_verify_logits(const ds41_b200_verify_args *p, cudaStrea
   if (e != cudaSuccess) return int(e);
   // transactions with a certification bit set: redone in the reference's order of operations, when the caller gave
   // the status words and room for two probability rows per CTA (the scratch-free entry point has neither)
-  if (!greedy && p->status && p->scratch_bytes >= streaming_need + verify_replay_scratch_bytes()) {
+  if (!greedy && p->status && p->scratch_bytes >= stats_bytes + verify_replay_scratch_bytes()) {
     VerifyReplayArgs r{p->target_logits, p->draft_logits, p->draft_ids, p->sequences, p->drafts, p->vocab, a.temperature,
                        p->top_p, p->seeds, p->steps, p->results, p->status,
-                       static_cast<unsigned char *>(p->scratch) + streaming_need};
+                       static_cast<unsigned char *>(p->scratch) + stats_bytes};
     e = launch_verify_replay(r, stream);
   }
   return int(e);

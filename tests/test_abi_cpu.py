@@ -94,3 +94,15 @@ def test_argument_checks_need_no_device(pkg):
     assert pkg.sample_scratch_bytes(1024, 129280) > 1024 * 129280 // 32
     assert pkg.fuse_head_fp8_workspace_bytes(4, 100) == 0
     assert lib.ds41_b200_verify_logits_static_max_rows() == 1024
+
+
+def test_verification_scratch_is_what_the_call_uses(pkg):
+    """48 bytes of statistics per logits row and the replay's rows (two CTAs: 28 bytes for each of 131072 ids), beyond 40 rows of at
+    least 16384 ids the batch path's work space too; and no more."""
+    replay = 2 * 131072 * 28
+    flat = lambda rows: rows * (16 + 2048 * 8 + 32 * 16 + 48 + 128 * 16 + 1024 * 8) + 256
+    for sequences, drafts, vocab in [(1, 0, 129280), (1, 5, 129280), (3, 2, 500), (8, 2, 129280), (9, 2, 129280), (32, 2, 131072),
+                                     (100, 5, 16383), (100, 5, 16384)]:
+        rows = sequences * (2 * drafts + 1)
+        want = 48 * rows + replay + (flat(rows) if rows > 40 and vocab >= 16384 else 0)
+        assert pkg.verify_scratch_bytes(sequences, drafts, vocab) == want, (sequences, drafts, vocab)
