@@ -3,7 +3,9 @@
  * Conventions are the reference plugins' own (components/fuse-head/include/ds41/fuse_head.h:8,
  * components/dense/include/ds41/dense.h:8-10, engine/third_party/spark/include/ds41/spark.h:35-36,116-120):
  *   - every tensor argument is DEVICE memory owned by the caller and alive until the stream reaches the call;
- *   - calls only enqueue work on the given stream: no allocation, no synchronisation, no hidden state;
+ *   - calls only enqueue work on the given stream: no allocation, no synchronisation, no hidden state.  A call's kernels may be
+ *     launched while the work in front of them on the stream still runs, but read and write nothing, weights included, before
+ *     all of it has finished: to the caller they are ordered like any others;
  *   - the return value is a cudaError_t as int (0 = enqueued); argument errors return cudaErrorInvalidValue and
  *     leave a message for ds41_spark_error();
  *   - DATA errors (non-finite logits, empty allowed set, impossible draft ...) are reported in band, per row,
@@ -69,7 +71,9 @@ int ds41_b200_head_fp8(const void *a_e4m3, const float *a_scale, const void *w_e
                        cudaStream_t stream);
 /* The same head, which also leaves per-row records (first maximum and its id, minimum, finiteness) of the logits it
  * produced in row_extremes [M] (DS41_B200_ROW_EXTREMES_BYTES each, 16-byte aligned, cleared by the call): pass them to
- * ds41_b200_sample_logits as args->row_extremes and the sampler's batch path skips its own first pass over the logits.
+ * ds41_b200_sample_logits as args->row_extremes and the sampler, in the batch path and for small batches in the cluster
+ * kernel, skips its own first pass over the logits of rows cut by top-p alone.  A row with a non-finite logit has its flag set,
+ * also one that has no maximum at all.
  * No counterpart in the reference (its sampler runs on the host). */
 #define DS41_B200_ROW_EXTREMES_BYTES 16
 int ds41_b200_head_fp8_stats(const void *a_e4m3, const float *a_scale, const void *w_e4m3, const float *w_scale,
@@ -165,7 +169,8 @@ typedef struct ds41_b200_sample_args {
                                  status 0 (the scratch holds the replay's rows too: about 10 MB). */
   size_t scratch_bytes;
   const void *row_extremes;   /* optional: the [rows] records ds41_b200_head_fp8_stats wrote for these logits (16 bytes
-                                 each); the batch path then skips its own maximum / minimum pass.  NULL otherwise. */
+                                 each), used with scratch for rows cut by top-p alone: the sampler then skips its own
+                                 maximum / minimum pass.  NULL otherwise. */
 } ds41_b200_sample_args;
 size_t ds41_b200_sample_scratch_bytes(int rows, int vocab);
 int ds41_b200_sample_logits(const ds41_b200_sample_args *args, cudaStream_t stream);
@@ -205,8 +210,7 @@ int ds41_b200_verify_logits(const ds41_b200_verify_args *args, cudaStream_t stre
  * the reference.  args->scratch and args->scratch_bytes are ignored: the per-row statistics live in a 48 KiB device
  * array built into the library, so sequences*(2*drafts+1) may not exceed
  * ds41_b200_verify_logits_static_max_rows() (1024); larger requests return cudaErrorInvalidValue with a message.
- * Small calls (up to five full-vocabulary rows, e.g. one sequence with two drafts) take the chunk + combine path and
- * keep their 544-byte chunk records in the same array, behind the statistics.
+ * Every row goes through the cluster kernel, and decisions inside the rounding bound keep their status bits.
  * The first call on each device looks up the array's address (make it before any stream capture); no call
  * allocates.  All calls share the array, so calls that could overlap on the GPU must be serialised by the caller. */
 int ds41_b200_verify_logits_static_max_rows(void);
@@ -214,11 +218,13 @@ int ds41_b200_verify_logits_static(const ds41_b200_verify_args *args, cudaStream
 
 /* ---- operators on probability rows: the reference sampler's C ABI on the device ------------------------------------------
  * For callers that keep the reference's own interface (logits -> probability row -> sample / verify:
- * engine/include/ds41/engine.hpp:211-227) instead of the fused calls above.  Every sum runs on one thread in index
- * order, as the reference's host loops do, so for the same probability rows the tokens and accept / reject records are
- * the reference's bit for bit; ds41_b200_probabilities follows ds41_spark_probabilities operation by operation and can
- * differ from the host's rows only in the last place of exp().  One CTA per row or transaction, milliseconds per
- * full-vocabulary row: compatibility and reporting paths, not the decode-rate path.
+ * engine/include/ds41/engine.hpp:211-227) instead of the fused calls above.  Every sum has the roundings of the reference's
+ * one-thread loop in index order (taken in parallel as integer sums inside each binade of the accumulator, or bounded so that
+ * the decision cannot differ), so for the same probability rows the tokens and accept / reject records are the reference's bit
+ * for bit; ds41_b200_probabilities follows ds41_spark_probabilities operation by operation and can differ from the host's rows
+ * only in the last place of exp().  Probability rows and the verification take a cluster of CTAs per row or transaction, tens of
+ * microseconds at the full vocabulary; the verification's undecided and greedy transactions, the sampling and the two gpu_v2
+ * calls one CTA each (a chain over 129280 ids is about 0.13 ms).
  *   ds41_b200_probabilities         <- ds41_spark_probabilities (spark.h:115; sampling.cpp:30-38), temperature floor of
  *                                      the engine adapter (engine/src/sampling.cpp:209-210); non-finite rows: status -1
  *   ds41_b200_sample_probabilities  <- ds41_spark_sample_v2     (spark.h:131; sampling.cpp:12-21,59), row r at the
