@@ -12,7 +12,10 @@
 
 namespace ds41 {
 
-constexpr int kOnePerSm = 96;   // CTAs
+// CTAs of the grids that get one CTA per SM (launch_rows).  One against two per SM, us: 12 rows of eight CTAs 25.8 / 30.3 (top-p) and
+// 11.9 / 14.0 (top-k), 14 rows 26.0 / 30.7, 16 rows 42.6 / 32.3: clusters of eight, which have to lie within one part of the GPU,
+// fill it at 112 to 120 CTAs already; rows of one or two CTAs at 148 (144 CTAs 25.6 / 29.9, 160 46.2 / 37.9).  96 is below both.
+constexpr int kOnePerSm = 96;
 
 int cluster_size_for(int vocab) {
   int n = 1;
@@ -61,7 +64,7 @@ cudaError_t launch_rows(const RowArgs &a, int rows, cudaStream_t stream) {
   }
   // left-over rows only: a persistent grid of two clusters per 8 SMs walks the status words
   const int clusters = a.only_uncovered ? (rows < 74 ? rows : 74) : rows;
-  // A grid that fits the GPU with one CTA per SM gets 128 registers per thread: no spills, and more of a step's loads and
+  // A grid that surely fits the GPU with one CTA per SM gets 128 registers per thread: no spills, and more of a step's loads and
   // FP64 chains in flight.  A larger one is better off with two CTAs per SM, which fill each other's waits at the barriers
   if (clusters * cl <= kOnePerSm) return launch_rows<kMode, 1>(args, clusters, cl, dev, stream);
   return launch_rows<kMode, 2>(args, clusters, cl, dev, stream);
@@ -154,10 +157,15 @@ extern "C" const char *ds41_spark_error(void) { return last_error(); }
 
 namespace {
 // Up to this many rows the cluster kernel takes a batch in one launch; larger ones go through the batch path (top-p alone)
-// or the streaming path (top-k, greedy).  Where the two meet, at 129280 ids: top-p 48 rows 65 us against 75, 64 rows 70
-// against 65; greedy 64 rows 18.5 us against 18.9, 96 rows 27 against 23.  Rows cut by top-k cost the cluster kernel the same at
-// any vocabulary of eight slices, and the streaming path what their ids take to read: 129280 ids 140 rows 71 us against 76, 200
-// rows 100 against 95; 40000 ids 65 rows 31 against 41, 100 rows 50 against 45.
+// or the streaming path (top-k, greedy).  The two constants are drawn for 129280 ids; cluster kernel / other path, us: top-p 48
+// rows 61 / 73, 64 rows 72 / 64 (with the head's records, which spare the batch path a pass: 32 rows 37 / 42, 48 rows 54 / 50);
+// greedy 32 rows 10.0 / 10.6, 64 rows 18 / 15.  With fewer ids they are not where the two meet: the cluster kernel's cost follows
+// its CTAs per row (eight beyond 32768 ids, two beyond 16384, else one), the other path's the ids.  40000 ids: top-p 64 rows
+// 48 / 53, 96 rows 71 / 62; greedy 32 rows 8.8 / 9.0, 48 rows 15 / 11.  16384 and 32768 ids: top-p 192 rows still 39 / 57 and
+// 57 / 65, greedy 128 rows 7.3 / 8.4 and 9.7 / 9.8.
+// Rows cut by top-k cost the cluster kernel the same at any vocabulary of eight slices, and the streaming path what their ids
+// take to read: 129280 ids 140 rows 71 us against 76, 200 rows 100 against 95; 40000 ids 65 rows 31 against 41, 100 rows 50
+// against 45: the limit follows the line through the two.
 constexpr int kClusterRows = 48, kClusterRowsGreedy = 64;
 int cluster_rows_topk(int vocab) { return vocab > 32768 ? 44 + vocab / 1114 : 256; }
 

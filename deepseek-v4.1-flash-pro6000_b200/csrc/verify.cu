@@ -216,7 +216,9 @@ __global__ void __launch_bounds__(kThreads, 2) verify_kernel(const __grid_consta
 namespace ds41 {
 namespace {
 // Up to this many rows the cluster kernel takes the statistics in one launch; beyond, the batch path's grid-wide passes do
-// (they need scratch).
+// (they need scratch).  Whole calls with either, us: 129280 ids 40 rows 56 / 63, 60 rows 68 / 83, 80 rows 90 / 73; 65536 ids 60 rows
+// 56 / 77, 80 rows 77 / 65: they meet at about 70 rows there, and the line lies below.  At 16384 and 32768 ids, one and two CTAs a
+// row, the cluster kernel is ahead up to 160 rows (49 / 63 and 64 / 67).
 constexpr int kClusterStatRows = 40;
 // The scratch begins with the row statistics; the replay's rows follow, then the batch path's scratch.
 size_t verify_stats_bytes(int sequences, int drafts) {
