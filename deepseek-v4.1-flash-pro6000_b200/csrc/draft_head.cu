@@ -362,8 +362,8 @@ cudaError_t launch_compact(const float *x, const void *w, float *y, int N, int K
   // One CTA of sixteen warps per SM (twelve, with 168 registers per thread, from M = 5 on).  Weight rows that share one read of
   // an activation fragment: per 512 bytes of weights and row M * 8 / rows cycles of shared memory, against the 22 cycles they
   // take to arrive: four rows (five at M = 5: 227 to 220 us), or what the registers hold (three at M = 8; five at M = 6 spill:
-  // 392 us).  A ring of 2, 3, 4 or 6 steps, what the activations leave room for.  129280 x 5120, us at M = 1 to 8: 194 190 193
-  // 194 220 257 375 355 (195 190 195 215 286 328 423 515 with the activations' fragments in place, 32 bytes a lane).
+  // 392 us).  A ring of 2, 3, 4 or 6 steps, what the activations leave room for.  129280 x 5120, us at M = 1 to 8: 195 192 194
+  // 196 223 257 353 332 (195 190 195 215 286 328 423 515 with the activations' fragments in place, 32 bytes a lane).
   constexpr int kRing = M == 5 ? 5 : M <= 7 ? 4 : 3, kRingThreads = M <= 4 ? 512 : 384;
   const size_t activations = size_t(M) * K * sizeof(float), step = size_t(kRingThreads / 32) * kRing * 512;
   const int room = int((227 * 1024 - activations) / step);

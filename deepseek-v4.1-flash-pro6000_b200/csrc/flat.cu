@@ -337,7 +337,7 @@ __device__ __forceinline__ unsigned mass_sub_region(const float *x, int left, co
 }
 
 // The FP64 pass: the weight of every id, per 1024-id sub-region the sum over all ids and over the ids before the window; a
-// warp takes a sub-region at a time.  Bound by issue slots (about 33 instructions per id) and by the FP64 and conversion
+// warp takes a sub-region at a time.  Bound by issue slots (38 instructions per id) and by the FP64 and conversion
 // pipes, not by memory.
 __global__ void __launch_bounds__(kFlatMassThreads, 6) flat_mass_kernel(FlatArgs a) {
   __shared__ double table[64];
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(kFlatMassThreads, 6) flat_mass_kernel(FlatArgs
 // One row per CTA of 128 threads (a sub-region each): orders the window's list, certifies the cut, draws.  The list is
 // ordered by bucket: 128 buckets by logit between the window's edges hold one to three ids each, so a count, a prefix sum and
 // a scatter leave only comparisons inside a bucket.  Small CTAs, because a row is a chain of short dependent steps: sixteen
-// rows per SM hide each other's waits (1024 rows in 20 us; 63 us with 512 threads per row and a bitonic sort).
+// rows per SM hide each other's waits (1024 rows in 17 us; 63 us with 512 threads per row and a bitonic sort).
 constexpr int kRT4 = kFlatMassThreads, kRW4 = kRT4 / 32;
 static_assert(kRT4 == kFlatSubs, "one sub-region per thread");
 struct ResolveSmem {

@@ -25,7 +25,7 @@ constexpr int kChunkK = 64, kRowPitch = kChunkK * 2 + 32;   // bytes; the skew k
 // Weight rows per lane, per warp (four lanes each), bytes of a stage (2.5 or 5 KB) and the most warps.  Up to three activation
 // rows twice the warps hide more latency than the second use of an activation saves (M = 1 to 6: 194 197 202 235 261 321 us with
 // two rows per lane, 196 200 208 232 255 252 with four); 129280 rows are 3.9 rounds of 148 SMs x 7 warps x 32 rows, or 14 x 16
-// (eight or sixteen warps: 3.4, the fourth half empty).
+// (eight or sixteen warps: 3.4, the fourth half empty).  With the shapes below, eight calls at a time: 197 200 203 221 253 259.
 template <int M>
 struct Shape {
   static constexpr int kLaneRows = M <= 3 ? 2 : 4, kWarpRows = 8 * kLaneRows, kStageBytes = kWarpRows * kRowPitch;

@@ -20,7 +20,7 @@ namespace {
 // finished.  The shape follows what an SM can hold beside the activations: one row of them leaves room for four small CTAs; up
 // to six rows take one CTA of 32 warps with two weight rows each; more rows, where the shared-memory reads of the activations
 // weigh in, sixteen warps with four weight rows, so that each is used four times.  HBM-bound; 129280 x 5120, us at M = 1 to 8
-// (405 at the rate of a plain copy): 411 432 434 439 422 429 455 491; sixteen warps of four rows throughout 440 443 434 442
+// (405 at the rate of a plain copy): 406 419 422 427 420 425 451 460; sixteen warps of four rows throughout 440 443 434 442
 // 449 450 448 459; CTAs of eight warps with two rows, as many as the activations allow, 405 621 684 688 731 1219 1240 1241.
 template <int M>
 struct F32Shape {

@@ -16,11 +16,12 @@
 // a ring of shared-memory stages, warp 1 issues four K=32 tcgen05.mma per 128-wide K block into one of four TMEM
 // accumulators, sixteen epilogue warps (lane quadrant x 32-column group) pull each finished K block out of TMEM
 // (tcgen05.ld), hand the accumulator back at once, scale and add in fp32 registers.
-// What bounds it (129280 x 4096, us with quantisation and launch): up to 32 rows the weights' 530 MB (88 and 96 against 77 to 81
-// for the copies alone); from 64 rows on the epilogue, whose hand-over of every K block and output of every tile the tensor
-// pipe waits for: 102 at 64, 119 at 128, 198 at 256, 690 at 1024 rows, where the copies alone take 81, 90, 121 and 404.  The
-// issuing warp waits as a whole and elects the lane that issues (108 to 104 at 64 rows against one lane on its own path), the
-// epilogue has the weight scales in shared memory and spends half the instructions on statistics and stores (735 to 690).
+// What bounds it (129280 x 4096, us with quantisation and launch, eight calls at a time at 1965 MHz): up to 32 rows the weights'
+// 530 MB (88 to 93 against 77 to 81 for the copies alone); from 64 rows on the epilogue, whose hand-over of every K block and
+// output of every tile the tensor pipe waits for: 99 at 64, 111 at 128, 187 at 256, 652 at 1024 rows, where the copies alone take
+// 81, 90, 121 and 404 (a sustained run meets the power cap: 125, 213 and 690 to 790).  The issuing warp waits as a whole and elects
+// the lane that issues (108 to 104 at 64 rows against one lane on its own path), the epilogue has the weight scales in shared
+// memory and spends half the instructions on statistics and stores (735 to 690 at 1024 rows, sustained).
 // Every wait is bounded; on expiry the kernel raises *error_flag, frees its TMEM and returns.
 #include "ds41_b200.h"
 #include "flat.cuh"
@@ -474,9 +475,9 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         }
       }
       // Lane l holds row l of the warp's 32 x 32 block.  Written as it is, one store instruction would touch 32 rows with 16
-      // bytes each; butterflies of the 16-byte column groups at lane distances 8 and 16 turn that into 8 rows with 64
-      // contiguous bytes, which the local L2 takes at its full rate, and one more at distance 4 into 4 rows with 128 bytes,
-      // which is what a peer GPU's memory wants to be written with.
+      // bytes each; butterflies of the 16-byte column groups at lane distances 8, 16 and 4 turn that into 4 rows with 128
+      // contiguous bytes, which the local L2 and a peer GPU's memory both want (without the third one, 8 rows of 64 bytes:
+      // 122 us against 119 at 128 rows).
       if (alive) {
         const bool scattered = p.rows_per_owner != 0;
         const bool plain = !scattered && whole && p.ldl % 4 == 0 && (reinterpret_cast<uintptr_t>(p.logits) & 15u) == 0;

@@ -10,7 +10,7 @@
 // host's rows in the last place of exp()).  Probability rows (prob_rows.cuh) and the verification take a cluster per row or
 // transaction; the other calls, and what the verification cannot certify from parallel sums, one CTA that follows the chains
 // (replay_core.cuh).  2 drafts + 3 target rows of 129280 to their verification record: 1475 us with one CTA for everything,
-// 882 with the certified verification, 133 with the clusters for the rows.
+// 882 with the certified verification, 136 with the clusters for the rows.
 #include "ds41_b200.h"
 #include "host_error.h"
 #include "launch.h"

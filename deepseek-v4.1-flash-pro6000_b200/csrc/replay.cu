@@ -8,11 +8,11 @@
 //     ids are ordered by p descending (ties: lower id first, std::stable_sort), mass += p[idx[k++]] while k < n and
 //     mass < top_p, the rest is zeroed and every p[i] divided by mass;
 //   draw (sampling.cpp:18-21): z = sum of p[i] in id order, t = u * z, c += p[i] until t < c.
-// The sums run on one thread, in order, so they round exactly as the reference's do; only exp() itself can differ from
-// the host library's in the last place, which moves a sum by a few 2^-53 relative instead of by vocab * 2^-53.  A
-// decision that is still closer than 16 * 2^-53 to its threshold keeps its status bit; every other replayed row
-// leaves with status 0.  The sums follow the reference's chain of roundings exactly but in parallel (integer prefix sums
-// inside each binade of the accumulator, replay_core.cuh), and the order is never put together: the top-p loop consumes
+// The sums have the roundings of the reference's one-thread loops, in the same order of terms, but are taken in parallel
+// (integer prefix sums inside each binade of the accumulator, replay_core.cuh); only exp() itself can differ from the host
+// library's in the last place, which moves a sum by a few 2^-53 relative instead of by vocab * 2^-53.  A decision that is
+// still closer than 16 * 2^-53 to its threshold keeps its status bit; every other replayed row leaves with status 0.  The
+// order is never put together: the top-p loop consumes
 // whole ranges of the key as integer sums and sorts only the few chunks in which it needs the terms one by one.  A
 // full-vocabulary row costs a little under a millisecond; the parallel bound flags a few rows in 10^5.
 #include "replay_core.cuh"
