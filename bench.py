@@ -46,17 +46,15 @@ DRAFT_SIGMA = 0.30
 NCU_TRAFFIC_PER_ROW = {
     # profiles/sampler_batch_kernels_256rows.md: one launch of each kernel at 256 rows x 129280 fp32 (132.38 MB per
     # pass over the logits), read + written
-    "flat_hist_kernel": 137.8e6 / 256, "flat_window_kernel": 4.23e6 / 256, "flat_mass_kernel": 132.76e6 / 256,
-    "flat_resolve_kernel": 2.40e6 / 256, "row_kernel": 0.07e6 / 256, "replay_sample_kernel": 0.07e6 / 256,
-    # not launched in that capture (the head's epilogue had left the row records): one read of the logits, extrapolated
-    "flat_stats_kernel": 132.38e6 / 256,
+    "flat_stats_kernel": 136.05e6 / 256, "flat_hist_kernel": 140.06e6 / 256, "flat_window_kernel": 4.26e6 / 256,
+    "flat_mass_kernel": 138.37e6 / 256, "flat_resolve_kernel": 2.39e6 / 256, "row_kernel": 0.07e6 / 256,
+    "replay_sample_kernel": 0.07e6 / 256,
 }
-EXTRAPOLATED_TRAFFIC = ("flat_stats_kernel",)
 NCU_TRAFFIC_PER_LAUNCH = {
-    # head_fp8_kernel<64,128>, 64 x 129280 x 4096: 530.38 MB read + 28.19 MB written (profiles/head_fp8_kernel_b64_full_vocab.md)
-    ("cfg2_b64", "head_fp8_kernel"): 558.6e6,
-    # row_kernel<0>, 64 flat rows: 33.195 MB read + 256 B written (profiles/row_kernel_64rows_flat.md); one read per row
-    ("cfg2_b64", "row_kernel"): 33.195e6,
+    # head_fp8_kernel<64,128>, 64 x 129280 x 4096: 530.05 MB read + 7.34 MB written (profiles/head_fp8_kernel_b64_full_vocab.md)
+    ("cfg2_b64", "head_fp8_kernel"): 537.4e6,
+    # row_kernel<0, 2>, 64 flat rows: 34.37 MB read + 0.07 MB written (profiles/row_kernel_64rows_flat.md); one read per row
+    ("cfg2_b64", "row_kernel"): 34.44e6,
 }
 
 
@@ -850,14 +848,11 @@ def main():
                 total = sum(phases.values()) or 1.0
                 top = max(phases, key=phases.get)
                 entry_["kernels"] = {k: {"ms": v, "share": v / total,
-                                         "traffic": ((NCU_TRAFFIC_PER_ROW.get(k) or 0) * rows_here or None) if v > 0.004 else None,
-                                         "traffic_extrapolated": k in EXTRAPOLATED_TRAFFIC}
+                                         "traffic": ((NCU_TRAFFIC_PER_ROW.get(k) or 0) * rows_here or None) if v > 0.004 else None}
                                      for k, v in phases.items()}
                 entry_["dominant_kernel"] = top
                 entry_["traffic"] = sampler_traffic(phases, rows_here)
-                entry_["traffic_note"] = ("per-kernel ncu captures at 256 rows, scaled by rows (streaming kernels)" +
-                                          ("; flat_stats_kernel extrapolated as one read of the logits"
-                                           if phases.get("flat_stats_kernel", 0) > 0.004 else ""))
+                entry_["traffic_note"] = "per-kernel ncu captures at 256 rows, scaled by rows (streaming kernels)"
             per_kernel.append(entry_)
         per_kernel.sort(key=lambda k: -k["kernel_ms"])
         roof = dict(per_kernel[0])

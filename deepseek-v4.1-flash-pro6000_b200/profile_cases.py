@@ -44,6 +44,8 @@ def main():
         blocks = w.view(args.vocab // 128, 128, args.hidden // 128, 128)
         ws = (blocks.abs().amax(dim=(1, 3)) / 448.0).clamp_min(1e-30)
         wq = (blocks / ws[:, None, :, None]).reshape(args.vocab, args.hidden).to(torch.float8_e4m3fn).view(torch.uint8)
+        del w, blocks
+        torch.cuda.empty_cache()   # a capture saves and restores what the process holds on the device
         a, a_scale = pkg.quantize_activations(x)
         flag = torch.zeros(1, dtype=torch.int32, device=dev)
         logits = torch.empty((rows, args.vocab), dtype=torch.float32, device=dev)
