@@ -1,5 +1,5 @@
 // Types of the sampler's batch path (kernels and launcher in flat.cu): top-p rows without penalties, mask or top-k,
-// decided by four grid-wide kernels over the whole batch.
+// decided by grid-wide kernels over the whole batch.
 #pragma once
 #include <cuda_runtime.h>
 #include <stddef.h>

@@ -68,15 +68,15 @@ def test_static_scratch_matches_caller_scratch_twice(pkg, oracle):
 
 
 @pytest.mark.parametrize("seqs,drafts,vocab,t,top", [
-    (1, 2, 129280, 0.6, 0.95),    # the common decode step: five rows, the chunk + combine path inside the static array
+    (1, 2, 129280, 0.6, 0.95),    # the common decode step: five rows
     (1, 1, 129280, 1.0, 1.0),
     (3, 0, 129280, 0.8, 0.9),     # no drafts: the bonus sample only
     (4, 2, 129280, 0.0, 1.0),     # greedy
     (1, 5, 50000, 0.7, 0.9),
 ])
 def test_static_scratch_small_calls(pkg, oracle, seqs, drafts, vocab, t, top):
-    """Calls small enough for the streaming path keep their chunk records in the built-in array too; the results are
-    those of the call with caller scratch, and a larger call right after still works (no record outlives its call)."""
+    """Small calls, whose statistics lie in the built-in array: the results are those of the call with caller scratch, and a
+    larger call right after still works (no record outlives its call)."""
     t_draw = t if t > 0 else 1.0
     target, draft, ids, seeds, steps = make_inputs(oracle, 70 + seqs + drafts, seqs, max(drafts, 1), vocab, t_draw, top)
     if drafts == 0:
