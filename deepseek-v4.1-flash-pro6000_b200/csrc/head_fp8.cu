@@ -7,21 +7,25 @@
 // group) by the reference's power-of-two rule (dense.cu:8-16) widened to the weight block.  It keeps the plugin
 // conventions of fuse_head.h:8 (caller-owned buffers, stream-ordered, no allocation, no synchronisation).
 //
-// Kernel shape: an output tile is kRows batch rows x 128 vocabulary ids.  The batch rows are the M dimension of
-// tcgen05.mma (one TMEM lane per batch row; M is always 128, the activation tile holds kRows = 16..128 real rows and
-// the lanes beyond them are never read), the 128 vocabulary rows of a weight tile are its N dimension (128 TMEM
-// columns).  With this orientation the combined scale a_scale[m,kb] * w_scale[n/128,kb] of a K block is ONE number
-// per epilogue thread (its batch row; the weight block is the whole tile), so the fp32 promotion of a K block is a
-// register-only loop of fused multiply-adds.  Per CTA: warp 0 streams W and A tiles with TMA (128-byte swizzle) into
-// a ring of shared-memory stages, warp 1 issues four K=32 tcgen05.mma per 128-wide K block into one of four TMEM
-// accumulators, sixteen epilogue warps (lane quadrant x 32-column group) pull each finished K block out of TMEM
-// (tcgen05.ld), hand the accumulator back at once, scale and add in fp32 registers.
-// What bounds it (129280 x 4096, us with quantisation and launch, eight calls at a time at 1965 MHz): up to 32 rows the weights'
-// 530 MB (88 to 93 against 77 to 81 for the copies alone); from 64 rows on the epilogue, whose hand-over of every K block and
-// output of every tile the tensor pipe waits for: 99 at 64, 111 at 128, 187 at 256, 652 at 1024 rows, where the copies alone take
-// 81, 90, 121 and 404 (a sustained run meets the power cap: 125, 213 and 690 to 790).  The issuing warp waits as a whole and elects
-// the lane that issues (108 to 104 at 64 rows against one lane on its own path), the epilogue has the weight scales in shared
-// memory and spends half the instructions on statistics and stores (735 to 690 at 1024 rows, sustained).
+// Two kernels, both persistent: warp 0 streams W and A tiles with TMA (128-byte swizzle) into a ring of shared-memory stages, warp
+// 1 issues four K=32 tcgen05.mma per 128-wide K block, the other warps pull each finished K block out of TMEM (tcgen05.ld), hand
+// its accumulator back at once, scale and add in fp32 registers.
+// * head_fp8_decode_kernel, up to 64 rows: 128 vocabulary ids are the M dimension (TMEM lanes), the 16, 32 or 64 batch rows N.  M is
+//   always 128, so this way an MMA reads and multiplies no row that is not there, and a K block takes the tensor core 160 to 192
+//   cycles instead of 256 (and beside the copies' writes to the same shared memory about 450, which made it the bound: weights
+//   arrive every 700).  A hand-over costs the issuing warp another 100, so that one covers a whole stage of two or four K blocks.
+//   A lane holds one id for all batch rows: a store writes 128 consecutive bytes of a row as it is.  The activation scale is another
+//   one for each column; its product with the weight scale is exact (a power of two), the sums are those of the other kernel.
+//   Eight epilogue warps: sixteen leave 96 registers, too few to have all columns of a stage in flight.
+// * head_fp8_kernel, more rows: the batch rows are the M dimension, 128 or 256 vocabulary ids N: the combined scale
+//   a_scale[m,kb] * w_scale[n/128,kb] of a K block is ONE number per epilogue thread (sixteen warps: lane quadrant x column group).
+// What bounds it (129280 x 4096, us with quantisation and launch; before: with the other kernel for every size): up to 64 rows the
+// weights' 530 MB and the logits (81 to 86 at the measured copy rate): 1 row 78 (88 before), 16 rows 80 (92), 32 rows 83 (95), 64 rows 90
+// (102); with the row records 79, 81, 84 and 98 (90, 95, 97, 105).  From 65 rows on the epilogue, whose hand-over of every K block
+// and output of every tile the tensor pipe waits for: 111 at 128 rows, 187 at 256, 652 at 1024, where the copies alone take 90, 121
+// and 404 (a sustained run meets the power cap: 125, 213 and 690 to 790).  The issuing warp waits as a whole and elects the lane that
+// issues (108 to 104 at 64 rows against one lane on its own path), the epilogue has the weight scales in shared memory and spends
+// half the instructions on statistics and stores (735 to 690 at 1024 rows, sustained).
 // Every wait is bounded; on expiry the kernel raises *error_flag, frees its TMEM and returns.
 #include "ds41_b200.h"
 #include "flat.cuh"
@@ -138,7 +142,7 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t *r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
       "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
@@ -149,7 +153,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
@@ -157,6 +161,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr)
       : "memory");
 }
+
+// Four bytes from global to shared memory without a register; copies_done() waits for all of the thread's.
+__device__ __forceinline__ void copy4_async(float *to, const float *from) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(to)), "l"(__cvta_generic_to_global(from)) : "memory");
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Two fp32 fused multiply-adds in one instruction (fma.rn.f32x2: each half is the same correctly rounded FMA as
 // fmaf): the promotion of a K block is 32 or 64 of them per thread, and the epilogue warps' issue slots are what the
@@ -174,23 +184,29 @@ __device__ __forceinline__ void fma2_acc(float &s0, float &s1, uint32_t d0, uint
   asm("mov.b64 {%0, %1}, %2;" : "=f"(s0), "=f"(s1) : "l"(out));
 }
 
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long v;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+
 // kRows batch rows x kVocab vocabulary ids per output tile (kVocab = UMMA N: 128, or 256 to halve the activation
 // traffic per output element when the batch is large and the kernel is bound by L2 -> shared-memory copies)
 template <int kRows, int kVocab>
 struct HeadSmem {
   static constexpr int kAccBufs = kTmemColumns / kVocab;
   static constexpr int kStageBytes = kVocab * kTileK + kRows * kTileK;
-  // the MMA reads 128 activation rows from every stage; with kRows < 128 the rows beyond the tile belong to the next
-  // stage (or to the pad after the last one) and only feed TMEM lanes nobody reads
-  static constexpr int kPadBytes = (128 - kRows) * kTileK;
+  // The MMA reads 128 activation rows from every stage; with kRows < 128 the rows beyond the tile are the weights behind it (the
+  // activations come first in a stage) and only feed TMEM lanes nobody reads.
+  static_assert(kVocab >= 128 - kRows, "the rows read beyond the activations lie in the stage");
   static constexpr int kMaxStages = 12;
-  // bytes beside the stages: alignment slack, pad, scale tables [K/128][kRows] and [warps][K/128], barriers and flags
+  // bytes beside the stages: alignment slack, scale tables [K/128][kRows] and [warps][2][K/128], barriers and flags
   static constexpr size_t fixed_bytes(int kblocks) {
-    return 1024 + kPadBytes + size_t(kblocks) * (kRows + kEpiWarps) * 4 + (2 * kMaxStages + 2 * kAccBufs) * 8 + 16;
+    return 1024 + size_t(kblocks) * (kRows + 2 * kEpiWarps) * 4 + (2 * kMaxStages + 2 * kAccBufs) * 8 + 16;
   }
   // a stage holds `group` consecutive K blocks (one TMA box per operand)
   static constexpr int stages(int kblocks, int group) {
-    const long long room = 226 * 1024 - (long long)fixed_bytes(kblocks);
+    const long long room = 227 * 1024 - (long long)fixed_bytes(kblocks);
     const int n = room < 0 ? 0 : int(room / (kStageBytes * group));
     return n > kMaxStages ? kMaxStages : n;
   }
@@ -220,6 +236,33 @@ struct HeadArgs {
   int group;             // K blocks per stage: every row of a weight tile is fetched as group*128 contiguous bytes
 };
 
+// Merges a thread's statistics of batch row m into the row's record.  id 0x7fffffff: no maximum (only NaN and -inf seen).
+__device__ __forceinline__ void merge_stats(const HeadArgs &p, int m, float best, int id, float low, bool bad) {
+  auto ordered = [](float v) {
+    const uint32_t bits = __float_as_uint(v == 0.f ? 0.f : v);  // -0 and +0 are the same logit
+    return bits ^ ((bits >> 31) ? 0xffffffffu : 0x80000000u);
+  };
+  const unsigned long long key = (unsigned long long)(ordered(best)) << 32 | (0xffffffffu - uint32_t(id + p.col_offset));
+  const bool any = id != 0x7fffffff;
+  if (p.owner_stats_offset) {
+    const int owner = m / p.rows_per_owner;
+    HeadRowStats *rs = reinterpret_cast<HeadRowStats *>(reinterpret_cast<unsigned char *>(p.owner_base[owner]) +
+                                                        p.owner_stats_offset) + (m - owner * p.rows_per_owner);
+    if (any) {
+      atomicMax_system(&rs->max_key, key);
+      atomicMax_system(&rs->min_key, ~ordered(low));
+    }
+    if (bad) atomicOr_system(&rs->flags, 1u);
+  } else {
+    HeadRowStats *rs = p.row_stats + m;
+    if (any) {
+      atomicMax(&rs->max_key, key);
+      atomicMax(&rs->min_key, ~ordered(low));
+    }
+    if (bad) atomicOr(&rs->flags, 1u);
+  }
+}
+
 template <int kRows, int kVocab>
 __global__ void __launch_bounds__(kHeadThreads, 1)
 head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, HeadArgs p) {
@@ -228,18 +271,18 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   constexpr int kStageBytes = Smem::kStageBytes;
   constexpr int kMaxStages = Smem::kMaxStages;
   const int kStages = p.stages, group = p.group;
-  const int stage_bytes = kStageBytes * group, w_bytes = kTileN * kTileK * group;  // [W g0..][A g0..]
+  const int stage_bytes = kStageBytes * group, a_bytes = kRows * kTileK * group;  // [A g0..][W g0..]
   constexpr uint32_t kTmemCols = kTmemColumns;
   constexpr int kQuads = (kRows + 31) / 32;          // lane quadrants that hold real batch rows
   constexpr int kGroups = 4, kMyCols = kTileN / kGroups;  // 32- or 64-column groups: warp (quadrant q, group g)
   constexpr int kEpiActive = 32 * kQuads * kGroups;  // epilogue threads that take part
   extern __shared__ __align__(1024) unsigned char smem[];
-  // carve: [stages][W tile 16 KB | A tile kRows*128 B], pad, then the activation-scale table, then barriers
+  // carve: [stages][A tiles kRows*128 B | W tiles 16 or 32 KB], then the scale tables, then barriers
   unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~uintptr_t(1023));
-  float *sa = reinterpret_cast<float *>(tiles + size_t(kStages) * stage_bytes + Smem::kPadBytes);  // [K/128][kRows]
+  float *sa = reinterpret_cast<float *>(tiles + size_t(kStages) * stage_bytes);  // [K/128][kRows]
   const int kblocks = p.K / kTileK;
-  float *sw = sa + size_t(kblocks) * kRows;                                                              // [epilogue warp][K/128]
-  uint64_t *bars = reinterpret_cast<uint64_t *>(sw + size_t(kblocks) * kEpiWarps);
+  float *sw = sa + size_t(kblocks) * kRows;                                                              // [epilogue warp][2][K/128]
+  uint64_t *bars = reinterpret_cast<uint64_t *>(sw + size_t(kblocks) * 2 * kEpiWarps);
   uint64_t *full = bars, *empty = bars + kMaxStages, *acc_full = bars + 2 * kMaxStages, *acc_empty = acc_full + kAccBufs;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + kAccBufs);
   int *abort_word = reinterpret_cast<int *>(tmem_slot + 1);
@@ -282,7 +325,7 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         const int nt = tile / b_tiles, bt = tile % b_tiles;
         for (int kb = 0; kb < kblocks; kb += group) {
           if (!mbar_wait(&empty[stage], phase ^ 1, ab)) break;
-          unsigned char *w_dst = tiles + size_t(stage) * stage_bytes, *a_dst = w_dst + w_bytes;
+          unsigned char *a_dst = tiles + size_t(stage) * stage_bytes, *w_dst = a_dst + a_bytes;
           mbar_expect_tx(&full[stage], uint32_t(stage_bytes));
           tma_load_3d(w_dst, &map_w, &full[stage], 0, nt * kTileN, kb, policy);
           tma_load_3d(a_dst, &map_a, &full[stage], 0, bt * kRows, kb);
@@ -301,7 +344,7 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       bool ok = true;
       for (int kb = 0; kb < kblocks && ok; kb += group) {
         if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], phase, ab))) break;
-        uint32_t w16 = tiles16 + stage * stage16, a16 = w16 + (w_bytes >> 4);  // addresses >> 4
+        uint32_t a16 = tiles16 + stage * stage16, w16 = a16 + (a_bytes >> 4);  // addresses >> 4
         for (int g = 0; g < group; ++g) {
           ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[acc], acc_phase ^ 1, ab));
           if (!ok) break;
@@ -331,7 +374,17 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const int row = quad * 32 + lane;   // batch row inside the tile
     const int et = (group * kQuads + quad) * 32 + lane;  // 0..kEpiActive-1
     const uint32_t lane_base = tmem_base + group * kMyCols + (uint32_t(quad * 32) << 16);
-    float *my_sw = sw + size_t(warp - 2) * kblocks;
+    float *my_sw = sw + size_t(warp - 2) * 2 * kblocks;
+    // fp32 scales of the 128-row weight block this warp's columns belong to (a 256-wide tile spans two blocks), on their way into
+    // shared memory
+    auto fetch_scales = [&](int tile, float *to) {
+      if (tile < total_tiles) {
+        const int w_block = min((tile / b_tiles * kTileN + group * kMyCols) / 128, (p.N + 127) / 128 - 1);
+        for (int i = lane; i < kblocks; i += 32) copy4_async(to + i, p.w_scale + size_t(w_block) * kblocks + i);
+      }
+    };
+    fetch_scales(blockIdx.x, my_sw);
+    int which = 0;
     uint32_t acc = 0, acc_phase = 0;
     int table_bt = -1;
     bool alive = true;  // warp-uniform; once false the remaining tiles are walked without waiting or computing,
@@ -350,32 +403,7 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     };
     auto flush_stats = [&](int bt_of) {
       const int m = bt_of * kRows + row;
-      if (stats_on && row < kRows && m < p.M) {
-        auto ordered = [](float v) {
-          const uint32_t bits = __float_as_uint(v == 0.f ? 0.f : v);  // -0 and +0 are the same logit
-          return bits ^ ((bits >> 31) ? 0xffffffffu : 0x80000000u);
-        };
-        const unsigned long long key = (unsigned long long)(ordered(st_best)) << 32 |
-                                       (0xffffffffu - uint32_t(st_id + p.col_offset));
-        const bool any = st_id != 0x7fffffff, bad = st_bad + st_bad1 != 0.f;   // (only NaN and -inf: no maximum, but the flag)
-        if (p.owner_stats_offset) {
-          const int owner = m / p.rows_per_owner;
-          HeadRowStats *rs = reinterpret_cast<HeadRowStats *>(reinterpret_cast<unsigned char *>(p.owner_base[owner]) +
-                                                              p.owner_stats_offset) + (m - owner * p.rows_per_owner);
-          if (any) {
-            atomicMax_system(&rs->max_key, key);
-            atomicMax_system(&rs->min_key, ~ordered(st_low));
-          }
-          if (bad) atomicOr_system(&rs->flags, 1u);
-        } else {
-          HeadRowStats *rs = p.row_stats + m;
-          if (any) {
-            atomicMax(&rs->max_key, key);
-            atomicMax(&rs->min_key, ~ordered(st_low));
-          }
-          if (bad) atomicOr(&rs->flags, 1u);
-        }
-      }
+      if (stats_on && row < kRows && m < p.M) merge_stats(p, m, st_best, st_id, st_low, st_bad + st_bad1 != 0.f);
       st_best = -CUDART_INF_F; st_low = CUDART_INF_F; st_bad = st_bad1 = 0.f; st_id = 0x7fffffff;
     };
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
@@ -391,12 +419,13 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         asm volatile("bar.sync 1, %0;" ::"n"(kEpiActive) : "memory");
         table_bt = bt;
       }
-      // fp32 scale of the 128-row weight block this warp's columns belong to (a 256-wide tile spans two blocks)
-      const int w_block = min((nt * kTileN + group * kMyCols) / 128, (p.N + 127) / 128 - 1);
-      const float *wsc = p.w_scale + size_t(w_block) * kblocks;
-      // copied once per tile: a global load in the loop below, even one that hits, delays the hand-over of each accumulator
-      for (int i = lane; i < kblocks; i += 32) my_sw[i] = load_input(wsc + i);
+      // The next tile's scales are fetched a tile ahead: they come from DRAM, and a load of them between two tiles would keep the
+      // accumulators waiting for longer than the MMAs can run ahead.
+      const float *tile_sw = my_sw + which * kblocks;
+      copies_done();
       __syncwarp();
+      which ^= 1;
+      fetch_scales(tile + gridDim.x, my_sw + which * kblocks);
       float sum[kMyCols];
 #pragma unroll
       for (int c = 0; c < kMyCols; ++c) sum[c] = 0.f;
@@ -404,7 +433,7 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         alive = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], acc_phase, ab));
         if (!alive) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const float scale = sa[kb * kRows + (row < kRows ? row : 0)] * my_sw[kb];
+        const float scale = sa[kb * kRows + (row < kRows ? row : 0)] * tile_sw[kb];
         const unsigned long long scale2 = pack2(scale, scale);
         if constexpr (kMyCols == 32) {
           uint32_t r[32];
@@ -547,6 +576,301 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 }
 
 // ---------------------------------------------------------------------------------------------------------------
+// Batches of up to 64 rows: the weights are the M dimension of the MMA, the batch its N.
+constexpr int kDecodeWarps = 8, kDecodeThreads = 64 + 32 * kDecodeWarps;   // epilogue warps; with TMA and MMA warp
+template <int kRows>
+struct DecodeSmem {
+  static constexpr int kStageBytes = (128 + kRows) * kTileK;
+  static constexpr int kMaxAccs = 16;
+  static constexpr int kMaxGroup = kRows <= 32 ? 4 : 2;                      // K blocks of a stage
+  static constexpr int kMaxStages = 12;
+  // for the statistics an epilogue warp turns its logits, kTurn batch rows at a time, in a block of shared memory (with four batch
+  // rows at a time the 16-row tile's ring still has its third stage)
+  static constexpr int kTurn = kRows == 16 ? 4 : 16, kTurnFloats = 36 * kTurn;
+  // bytes beside the stages: alignment slack, blocks, scale tables [K/128][kRows] and [warps][2][K/128], barriers and flags
+  static constexpr size_t fixed_bytes(int kblocks) {
+    return 1024 + kDecodeWarps * kTurnFloats * 4 + size_t(kblocks) * (kRows + 2 * kDecodeWarps) * 4 +
+           (2 * kMaxStages + 2 * kMaxAccs) * 8 + 16;
+  }
+  static constexpr int stages(int kblocks, int group) {
+    const long long room = 227 * 1024 - (long long)fixed_bytes(kblocks);
+    const int n = room < 0 ? 0 : int(room / (kStageBytes * group));
+    return n > kMaxStages ? kMaxStages : n;
+  }
+};
+
+template <int kN>
+struct Blocks { static constexpr int value = kN; };
+template <int kCols>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t *r) {
+  if constexpr (kCols == 8) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr) : "memory");
+  } else if constexpr (kCols == 16) {
+    tmem_ld16(taddr, r);
+  } else {
+    static_assert(kCols == 32, "8, 16 or 32 columns");
+    tmem_ld32(taddr, r);
+  }
+}
+template <int kRows>
+__global__ void __launch_bounds__(kDecodeThreads, 1)
+head_fp8_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ HeadArgs p) {
+  using Smem = DecodeSmem<kRows>;
+  constexpr int kMaxAccs = Smem::kMaxAccs, kMaxStages = Smem::kMaxStages, kStageBytes = Smem::kStageBytes;
+  constexpr int kCols = kRows / 2;   // batch rows of an epilogue warp: warp = (lane quadrant, half of the batch rows)
+  const int kStages = p.stages, group = p.group;
+  const int accs = min(kMaxAccs, kTmemColumns / (kRows * group));   // sets of accumulators: one per K block of a stage, kRows columns each
+  const int stage_bytes = kStageBytes * group, w_bytes = 128 * kTileK * group;   // [W g0..][A g0..]
+  extern __shared__ __align__(1024) unsigned char smem[];
+  unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~uintptr_t(1023));
+  float *turn = reinterpret_cast<float *>(tiles + size_t(kStages) * stage_bytes);   // [epilogue warp][kTurn][36]
+  float *sa = turn + kDecodeWarps * Smem::kTurnFloats;                              // [K/128][kRows]
+  const int kblocks = p.K / kTileK;
+  float *sw = sa + size_t(kblocks) * kRows;                                         // [epilogue warp][2][K/128]
+  uint64_t *bars = reinterpret_cast<uint64_t *>(sw + size_t(kblocks) * 2 * kDecodeWarps);
+  uint64_t *full = bars, *empty = bars + kMaxStages, *acc_full = bars + 2 * kMaxStages, *acc_empty = acc_full + kMaxAccs;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + kMaxAccs);
+  int *abort_word = reinterpret_cast<int *>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int total_tiles = (p.N + 127) / 128;
+  const int active = p.M > kCols ? 2 : 1;   // halves with a batch row in them
+  Abort ab{abort_word};
+
+  if (threadIdx.x == 0) {
+    *abort_word = 0;
+    for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int b = 0; b < accs; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4 * active); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {  // TMEM allocation by one full warp; the address lands in shared memory
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)), "r"(uint32_t(kTmemColumns)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      uint32_t stage = 0, phase = 0;
+      // every weight is read once per step, and 530 MB of them would push everything else out of the L2 -- the logits, the
+      // activations, the code of the kernels around this one
+      uint64_t policy;
+      asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+      // the ring's first weights are on their way to the L2 while the kernel in front of this one (the quantiser) finishes
+      const int early = kblocks / group < kStages ? kblocks / group : kStages;
+      for (int s = 0; s < early; ++s) tma_prefetch_3d(&map_w, 0, int(blockIdx.x) * 128, s * group, policy);
+      cudaGridDependencySynchronize();
+      cudaTriggerProgrammaticLaunchCompletion();
+      for (int tile = blockIdx.x; tile < total_tiles && !ab.set(); tile += gridDim.x) {
+        for (int kb = 0; kb < kblocks; kb += group) {
+          if (!mbar_wait(&empty[stage], phase ^ 1, ab)) break;
+          unsigned char *w_dst = tiles + size_t(stage) * stage_bytes, *a_dst = w_dst + w_bytes;
+          mbar_expect_tx(&full[stage], uint32_t(stage_bytes));
+          tma_load_3d(w_dst, &map_w, &full[stage], 0, tile * 128, kb, policy);
+          tma_load_3d(a_dst, &map_a, &full[stage], 0, 0, kb);
+          if (++stage == kStages) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer: the warp waits together, one lane issues
+    cudaGridDependencySynchronize();
+    constexpr uint32_t idesc = umma_idesc(kRows);
+    const uint32_t tiles16 = smem_addr(tiles) >> 4, stage16 = uint32_t(stage_bytes) >> 4;
+    const bool leader = elect_one();
+    uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+    for (int tile = blockIdx.x; tile < total_tiles && !__any_sync(0xffffffffu, ab.set()); tile += gridDim.x) {
+      bool ok = true;
+      for (int kb = 0; kb < kblocks && ok; kb += group) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], phase, ab))) break;
+        uint32_t w16 = tiles16 + stage * stage16, a16 = w16 + (uint32_t(w_bytes) >> 4);  // addresses >> 4
+        ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[acc], acc_phase ^ 1, ab));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (leader) {
+          uint32_t d_addr = tmem_base + acc * group * kRows;
+          for (int g = 0; g < group; ++g) {
+            // D[vocabulary id, batch row] (+)= W[vocabulary id, k] * A[batch row, k], K = 32 bytes per instruction
+            umma_f8<false>(d_addr, umma_desc16(w16), umma_desc16(a16), idesc);
+            umma_f8<true>(d_addr, umma_desc16(w16 + 2), umma_desc16(a16 + 2), idesc);
+            umma_f8<true>(d_addr, umma_desc16(w16 + 4), umma_desc16(a16 + 4), idesc);
+            umma_f8<true>(d_addr, umma_desc16(w16 + 6), umma_desc16(a16 + 6), idesc);
+            d_addr += kRows; w16 += (128 * kTileK) >> 4; a16 += (kRows * kTileK) >> 4;
+          }
+          umma_commit(&acc_full[acc]);   // the accumulators of these K blocks are complete
+          umma_commit(&empty[stage]);    // the stage may be refilled: these MMAs have read it
+        }
+        __syncwarp();
+        if (++acc == uint32_t(accs)) { acc = 0; acc_phase ^= 1; }
+        if (++stage == kStages) { stage = 0; phase ^= 1; }
+      }
+    }
+  } else if (((warp - 2) >> 2) < active) {
+    // ------------------------------------------------------------------ epilogue: warp = (lane quadrant, half of the batch rows)
+    cudaGridDependencySynchronize();
+    const int quad = warp & 3;            // TMEM lanes [32*quad, 32*quad+32) are readable by this warp: vocabulary ids
+    const int first = ((warp - 2) >> 2) * kCols, et = threadIdx.x - 64;   // batch rows [first, first + kCols)
+    const int epi_threads = 128 * active;
+    const uint32_t lane_base = tmem_base + first + (uint32_t(quad * 32) << 16);
+    float *my_sw = sw + size_t(warp - 2) * 2 * kblocks;
+    auto fetch_scales = [&](int tile, float *to) {   // the tile's weight scales on their way into shared memory
+      if (tile < total_tiles)
+        for (int i = lane; i < kblocks; i += 32) copy4_async(to + i, p.w_scale + size_t(tile) * kblocks + i);
+    };
+    fetch_scales(blockIdx.x, my_sw);
+    int which = 0;
+    for (int i = et; i < kblocks * kRows; i += epi_threads) {   // activation scales: sa[kb][row]
+      const int r = i / kblocks, kb = i % kblocks;
+      sa[kb * kRows + r] = r < p.M ? load_input(p.a_scale + size_t(r) * kblocks + kb) : 0.f;
+    }
+    asm volatile("bar.sync 1, %0;" ::"r"(epi_threads) : "memory");
+    uint32_t acc = 0, acc_phase = 0;
+    bool alive = true;  // warp-uniform
+    // Statistics: in each turn a lane looks at kTurn consecutive ids of one of kTurn batch rows (tiles come in ascending order, so
+    // a strict comparison keeps the first maximum).
+    constexpr int kTurn = Smem::kTurn, kTurns = kCols / kTurn;
+    float st_best[kTurns], st_low[kTurns], st_bad[kTurns];   // (st_bad: NaN once a logit is NaN or infinite)
+    int st_id[kTurns];
+#pragma unroll
+    for (int h = 0; h < kTurns; ++h) { st_best[h] = -CUDART_INF_F; st_low[h] = CUDART_INF_F; st_id[h] = 0x7fffffff; st_bad[h] = 0.f; }
+    float *my_turn = turn + (warp - 2) * Smem::kTurnFloats;
+    const bool stats_on = p.row_stats != nullptr || p.owner_stats_offset != 0;
+    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
+      // The next tile's scales are fetched a tile ahead: they come from DRAM.
+      const float *tile_sw = my_sw + which * kblocks;
+      copies_done();
+      __syncwarp();
+      which ^= 1;
+      fetch_scales(tile + gridDim.x, my_sw + which * kblocks);
+      float sum[kCols];
+#pragma unroll
+      for (int c = 0; c < kCols; ++c) sum[c] = 0.f;
+      for (int kb = 0; kb < kblocks;) {
+        alive = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], acc_phase, ab));
+        if (!alive) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        auto consume = [&](auto blocks) {   // that many K blocks: all loads in flight together, one wait
+          constexpr int kBlocks = decltype(blocks)::value;
+          const uint32_t taddr = lane_base + acc * kBlocks * kRows;
+          uint32_t r[kBlocks * kCols];
+#pragma unroll
+          for (int u = 0; u < kBlocks; ++u) tmem_ld<kCols>(taddr + u * kRows, r + u * kCols);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          // the values are in registers: the accumulators can be refilled while they are scaled and added
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_empty[acc]);
+#pragma unroll
+          for (int u = 0; u < kBlocks; ++u, ++kb) {
+            const unsigned long long w_scale = pack2(tile_sw[kb], tile_sw[kb]);
+            const ulonglong2 *row_scale = reinterpret_cast<const ulonglong2 *>(sa + kb * kRows + first);
+#pragma unroll
+            for (int c = 0; c < kCols; c += 4) {
+              const ulonglong2 s = row_scale[c >> 2];
+              const uint32_t *d = r + u * kCols + c;
+              fma2_acc(sum[c], sum[c + 1], d[0], d[1], mul2(s.x, w_scale));
+              fma2_acc(sum[c + 2], sum[c + 3], d[2], d[3], mul2(s.y, w_scale));
+            }
+          }
+        };
+        if (Smem::kMaxGroup >= 4 && group == 4) consume(Blocks<Smem::kMaxGroup >= 4 ? 4 : 1>{});
+        else if (group == 2) consume(Blocks<2>{});
+        else consume(Blocks<1>{});
+        if (++acc == uint32_t(accs)) { acc = 0; acc_phase ^= 1; }
+      }
+      if (!alive) break;
+      const int n0 = tile * 128 + 32 * quad, n = n0 + lane;
+      const bool in = n < p.N;
+      // a store instruction writes 128 contiguous bytes of a row
+      int owner = p.rows_per_owner ? first / p.rows_per_owner : 0, left = p.rows_per_owner ? (owner + 1) * p.rows_per_owner - first : kRows;
+      float *dst = p.rows_per_owner ? p.owner_base[owner] + size_t(p.rows_per_owner - left) * p.ldl + p.col_offset + n
+                                    : p.logits + size_t(first) * p.ldl + n;
+#pragma unroll
+      for (int c = 0; c < kCols; ++c, dst += p.ldl) {
+        if (left-- == 0) {              // the next owner's rows (a batch row's buffer exists)
+          if (first + c < p.M) dst = p.owner_base[++owner] + p.col_offset + n;
+          left = p.rows_per_owner - 1;
+        }
+        if (in && first + c < p.M) *dst = sum[c];
+      }
+      if (stats_on) {
+        const int turn_row = lane % kTurn, turn_id = lane / kTurn * kTurn, ids = min(kTurn, p.N - n0 - turn_id);
+#pragma unroll
+        for (int h = 0; h < kTurns; ++h) {
+          __syncwarp();
+#pragma unroll
+          for (int c = 0; c < kTurn; ++c) my_turn[36 * c + lane] = sum[h * kTurn + c];
+          __syncwarp();
+          float v[kTurn];
+#pragma unroll
+          for (int c = 0; c < kTurn; c += 4)
+            *reinterpret_cast<float4 *>(v + c) = *reinterpret_cast<const float4 *>(my_turn + 36 * turn_row + turn_id + c);
+          if (ids < kTurn)             // the last ids of the vocabulary: those beyond it repeat the last one (or are left out)
+#pragma unroll
+            for (int c = 1; c < kTurn; ++c) v[c] = c < ids ? v[c] : v[c - 1];
+          float hi = v[0], low = v[0], bad = st_bad[h];
+#pragma unroll
+          for (int c = 0; c < kTurn; ++c) { hi = fmaxf(hi, v[c]); low = fminf(low, v[c]); bad = fmaf(v[c], 0.f, bad); }
+          if (ids <= 0) { hi = -CUDART_INF_F; low = CUDART_INF_F; bad = st_bad[h]; }
+          st_bad[h] = bad;
+          st_low[h] = fminf(st_low[h], low);
+          if (__any_sync(0xffffffffu, hi > st_best[h])) {
+            int at = 0;
+#pragma unroll
+            for (int c = kTurn - 1; c > 0; --c) at = v[c] == hi ? c : at;
+            if (v[0] == hi) at = 0;
+            if (hi > st_best[h]) { st_best[h] = hi; st_id[h] = n0 + turn_id + at; }
+          }
+        }
+      }
+    }
+    if (stats_on) {
+      // The four lane quadrants' records of a batch row are merged here: all CTAs raise the same few lines at the end.  (The ring is
+      // free: the last accumulators have been waited for.)
+      struct Record { float best, low; int id, bad; };
+      Record *records = reinterpret_cast<Record *>(tiles);   // [quadrant][kRows]
+#pragma unroll
+      for (int h = 0; h < kTurns; ++h) {
+        int bad = st_bad[h] == 0.f ? 0 : 1;
+        for (int o = kTurn; o < 32; o <<= 1) {
+          const float best = __shfl_xor_sync(0xffffffffu, st_best[h], o);
+          const int id = __shfl_xor_sync(0xffffffffu, st_id[h], o);
+          if (best > st_best[h] || (best == st_best[h] && id < st_id[h])) { st_best[h] = best; st_id[h] = id; }
+          st_low[h] = fminf(st_low[h], __shfl_xor_sync(0xffffffffu, st_low[h], o));
+          bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+        }
+        if (alive && lane < kTurn) records[quad * kRows + first + h * kTurn + lane] = Record{st_best[h], st_low[h], st_id[h], bad};
+      }
+      asm volatile("bar.sync 1, %0;" ::"r"(epi_threads) : "memory");
+      if (alive && et < p.M) {
+        Record all = records[et];
+#pragma unroll
+        for (int q = 1; q < 4; ++q) {
+          const Record r = records[q * kRows + et];
+          if (r.best > all.best || (r.best == all.best && r.id < all.id)) { all.best = r.best; all.id = r.id; }
+          all.low = fminf(all.low, r.low);
+          all.bad |= r.bad;
+        }
+        merge_stats(p, et, all.best, all.id, all.low, all.bad != 0);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(uint32_t(kTmemColumns)));
+  }
+  if (threadIdx.x == 0 && *abort_word && p.error_flag) atomicExch(p.error_flag, 1);
+}
+
+// ---------------------------------------------------------------------------------------------------------------
 // Activation quantisation: per (row, 128-wide K group) scale = 2^ceil(log2(max(amax,1e-4)/448)), e4m3 round to
 // nearest even with saturation (components/dense/src/dense.cu:8-16 with the group widened from 32 to 128).
 __global__ void quantize_kernel(const __nv_bfloat16 *x, uint8_t *a, float *scale, int groups) {
@@ -636,6 +960,26 @@ cudaError_t launch_head(const CUtensorMap &mw, const CUtensorMap &ma, const Head
   int grid = tiles < sms ? tiles : sms;
   if (b_tiles <= grid) grid -= grid % b_tiles;  // every CTA then keeps one batch tile (and its scale table) for good
   return launch_early(head_fp8_kernel<kRows, kVocab>, grid, kHeadThreads, smem, stream, mw, ma, q);
+}
+
+template <int kRows>
+cudaError_t launch_decode(const CUtensorMap &mw, const CUtensorMap &ma, const HeadArgs &p, int sms, cudaStream_t stream) {
+  using Smem = DecodeSmem<kRows>;
+  HeadArgs q = p;
+  q.stages = Smem::stages(p.K / kTileK, p.group);
+  if (q.stages < 2) return cudaErrorInvalidValue;
+  const size_t smem = Smem::fixed_bytes(p.K / kTileK) + size_t(q.stages) * Smem::kStageBytes * p.group;
+  static thread_local int configured = -1;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (configured != dev) {
+    e = cudaFuncSetAttribute(head_fp8_decode_kernel<kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return e;
+    configured = dev;
+  }
+  const int tiles = (p.N + 127) / 128;
+  return launch_early(head_fp8_decode_kernel<kRows>, tiles < sms ? tiles : sms, kDecodeThreads, smem, stream, mw, ma, q);
 }
 
 }  // namespace
@@ -733,6 +1077,7 @@ int run_head(const void *a_e4m3, const float *a_scale, const void *w_e4m3, const
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return int(e);
+  constexpr int kDecodeRows = 64;
   const int cols = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
   // Vocabulary tile: 256 wide once the batch spans several tiles (then the kernel is bound by L2 -> shared-memory
   // copies and a wider tile re-reads the activations half as often), else 128.
@@ -742,15 +1087,16 @@ int run_head(const void *a_e4m3, const float *a_scale, const void *w_e4m3, const
   const int kblocks = K / kTileK;
   auto ring = [&](int g) {
     return vocab_tile == 256 ? HeadSmem<128, 256>::stages(kblocks, g)
-         : cols == 16 ? HeadSmem<16, 128>::stages(kblocks, g) : cols == 32 ? HeadSmem<32, 128>::stages(kblocks, g)
-         : cols == 64 ? HeadSmem<64, 128>::stages(kblocks, g) : HeadSmem<128, 128>::stages(kblocks, g);
+         : cols == 16 ? DecodeSmem<16>::stages(kblocks, g) : cols == 32 ? DecodeSmem<32>::stages(kblocks, g)
+         : cols == 64 ? DecodeSmem<64>::stages(kblocks, g) : HeadSmem<128, 128>::stages(kblocks, g);
   };
   int group = 1;
-  for (int g = 4; g > 1; g >>= 1)
+  const int most = M > kDecodeRows || cols <= 32 ? 4 : 2;
+  for (int g = most; g > 1; g >>= 1)
     if (kblocks % g == 0 && ring(g) >= 2) { group = g; break; }
   if (const char *forced = getenv("DS41_HEAD_GROUP")) {
     const int g = atoi(forced);
-    if ((g == 1 || g == 2 || g == 4) && kblocks % g == 0 && ring(g) >= 2) group = g;
+    if ((g == 1 || g == 2 || g == 4) && g <= most && kblocks % g == 0 && ring(g) >= 2) group = g;
   }
   p.group = group;
   CUtensorMap mw, ma;
@@ -758,11 +1104,11 @@ int run_head(const void *a_e4m3, const float *a_scale, const void *w_e4m3, const
       !make_map(&ma, a_e4m3, uint64_t(M), uint64_t(K), uint32_t(cols), uint32_t(group)))
     return invalid("cuTensorMapEncodeTiled failed");
   if (vocab_tile == 256) return int(launch_head<128, 256>(mw, ma, p, sms, stream));
+  if (M > kDecodeRows) return int(launch_head<128, 128>(mw, ma, p, sms, stream));
   switch (cols) {
-    case 16: e = launch_head<16, 128>(mw, ma, p, sms, stream); break;
-    case 32: e = launch_head<32, 128>(mw, ma, p, sms, stream); break;
-    case 64: e = launch_head<64, 128>(mw, ma, p, sms, stream); break;
-    default: e = launch_head<128, 128>(mw, ma, p, sms, stream); break;
+    case 16: e = launch_decode<16>(mw, ma, p, sms, stream); break;
+    case 32: e = launch_decode<32>(mw, ma, p, sms, stream); break;
+    default: e = launch_decode<64>(mw, ma, p, sms, stream); break;
   }
   return int(e);
 }
