@@ -7,25 +7,31 @@
 // group) by the reference's power-of-two rule (dense.cu:8-16) widened to the weight block.  It keeps the plugin
 // conventions of fuse_head.h:8 (caller-owned buffers, stream-ordered, no allocation, no synchronisation).
 //
-// Two kernels, both persistent: warp 0 streams W and A tiles with TMA (128-byte swizzle) into a ring of shared-memory stages, warp
-// 1 issues four K=32 tcgen05.mma per 128-wide K block, the other warps pull each finished K block out of TMEM (tcgen05.ld), hand
-// its accumulator back at once, scale and add in fp32 registers.
+// Three kernels, all persistent: a warp streams W and A tiles with TMA (128-byte swizzle) into a ring of shared-memory stages, one
+// issues four K=32 tcgen05.mma per 128-wide K block, the others pull each finished K block out of TMEM (tcgen05.ld), hand its
+// accumulator back at once, scale and add in fp32 registers.
 // * head_fp8_decode_kernel, up to 64 rows: 128 vocabulary ids are the M dimension (TMEM lanes), the 16, 32 or 64 batch rows N.  M is
 //   always 128, so this way an MMA reads and multiplies no row that is not there, and a K block takes the tensor core 160 to 192
 //   cycles instead of 256 (and beside the copies' writes to the same shared memory about 450, which made it the bound: weights
 //   arrive every 700).  A hand-over costs the issuing warp another 100, so that one covers a whole stage of two or four K blocks.
 //   A lane holds one id for all batch rows: a store writes 128 consecutive bytes of a row as it is.  The activation scale is another
-//   one for each column; its product with the weight scale is exact (a power of two), the sums are those of the other kernel.
+//   one for each column; its product with the weight scale is exact (a power of two), the sums are those of the other kernels.
 //   Eight epilogue warps: sixteen leave 96 registers, too few to have all columns of a stage in flight.
-// * head_fp8_kernel, more rows: the batch rows are the M dimension, 128 or 256 vocabulary ids N: the combined scale
-//   a_scale[m,kb] * w_scale[n/128,kb] of a K block is ONE number per epilogue thread (sixteen warps: lane quadrant x column group).
-// What bounds it (129280 x 4096, us with quantisation and launch; before: with the other kernel for every size): up to 64 rows the
-// weights' 530 MB and the logits (81 to 86 at the measured copy rate): 1 row 78 (88 before), 16 rows 80 (92), 32 rows 83 (95), 64 rows 90
-// (102); with the row records 79, 81, 84 and 98 (90, 95, 97, 105).  From 65 rows on the epilogue, whose hand-over of every K block
-// and output of every tile the tensor pipe waits for: 111 at 128 rows, 187 at 256, 652 at 1024, where the copies alone take 90, 121
-// and 404 (a sustained run meets the power cap: 125, 213 and 690 to 790).  The issuing warp waits as a whole and elects the lane that
-// issues (108 to 104 at 64 rows against one lane on its own path), the epilogue has the weight scales in shared memory and spends
-// half the instructions on statistics and stores (735 to 690 at 1024 rows, sustained).
+// * head_fp8_kernel, 65 to 128 rows: the batch rows are the M dimension, 128 ids N: the combined scale
+//   a_scale[m,kb] * w_scale[n/128,kb] of a K block is ONE number per epilogue thread.  (The decode kernel with N = 128 takes 127 to 139
+//   us here instead of 106 to 120: eight warps with 64 columns each, or sixteen without the registers.)
+// * head_fp8_pair_kernel, more rows: the same with a pair of SMs on 256 batch rows x 256 ids (cta_group::2).  Each CTA fetches its own
+//   128 rows of A and half of the ids' rows, 32 KB a K block instead of the 48 KB of a 128 x 256 tile alone, which alone took 404 of
+//   652 us at 1024 rows.  Both CTAs' copies count on the leading CTA's barriers, its one warp issues, and the epilogues of both
+//   hand accumulators back to it.
+// What bounds it (129280 x 4096, us with quantisation and launch; before: with head_fp8_kernel for every size, 128 x 256 tiles from 129
+// rows on): up to 64 rows the weights' 530 MB and the logits (81 to 86 at the measured copy rate): 1 row 78 (88 before), 16 rows
+// 80 (92), 32 rows 83 (95), 64 rows 90 (102); with the row records 79, 81, 84 and 98 (90, 95, 97, 105).  From 65 rows on the epilogue
+// (106 at 65 rows, 120 at 128): beside the MMAs' operands and the copies, which fill the shared memory's bandwidth, every access of the
+// epilogue to it, waits and scales included, takes 100 to 230 cycles.  Run without pause, as in a decode loop, the power cap (about
+// 1.6 GHz) counts as much: 256 rows 168 to 200 (198 to 222 before), 512 rows 342 to 361 (403), 1024 rows 689 to 707 (764 to 778); with the
+// row records 713 to 735 (801 to 810).  The issuing warp waits as a whole and elects the lane that issues (108 to 104 at 64 rows
+// against one lane on its own path).
 // Every wait is bounded; on expiry the kernel raises *error_flag, frees its TMEM and returns.
 #include "ds41_b200.h"
 #include "flat.cuh"
@@ -44,7 +50,7 @@ namespace {
 
 constexpr int kTmemColumns = 512;  // all of an SM's tensor memory: 4 accumulators of 128 columns or 2 of 256
 constexpr int kTileK = 128;   // K elements per block = one 128-byte swizzle row of e4m3
-constexpr int kEpiWarps = 16, kHeadThreads = 64 + 32 * kEpiWarps;
+constexpr int kEpiWarps = 16, kHeadThreads = 64 + 32 * kEpiWarps, kPairThreads = 128 + 32 * kEpiWarps;
 constexpr uint32_t kSpinLimit = 1u << 22;
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return uint32_t(__cvta_generic_to_shared(p)); }
@@ -75,17 +81,26 @@ __device__ __forceinline__ bool mbar_try(uint64_t *bar, uint32_t parity) {
       : "memory");
   return done != 0;
 }
-__device__ __noinline__ bool mbar_wait_slow(uint64_t *bar, uint32_t parity, volatile int *flag) {
-  for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
-    if (mbar_try(bar, parity)) return true;
-    if ((spin & 255u) == 255u && *flag != 0) return false;
-  }
-  *flag = 1;
-  return false;
+// Without waiting at all.
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(done)
+      : "r"(smem_addr(bar)), "r"(parity)
+      : "memory");
+  return done != 0;
 }
+// (In line: around a call the 64 sums of an epilogue thread would be spilled.)
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, const Abort &ab) {
   if (mbar_try(bar, parity)) return true;
-  return mbar_wait_slow(bar, parity, ab.flag);
+#pragma unroll 1
+  for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
+    if (mbar_try(bar, parity)) return true;
+    if ((spin & 255u) == 255u && ab.set()) return false;
+  }
+  *ab.flag = 1;
+  return false;
 }
 
 // Box {128 bytes, rows, K blocks} of the operand seen as [K/128][rows][128 bytes] (see make_map).
@@ -168,6 +183,12 @@ __device__ __forceinline__ void copy4_async(float *to, const float *from) {
 }
 __device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr) : "memory");
+}
+
 // Two fp32 fused multiply-adds in one instruction (fma.rn.f32x2: each half is the same correctly rounded FMA as
 // fmaf): the promotion of a K block is 32 or 64 of them per thread, and the epilogue warps' issue slots are what the
 // tensor pipe ends up waiting for.
@@ -190,19 +211,74 @@ __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigne
   return v;
 }
 
-// kRows batch rows x kVocab vocabulary ids per output tile (kVocab = UMMA N: 128, or 256 to halve the activation
-// traffic per output element when the batch is large and the kernel is bound by L2 -> shared-memory copies)
-template <int kRows, int kVocab>
-struct HeadSmem {
-  static constexpr int kAccBufs = kTmemColumns / kVocab;
-  static constexpr int kStageBytes = kVocab * kTileK + kRows * kTileK;
-  // The MMA reads 128 activation rows from every stage; with kRows < 128 the rows beyond the tile are the weights behind it (the
-  // activations come first in a stage) and only feed TMEM lanes nobody reads.
-  static_assert(kVocab >= 128 - kRows, "the rows read beyond the activations lie in the stage");
-  static constexpr int kMaxStages = 12;
-  // bytes beside the stages: alignment slack, scale tables [K/128][kRows] and [warps][2][K/128], barriers and flags
+// ---- a pair of CTAs (a cluster of two) on one tile
+__device__ __forceinline__ uint32_t pair_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// All threads of both CTAs: what each has done before is seen by the other behind it.
+__device__ __forceinline__ void pair_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address of the leading CTA's copy of a shared variable.
+__device__ __forceinline__ uint32_t in_leader(const void *p) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_addr(p)));
+  return a;
+}
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Into this CTA's shared memory; the bytes are counted by a barrier of the leading CTA.
+__device__ __forceinline__ void tma_load_pair(void *dst, const CUtensorMap *map, uint32_t leader_bar, int x, int row, int kb, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2.L2::cache_hint [%0], "
+      "[%1, {%3, %4, %5}], [%2], %6;" ::"r"(smem_addr(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(leader_bar), "r"(x), "r"(row), "r"(kb), "l"(policy)
+      : "memory");
+}
+// Instruction descriptor as umma_idesc, M = 256: 128 rows of A from each CTA, 128 of the 256 rows of B from each.
+constexpr uint32_t kPairIdesc = (1u << 4) | (uint32_t(256 >> 3) << 17) | (uint32_t(256 >> 4) << 24);
+template <bool kAccumulate>
+__device__ __forceinline__ void umma_f8_pair(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
+      "l"(a_desc), "l"(b_desc), "r"(kPairIdesc), "n"(kAccumulate ? 1 : 0)
+      : "memory");
+}
+// Arrives at both CTAs' copies of the barrier.
+__device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_addr(bar)),
+               "h"(uint16_t(3))
+               : "memory");
+}
+
+// 128 batch rows of each CTA of a pair x 256 vocabulary ids.  A stage is one K block: 128 rows of activations and 128 of the ids' rows.
+struct PairSmem {
+  static constexpr int kAccBufs = 2;
+  static constexpr int kStageBytes = 2 * 128 * kTileK, kStages = 5;
+  static constexpr int kOutFloats = 32 * 16;   // an epilogue warp's 32 rows x 16 ids on their way out
+  // bytes beside the stages: alignment slack, output blocks, statistics, scale tables [K/128][128] and [warps][2][K/128], barriers and flags
   static constexpr size_t fixed_bytes(int kblocks) {
-    return 1024 + size_t(kblocks) * (kRows + 2 * kEpiWarps) * 4 + (2 * kMaxStages + 2 * kAccBufs) * 8 + 16;
+    return 1024 + kEpiWarps * (kOutFloats * 4 + 32 * 16) + size_t(kblocks) * (128 + 2 * kEpiWarps) * 4 + (2 * kStages + 2 * kAccBufs) * 8 + 16;
+  }
+  static constexpr int stages(int kblocks) {
+    const long long room = 227 * 1024 - (long long)fixed_bytes(kblocks);
+    const int n = room < 0 ? 0 : int(room / kStageBytes);
+    return n > kStages ? kStages : n;
+  }
+};
+
+// 128 batch rows x 128 vocabulary ids
+struct HeadSmem {
+  static constexpr int kAccBufs = kTmemColumns / 128;
+  static constexpr int kStageBytes = 2 * 128 * kTileK;
+  static constexpr int kMaxStages = 12;
+  // bytes beside the stages: alignment slack, scale tables [K/128][128] and [warps][K/128], barriers and flags
+  static constexpr size_t fixed_bytes(int kblocks) {
+    return 1024 + size_t(kblocks) * (128 + kEpiWarps) * 4 + (2 * kMaxStages + 2 * kAccBufs) * 8 + 16;
   }
   // a stage holds `group` consecutive K blocks (one TMA box per operand)
   static constexpr int stages(int kblocks, int group) {
@@ -232,7 +308,7 @@ struct HeadArgs {
   // The same records in the row-scattered variant: row m's record lies owner_stats_offset bytes behind owner_base[owner]
   // at index m % rows_per_owner (0: none).  Several GPUs merge into one record, so those atomics have system scope.
   long long owner_stats_offset;
-  int stages;            // shared-memory stages of the TMA ring (host: HeadSmem::stages)
+  int stages;            // shared-memory stages of the TMA ring (host: PairSmem::stages)
   int group;             // K blocks per stage: every row of a weight tile is fetched as group*128 contiguous bytes
 };
 
@@ -263,43 +339,39 @@ __device__ __forceinline__ void merge_stats(const HeadArgs &p, int m, float best
   }
 }
 
-template <int kRows, int kVocab>
+// 65 to 128 rows: 128 batch rows x 128 vocabulary ids a tile.
 __global__ void __launch_bounds__(kHeadThreads, 1)
-head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, HeadArgs p) {
-  using Smem = HeadSmem<kRows, kVocab>;
-  constexpr int kTileN = kVocab, kAccBufs = Smem::kAccBufs;
+head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ HeadArgs p) {
+  using Smem = HeadSmem;
+  constexpr int kRows = 128, kTileN = 128, kAccBufs = Smem::kAccBufs;
   constexpr int kStageBytes = Smem::kStageBytes;
   constexpr int kMaxStages = Smem::kMaxStages;
   const int kStages = p.stages, group = p.group;
   const int stage_bytes = kStageBytes * group, a_bytes = kRows * kTileK * group;  // [A g0..][W g0..]
-  constexpr uint32_t kTmemCols = kTmemColumns;
-  constexpr int kQuads = (kRows + 31) / 32;          // lane quadrants that hold real batch rows
-  constexpr int kGroups = 4, kMyCols = kTileN / kGroups;  // 32- or 64-column groups: warp (quadrant q, group g)
-  constexpr int kEpiActive = 32 * kQuads * kGroups;  // epilogue threads that take part
+  constexpr int kMyCols = 32, kEpiThreads = 32 * kEpiWarps;   // epilogue warp = (lane quadrant, group of 32 columns)
   extern __shared__ __align__(1024) unsigned char smem[];
-  // carve: [stages][A tiles kRows*128 B | W tiles 16 or 32 KB], then the scale tables, then barriers
+  // carve: [stages][A tiles 16 KB | W tiles 16 KB], then the scale tables, then barriers
   unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~uintptr_t(1023));
   float *sa = reinterpret_cast<float *>(tiles + size_t(kStages) * stage_bytes);  // [K/128][kRows]
   const int kblocks = p.K / kTileK;
-  float *sw = sa + size_t(kblocks) * kRows;                                                              // [epilogue warp][2][K/128]
-  uint64_t *bars = reinterpret_cast<uint64_t *>(sw + size_t(kblocks) * 2 * kEpiWarps);
+  float *sw = sa + size_t(kblocks) * kRows;                                                              // [epilogue warp][K/128]
+  uint64_t *bars = reinterpret_cast<uint64_t *>(sw + size_t(kblocks) * kEpiWarps);
   uint64_t *full = bars, *empty = bars + kMaxStages, *acc_full = bars + 2 * kMaxStages, *acc_empty = acc_full + kAccBufs;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + kAccBufs);
   int *abort_word = reinterpret_cast<int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_tiles = (p.N + kTileN - 1) / kTileN, b_tiles = (p.M + kRows - 1) / kRows;
-  const int total_tiles = n_tiles * b_tiles;  // tile t = (vocabulary tile t / b_tiles, batch tile t % b_tiles)
+  const int total_tiles = (p.N + kTileN - 1) / kTileN;
   Abort ab{abort_word};
 
   if (threadIdx.x == 0) {
     *abort_word = 0;
     for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int b = 0; b < kAccBufs; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], kQuads * kGroups); }
+    for (int b = 0; b < kAccBufs; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], kEpiWarps); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {  // TMEM allocation by one full warp; the address lands in shared memory
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)), "r"(kTmemCols));
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)), "r"(uint32_t(kTmemColumns)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -311,24 +383,22 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       uint32_t stage = 0, phase = 0;
-      // one batch tile: every weight is read once per step, and 530 MB of them would push everything else out of the L2 --
-      // the logits, the activations, the code of the kernels around this one
+      // every weight is read once per step, and 530 MB of them would push everything else out of the L2 -- the logits, the
+      // activations, the code of the kernels around this one
       uint64_t policy;
-      if (b_tiles == 1) asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
-      else asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
+      asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
       // the ring's first weights are on their way to the L2 while the kernel in front of this one (the quantiser) finishes
       const int early = kblocks / group < kStages ? kblocks / group : kStages;
-      for (int s = 0; s < early; ++s) tma_prefetch_3d(&map_w, 0, int(blockIdx.x) / b_tiles * kTileN, s * group, policy);
+      for (int s = 0; s < early; ++s) tma_prefetch_3d(&map_w, 0, int(blockIdx.x) * kTileN, s * group, policy);
       cudaGridDependencySynchronize();
       cudaTriggerProgrammaticLaunchCompletion();
       for (int tile = blockIdx.x; tile < total_tiles && !ab.set(); tile += gridDim.x) {
-        const int nt = tile / b_tiles, bt = tile % b_tiles;
         for (int kb = 0; kb < kblocks; kb += group) {
           if (!mbar_wait(&empty[stage], phase ^ 1, ab)) break;
           unsigned char *a_dst = tiles + size_t(stage) * stage_bytes, *w_dst = a_dst + a_bytes;
           mbar_expect_tx(&full[stage], uint32_t(stage_bytes));
-          tma_load_3d(w_dst, &map_w, &full[stage], 0, nt * kTileN, kb, policy);
-          tma_load_3d(a_dst, &map_a, &full[stage], 0, bt * kRows, kb);
+          tma_load_3d(w_dst, &map_w, &full[stage], 0, tile * kTileN, kb, policy);
+          tma_load_3d(a_dst, &map_a, &full[stage], 0, 0, kb);
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
       }
@@ -366,31 +436,19 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         if (++stage == kStages) { stage = 0; phase ^= 1; }
       }
     }
-  } else if ((warp & 3) < kQuads) {
+  } else if (warp >= 2) {
     // ------------------------------------------------------------------ epilogue: warp = (lane quadrant, column group)
     cudaGridDependencySynchronize();
     const int quad = warp & 3;          // TMEM lanes [32*quad, 32*quad+32) are readable by this warp: batch rows
     const int group = (warp - 2) >> 2;  // vocabulary ids [32*group, 32*group+32) of the tile
     const int row = quad * 32 + lane;   // batch row inside the tile
-    const int et = (group * kQuads + quad) * 32 + lane;  // 0..kEpiActive-1
+    const int et = threadIdx.x - 64;
     const uint32_t lane_base = tmem_base + group * kMyCols + (uint32_t(quad * 32) << 16);
-    float *my_sw = sw + size_t(warp - 2) * 2 * kblocks;
-    // fp32 scales of the 128-row weight block this warp's columns belong to (a 256-wide tile spans two blocks), on their way into
-    // shared memory
-    auto fetch_scales = [&](int tile, float *to) {
-      if (tile < total_tiles) {
-        const int w_block = min((tile / b_tiles * kTileN + group * kMyCols) / 128, (p.N + 127) / 128 - 1);
-        for (int i = lane; i < kblocks; i += 32) copy4_async(to + i, p.w_scale + size_t(w_block) * kblocks + i);
-      }
-    };
-    fetch_scales(blockIdx.x, my_sw);
-    int which = 0;
+    float *my_sw = sw + size_t(warp - 2) * kblocks;
     uint32_t acc = 0, acc_phase = 0;
-    int table_bt = -1;
-    bool alive = true;  // warp-uniform; once false the remaining tiles are walked without waiting or computing,
-                        // so that all epilogue threads still meet at every named barrier
-    // running statistics of this thread's batch row over the tiles of one batch tile (vocabulary tiles come in ascending
-    // order, so a strict comparison keeps the first maximum).  With 32 columns a thread the column is looked for only in a tile
+    bool alive = true;  // warp-uniform
+    // running statistics of this thread's batch row over its tiles (vocabulary tiles come in ascending
+    // order, so a strict comparison keeps the first maximum).  The column is looked for only in a tile
     // that raises the maximum of one of the warp's rows.  (Looking it up in the logits when the row is left took 10 us at 128
     // rows and 28 at 256: the reads stand behind everything that the GPU has just written.)
     float st_best = -CUDART_INF_F, st_low = CUDART_INF_F, st_bad = 0.f, st_bad1 = 0.f;
@@ -401,31 +459,16 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       const int owner = m / p.rows_per_owner;
       return p.owner_base[owner] + size_t(m - owner * p.rows_per_owner) * p.ldl + p.col_offset;
     };
-    auto flush_stats = [&](int bt_of) {
-      const int m = bt_of * kRows + row;
-      if (stats_on && row < kRows && m < p.M) merge_stats(p, m, st_best, st_id, st_low, st_bad + st_bad1 != 0.f);
-      st_best = -CUDART_INF_F; st_low = CUDART_INF_F; st_bad = st_bad1 = 0.f; st_id = 0x7fffffff;
-    };
-    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-      const int nt = tile / b_tiles, bt = tile % b_tiles;
-      if (bt != table_bt) {  // activation scales of this batch tile: sa[kb][row] (a grid that is a multiple of b_tiles
-                             // keeps bt fixed per CTA, so this normally happens once)
-        if (table_bt >= 0) flush_stats(table_bt);
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiActive) : "memory");  // readers of the previous table are done
-        for (int i = et; i < kblocks * kRows; i += kEpiActive) {
-          const int r = i / kblocks, kb = i % kblocks, m = bt * kRows + r;
-          sa[kb * kRows + r] = m < p.M ? load_input(p.a_scale + size_t(m) * kblocks + kb) : 0.f;
-        }
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiActive) : "memory");
-        table_bt = bt;
-      }
-      // The next tile's scales are fetched a tile ahead: they come from DRAM, and a load of them between two tiles would keep the
-      // accumulators waiting for longer than the MMAs can run ahead.
-      const float *tile_sw = my_sw + which * kblocks;
-      copies_done();
+    for (int i = et; i < kblocks * kRows; i += kEpiThreads) {   // activation scales: sa[kb][row]
+      const int r = i / kblocks, kb = i % kblocks;
+      sa[kb * kRows + r] = r < p.M ? load_input(p.a_scale + size_t(r) * kblocks + kb) : 0.f;
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+    for (int tile = blockIdx.x; tile < total_tiles && alive; tile += gridDim.x) {
+      // fp32 scales of the tile's weight block, copied once per tile: a global load in the loop below, even one that hits, delays the
+      // hand-over of each accumulator.  (Fetched a tile ahead, as the other two kernels do: 107.5 us at 65 rows instead of 106.5.)
+      for (int i = lane; i < kblocks; i += 32) my_sw[i] = load_input(p.w_scale + size_t(tile) * kblocks + i);
       __syncwarp();
-      which ^= 1;
-      fetch_scales(tile + gridDim.x, my_sw + which * kblocks);
       float sum[kMyCols];
 #pragma unroll
       for (int c = 0; c < kMyCols; ++c) sum[c] = 0.f;
@@ -433,38 +476,21 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         alive = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], acc_phase, ab));
         if (!alive) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const float scale = sa[kb * kRows + (row < kRows ? row : 0)] * tile_sw[kb];
+        const float scale = sa[kb * kRows + row] * my_sw[kb];
         const unsigned long long scale2 = pack2(scale, scale);
-        if constexpr (kMyCols == 32) {
-          uint32_t r[32];
-          tmem_ld32(lane_base + acc * kTileN, r);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          // the values are in registers: the accumulator can be refilled while they are scaled and added
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&acc_empty[acc]);
+        uint32_t r[32];
+        tmem_ld32(lane_base + acc * kTileN, r);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        // the values are in registers: the accumulator can be refilled while they are scaled and added
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[acc]);
 #pragma unroll
-          for (int c = 0; c < 32; c += 2) fma2_acc(sum[c], sum[c + 1], r[c], r[c + 1], scale2);
-        } else {
-          // 64 columns per thread: four 16-column loads, one in flight at a time (what the registers of 576 threads leave room for)
-#pragma unroll
-          for (int c0 = 0; c0 < kMyCols; c0 += 16) {
-            uint32_t r[32];
-            tmem_ld16(lane_base + acc * kTileN + c0, r);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (c0 + 16 == kMyCols) {
-              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&acc_empty[acc]);
-            }
-#pragma unroll
-            for (int c = 0; c < 16; c += 2) fma2_acc(sum[c0 + c], sum[c0 + c + 1], r[c], r[c + 1], scale2);
-          }
-        }
+        for (int c = 0; c < 32; c += 2) fma2_acc(sum[c], sum[c + 1], r[c], r[c + 1], scale2);
         if (++acc == kAccBufs) { acc = 0; acc_phase ^= 1; }
       }
       // Output, while the tensor cores wait: as few instructions as it takes.
-      const int n0 = nt * kTileN + group * kMyCols;
+      const int n0 = tile * kTileN + group * kMyCols;
       const bool whole = n0 + kMyCols <= p.N;
       if (alive && stats_on) {
         if (whole) {
@@ -472,25 +498,17 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 #pragma unroll
           for (int c = 0; c < kMyCols; c += 2)   // NaN once any logit is NaN or infinite
             fma2_acc(st_bad, st_bad1, __float_as_uint(sum[c]), __float_as_uint(sum[c + 1]), zero2);
-          if constexpr (kMyCols == 32) {
-            float hi = sum[0], low = sum[0];
+          float hi = sum[0], low = sum[0];
 #pragma unroll
-            for (int c = 1; c < kMyCols; ++c) { hi = fmaxf(hi, sum[c]); low = fminf(low, sum[c]); }
-            if (__any_sync(0xffffffffu, hi > st_best)) {
-              int at = 0;
+          for (int c = 1; c < kMyCols; ++c) { hi = fmaxf(hi, sum[c]); low = fminf(low, sum[c]); }
+          if (__any_sync(0xffffffffu, hi > st_best)) {
+            int at = 0;
 #pragma unroll
-              for (int c = kMyCols - 1; c > 0; --c) at = sum[c] == hi ? c : at;
-              if (sum[0] == hi) at = 0;
-              if (hi > st_best) { st_best = hi; st_id = n0 + at; }
-            }
-            st_low = fminf(st_low, low);
-          } else {                               // (no registers to spare)
-#pragma unroll
-            for (int c = 0; c < kMyCols; ++c) {
-              if (sum[c] > st_best) { st_best = sum[c]; st_id = n0 + c; }
-              st_low = fminf(st_low, sum[c]);
-            }
+            for (int c = kMyCols - 1; c > 0; --c) at = sum[c] == hi ? c : at;
+            if (sum[0] == hi) at = 0;
+            if (hi > st_best) { st_best = hi; st_id = n0 + at; }
           }
+          st_low = fminf(st_low, low);
         } else {
 #pragma unroll
           for (int c = 0; c < kMyCols; ++c) {
@@ -510,52 +528,335 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       if (alive) {
         const bool scattered = p.rows_per_owner != 0;
         const bool plain = !scattered && whole && p.ldl % 4 == 0 && (reinterpret_cast<uintptr_t>(p.logits) & 15u) == 0;
+        float4 x[8];
 #pragma unroll
-        for (int half = 0; half < kMyCols / 32; ++half) {
-          float4 x[8];
+        for (int c = 0; c < 8; ++c)
+          x[c] = make_float4(sum[4 * c], sum[4 * c + 1], sum[4 * c + 2], sum[4 * c + 3]);
+        auto exchange = [&](int bit, int dist) {   // column group bit of the index <-> the lane bit of that distance
+          const bool upper = (lane & dist) != 0;
 #pragma unroll
-          for (int c = 0; c < 8; ++c)
-            x[c] = make_float4(sum[32 * half + 4 * c], sum[32 * half + 4 * c + 1], sum[32 * half + 4 * c + 2], sum[32 * half + 4 * c + 3]);
-          auto exchange = [&](int bit, int dist) {   // column group bit of the index <-> the lane bit of that distance
-            const bool upper = (lane & dist) != 0;
+          for (int c = 0; c < 8; ++c) {
+            if ((c >> bit) & 1) continue;
+            const int c2 = c | (1 << bit);
+            const float4 give = upper ? x[c] : x[c2];
+            float4 take;
+            take.x = __shfl_xor_sync(0xffffffffu, give.x, dist);
+            take.y = __shfl_xor_sync(0xffffffffu, give.y, dist);
+            take.z = __shfl_xor_sync(0xffffffffu, give.z, dist);
+            take.w = __shfl_xor_sync(0xffffffffu, give.w, dist);
+            if (upper) x[c] = take; else x[c2] = take;
+          }
+        };
+        exchange(0, 8);
+        exchange(1, 16);
+        exchange(2, 4);
+        // x[c] = columns [4 * (lane / 8) + 16 * (lane / 4 % 2), +4) of block row 8 * (c % 4) + 4 * (c / 4) + lane % 4
+        if (plain) {
+          const int r = quad * 32 + (lane & 3), rows = p.M - r;
+          float *dst = p.logits + size_t(r) * p.ldl + n0 + 4 * (lane >> 3) + 16 * ((lane >> 2) & 1);
+          const long long step = 4 * p.ldl;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-              if ((c >> bit) & 1) continue;
-              const int c2 = c | (1 << bit);
-              const float4 give = upper ? x[c] : x[c2];
-              float4 take;
-              take.x = __shfl_xor_sync(0xffffffffu, give.x, dist);
-              take.y = __shfl_xor_sync(0xffffffffu, give.y, dist);
-              take.z = __shfl_xor_sync(0xffffffffu, give.z, dist);
-              take.w = __shfl_xor_sync(0xffffffffu, give.w, dist);
-              if (upper) x[c] = take; else x[c2] = take;
+          for (int c = 0; c < 8; ++c) {
+            if (4 * c < rows) *reinterpret_cast<float4 *>(dst) = x[(c >> 1) | ((c & 1) << 2)];
+            dst += step;
+          }
+        } else {
+          const int n = n0 + 4 * (lane >> 3) + 16 * ((lane >> 2) & 1);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const int m = quad * 32 + 8 * (c & 3) + 4 * (c >> 2) + (lane & 3);
+            if (m >= p.M || n >= p.N) continue;
+            float *dst = row_of(m) + n;
+            if (n + 4 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
+              *reinterpret_cast<float4 *>(dst) = x[c];
+            } else {
+              const float v[4] = {x[c].x, x[c].y, x[c].z, x[c].w};
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                if (n + k < p.N) dst[k] = v[k];
             }
-          };
-          exchange(0, 8);
-          exchange(1, 16);
-          exchange(2, 4);
-          // x[c] = columns [4 * (lane / 8) + 16 * (lane / 4 % 2), +4) of block row 8 * (c % 4) + 4 * (c / 4) + lane % 4
-          if (plain) {
-            const int r = quad * 32 + (lane & 3), rows = min(kRows, p.M - bt * kRows) - r;
-            float *dst = p.logits + size_t(bt * kRows + r) * p.ldl + n0 + 32 * half + 4 * (lane >> 3) + 16 * ((lane >> 2) & 1);
-            const long long step = 4 * p.ldl;
+          }
+        }
+      }
+    }
+    if (alive && stats_on && row < p.M) merge_stats(p, row, st_best, st_id, st_low, st_bad + st_bad1 != 0.f);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(uint32_t(kTmemColumns)));
+  }
+  if (threadIdx.x == 0 && *abort_word && p.error_flag) atomicExch(p.error_flag, 1);
+}
+
+// Larger batches: pairs of CTAs, 256 batch rows x 256 vocabulary ids a tile.  An epilogue thread keeps 64 sums, so every register
+// counts: 112 each (the warps beside them give theirs up), statistics in shared memory between the tiles (737 -> 713 us with the
+// records at 1024 rows), waits in line (around a call all sums would be spilled).  The hand-back to the leading CTA is a relaxed
+// arrival: with release semantics at cluster scope a K block took 1870 cycles instead of 840.  Tried without gain: 128 ids a tile, four
+// accumulators, 32 sums and boxes stored by TMA (829 us: 24 KB a K block of half the size); the next K block's scales, its wait or its
+// first load ahead (721 to 850: spills); sixteen columns a load (740).
+__global__ void __launch_bounds__(kPairThreads, 1)
+head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ HeadArgs p) {
+  using Smem = PairSmem;
+  constexpr int kAccBufs = Smem::kAccBufs, kStageBytes = Smem::kStageBytes, kMaxStages = Smem::kStages;
+  constexpr int kCols = 64;             // ids of an epilogue warp: warp = (lane quadrant, group of 64 ids)
+  const int kStages = p.stages;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  // carve: [stages][A 16 KB | W 16 KB], then output blocks, scale tables, barriers; the same places in both CTAs
+  unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~uintptr_t(1023));
+  float *out = reinterpret_cast<float *>(tiles + size_t(kStages) * kStageBytes);   // [epilogue warp][32][20]
+  float4 *stats = reinterpret_cast<float4 *>(out + kEpiWarps * Smem::kOutFloats);  // [epilogue thread] maximum, minimum, its id, not finite
+  float *sa = reinterpret_cast<float *>(stats + kEpiWarps * 32);                   // [K/128][128]
+  const int kblocks = p.K / kTileK;
+  float *sw = sa + size_t(kblocks) * 128;                                          // [epilogue warp][2][K/128]
+  uint64_t *bars = reinterpret_cast<uint64_t *>(sw + size_t(kblocks) * 2 * kEpiWarps);
+  uint64_t *full = bars, *empty = bars + kMaxStages, *acc_full = bars + 2 * kMaxStages, *acc_empty = acc_full + kAccBufs;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + kAccBufs);
+  int *abort_word = reinterpret_cast<int *>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = int(pair_rank()), pair = int(blockIdx.x) >> 1, pairs = int(gridDim.x) >> 1;
+  const int b_tiles = (p.M + 255) / 256, total_tiles = (p.N + 255) / 256 * b_tiles;
+  // tile t = (vocabulary tile t / b_tiles, batch tile t % b_tiles)
+  const int active = p.M > 128 ? 2 : 1;   // CTAs of a pair that have batch rows at all
+  Abort ab{abort_word};
+
+  if (threadIdx.x == 0) {
+    *abort_word = 0;
+    for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int b = 0; b < kAccBufs; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], kEpiWarps * active); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {  // TMEM allocation by one full warp of each CTA; the address lands in shared memory
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)), "r"(uint32_t(kTmemColumns)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  pair_barrier();   // both CTAs have started and set up their barriers
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer, one in each CTA
+    if (lane == 0) {
+      uint32_t stage = 0, phase = 0;
+      // one batch tile: every weight is read once per step, and 530 MB of them would push everything else out of the L2 --
+      // the logits, the activations, the code of the kernels around this one
+      uint64_t policy, keep;
+      if (b_tiles == 1) asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+      else asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
+      asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(keep));
+      // the ring's first weights are on their way to the L2 while the kernel in front of this one (the quantiser) finishes
+      const int early = kblocks < kStages ? kblocks : kStages;
+      for (int s = 0; s < early; ++s) tma_prefetch_3d(&map_w, 0, pair / b_tiles * 256 + 128 * rank, s, policy);
+      cudaGridDependencySynchronize();
+      cudaTriggerProgrammaticLaunchCompletion();
+      const uint32_t leader_full = in_leader(full);
+      for (int tile = pair; tile < total_tiles && !ab.set(); tile += pairs) {
+        const int id = tile / b_tiles * 256 + 128 * rank, first = tile % b_tiles * 256, mine = first + 128 * rank;
+        // (a second half without batch rows is not fetched: what the MMA makes of the rows' place nobody reads)
+        const uint32_t bytes = kStageBytes + 128 * kTileK + (first + 128 < p.M ? 128 * kTileK : 0);
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!mbar_wait(&empty[stage], phase ^ 1, ab)) break;
+          unsigned char *a_dst = tiles + size_t(stage) * kStageBytes, *w_dst = a_dst + 128 * kTileK;
+          if (rank == 0) mbar_expect_tx(&full[stage], bytes);   // of both CTAs
+          tma_load_pair(w_dst, &map_w, leader_full + 8 * stage, 0, id, kb, policy);
+          if (mine < p.M) tma_load_pair(a_dst, &map_a, leader_full + 8 * stage, 0, mine, kb, keep);
+          if (++stage == uint32_t(kStages)) { stage = 0; phase ^= 1; }
+        }
+      }
+      // every release has arrived before this CTA's shared memory goes away
+      for (int s = 0; s < kStages && !ab.set(); ++s) {
+        mbar_wait(&empty[stage], phase ^ 1, ab);
+        if (++stage == uint32_t(kStages)) { stage = 0; phase ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer of the leading CTA: the warp waits together, one lane issues
+    cudaGridDependencySynchronize();
+    if (rank == 0) {
+      const uint32_t tiles16 = smem_addr(tiles) >> 4;
+      const bool leader = elect_one();
+      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+      for (int tile = pair; tile < total_tiles && !__any_sync(0xffffffffu, ab.set()); tile += pairs) {
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], phase, ab))) break;
+          if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[acc], acc_phase ^ 1, ab))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a16 = tiles16 + stage * (kStageBytes >> 4), w16 = a16 + ((128 * kTileK) >> 4);  // addresses >> 4
+          const uint32_t d_addr = tmem_base + acc * 256;
+          if (leader) {
+            // D[batch row, vocabulary id] (+)= A[batch row, k] * W[vocabulary id, k], K = 32 bytes per instruction
+            umma_f8_pair<false>(d_addr, umma_desc16(a16), umma_desc16(w16));
+            umma_f8_pair<true>(d_addr, umma_desc16(a16 + 2), umma_desc16(w16 + 2));
+            umma_f8_pair<true>(d_addr, umma_desc16(a16 + 4), umma_desc16(w16 + 4));
+            umma_f8_pair<true>(d_addr, umma_desc16(a16 + 6), umma_desc16(w16 + 6));
+            umma_commit_pair(&acc_full[acc]);   // accumulator of this K block is complete
+            umma_commit_pair(&empty[stage]);    // the stage may be refilled: these MMAs have read it
+          }
+          __syncwarp();
+          if (++acc == kAccBufs) { acc = 0; acc_phase ^= 1; }
+          if (++stage == uint32_t(kStages)) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else {
+    cudaGridDependencySynchronize();
+  }
+  } else {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+  if (rank < active) {
+    // ------------------------------------------------------------------ epilogue: warp = (lane quadrant, column group)
+    cudaGridDependencySynchronize();
+    const int quad = warp & 3;          // TMEM lanes [32*quad, 32*quad+32) are readable by this warp: batch rows
+    const int group = (warp - 4) >> 2;  // vocabulary ids [64*group, 64*group+64) of the tile
+    const int row = quad * 32 + lane;   // batch row inside the CTA's 128
+    const int et = threadIdx.x - 128;
+    const uint32_t lane_base = tmem_base + group * kCols + (uint32_t(quad * 32) << 16);
+    const uint32_t leader_empty = in_leader(acc_empty);
+    float *my_sw = sw + size_t(warp - 4) * 2 * kblocks;
+    float *my_out = out + (warp - 4) * Smem::kOutFloats;
+    // fp32 scales of the 128-row weight block this warp's columns belong to, on their way into shared memory
+    auto fetch_scales = [&](int tile, float *to) {
+      if (tile < total_tiles) {
+        const int w_block = min(tile / b_tiles * 2 + (group >> 1), (p.N + 127) / 128 - 1);
+        for (int i = lane; i < kblocks; i += 32) copy4_async(to + i, p.w_scale + size_t(w_block) * kblocks + i);
+      }
+    };
+    fetch_scales(pair, my_sw);
+    int which = 0;
+    uint32_t acc = 0, acc_phase = 0;
+    int table_bt = -1;
+    bool alive = true;  // warp-uniform; once false the remaining tiles are walked without waiting or computing,
+                        // so that all epilogue threads still meet at every named barrier
+    // running statistics of this thread's batch row over the tiles of one batch tile (vocabulary tiles come in ascending
+    // order, so a strict comparison keeps the first maximum)
+    const float4 nothing = make_float4(-CUDART_INF_F, CUDART_INF_F, __int_as_float(0x7fffffff), 0.f);
+    stats[et] = nothing;   // (in shared memory: the registers are the sums')
+    const bool stats_on = p.row_stats != nullptr || p.owner_stats_offset != 0;
+    auto row_of = [&](int m) {   // batch row m of the output
+      if (p.rows_per_owner == 0) return p.logits + size_t(m) * p.ldl;
+      const int owner = m / p.rows_per_owner;
+      return p.owner_base[owner] + size_t(m - owner * p.rows_per_owner) * p.ldl + p.col_offset;
+    };
+    auto flush_stats = [&](int bt_of) {
+      const int m = bt_of * 256 + 128 * rank + row;
+      const float4 st = stats[et];
+      if (stats_on && m < p.M) merge_stats(p, m, st.x, __float_as_int(st.z), st.y, st.w != 0.f);
+      stats[et] = nothing;
+    };
+    for (int tile = pair; tile < total_tiles; tile += pairs) {
+      const int nt = tile / b_tiles, bt = tile % b_tiles, m0 = bt * 256 + 128 * rank;
+      if (bt != table_bt) {  // activation scales of this CTA's rows: sa[kb][row] (a number of pairs that is a multiple of b_tiles
+                             // keeps bt fixed per CTA, so this normally happens once)
+        if (table_bt >= 0) flush_stats(table_bt);
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");  // readers of the previous table are done
+        for (int i = et; i < kblocks * 128; i += 32 * kEpiWarps) {
+          const int r = i / kblocks, kb = i % kblocks, m = m0 + r;
+          sa[kb * 128 + r] = m < p.M ? load_input(p.a_scale + size_t(m) * kblocks + kb) : 0.f;
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
+        table_bt = bt;
+      }
+      // The next tile's scales are fetched a tile ahead: they come from DRAM, and a load of them between two tiles would keep the
+      // accumulators waiting.
+      const float *tile_sw = my_sw + which * kblocks;
+      copies_done();
+      __syncwarp();
+      which ^= 1;
+      fetch_scales(tile + pairs, my_sw + which * kblocks);
+      float sum[kCols];
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-              if (4 * c < rows) *reinterpret_cast<float4 *>(dst) = x[(c >> 1) | ((c & 1) << 2)];
-              dst += step;
+      for (int c = 0; c < kCols; ++c) sum[c] = 0.f;
+      for (int kb = 0; kb < kblocks && alive; ++kb) {
+        const float scale = sa[kb * 128 + row] * tile_sw[kb];
+        const unsigned long long scale2 = pack2(scale, scale);
+        alive = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], acc_phase, ab));
+        if (!alive) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        uint32_t r[2][8];
+        tmem_ld8(lane_base + acc * 256, r[0]);
+#pragma unroll
+        for (int q = 0; q < kCols / 8; ++q) {
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (q + 1 < kCols / 8) {
+            tmem_ld8(lane_base + acc * 256 + 8 * (q + 1), r[(q + 1) & 1]);
+          } else {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_leader(leader_empty + 8 * acc);
+          }
+#pragma unroll
+          for (int c = 0; c < 8; c += 2) fma2_acc(sum[8 * q + c], sum[8 * q + c + 1], r[q & 1][c], r[q & 1][c + 1], scale2);
+        }
+        if (++acc == kAccBufs) { acc = 0; acc_phase ^= 1; }
+      }
+      // Output, while the tensor cores wait: as few instructions as it takes.
+      const int n0 = nt * 256 + group * kCols;
+      const bool whole = n0 + kCols <= p.N;
+      if (alive && stats_on) {
+        const float4 st = stats[et];
+        float st_best = st.x, st_low = st.y, st_bad = st.w, st_bad1 = 0.f;
+        int st_id = __float_as_int(st.z);
+        if (whole) {
+          const unsigned long long zero2 = pack2(0.f, 0.f);
+#pragma unroll
+          for (int c = 0; c < kCols; c += 2)   // NaN once any logit is NaN or infinite
+            fma2_acc(st_bad, st_bad1, __float_as_uint(sum[c]), __float_as_uint(sum[c + 1]), zero2);
+#pragma unroll
+          for (int c = 0; c < kCols; ++c) {
+            if (sum[c] > st_best) { st_best = sum[c]; st_id = n0 + c; }
+            st_low = fminf(st_low, sum[c]);
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < kCols; ++c) {
+            const float v = sum[c];
+            if (n0 + c < p.N) {
+              st_bad = fmaf(v, 0.f, st_bad);
+              if (v > st_best) { st_best = v; st_id = n0 + c; }
+              st_low = fminf(st_low, v);
+            }
+          }
+        }
+        stats[et] = make_float4(st_best, st_low, __int_as_float(st_id), st_bad + st_bad1);
+      }
+      // Lane l holds row l of the warp's 32 x 64 block.  Sixteen ids at a time go through shared memory, so that a store instruction
+      // writes 64 contiguous bytes of eight rows (rows 80 bytes apart: neither side has a bank conflict).
+      if (alive) {
+        const bool plain = p.rows_per_owner == 0 && whole && p.ldl % 4 == 0 && (reinterpret_cast<uintptr_t>(p.logits) & 15u) == 0;
+        const int r0 = quad * 32 + (lane >> 2), col = 4 * (lane & 3);
+#pragma unroll
+        for (int q = 0; q < kCols / 16; ++q) {
+          __syncwarp();
+#pragma unroll
+          for (int c = 0; c < 16; c += 4)
+            *reinterpret_cast<float4 *>(my_out + lane * 16 + (c ^ (4 * ((lane >> 1) & 3)))) =
+                make_float4(sum[16 * q + c], sum[16 * q + c + 1], sum[16 * q + c + 2], sum[16 * q + c + 3]);
+          __syncwarp();
+          if (plain) {
+            float *dst = p.logits + size_t(m0 + r0) * p.ldl + n0 + 16 * q + col;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float4 v = *reinterpret_cast<const float4 *>(my_out + ((lane >> 2) + 8 * i) * 16 + (col ^ (4 * ((lane >> 3) & 3))));
+              if (m0 + r0 + 8 * i < p.M) *reinterpret_cast<float4 *>(dst) = v;
+              dst += 8 * p.ldl;
             }
           } else {
-            const int n = n0 + 32 * half + 4 * (lane >> 3) + 16 * ((lane >> 2) & 1);
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-              const int r = quad * 32 + 8 * (c & 3) + 4 * (c >> 2) + (lane & 3), m = bt * kRows + r;
-              if (r >= kRows || m >= p.M || n >= p.N) continue;
+            const int n = n0 + 16 * q + col;
+#pragma unroll 1
+            for (int i = 0; i < 4; ++i) {
+              const int m = m0 + r0 + 8 * i;
+              const float *v = my_out + ((lane >> 2) + 8 * i) * 16 + (col ^ (4 * ((lane >> 3) & 3)));
+              if (m >= p.M || n >= p.N) continue;
               float *dst = row_of(m) + n;
               if (n + 4 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
-                *reinterpret_cast<float4 *>(dst) = x[c];
+                *reinterpret_cast<float4 *>(dst) = *reinterpret_cast<const float4 *>(v);
               } else {
-                const float v[4] = {x[c].x, x[c].y, x[c].z, x[c].w};
-#pragma unroll
                 for (int k = 0; k < 4; ++k)
                   if (n + k < p.N) dst[k] = v[k];
               }
@@ -565,14 +866,19 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       }
     }
     if (alive && table_bt >= 0) flush_stats(table_bt);
+  } else {
+    cudaGridDependencySynchronize();
+  }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  pair_barrier();   // no CTA leaves, or gives its tensor memory back, while the other's MMAs and arrivals can still reach it
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols));
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(uint32_t(kTmemColumns)));
   }
   if (threadIdx.x == 0 && *abort_word && p.error_flag) atomicExch(p.error_flag, 1);
+  pair_barrier();
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -604,9 +910,7 @@ struct Blocks { static constexpr int value = kN; };
 template <int kCols>
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t *r) {
   if constexpr (kCols == 8) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr) : "memory");
+    tmem_ld8(taddr, r);
   } else if constexpr (kCols == 16) {
     tmem_ld16(taddr, r);
   } else {
@@ -937,29 +1241,51 @@ bool make_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, 
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int kRows, int kVocab>
 cudaError_t launch_head(const CUtensorMap &mw, const CUtensorMap &ma, const HeadArgs &p, int sms, cudaStream_t stream) {
-  using Smem = HeadSmem<kRows, kVocab>;
-  const int stages = Smem::stages(p.K / kTileK, p.group);
-  if (stages < 2) return cudaErrorInvalidValue;
-  const size_t smem = Smem::fixed_bytes(p.K / kTileK) + size_t(stages) * Smem::kStageBytes * p.group;
   HeadArgs q = p;
-  q.stages = stages;
+  q.stages = HeadSmem::stages(p.K / kTileK, p.group);
+  if (q.stages < 2) return cudaErrorInvalidValue;
+  const size_t smem = HeadSmem::fixed_bytes(p.K / kTileK) + size_t(q.stages) * HeadSmem::kStageBytes * p.group;
   static thread_local int configured = -1;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (configured != dev) {
-    e = cudaFuncSetAttribute(head_fp8_kernel<kRows, kVocab>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    e = cudaFuncSetAttribute(head_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
     configured = dev;
   }
-  if (smem > 227 * 1024) return cudaErrorInvalidValue;
-  const int b_tiles = (p.M + kRows - 1) / kRows;
-  const int tiles = ((p.N + kVocab - 1) / kVocab) * b_tiles;
-  int grid = tiles < sms ? tiles : sms;
-  if (b_tiles <= grid) grid -= grid % b_tiles;  // every CTA then keeps one batch tile (and its scale table) for good
-  return launch_early(head_fp8_kernel<kRows, kVocab>, grid, kHeadThreads, smem, stream, mw, ma, q);
+  const int tiles = (p.N + 127) / 128;   // one batch tile
+  return launch_early(head_fp8_kernel, tiles < sms ? tiles : sms, kHeadThreads, smem, stream, mw, ma, q);
+}
+
+cudaError_t launch_pairs(const CUtensorMap &mw, const CUtensorMap &ma, const HeadArgs &p, int sms, cudaStream_t stream) {
+  HeadArgs q = p;
+  q.stages = PairSmem::stages(p.K / kTileK);
+  if (q.stages < 2) return cudaErrorInvalidValue;
+  static thread_local int configured = -1;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (configured != dev) {
+    e = cudaFuncSetAttribute(head_fp8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return e;
+    configured = dev;
+  }
+  const int b_tiles = (p.M + 255) / 256, tiles = ((p.N + 255) / 256) * b_tiles;
+  int pairs = tiles < sms / 2 ? tiles : sms / 2;
+  if (b_tiles <= pairs) pairs -= pairs % b_tiles;  // every CTA then keeps one batch tile (and its scale table) for good
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(2 * pairs));
+  cfg.blockDim = dim3(kPairThreads);
+  cfg.dynamicSmemBytes = PairSmem::fixed_bytes(p.K / kTileK) + size_t(q.stages) * PairSmem::kStageBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1] = programmatic_launch();
+  cfg.attrs = attr; cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, head_fp8_pair_kernel, mw, ma, q);
 }
 
 template <int kRows>
@@ -1077,21 +1403,23 @@ int run_head(const void *a_e4m3, const float *a_scale, const void *w_e4m3, const
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return int(e);
-  constexpr int kDecodeRows = 64;
-  const int cols = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
-  // Vocabulary tile: 256 wide once the batch spans several tiles (then the kernel is bound by L2 -> shared-memory
-  // copies and a wider tile re-reads the activations half as often), else 128.
-  const int vocab_tile = (M > 128 && N >= 256) ? 256 : 128;
-  // K blocks per stage: the largest of 4, 2, 1 that divides K/128 and still leaves a ring of at least 2 stages
-  // (measured: longer contiguous runs per weight row beat a deeper ring of shorter ones)
   const int kblocks = K / kTileK;
+  CUtensorMap mw, ma;
+  if (M > 128) {
+    if (!make_map(&mw, w_e4m3, uint64_t(N), uint64_t(K), 128, 1) || !make_map(&ma, a_e4m3, uint64_t(M), uint64_t(K), 128, 1))
+      return invalid("cuTensorMapEncodeTiled failed");
+    return int(launch_pairs(mw, ma, p, sms, stream));
+  }
+  const int rows = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
+  // K blocks per stage: the largest number that divides K/128 and still leaves a ring of at least 2 stages (longer contiguous
+  // runs per weight row and fewer hand-overs beat a deeper ring of shorter stages; 64 rows take at most two, whose columns an epilogue
+  // thread has the registers for)
   auto ring = [&](int g) {
-    return vocab_tile == 256 ? HeadSmem<128, 256>::stages(kblocks, g)
-         : cols == 16 ? DecodeSmem<16>::stages(kblocks, g) : cols == 32 ? DecodeSmem<32>::stages(kblocks, g)
-         : cols == 64 ? DecodeSmem<64>::stages(kblocks, g) : HeadSmem<128, 128>::stages(kblocks, g);
+    return rows == 16 ? DecodeSmem<16>::stages(kblocks, g) : rows == 32 ? DecodeSmem<32>::stages(kblocks, g)
+         : rows == 64 ? DecodeSmem<64>::stages(kblocks, g) : HeadSmem::stages(kblocks, g);
   };
   int group = 1;
-  const int most = M > kDecodeRows || cols <= 32 ? 4 : 2;
+  const int most = rows == 64 ? DecodeSmem<64>::kMaxGroup : 4;
   for (int g = most; g > 1; g >>= 1)
     if (kblocks % g == 0 && ring(g) >= 2) { group = g; break; }
   if (const char *forced = getenv("DS41_HEAD_GROUP")) {
@@ -1099,16 +1427,14 @@ int run_head(const void *a_e4m3, const float *a_scale, const void *w_e4m3, const
     if ((g == 1 || g == 2 || g == 4) && g <= most && kblocks % g == 0 && ring(g) >= 2) group = g;
   }
   p.group = group;
-  CUtensorMap mw, ma;
-  if (!make_map(&mw, w_e4m3, uint64_t(N), uint64_t(K), uint32_t(vocab_tile), uint32_t(group)) ||
-      !make_map(&ma, a_e4m3, uint64_t(M), uint64_t(K), uint32_t(cols), uint32_t(group)))
+  if (!make_map(&mw, w_e4m3, uint64_t(N), uint64_t(K), 128, uint32_t(group)) ||
+      !make_map(&ma, a_e4m3, uint64_t(M), uint64_t(K), uint32_t(rows), uint32_t(group)))
     return invalid("cuTensorMapEncodeTiled failed");
-  if (vocab_tile == 256) return int(launch_head<128, 256>(mw, ma, p, sms, stream));
-  if (M > kDecodeRows) return int(launch_head<128, 128>(mw, ma, p, sms, stream));
-  switch (cols) {
+  switch (rows) {
     case 16: e = launch_decode<16>(mw, ma, p, sms, stream); break;
     case 32: e = launch_decode<32>(mw, ma, p, sms, stream); break;
-    default: e = launch_decode<64>(mw, ma, p, sms, stream); break;
+    case 64: e = launch_decode<64>(mw, ma, p, sms, stream); break;
+    default: e = launch_head(mw, ma, p, sms, stream); break;
   }
   return int(e);
 }

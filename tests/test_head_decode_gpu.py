@@ -1,4 +1,4 @@
-"""The FP8 head for batches of up to 64 rows (csrc/head_fp8.cu, head_fp8_decode_kernel): batch sizes around its tiles of 16, 32
+"""The kernels of the FP8 head (csrc/head_fp8.cu).  Up to 64 rows (head_fp8_decode_kernel): batch sizes around its tiles of 16, 32
 and 64 rows and around the halves that a tile is split into, vocabularies whose last tile is cut and that take a CTA several
 tiles, stages of one, two and four K blocks; with the row records, against the product in 64 bits."""
 import numpy as np
@@ -25,6 +25,18 @@ def unorder(o):
 @pytest.mark.parametrize("N,K", [(129, 128), (1000, 512), (20011, 384), (40000, 256), (300, 16384)])
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 63, 64, 65])
 def test_product_and_records(pkg, M, N, K):
+    check_product_and_records(pkg, M, N, K)
+
+
+@pytest.mark.parametrize("N,K", [(100, 128), (257, 512), (20011, 384), (40000, 256), (300, 16384)])
+@pytest.mark.parametrize("M", [127, 128, 129, 256, 257, 385, 700])
+def test_larger_batches(pkg, M, N, K):
+    """Around one CTA's 128 rows and a pair's 256 (head_fp8_kernel, head_fp8_pair_kernel): a second half without rows, several batch
+    tiles, vocabularies shorter than a tile, fewer K blocks than stages."""
+    check_product_and_records(pkg, M, N, K)
+
+
+def check_product_and_records(pkg, M, N, K):
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     x = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
     blocks, kb = (N + 127) // 128, K // 128
