@@ -240,6 +240,11 @@ __device__ __forceinline__ RowCtx make_ctx(RowSmem *s, int vocab) {
 __device__ __forceinline__ void cluster_announce() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_await() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
 
+// The two halves of a barrier of the cluster, for a CTA that has nothing more to do with the others' shared memory (nor they with
+// its own) but goes on by itself: behind its arrival the others may leave, or begin their next row.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_complete() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
 // All-gather of one Slot per CTA.  Every thread of the CTA must pass the same `mine`.  Two buffers alternate, so a
 // fast CTA's next exchange cannot overwrite values a slower CTA is still reading (a third exchange can only start
 // after the second one's cluster barrier, which every CTA reaches after it has finished reading the first).

@@ -82,8 +82,9 @@ __device__ __forceinline__ int warp_find(int lane, const double *run, int n, Sto
 }
 
 // cutoff: a logit that at least top_k ids of the row reach (from the CTAs' sampled thresholds; -inf: none known).  `draw`: draw a token with uniform u; otherwise only the statistics are produced.
+// release: the CTAs that have no part in the end of the row do not wait for it.
 __device__ __forceinline__ FastOutcome fast_small_support(RowCtx &c, float max_logit, double t, int allowed, int top_k,
-                                                          double top_p, float cutoff, double u, bool draw) {
+                                                          double top_p, float cutoff, double u, bool draw, bool release) {
   RowSmem *s = c.s;
   FastOutcome out{};
   const bool count_mode = top_k > 0 && top_k < allowed;
@@ -186,6 +187,7 @@ __device__ __forceinline__ FastOutcome fast_small_support(RowCtx &c, float max_l
   unsigned long long *keys = s->work.n.sorted;
   const Lists lists(c);
   for (int i = c.tid; i < n; i += kThreads) s->work.n.all[i] = lists.key(c, i);
+  if (release) cluster_arrive();   // the row is this CTA's alone from here on, a quarter of its time: the others need not wait for it
   __syncthreads();
   for (int i0 = 0; i0 < n; i0 += kThreads / 4) {
     const int i = i0 + (c.tid >> 2);

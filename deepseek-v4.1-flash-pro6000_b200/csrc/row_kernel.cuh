@@ -43,6 +43,7 @@ struct RowArgs {
   int only_uncovered;  // 1: process only rows the streaming path reported as not covered, leave the others alone
   const int *pending;  // optional, with only_uncovered: number of such rows; 0 = nothing to do, every CTA returns at once
   int rows;            // set by launch_rows: a cluster walks rows cluster, cluster + clusters, ... below this
+  int resident;        // set by launch_rows: about as many clusters run at a time; rows this far on wait for a place
 };
 
 // Region sums of a non-negative per-id value (value(j) for local index j < len, 0 for ids outside the support):
@@ -535,9 +536,15 @@ __device__ __forceinline__ bool row_body(const RowArgs &a, RowCtx &c, RowSmem *s
       }
       recorded = true;
     } else {
-      const FastOutcome f = fast_small_support(c, max_logit, t, allowed, a.top_k, a.top_p, cutoff, draw ? s->u : 0.0, draw);
+      const FastOutcome f = fast_small_support(c, max_logit, t, allowed, a.top_k, a.top_p, cutoff, draw ? s->u : 0.0, draw,
+                                               row + a.resident < a.rows);
       if (f.applicable) {
         decided = true;
+        if (row + a.resident < a.rows && c.rank == 0) {   // (it has arrived at the barrier that the others end the row with)
+          cluster_complete();
+          __syncthreads();               // (its other warps do not begin the next row beside the one that ends this one)
+          closed = true;
+        }
         status = f.status; token = f.token; cut = f.cut; kept = f.kept; entered = f.entered; z = f.z; e_kept = f.e_kept;
       }
     }

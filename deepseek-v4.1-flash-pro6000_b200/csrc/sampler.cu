@@ -17,6 +17,11 @@ namespace ds41 {
 // fill it at 112 to 120 CTAs already; rows of one or two CTAs at 148 (144 CTAs 25.6 / 29.9, 160 46.2 / 37.9).  96 is below both.
 constexpr int kOnePerSm = 96;
 
+// CTAs that the GPU holds at a time, two per SM.  A cluster lets its CTAs go before the end of its row only where another row waits for
+// their place: 256 constrained rows 209 -> 194 us.  Without one it is the next launch that moves in, around the CTAs that are still
+// at work, and lies badly: 32 rows 21.9 -> 26.8 us in a row of launches.
+constexpr int kResidentCtas = 296;
+
 int cluster_size_for(int vocab) {
   int n = 1;
   while (n < kMaxCluster && vocab > n * kSliceCap) n <<= 1;
@@ -55,6 +60,7 @@ cudaError_t launch_rows(const RowArgs &a, int rows, cudaStream_t stream) {
   const int cl = cluster_size_for(a.vocab);
   RowArgs args = a;
   args.rows = rows;
+  args.resident = kResidentCtas / cl;
   if (!args.logits2) args.split = rows;
   if (!(args.bound_scale > 0)) args.bound_scale = 1.0;
   if (a.temperature > 0) {
