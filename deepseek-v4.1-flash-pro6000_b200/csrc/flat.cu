@@ -6,6 +6,7 @@
 //                                    that adds 1 to the bin's count and the id's place inside the bin (0..127) to the
 //                                    bin's place sum.  Count and first moment bracket the bin's mass from both sides
 //                                    (Jensen below, the chord above) to a few 1e-5.
+//   (smaller batches: flat_front_kernel, one cluster per row, does what these two and the next one do in one launch)
 //   flat_window_kernel  (row)        bracketed running mass -> the window of bins that provably holds the top-p crossing,
 //                                    exact id counts before and inside it.  Rows this path does not fit get status -8
 //                                    (the caller sends them to the other paths), non-finite rows -1.
@@ -21,6 +22,7 @@
 
 #include "launch.h"
 #include "phase_events.h"
+#include "cluster.cuh"
 #include "window.cuh"
 
 namespace ds41 {
@@ -189,6 +191,20 @@ __global__ void __launch_bounds__(kFT) flat_hist_kernel(FlatArgs a) {
   if (threadIdx.x == 0 && seen != end - begin) atomicOr(&a.s.lcount[row * 4 + 1], 1);
 }
 
+// The window [w0, w1] (w0 = 0x7fffffff: none was found) with the ids before and through it.
+__device__ __forceinline__ void window_found(const FlatArgs &a, FlatInfo &info, float m, float scale, int w0, int w1, int before, int through) {
+  const int inside = through - before;
+  // the mass pass draws the window a quarter of a bin wider on both sides; what does not fit the list it reports itself
+  const bool ok = w0 != 0x7fffffff && w1 >= w0 && inside >= 1 && inside <= kFlatList;
+  info.applicable = ok ? 1 : 0; info.w0 = w0; info.w1 = w1; info.n_before = before; info.n_window = inside;
+  info.pad[1] = ok ? 0 : 1;
+  if (ok) {
+    const double quarter = double(kFlatFrac / 4);
+    info.y_sure = float(double(m) - (double(kFlatFrac) * w0 - quarter) / double(scale));
+    info.y_tail = float(double(m) - (double(kFlatFrac) * (w1 + 1) + quarter) / double(scale));
+  }
+}
+
 __global__ void __launch_bounds__(kFlatWindowThreads) flat_window_kernel(FlatArgs a) {
   constexpr int kWarpsHere = kFlatWindowThreads / 32, kPer = kFlatBins / kFlatWindowThreads;  // 8 consecutive bins per thread
   __shared__ double part_lo[kWarpsHere], part_hi[kWarpsHere];
@@ -214,8 +230,8 @@ __global__ void __launch_bounds__(kFlatWindowThreads) flat_window_kernel(FlatArg
       info.applicable = usable ? 1 : 0;
       info.w0 = kFlatBins; info.w1 = kFlatBins - 1; info.n_before = a.vocab; info.n_window = 0;
       info.y_sure = -CUDART_INF_F; info.y_tail = CUDART_INF_F;  // every (finite) logit is before the window
+      if (!usable) { info.pad[1] = 1; leave_row(a, row, kNotCovered); }
       a.s.info[row] = info;
-      if (!usable) { leave_row(a, row, kNotCovered); atomicAdd(a.s.pending, 1); }
     }
     return;
   }
@@ -269,19 +285,181 @@ __global__ void __launch_bounds__(kFlatWindowThreads) flat_window_kernel(FlatArg
   }
   __syncthreads();
   if (tid == 0) {
-    const int w0 = first[0];
     const bool ends = first[1] == 0x7fffffff;   // never surely reached: the window runs to the end
-    const int w1 = ends ? kFlatBins - 1 : first[1], before = ids[0], inside = (ends ? a.vocab : ids[1]) - before;
-    // the mass pass draws the window a quarter of a bin wider on both sides; what does not fit the list it reports itself
-    const bool ok = w0 != 0x7fffffff && w1 >= w0 && inside >= 1 && inside <= kFlatList;
-    info.applicable = ok ? 1 : 0; info.w0 = w0; info.w1 = w1; info.n_before = before; info.n_window = inside;
-    if (ok) {
-      const double quarter = double(kFlatFrac / 4);
-      info.y_sure = float(double(b.m) - (double(kFlatFrac) * w0 - quarter) / double(b.scale));
-      info.y_tail = float(double(b.m) - (double(kFlatFrac) * (w1 + 1) + quarter) / double(b.scale));
-    }
+    window_found(a, info, b.m, b.scale, first[0], ends ? kFlatBins - 1 : first[1], ids[0], ends ? a.vocab : ids[1]);
+    if (info.pad[1]) leave_row(a, row, kNotCovered);
     a.s.info[row] = info;
-    if (!ok) { leave_row(a, row, kNotCovered); atomicAdd(a.s.pending, 1); }
+  }
+}
+
+// The front of the path for batches that leave the GPU idle between its passes: statistics (unless the head left them), histogram and
+// window search of a row by one cluster of eight CTAs.  A slice is read once, into registers, and the CTAs agree through their
+// shared memory: no partial results, no merging with global atomics, and nothing to clear in front (a memset would also wait for
+// everything in front of it).  Bound by latency: a slice's load, 16160 shared-memory atomics per CTA and three or four barriers.
+constexpr int kFrontRanks = 8;                 // CTAs per row, of 32 ids a thread
+static_assert(kFrontRanks * 32 * kFT >= kFlatSub * kFlatSubs, "a row fits");
+struct FrontExtremes { float max, min; int argmax, flags; };
+struct FrontTotals { double lo, hi; int n, pad[3]; };
+template <bool kKnown>
+__global__ void __launch_bounds__(kFT, 2) flat_front_kernel(const __grid_constant__ FlatArgs a) {
+  constexpr int kShare = kFlatBins / kFrontRanks, kShareWarps = kShare / 32;   // bins that this CTA totals, one per thread
+  __shared__ unsigned bins[kFlatBins];
+  __shared__ __align__(16) FrontExtremes extremes, warp_extremes[kFW];
+  __shared__ __align__(16) FrontTotals totals;
+  __shared__ double part_lo[kShareWarps], part_hi[kShareWarps];
+  __shared__ int part_n[kShareWarps];
+  __shared__ FlatPartial ext;
+  __shared__ struct { float m, scale; double kappa; int ok; } map;
+  __shared__ unsigned long long found[2];        // of rank 0: first bin that may / surely reaches the target << 32 | ids before / through it
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = int(cluster_rank()), row = blockIdx.x / kFrontRanks;
+  for (int j = tid; j < kFlatBins; j += kFT) bins[j] = 0u;
+  if (tid < 2) found[tid] = ~0ull;
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+  if (blockIdx.x == 0 && tid < 4) a.s.pending[tid] = 0;            // (counted in from the resolve kernel on)
+  if (rank == 0 && tid < 4) a.s.lcount[row * 4 + tid] = 0;
+  const int stride = ((a.vocab + kFrontRanks - 1) / kFrontRanks + 3) & ~3;
+  const int begin = min(a.vocab, rank * stride), len = min(a.vocab, begin + stride) - begin;
+  const float *x = row_logits(a, row) + begin;
+  const bool aligned = row_aligned(x);
+  // id 4 (tid + 512 i) + k of the slice
+  auto fetch = [&](int i) {
+    const int id = 4 * (tid + kFT * i);
+    if (id + 4 <= len) return load4(x + id, aligned);
+    const float none = __int_as_float(0x7fffffff);   // beyond the slice; the places are told apart by `id`
+    return make_float4(id < len ? load_input(x + id) : none, id + 1 < len ? load_input(x + id + 1) : none,
+                       id + 2 < len ? load_input(x + id + 2) : none, none);
+  };
+  auto each = [&](const float4 &q, int i, auto f) {
+    const int id = 4 * (tid + kFT * i);
+    if (id + 4 <= len) { f(q.x, id); f(q.y, id + 1); f(q.z, id + 2); f(q.w, id + 3); }
+    else { if (id < len) f(q.x, id); if (id + 1 < len) f(q.y, id + 1); if (id + 2 < len) f(q.z, id + 2); }
+  };
+  float4 v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = fetch(i);
+  if constexpr (kKnown) {
+    if (tid == 0) ext = row_extremes(a, row);
+  } else {
+    float best = -CUDART_INF_F, low = CUDART_INF_F, poison = 0.f;
+    int id_best = 0x7fffffff;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      each(v[i], i, [&](float y, int id) {
+        poison = fmaf(y, 0.f, poison);           // NaN once a logit is NaN or infinite
+        if (y > best) { best = y; id_best = id; }
+        low = fminf(low, y);
+      });
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, id_best, o);
+      if (ov > best || (ov == best && oi < id_best)) { best = ov; id_best = oi; }
+      low = fminf(low, __shfl_xor_sync(0xffffffffu, low, o));
+    }
+    const bool bad = __any_sync(0xffffffffu, !(poison == 0.f));
+    if (lane == 0) warp_extremes[warp] = FrontExtremes{best, low, id_best, bad ? 1 : 0};
+    __syncthreads();
+    auto reduce = [&](FrontExtremes e) {         // over the lanes of a warp; ids ascend with the lanes' sources
+#pragma unroll
+      for (int o = 16; o; o >>= 1) {
+        const float om = __shfl_xor_sync(0xffffffffu, e.max, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, e.argmax, o);
+        if (om > e.max || (om == e.max && oi < e.argmax)) { e.max = om; e.argmax = oi; }
+        e.min = fminf(e.min, __shfl_xor_sync(0xffffffffu, e.min, o));
+      }
+      e.flags = int(__reduce_or_sync(0xffffffffu, unsigned(e.flags)));
+      return e;
+    };
+    if (warp == 0) {
+      FrontExtremes e = reduce(warp_extremes[lane & (kFW - 1)]);
+      if (e.argmax != 0x7fffffff) e.argmax += begin;
+      if (lane == 0) extremes = e;
+    }
+    cluster_barrier();
+    if (warp == 0) {
+      const uint4 q = peer_load_u128(peer_addr(&extremes, lane & (kFrontRanks - 1)));
+      const FrontExtremes e = reduce(FrontExtremes{__uint_as_float(q.x), __uint_as_float(q.y), int(q.z), int(q.w)});
+      if (lane == 0) ext = FlatPartial{e.max, e.min, e.argmax, e.flags};
+    }
+  }
+  if (tid == 0) {
+    const FlatMap b = make_map(ext.max, ext.min, a.log2e_t);
+    map.m = b.m; map.scale = b.scale; map.kappa = b.kappa; map.ok = b.ok && !ext.flags ? 1 : 0;
+  }
+  __syncthreads();
+  const bool placed = map.ok != 0;               // the same in every CTA
+  if (placed) {
+    FlatMap b;
+    b.m = map.m; b.scale = map.scale;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) each(v[i], i, [&](float y, int) { bin_add(bins, y, b); });
+  }
+  cluster_barrier();                             // every CTA's histogram is complete
+  double lo = 0, hi = 0, run_lo = 0, run_hi = 0;
+  int n = 0, run_n = 0;
+  if (placed && tid < kShare) {
+    unsigned w[kFrontRanks], sum = 0;
+#pragma unroll
+    for (int r = 0; r < kFrontRanks; ++r) w[r] = peer_load_u32(peer_addr(&bins[rank * kShare + tid], r));
+#pragma unroll
+    for (int r = 0; r < kFrontRanks; ++r) { n += int(w[r] >> 18); sum += w[r] & 0x3ffffu; }
+    const BinBracket bracket(map.kappa);
+    double e[2];
+    bracket.prefactors(rank * kShare + tid, e);
+    bracket.mass(e, double(n), double(sum), &lo, &hi);
+    run_lo = lanes_scan(lane, lo); run_hi = lanes_scan(lane, hi); run_n = lanes_scan(lane, n);
+    if (lane == 31) { part_lo[warp] = run_lo; part_hi[warp] = run_hi; part_n[warp] = run_n; }
+    run_lo -= lo; run_hi -= hi; run_n -= n;
+  }
+  __syncthreads();
+  if (placed && tid < kShare) {
+    const bool in = lane < kShareWarps;
+    const double wl = lanes_scan(lane, in ? part_lo[lane] : 0.0), wh = lanes_scan(lane, in ? part_hi[lane] : 0.0);
+    const int wn = lanes_scan(lane, in ? part_n[lane] : 0);
+    if (warp > 0) {
+      run_lo += __shfl_sync(0xffffffffu, wl, warp - 1); run_hi += __shfl_sync(0xffffffffu, wh, warp - 1);
+      run_n += __shfl_sync(0xffffffffu, wn, warp - 1);
+    }
+    if (tid == 31) totals = FrontTotals{wl, wh, wn, {0, 0, 0}};
+  }
+  cluster_barrier();                             // every CTA's totals are there
+  int counted = 0;
+  if (placed && tid < kShare) {
+    const uint32_t from = peer_addr(&totals, lane & (kFrontRanks - 1));
+    const uint4 q = peer_load_u128(from);
+    const bool in = lane < kFrontRanks;
+    const double l = __hiloint2double(int(q.y), int(q.x)), h = __hiloint2double(int(q.w), int(q.z));
+    const double sl = lanes_scan(lane, in ? l : 0.0), sh = lanes_scan(lane, in ? h : 0.0);
+    const int sn = lanes_scan(lane, in ? int(peer_load_u32(from + 16)) : 0);
+    if (rank > 0) {
+      run_lo += __shfl_sync(0xffffffffu, sl, rank - 1); run_hi += __shfl_sync(0xffffffffu, sh, rank - 1);
+      run_n += __shfl_sync(0xffffffffu, sn, rank - 1);
+    }
+    counted = __shfl_sync(0xffffffffu, sn, 31);
+    // (the allowances as in flat_window_kernel)
+    const double t_lo = a.top_p * __shfl_sync(0xffffffffu, sl, 31) * (1.0 - 1e-9), t_hi = a.top_p * __shfl_sync(0xffffffffu, sh, 31) * (1.0 + 1e-9);
+    const int bin = rank * kShare + tid;
+    if (run_hi < t_lo && run_hi + hi >= t_lo) peer_store_u64(peer_addr(&found[0], 0), (unsigned long long)(unsigned(bin)) << 32 | unsigned(run_n));
+    if (run_lo < t_hi && run_lo + lo >= t_hi) peer_store_u64(peer_addr(&found[1], 0), (unsigned long long)(unsigned(bin)) << 32 | unsigned(run_n + n));
+  }
+  cluster_barrier();                             // (also: nobody reads another CTA's shared memory any more)
+  if (rank == 0 && tid == 0) {
+    FlatInfo info{};
+    info.max = ext.max; info.min = ext.min; info.argmax = ext.argmax;
+    if (ext.flags) {
+      leave_row(a, row, -1);
+    } else if (!placed || counted != a.vocab) {  // no range to place the ids on; a bin's word that overflowed
+      info.w0 = kFlatBins; info.w1 = kFlatBins - 1; info.n_before = a.vocab;
+      info.pad[1] = 1;
+    } else {
+      const unsigned long long f0 = found[0], f1 = found[1];
+      const bool ends = f1 == ~0ull;             // never surely reached: the window runs to the end
+      window_found(a, info, map.m, map.scale, f0 == ~0ull ? 0x7fffffff : int(unsigned(f0 >> 32)),
+                   ends ? kFlatBins - 1 : int(unsigned(f1 >> 32)), int(unsigned(f0)), ends ? a.vocab : int(unsigned(f1)));
+    }
+    if (info.pad[1]) leave_row(a, row, kNotCovered);
+    a.s.info[row] = info;
   }
 }
 
@@ -435,7 +613,10 @@ __global__ void __launch_bounds__(kRT4) flat_resolve_kernel(FlatArgs a) {
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();
   const FlatInfo info = a.s.info[row];
-  if (!info.applicable) return;
+  if (!info.applicable) {
+    if (tid == 0 && info.pad[1]) atomicAdd(a.s.pending, 1);
+    return;
+  }
   const int listed = a.s.lcount[row * 4], flags = a.s.lcount[row * 4 + 1];
   const float *x = row_logits(a, row);
   const bool full = info.w0 >= kFlatBins;  // top_p = 1: every id is kept
@@ -675,6 +856,14 @@ FlatInfo *flat_info(void *scratch, int rows) {
   return reinterpret_cast<FlatInfo *>(static_cast<unsigned char *>(scratch) + 4 * sizeof(int) + size_t(rows) * before);
 }
 
+// Up to this many rows flat_front_kernel takes the place of three passes and the clearing in front of them.  Some 32 rows are at work at
+// a time, each as long as a chain of barriers takes, while the passes fill the GPU whatever the batch: whole calls at 129280 ids, us,
+// front / passes: 49 rows 44 / 67, 64 48 / 58, 100 66 / 73, 120 77 / 84, 160 96 / 91, 256 148 / 130 (40000 ids: 64 rows 42 / 51);
+// verification of 45 logits rows 46 / 68, 110 rows 81 / 89, 160 rows 107 / 102; with the head's records, which spare the passes one
+// of them, a decode step of 49 rows 132 / 139, 64 141 / 143, 100 174 / 175, 128 191 / 186.  Up to 32768 ids the cluster kernel takes
+// batches of these sizes (sampler.cu).
+constexpr int kFrontMinVocab = 32768, kFrontRows = 130, kFrontRowsKnown = 100;
+
 cudaError_t launch_flat(FlatArgs a, void *scratch, cudaStream_t stream) {
   if (!a.logits2) a.split = a.rows;
   a.log2e_t = kLog2e / a.t;
@@ -696,17 +885,35 @@ cudaError_t launch_flat(FlatArgs a, void *scratch, cudaStream_t stream) {
   while (parts < kFlatMaxParts && a.rows * parts < 1024) parts <<= 1;
   a.parts = parts;
   const bool full = a.top_p >= 1.0;
-  const size_t zeroed = 4 * sizeof(int) + rows * 4 * sizeof(int) + (parts > 1 && !full ? rows * kFlatBins * sizeof(unsigned long long) : 0);
-  cudaError_t e = cudaMemsetAsync(scratch, 0, zeroed, stream);
-  if (e != cudaSuccess) return e;
-  phase_restart();
-  phase_mark(stream);
-  if (!a.head_stats && (e = launch_early(flat_stats_kernel, a.rows * parts, kFT, 0, stream, a)) != cudaSuccess) return e;
-  phase_mark(stream);
-  if (!full && (e = launch_early(flat_hist_kernel, a.rows * parts, kFT, 0, stream, a)) != cudaSuccess) return e;
-  phase_mark(stream);
-  if ((e = launch_early(flat_window_kernel, a.rows, kFlatWindowThreads, 0, stream, a)) != cudaSuccess) return e;
-  phase_mark(stream);
+  cudaError_t e;
+  if (!full && a.vocab > kFrontMinVocab && a.rows <= (a.head_stats ? kFrontRowsKnown : kFrontRows)) {
+    phase_restart();
+    phase_mark(stream);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(a.rows) * kFrontRanks);
+    cfg.blockDim = dim3(kFT);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kFrontRanks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1] = programmatic_launch();
+    cfg.attrs = attr; cfg.numAttrs = 2;
+    e = a.head_stats ? cudaLaunchKernelEx(&cfg, flat_front_kernel<true>, a) : cudaLaunchKernelEx(&cfg, flat_front_kernel<false>, a);
+    if (e != cudaSuccess) return e;
+    for (int i = 0; i < 3; ++i) phase_mark(stream);   // (statistics, histogram and window search in one)
+  } else {
+    const size_t zeroed = 4 * sizeof(int) + rows * 4 * sizeof(int) + (parts > 1 && !full ? rows * kFlatBins * sizeof(unsigned long long) : 0);
+    e = cudaMemsetAsync(scratch, 0, zeroed, stream);
+    if (e != cudaSuccess) return e;
+    phase_restart();
+    phase_mark(stream);
+    if (!a.head_stats && (e = launch_early(flat_stats_kernel, a.rows * parts, kFT, 0, stream, a)) != cudaSuccess) return e;
+    phase_mark(stream);
+    if (!full && (e = launch_early(flat_hist_kernel, a.rows * parts, kFT, 0, stream, a)) != cudaSuccess) return e;
+    phase_mark(stream);
+    if ((e = launch_early(flat_window_kernel, a.rows, kFlatWindowThreads, 0, stream, a)) != cudaSuccess) return e;
+    phase_mark(stream);
+  }
   // the mass pass: four warps per CTA, one 1024-id sub-region per warp and round.  Six CTAs fit an SM (888 at a time on
   // the GPU), so the rows are cut into as many pieces as give about four waves or more: a grid of 1.4 waves (256 rows x
   // 4 pieces) left a third of the SMs idle through its second wave

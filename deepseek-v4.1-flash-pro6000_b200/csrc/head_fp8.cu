@@ -34,6 +34,7 @@
 // against one lane on its own path).
 // Every wait is bounded; on expiry the kernel raises *error_flag, frees its TMEM and returns.
 #include "ds41_b200.h"
+#include "cluster.cuh"
 #include "flat.cuh"
 #include "host_error.h"
 #include "launch.h"
@@ -53,7 +54,7 @@ constexpr int kTileK = 128;   // K elements per block = one 128-byte swizzle row
 constexpr int kEpiWarps = 16, kHeadThreads = 64 + 32 * kEpiWarps, kPairThreads = 128 + 32 * kEpiWarps;
 constexpr uint32_t kSpinLimit = 1u << 22;
 
-__device__ __forceinline__ uint32_t smem_addr(const void *p) { return uint32_t(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ uint32_t smem_addr(const void *p) { return shared_addr(p); }
 
 struct Abort {  // shared flag: once set every later wait returns immediately
   volatile int *flag;
@@ -212,21 +213,6 @@ __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigne
 }
 
 // ---- a pair of CTAs (a cluster of two) on one tile
-__device__ __forceinline__ uint32_t pair_rank() {
-  uint32_t r;
-  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// All threads of both CTAs: what each has done before is seen by the other behind it.
-__device__ __forceinline__ void pair_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// The address of the leading CTA's copy of a shared variable.
-__device__ __forceinline__ uint32_t in_leader(const void *p) {
-  uint32_t a;
-  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_addr(p)));
-  return a;
-}
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -616,7 +602,7 @@ head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   int *abort_word = reinterpret_cast<int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = int(pair_rank()), pair = int(blockIdx.x) >> 1, pairs = int(gridDim.x) >> 1;
+  const int rank = int(cluster_rank()), pair = int(blockIdx.x) >> 1, pairs = int(gridDim.x) >> 1;
   const int b_tiles = (p.M + 255) / 256, total_tiles = (p.N + 255) / 256 * b_tiles;
   // tile t = (vocabulary tile t / b_tiles, batch tile t % b_tiles)
   const int active = p.M > 128 ? 2 : 1;   // CTAs of a pair that have batch rows at all
@@ -634,7 +620,7 @@ head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  pair_barrier();   // both CTAs have started and set up their barriers
+  cluster_barrier();   // both CTAs have started and set up their barriers
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
 
@@ -655,7 +641,7 @@ head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       for (int s = 0; s < early; ++s) tma_prefetch_3d(&map_w, 0, pair / b_tiles * 256 + 128 * rank, s, policy);
       cudaGridDependencySynchronize();
       cudaTriggerProgrammaticLaunchCompletion();
-      const uint32_t leader_full = in_leader(full);
+      const uint32_t leader_full = peer_addr(full, 0);
       for (int tile = pair; tile < total_tiles && !ab.set(); tile += pairs) {
         const int id = tile / b_tiles * 256 + 128 * rank, first = tile % b_tiles * 256, mine = first + 128 * rank;
         // (a second half without batch rows is not fetched: what the MMA makes of the rows' place nobody reads)
@@ -717,7 +703,7 @@ head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     const int row = quad * 32 + lane;   // batch row inside the CTA's 128
     const int et = threadIdx.x - 128;
     const uint32_t lane_base = tmem_base + group * kCols + (uint32_t(quad * 32) << 16);
-    const uint32_t leader_empty = in_leader(acc_empty);
+    const uint32_t leader_empty = peer_addr(acc_empty, 0);
     float *my_sw = sw + size_t(warp - 4) * 2 * kblocks;
     float *my_out = out + (warp - 4) * Smem::kOutFloats;
     // fp32 scales of the 128-row weight block this warp's columns belong to, on their way into shared memory
@@ -872,13 +858,13 @@ head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  pair_barrier();   // no CTA leaves, or gives its tensor memory back, while the other's MMAs and arrivals can still reach it
+  cluster_barrier();   // no CTA leaves, or gives its tensor memory back, while the other's MMAs and arrivals can still reach it
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(uint32_t(kTmemColumns)));
   }
   if (threadIdx.x == 0 && *abort_word && p.error_flag) atomicExch(p.error_flag, 1);
-  pair_barrier();
+  cluster_barrier();
 }
 
 // ---------------------------------------------------------------------------------------------------------------
