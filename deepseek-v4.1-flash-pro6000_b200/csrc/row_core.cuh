@@ -26,6 +26,7 @@ constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
 constexpr int kSliceCap = 16384;   // fp32 logits staged per CTA
 constexpr int kMaxCluster = 8;     // portable cluster size
+constexpr int kResidentRows = 32;  // rows of that many CTAs that run at a time
 constexpr int kBins = 1024;        // histogram bins per search level
 constexpr int kListCap = 1024;     // candidates resolved exactly (sorted) at the cut
 constexpr int kMaxLevels = 6;

@@ -17,10 +17,11 @@ namespace ds41 {
 // fill it at 112 to 120 CTAs already; rows of one or two CTAs at 148 (144 CTAs 25.6 / 29.9, 160 46.2 / 37.9).  96 is below both.
 constexpr int kOnePerSm = 96;
 
-// CTAs that the GPU holds at a time, two per SM.  A cluster lets its CTAs go before the end of its row only where another row waits for
-// their place: 256 constrained rows 209 -> 194 us.  Without one it is the next launch that moves in, around the CTAs that are still
-// at work, and lies badly: 32 rows 21.9 -> 26.8 us in a row of launches.
-constexpr int kResidentCtas = 296;
+// Rows of one, two or eight CTAs that the GPU holds at a time, two CTAs per SM (clusters of eight have to lie within one part of the
+// GPU: four in each of eight).  A cluster lets its CTAs go before the end of its row only where another row waits for their place: 256
+// constrained rows 209 -> 192 us.  Without one it is the next launch that moves in, around the CTAs that are still at work, and lies
+// badly: 32 rows 21.9 -> 26.8 us in a row of launches.
+int resident_rows(int cl) { return cl == kMaxCluster ? kResidentRows : 296 / cl; }
 
 int cluster_size_for(int vocab) {
   int n = 1;
@@ -60,7 +61,7 @@ cudaError_t launch_rows(const RowArgs &a, int rows, cudaStream_t stream) {
   const int cl = cluster_size_for(a.vocab);
   RowArgs args = a;
   args.rows = rows;
-  args.resident = kResidentCtas / cl;
+  args.resident = resident_rows(cl);
   if (!args.logits2) args.split = rows;
   if (!(args.bound_scale > 0)) args.bound_scale = 1.0;
   if (a.temperature > 0) {
@@ -163,17 +164,19 @@ extern "C" const char *ds41_spark_error(void) { return last_error(); }
 
 namespace {
 // Up to this many rows the cluster kernel takes a batch in one launch; larger ones go through the batch path (top-p alone)
-// or the streaming path (top-k, greedy).  The two constants are drawn for 129280 ids; cluster kernel / other path, us: top-p 48
-// rows 61 / 73, 64 rows 72 / 64 (with the head's records, which spare the batch path a pass: 32 rows 37 / 42, 48 rows 54 / 50);
-// greedy 32 rows 10.0 / 10.6, 64 rows 18 / 15.  With fewer ids they are not where the two meet: the cluster kernel's cost follows
-// its CTAs per row (eight beyond 32768 ids, two beyond 16384, else one), the other path's the ids.  40000 ids: top-p 64 rows
-// 48 / 53, 96 rows 71 / 62; greedy 32 rows 8.8 / 9.0, 48 rows 15 / 11.  16384 and 32768 ids: top-p 192 rows still 39 / 57 and
-// 57 / 65, greedy 128 rows 7.3 / 8.4 and 9.7 / 9.8.
+// or the streaming path (top-k, greedy).  Cluster kernel / other path, us a call:
+// Top-p, rows of eight CTAs (beyond 32768 ids): the line is the number of such clusters that run at a time.  129280 ids: 20 rows 30 / 31,
+// 37 rows 52 / 40, 48 rows 54 / 43; 40000 ids: 20 rows 24 / 29, 37 rows 44 / 35; decode steps of 30 rows 114.5 / 119.4, of 37 rows 142 / 126.
+// With fewer ids a row takes one or two CTAs and the batch path as many launches: 16384 ids 192 rows 37 / 56, 256 rows 37 / 55; 24000 ids
+// 148 rows 32 / 53, 256 rows 58 / 61; 32768 ids 256 rows 63 / 67.
+// Greedy (drawn for 129280 ids): 32 rows 10.0 / 10.6, 64 rows 18 / 15; 40000 ids: 32 rows 8.8 / 9.0, 48 rows 15 / 11; 16384 and 32768
+// ids: 128 rows 7.3 / 8.4 and 9.7 / 9.8.
 // Rows cut by top-k cost the cluster kernel the same at any vocabulary of eight slices, and the streaming path what their ids
-// take to read: 129280 ids 140 rows 71 us against 76, 200 rows 100 against 95; 40000 ids 65 rows 31 against 41, 100 rows 50
-// against 45: the limit follows the line through the two.
-constexpr int kClusterRows = 48, kClusterRowsGreedy = 64;
-int cluster_rows_topk(int vocab) { return vocab > 32768 ? 44 + vocab / 1114 : 256; }
+// take to read: 40000 ids 160 rows 66 / 73, 200 rows 79 / 75; 129280 ids 200 rows 94 / 119, 256 rows 117 / 133 (and the two
+// meet, from their slopes, at about 345): the limit follows the line through the two.
+constexpr int kClusterRowsGreedy = 64;
+int cluster_rows(int vocab) { return vocab > 32768 ? kResidentRows : 256; }
+int cluster_rows_topk(int vocab) { return vocab > 32768 ? 113 + vocab / 558 : 256; }
 
 // One launch that decides every row, and, for rows cut by top-p alone, the replay of those it could not certify.
 int sample_by_clusters(RowArgs a, const ds41_b200_sample_args &p, cudaStream_t stream) {
@@ -224,7 +227,7 @@ extern "C" int ds41_b200_sample_logits(const ds41_b200_sample_args *p, cudaStrea
   // With scratch: small batches by the cluster kernel alone; larger ones of rows that are only cut by top-p first go through
   // the batch path, which answers the rows it fits and marks the others -8 / -9, and the paths below then only touch those.
   const bool top_p_only = p->top_k == 0 && p->temperature > 0;
-  const int by_clusters = top_p_only ? kClusterRows : p->temperature > 0 ? cluster_rows_topk(p->vocab) : kClusterRowsGreedy;
+  const int by_clusters = top_p_only ? cluster_rows(p->vocab) : p->temperature > 0 ? cluster_rows_topk(p->vocab) : kClusterRowsGreedy;
   if (scratch_ok && p->rows <= by_clusters) return sample_by_clusters(a, *p, stream);
   const bool flat = scratch_ok && flat_shape(p->rows, p->vocab) && top_p_only && p->logits_stride != 0;
   // the streaming path covers small nuclei only: a full-vocabulary draw never fits its candidate sets

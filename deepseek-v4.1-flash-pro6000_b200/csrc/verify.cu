@@ -215,11 +215,12 @@ __global__ void __launch_bounds__(kThreads, 2) verify_kernel(const __grid_consta
 
 namespace ds41 {
 namespace {
-// Up to this many rows the cluster kernel takes the statistics in one launch; beyond, the batch path's grid-wide passes do
-// (they need scratch).  Whole calls with either, us: 129280 ids 40 rows 56 / 63, 60 rows 68 / 83, 80 rows 90 / 73; 65536 ids 60 rows
-// 56 / 77, 80 rows 77 / 65: they meet at about 70 rows there, and the line lies below.  At 16384 and 32768 ids, one and two CTAs a
-// row, the cluster kernel is ahead up to 160 rows (49 / 63 and 64 / 67).
+// Up to this many rows the cluster kernel takes the statistics in one launch; beyond, the batch path's grid-wide passes do (they need
+// the scratch that begins with the 41st row).  Whole calls with either, us: 129280 ids 40 rows 61 / 51, 80 rows 91 / 66, 160 rows 155 /
+// 108; 40000 ids 40 rows 48 / 41, 80 rows 74 / 57 (they meet at 32 rows, where the clusters of eight CTAs no longer run all at a time).
+// Up to 32768 ids, one and two CTAs a row, the cluster kernel is ahead: 24000 ids 40 rows 32 / 61, 80 rows 41 / 60, 160 rows 61 / 64.
 constexpr int kClusterStatRows = 40;
+int cluster_stat_rows(int vocab) { return vocab > 32768 ? kClusterStatRows : 160; }
 // The scratch begins with the row statistics; the replay's rows follow, then the batch path's scratch.
 size_t verify_stats_bytes(int sequences, int drafts) {
   static_assert(sizeof(RowStats) % 16 == 0, "what follows is aligned");
@@ -275,7 +276,7 @@ extern "C" int ds41_b200_verify_logits(const ds41_b200_verify_args *p, cudaStrea
     }
   }
   cudaError_t e;
-  if (!greedy && stat_launch_rows > kClusterStatRows && p->vocab >= kFlatMinVocab &&
+  if (!greedy && stat_launch_rows > cluster_stat_rows(p->vocab) && p->vocab >= kFlatMinVocab &&
       p->scratch_bytes >= ds41_b200_verify_scratch_bytes_for(p->sequences, p->drafts, p->vocab)) {
     FlatArgs f{};
     f.logits = a.logits; f.logits2 = a.logits2; f.split = p->drafts ? a.split : stat_launch_rows;
