@@ -1391,6 +1391,19 @@ int run_head(const void *a_e4m3, const float *a_scale, const void *w_e4m3, const
   if (e != cudaSuccess) return int(e);
   const int kblocks = K / kTileK;
   CUtensorMap mw, ma;
+  // Three, five ... times 128 rows: what is behind the last whole pair tile would take half of one for its own, and goes to a launch
+  // by itself instead, by the kernel of its size.  One launch / two, us in a loop (128 x 256 tiles before: 289 to 317, 478 to 500, 652 to 662):
+  // 257 rows 340 / 262, 352 rows 345 / 311, 384 rows 352 / 318, 513 rows 521 / 429, 640 rows 523 / 486, 770 rows 685 / 609, 880 rows
+  // 684 / 661.  (Rows of several owners stay together: an owner's rows are told apart by their place in the batch.)
+  if (M > 256 && p.rows_per_owner == 0 && ((M + 127) / 128 & 1)) {
+    const int whole = M & ~255;
+    HeadArgs rest = p;
+    p.M = whole; rest.M = M - whole;
+    rest.a_scale += size_t(whole) * (K / kTileK); rest.logits += size_t(whole) * p.ldl;
+    if (rest.row_stats) rest.row_stats += whole;
+    const int rc = run_head(a_e4m3, a_scale, w_e4m3, w_scale, p, stream);
+    return rc ? rc : run_head(static_cast<const uint8_t *>(a_e4m3) + size_t(whole) * K, rest.a_scale, w_e4m3, w_scale, rest, stream);
+  }
   if (M > 128) {
     if (!make_map(&mw, w_e4m3, uint64_t(N), uint64_t(K), 128, 1) || !make_map(&ma, a_e4m3, uint64_t(M), uint64_t(K), 128, 1))
       return invalid("cuTensorMapEncodeTiled failed");
