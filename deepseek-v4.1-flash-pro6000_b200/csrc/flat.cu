@@ -479,8 +479,7 @@ __device__ __forceinline__ void flush_window(const FlatArgs &a, int row, int lan
 }
 
 // One sub-region by one warp, eight rounds of four ids per lane: *z, *sure (this lane's shares), and a bit (4 i + k: id k of
-// round i) for every id that lies in the window.  Two loads are consumed while the next two are in flight; two rounds per
-// trip, so that the two register sets alternate without copies.
+// round i) for every id that lies in the window.  Two loads are consumed while the next two are in flight.
 template <bool kWhole>
 __device__ __forceinline__ unsigned mass_sub_region(const float *x, int left, const RowWeights &w, float y_sure, float y_tail,
                                                     int lane, double *z_out, double *sure_out) {
@@ -502,22 +501,24 @@ __device__ __forceinline__ unsigned mass_sub_region(const float *x, int left, co
     z += (e[0] + e[1]) + (e[2] + e[3]);
     inside |= sort_out4(sure, e, y, y_sure, y_tail) << (4 * i);
   };
-  float4 a0 = fetch(0), a1 = fetch(1), b0, b1;
+  float4 a0 = fetch(0), a1 = fetch(1);
 #pragma unroll 1
-  for (int i = 0; i < 8; i += 4) {
-    b0 = fetch(i + 2); b1 = fetch(i + 3);
-    consume(a0, i); consume(a1, i + 1);
-    if (i == 0) { a0 = fetch(4); a1 = fetch(5); }
-    consume(b0, i + 2); consume(b1, i + 3);
+  for (int i = 0; i < 8; i += 2) {
+    float4 b0 = a0, b1 = a1;
+    if (i < 6) { a0 = fetch(i + 2); a1 = fetch(i + 3); }
+    consume(b0, i);
+    consume(b1, i + 1);
   }
   *z_out = z; *sure_out = sure;
   return inside;
 }
 
 // The FP64 pass: the weight of every id, per 1024-id sub-region the sum over all ids and over the ids before the window; a
-// warp takes a sub-region at a time.  Bound by issue slots (38 instructions per id) and by the FP64 and conversion
-// pipes, not by memory.
-__global__ void __launch_bounds__(kFlatMassThreads, 6) flat_mass_kernel(FlatArgs a) {
+// warp takes a sub-region at a time.  Bound by the latency of its loads, conversions and FP64 chains as much as by issue slots (38
+// instructions per id), not by memory: eight CTAs an SM with 64 registers and two loads ahead instead of six with 80 and four
+// take the sampling call of 1024 rows from 342 to 326 us, of 256 rows from 115 to 109.  (A table of 16 entries, free of bank
+// conflicts, with one more multiply-add: 350.)
+__global__ void __launch_bounds__(kFlatMassThreads, 8) flat_mass_kernel(FlatArgs a) {
   __shared__ double table[64];
   __shared__ WarpWindow windows[kFlatMassThreads / 32];
   if (threadIdx.x < 64) table[threadIdx.x] = kPow2Neg64[threadIdx.x];
@@ -914,11 +915,11 @@ cudaError_t launch_flat(FlatArgs a, void *scratch, cudaStream_t stream) {
     if ((e = launch_early(flat_window_kernel, a.rows, kFlatWindowThreads, 0, stream, a)) != cudaSuccess) return e;
     phase_mark(stream);
   }
-  // the mass pass: four warps per CTA, one 1024-id sub-region per warp and round.  Six CTAs fit an SM (888 at a time on
-  // the GPU), so the rows are cut into as many pieces as give about four waves or more: a grid of 1.4 waves (256 rows x
-  // 4 pieces) left a third of the SMs idle through its second wave
+  // the mass pass: four warps per CTA, one 1024-id sub-region per warp and round.  Eight CTAs fit an SM (1184 at a time on
+  // the GPU), so the rows are cut into as many pieces as give about three waves or more, down to a sub-region per warp (64 rows: 16
+  // pieces 50.9 us, 32 pieces 49.2, the whole call)
   int mass_parts = 4;
-  while (mass_parts < 16 && a.rows * mass_parts < 2960) mass_parts <<= 1;
+  while (mass_parts < 32 && a.rows * mass_parts < 3600) mass_parts <<= 1;
   FlatArgs m = a;
   m.parts = mass_parts;
   if ((e = launch_early(flat_mass_kernel, a.rows * mass_parts, kFlatMassThreads, 0, stream, m)) != cudaSuccess) return e;

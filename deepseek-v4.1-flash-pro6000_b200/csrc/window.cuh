@@ -118,7 +118,11 @@ __device__ __forceinline__ void row_weights(const float (&y)[kN], const RowWeigh
 #pragma unroll
   for (int k = 0; k < kN; ++k) t[k] = fma(d[k], w.k64, w.magic);
 #pragma unroll
-  for (int k = 0; k < kN; ++k) tb[k] = w.table[__double2loint(t[k]) & 63];
+  for (int k = 0; k < kN; ++k) {   // (the power of two goes to the table's entry, beside the polynomial's chain)
+    const int n = __double2loint(t[k]);
+    const double entry = w.table[n & 63];
+    tb[k] = __hiloint2double(__double2hiint(entry) - ((n & ~63) << 14), __double2loint(entry));
+  }
 #pragma unroll
   for (int k = 0; k < kN; ++k) d[k] = fma(d[k], w.k64, -(t[k] - w.magic));
 #pragma unroll
@@ -130,10 +134,7 @@ __device__ __forceinline__ void row_weights(const float (&y)[kN], const RowWeigh
 #pragma unroll
   for (int k = 0; k < kN; ++k) q[k] *= d[k];
 #pragma unroll
-  for (int k = 0; k < kN; ++k) {
-    const double x = fma(tb[k], q[k], tb[k]);
-    e[k] = __hiloint2double(__double2hiint(x) - ((__double2loint(t[k]) & ~63) << 14), __double2loint(x));
-  }
+  for (int k = 0; k < kN; ++k) e[k] = fma(tb[k], q[k], tb[k]);
 }
 // sum += e if y > sure; else, if y >= tail, bit kBit of mask is set.  Predicated, without selects.
 template <int kBit>
