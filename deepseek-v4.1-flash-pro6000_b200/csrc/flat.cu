@@ -102,12 +102,29 @@ __device__ __forceinline__ FlatPartial row_extremes(const FlatArgs &a, int row) 
   return r;
 }
 
+// What the kernels behind count in, by the threads of a row's piece: the pending rows, the row's list, and its histogram, which the pieces
+// add to if there are several.  (A memset instead would stand between two programmatic launches and wait for everything in front.)
+__device__ __forceinline__ void clear_piece(const FlatArgs &a, int row, int part) {
+  if (blockIdx.x == 0 && threadIdx.x < 4) a.s.pending[threadIdx.x] = 0;
+  if (part == 0 && threadIdx.x < 4) a.s.lcount[row * 4 + threadIdx.x] = 0;
+  if (a.parts > 1 && a.top_p < 1.0)
+    for (int j = threadIdx.x; j < kFlatBins / a.parts; j += blockDim.x)
+      a.s.hist[size_t(row) * kFlatBins + part * (kFlatBins / a.parts) + j] = 0ull;
+}
+// Where the head left the statistics no pass over the logits comes before the histogram's.
+__global__ void __launch_bounds__(kFT) flat_clear_kernel(FlatArgs a) {
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+  clear_piece(a, blockIdx.x / a.parts, blockIdx.x % a.parts);
+}
+
 __global__ void __launch_bounds__(kFT) flat_stats_kernel(FlatArgs a) {
   __shared__ FlatRed red;
   const int row = blockIdx.x / a.parts, part = blockIdx.x % a.parts;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();
+  clear_piece(a, row, part);
   int begin, end;
   piece(a, part, &begin, &end);
   const float *x = row_logits(a, row);
@@ -875,7 +892,7 @@ cudaError_t launch_flat(FlatArgs a, void *scratch, cudaStream_t stream) {
   if (!a.logits2) a.split = a.rows;
   a.log2e_t = kLog2e / a.t;
   a.floor_gap = float(650.0 / kLog2e * a.t);
-  // carve (every array is a multiple of 16 bytes per row; the zeroed ones come first, in one block)
+  // carve (every array is a multiple of 16 bytes per row)
   unsigned char *p = static_cast<unsigned char *>(scratch);
   const size_t rows = size_t(a.rows);
   a.s.pending = reinterpret_cast<int *>(p); p += 4 * sizeof(int);
@@ -909,12 +926,10 @@ cudaError_t launch_flat(FlatArgs a, void *scratch, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     for (int i = 0; i < 3; ++i) phase_mark(stream);   // (statistics, histogram and window search in one)
   } else {
-    const size_t zeroed = 4 * sizeof(int) + rows * 4 * sizeof(int) + (parts > 1 && !full ? rows * kFlatBins * sizeof(unsigned long long) : 0);
-    e = cudaMemsetAsync(scratch, 0, zeroed, stream);
-    if (e != cudaSuccess) return e;
     phase_restart();
     phase_mark(stream);
-    if (!a.head_stats && (e = launch_early(flat_stats_kernel, a.rows * parts, kFT, 0, stream, a)) != cudaSuccess) return e;
+    e = a.head_stats ? launch_early(flat_clear_kernel, a.rows * parts, kFT, 0, stream, a) : launch_early(flat_stats_kernel, a.rows * parts, kFT, 0, stream, a);
+    if (e != cudaSuccess) return e;
     phase_mark(stream);
     if (!full && (e = launch_early(flat_hist_kernel, a.rows * parts, kFT, 0, stream, a)) != cudaSuccess) return e;
     phase_mark(stream);
