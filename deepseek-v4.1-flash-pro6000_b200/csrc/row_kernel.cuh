@@ -322,7 +322,7 @@ static __device__ __noinline__ SearchOut general_search(RowCtx &c, SearchArgs a)
 
 // One row, start to finish, by the whole cluster.  Shared memory needs no particular content on entry.  Returns true if a
 // barrier of the cluster already lies behind the last access to another CTA's shared memory.
-template <int kMode>
+template <int kMode, int kPerSm>
 __device__ __forceinline__ bool row_body(const RowArgs &a, RowCtx &c, RowSmem *s, const int row) {
   const float *logits = row < a.split ? a.logits + size_t(row) * a.logits_stride
                                       : a.logits2 + size_t(row - a.split) * a.logits_stride;
@@ -509,6 +509,7 @@ __device__ __forceinline__ bool row_body(const RowArgs &a, RowCtx &c, RowSmem *s
   // With the head's record nothing has been exchanged yet: where the histogram's barrier will not come first either, one here.
   if (known && (status != 0 || a.top_p >= 1.0 || !s->map.ok)) c.cluster.sync();
 
+  const bool release = kPerSm > 1 && row + a.resident < a.rows;   // (a grid of one CTA per SM fits the GPU)
   Cut cut{-CUDART_INF_F, -1};
   int entered = allowed, kept = allowed;
   double z = 0, e_kept = 0;
@@ -536,11 +537,10 @@ __device__ __forceinline__ bool row_body(const RowArgs &a, RowCtx &c, RowSmem *s
       }
       recorded = true;
     } else {
-      const FastOutcome f = fast_small_support(c, max_logit, t, allowed, a.top_k, a.top_p, cutoff, draw ? s->u : 0.0, draw,
-                                               row + a.resident < a.rows);
+      const FastOutcome f = fast_small_support(c, max_logit, t, allowed, a.top_k, a.top_p, cutoff, draw ? s->u : 0.0, draw, release);
       if (f.applicable) {
         decided = true;
-        if (row + a.resident < a.rows && c.rank == 0) {   // (it has arrived at the barrier that the others end the row with)
+        if (release && c.rank == 0) {    // (it has arrived at the barrier that the others end the row with)
           cluster_complete();
           __syncthreads();               // (its other warps do not begin the next row beside the one that ends this one)
           closed = true;
@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(kThreads, kPerSm) row_kernel(const __grid_cons
       if (!handed_on(st)) continue;
     }
     // no CTA may exit, or stage the next row, while a peer can still address its shared memory
-    if (!row_body<kMode>(a, c, s, row)) c.cluster.sync();
+    if (!row_body<kMode, kPerSm>(a, c, s, row)) c.cluster.sync();
     if (c.timed_out) {  // a bounded wait expired: this cluster reports its remaining rows and stops
       if (c.rank == 0 && c.tid == 0) {
         for (int r = row + clusters; r < a.rows; r += clusters) {
