@@ -212,20 +212,20 @@ class HeadSample:
         self.sharded = None
         self.exchange_note = None
         self.sampler_rows = batch
-        # own kernels per step: quantise, clearing of the row records, head, then the sampler call: the cluster kernel and the
-        # replay kernel up to 48 rows, else flat_hist / flat_window / flat_mass / flat_resolve, the cluster kernel's
-        # persistent grid for rows handed on and the replay kernel for uncertified rows (both return at once when there is
-        # nothing for them); flat_stats is not launched: the head's epilogue left its records
-        self.launches_per_step = 5 if batch <= 48 else 9
+        # own kernels per step: quantise, clearing of the row records, head (two launches where rows are left behind its whole pair
+        # tiles), then the sampler call: the cluster kernel and the replay kernel up to 32 rows, else flat_front (up to 100 rows) or
+        # flat_clear / flat_hist / flat_window, flat_mass / flat_resolve, the cluster kernel's persistent grid for rows handed on
+        # and the replay kernel for uncertified rows (both return at once when there is nothing for them); flat_stats is not
+        # launched: the head's epilogue left its records
+        self.launches_per_step = (5 if batch <= 32 else 8 if batch <= 100 else 10) + (batch > 256 and -(-batch // 128) % 2)
         if world > 1:
             self.sharded = import_module("ds41_b200.sharded").ShardedDecodeTail(pkg, device, batch, self.v0, self.vn,
                                                                               VOCAB, temperature, top_p, strategy,
                                                                               vocab_ranks=self.vocab_ranks)
             strategy = self.sharded.strategy  # "candidates" if the peer buffers could not be mapped
             self.exchange_note = self.sharded.exchange_error
-            # rows: quantise, head (+ peer stores and the row records merged into the owners), flat_hist / window / mass /
-            # resolve, cluster kernel, replay
-            self.launches_per_step = 8 if strategy == "rows" else 6
+            # rows: quantise, head (+ peer stores and the row records merged into the owners), the sampler as above
+            self.launches_per_step = (4 if my_rows <= 32 else 7 if my_rows <= 100 else 9) if strategy == "rows" else 6
             if strategy == "rows":
                 self.sampler_rows = self.sharded.exchange.my_rows
 

@@ -924,12 +924,12 @@ cudaError_t launch_flat(FlatArgs a, void *scratch, cudaStream_t stream) {
     cfg.attrs = attr; cfg.numAttrs = 2;
     e = a.head_stats ? cudaLaunchKernelEx(&cfg, flat_front_kernel<true>, a) : cudaLaunchKernelEx(&cfg, flat_front_kernel<false>, a);
     if (e != cudaSuccess) return e;
-    for (int i = 0; i < 3; ++i) phase_mark(stream);   // (statistics, histogram and window search in one)
+    for (int i = 0; i < 3; ++i) phase_mark(stream);   // (its time is the first of the three phases that it stands for)
   } else {
+    if (a.head_stats && (e = launch_early(flat_clear_kernel, a.rows * parts, kFT, 0, stream, a)) != cudaSuccess) return e;
     phase_restart();
     phase_mark(stream);
-    e = a.head_stats ? launch_early(flat_clear_kernel, a.rows * parts, kFT, 0, stream, a) : launch_early(flat_stats_kernel, a.rows * parts, kFT, 0, stream, a);
-    if (e != cudaSuccess) return e;
+    if (!a.head_stats && (e = launch_early(flat_stats_kernel, a.rows * parts, kFT, 0, stream, a)) != cudaSuccess) return e;
     phase_mark(stream);
     if (!full && (e = launch_early(flat_hist_kernel, a.rows * parts, kFT, 0, stream, a)) != cudaSuccess) return e;
     phase_mark(stream);
