@@ -518,7 +518,7 @@ __device__ __forceinline__ unsigned mass_sub_region(const float *x, int left, co
     for (int h = 0; h < 4; h += 2) {   // (four in lockstep need more registers, and moves between them: 326 us against 323 at 1024 rows)
       const float pair[2] = {y[h], y[h + 1]};
       double weight[2];
-      row_weights<2>(pair, w, weight);
+      row_weights<2, true>(pair, w, weight);
       e[h] = weight[0]; e[h + 1] = weight[1];
     }
     z += (e[0] + e[1]) + (e[2] + e[3]);

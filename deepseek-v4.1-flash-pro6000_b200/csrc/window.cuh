@@ -110,7 +110,9 @@ __device__ __forceinline__ RowWeights make_weights(float max_logit, double log2e
   asm("" : "+d"(w.k64), "+d"(w.magic), "+d"(w.b1), "+d"(w.b2), "+d"(w.b3), "+d"(w.b4));
   return w;
 }
-template <int kN>
+// kBeside: the power of two goes to the table's entry, beside the polynomial's chain (the batch path's pass: 347 -> 342 us at 1024 rows), not
+// to the product behind it (the cluster kernels, whose registers it strains: 11 verified rows 32.9 us against 33.2).
+template <int kN, bool kBeside = false>
 __device__ __forceinline__ void row_weights(const float (&y)[kN], const RowWeights &w, double (&e)[kN]) {
   double d[kN], t[kN], q[kN], tb[kN];
 #pragma unroll
@@ -118,10 +120,10 @@ __device__ __forceinline__ void row_weights(const float (&y)[kN], const RowWeigh
 #pragma unroll
   for (int k = 0; k < kN; ++k) t[k] = fma(d[k], w.k64, w.magic);
 #pragma unroll
-  for (int k = 0; k < kN; ++k) {   // (the power of two goes to the table's entry, beside the polynomial's chain)
+  for (int k = 0; k < kN; ++k) {
     const int n = __double2loint(t[k]);
-    const double entry = w.table[n & 63];
-    tb[k] = __hiloint2double(__double2hiint(entry) - ((n & ~63) << 14), __double2loint(entry));
+    tb[k] = w.table[n & 63];
+    if (kBeside) tb[k] = __hiloint2double(__double2hiint(tb[k]) - ((n & ~63) << 14), __double2loint(tb[k]));
   }
 #pragma unroll
   for (int k = 0; k < kN; ++k) d[k] = fma(d[k], w.k64, -(t[k] - w.magic));
@@ -134,7 +136,10 @@ __device__ __forceinline__ void row_weights(const float (&y)[kN], const RowWeigh
 #pragma unroll
   for (int k = 0; k < kN; ++k) q[k] *= d[k];
 #pragma unroll
-  for (int k = 0; k < kN; ++k) e[k] = fma(tb[k], q[k], tb[k]);
+  for (int k = 0; k < kN; ++k) {
+    const double x = fma(tb[k], q[k], tb[k]);
+    e[k] = kBeside ? x : __hiloint2double(__double2hiint(x) - ((__double2loint(t[k]) & ~63) << 14), __double2loint(x));
+  }
 }
 // sum += e if y > sure; else, if y >= tail, bit kBit of mask is set.  Predicated, without selects.
 template <int kBit>
