@@ -46,13 +46,13 @@ DRAFT_SIGMA = 0.30
 NCU_TRAFFIC_PER_ROW = {
     # profiles/sampler_batch_kernels_256rows.md: one launch of each kernel at 256 rows x 129280 fp32 (132.38 MB per
     # pass over the logits), read + written
-    "flat_stats_kernel": 136.05e6 / 256, "flat_hist_kernel": 140.06e6 / 256, "flat_window_kernel": 4.26e6 / 256,
-    "flat_mass_kernel": 138.37e6 / 256, "flat_resolve_kernel": 2.39e6 / 256, "row_kernel": 0.07e6 / 256,
+    "flat_stats_kernel": 140.24e6 / 256, "flat_hist_kernel": 140.18e6 / 256, "flat_window_kernel": 4.26e6 / 256,
+    "flat_mass_kernel": 137.27e6 / 256, "flat_resolve_kernel": 2.40e6 / 256, "row_kernel": 0.07e6 / 256,
     "replay_sample_kernel": 0.07e6 / 256,
 }
 NCU_TRAFFIC_PER_LAUNCH = {
-    # head_fp8_kernel<64,128>, 64 x 129280 x 4096: 530.05 MB read + 7.34 MB written (profiles/head_fp8_kernel_b64_full_vocab.md)
-    ("cfg2_b64", "head_fp8_kernel"): 537.4e6,
+    # head_fp8_decode_kernel<64>, 64 x 129280 x 4096: 529.99 MB read + 7.70 MB written (profiles/head_fp8_kernel_b64_full_vocab.md)
+    ("cfg2_b64", "head_fp8_kernel"): 537.7e6,
     # row_kernel<0, 2>, 64 flat rows: 34.37 MB read + 0.07 MB written (profiles/row_kernel_64rows_flat.md); one read per row
     ("cfg2_b64", "row_kernel"): 34.44e6,
 }
