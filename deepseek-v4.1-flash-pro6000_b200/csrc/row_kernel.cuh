@@ -509,7 +509,8 @@ __device__ __forceinline__ bool row_body(const RowArgs &a, RowCtx &c, RowSmem *s
   // With the head's record nothing has been exchanged yet: where the histogram's barrier will not come first either, one here.
   if (known && (status != 0 || a.top_p >= 1.0 || !s->map.ok)) c.cluster.sync();
 
-  const bool release = kPerSm > 1 && row + a.resident < a.rows;   // (a grid of one CTA per SM fits the GPU)
+  // (a grid of one CTA per SM fits the GPU; statistics are taken of rows cut by top-p, whose end all CTAs have a part in)
+  const bool release = kPerSm > 1 && kMode == kModeSample && row + a.resident < a.rows;
   Cut cut{-CUDART_INF_F, -1};
   int entered = allowed, kept = allowed;
   double z = 0, e_kept = 0;
