@@ -73,13 +73,23 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 // Bounded wait on a phase parity.  Returns false (and raises the abort flag) if the phase never completed.  The first
 // probe carries no other work: the single threads that issue the copies and the MMAs call this once or twice per K
 // block, and every instruction on their path delays the tensor pipe.
+// kCluster: what completes the phase are relaxed arrivals of another CTA (mbar_arrive_leader), so the wait has the cluster for its scope as
+// they have; as there, the order of the tensor memory's accesses comes from the tcgen05 fences on both sides.
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_try(uint64_t *bar, uint32_t parity) {
   uint32_t done;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(done)
-      : "r"(smem_addr(bar)), "r"(parity)
-      : "memory");
+  if constexpr (kCluster)
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(done)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(done)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
   return done != 0;
 }
 // Without waiting at all.
@@ -93,11 +103,12 @@ __device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
   return done != 0;
 }
 // (In line: around a call the 64 sums of an epilogue thread would be spilled.)
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, const Abort &ab) {
-  if (mbar_try(bar, parity)) return true;
+  if (mbar_try<kCluster>(bar, parity)) return true;
 #pragma unroll 1
   for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
-    if (mbar_try(bar, parity)) return true;
+    if (mbar_try<kCluster>(bar, parity)) return true;
     if ((spin & 255u) == 255u && ab.set()) return false;
   }
   *ab.flag = 1;
@@ -671,7 +682,7 @@ head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       for (int tile = pair; tile < total_tiles && !__any_sync(0xffffffffu, ab.set()); tile += pairs) {
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], phase, ab))) break;
-          if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[acc], acc_phase ^ 1, ab))) break;
+          if (!__all_sync(0xffffffffu, mbar_wait<true>(&acc_empty[acc], acc_phase ^ 1, ab))) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a16 = tiles16 + stage * (kStageBytes >> 4), w16 = a16 + ((128 * kTileK) >> 4);  // addresses >> 4
           const uint32_t d_addr = tmem_base + acc * 256;

@@ -152,3 +152,24 @@ def test_only_the_clearing_kernel_signals_before_its_wait():
         if signal in body and body.index(signal) < body.index(WAIT):
             before.add(kernel)
     assert before == {"clear_stats_kernel"}
+
+
+def test_waits_for_another_ctas_arrivals_have_the_clusters_scope():
+    """A barrier that another CTA arrives at with the cluster's scope is waited on with that scope, and the wait has the order that the
+    arrival has (relaxed: the tensor memory's accesses are ordered by the tcgen05 fences around both)."""
+    text = source("head_fp8.cu")
+    arrival = braced(text, text.index("void mbar_arrive_leader("))
+    assert "mbarrier.arrive.relaxed.cluster.shared::cluster" in arrival
+    probe = braced(text, text.index("bool mbar_try("))
+    wide = probe[probe.index("if constexpr (kCluster)"):probe.index("else")]
+    assert "mbarrier.try_wait.parity.relaxed.cluster.shared::cta" in wide
+    waits = braced(text, text.index("bool mbar_wait("))
+    assert set(re.findall(r"mbar_try(<\w+>)?\(", waits)) == {"<kCluster>"}
+    seen = []
+    for name, kernel, _, body in kernels():
+        for address in set(re.findall(r"\bmbar_arrive_leader\((\w+)", body)):
+            barrier = re.search(rf"\b{address} = peer_addr\((\w+), 0\);", body).group(1)
+            found = re.findall(rf"mbar_wait(<true>)?\(&{barrier}\[", body)
+            assert found and set(found) == {"<true>"}, (kernel, barrier)
+            seen.append((kernel, barrier))
+    assert seen == [("head_fp8_pair_kernel", "acc_empty")]
