@@ -293,17 +293,18 @@ struct HeadArgs {
   long long ldl;
   int M, N, K;
   int *error_flag;       // device word, raised on a wait timeout (may be null)
-  // Row-scattered output (vocabulary-sharded head): batch row m goes to owner m / rows_per_owner, into
-  // owner_base[owner] + (m % rows_per_owner) * ldl + col_offset + n.  The bases may be peer GPUs' memory; the epilogue
+  // Row-scattered output (vocabulary-sharded head): batch row m, the call's row g = first_row + m, goes to owner g / rows_per_owner, into
+  // owner_base[owner] + (g % rows_per_owner) * ldl + col_offset + n.  The bases may be peer GPUs' memory; the epilogue
   // writes them with plain stores, so the vocabulary-to-row transposition rides on the GEMM.  rows_per_owner == 0: off.
   float *owner_base[kMaxOwners];
   int rows_per_owner, col_offset;
+  int first_row;         // rows of the call in front of this launch's (a call may take two, see run_head)
   // Optional per-row statistics for the sampler (zero-initialised by the host): every epilogue thread keeps the first
   // maximum, the minimum and a finiteness flag of the logits it produces for its batch row and merges them with atomic
   // maxima when it leaves the row, so the sampler's own pass over the logits for these three numbers can be skipped.
   HeadRowStats *row_stats;
   // The same records in the row-scattered variant: row m's record lies owner_stats_offset bytes behind owner_base[owner]
-  // at index m % rows_per_owner (0: none).  Several GPUs merge into one record, so those atomics have system scope.
+  // at index (first_row + m) % rows_per_owner (0: none).  Several GPUs merge into one record, so those atomics have system scope.
   long long owner_stats_offset;
   int stages;            // shared-memory stages of the TMA ring (host: PairSmem::stages)
   int group;             // K blocks per stage: every row of a weight tile is fetched as group*128 contiguous bytes
@@ -318,9 +319,9 @@ __device__ __forceinline__ void merge_stats(const HeadArgs &p, int m, float best
   const unsigned long long key = (unsigned long long)(ordered(best)) << 32 | (0xffffffffu - uint32_t(id + p.col_offset));
   const bool any = id != 0x7fffffff;
   if (p.owner_stats_offset) {
-    const int owner = m / p.rows_per_owner;
+    const int g = p.first_row + m, owner = g / p.rows_per_owner;
     HeadRowStats *rs = reinterpret_cast<HeadRowStats *>(reinterpret_cast<unsigned char *>(p.owner_base[owner]) +
-                                                        p.owner_stats_offset) + (m - owner * p.rows_per_owner);
+                                                        p.owner_stats_offset) + (g - owner * p.rows_per_owner);
     if (any) {
       atomicMax_system(&rs->max_key, key);
       atomicMax_system(&rs->min_key, ~ordered(low));
@@ -453,8 +454,8 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const bool stats_on = p.row_stats != nullptr || p.owner_stats_offset != 0;
     auto row_of = [&](int m) {   // batch row m of the output
       if (p.rows_per_owner == 0) return p.logits + size_t(m) * p.ldl;
-      const int owner = m / p.rows_per_owner;
-      return p.owner_base[owner] + size_t(m - owner * p.rows_per_owner) * p.ldl + p.col_offset;
+      const int g = p.first_row + m, owner = g / p.rows_per_owner;
+      return p.owner_base[owner] + size_t(g - owner * p.rows_per_owner) * p.ldl + p.col_offset;
     };
     for (int i = et; i < kblocks * kRows; i += kEpiThreads) {   // activation scales: sa[kb][row]
       const int r = i / kblocks, kb = i % kblocks;
@@ -737,8 +738,8 @@ head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     const bool stats_on = p.row_stats != nullptr || p.owner_stats_offset != 0;
     auto row_of = [&](int m) {   // batch row m of the output
       if (p.rows_per_owner == 0) return p.logits + size_t(m) * p.ldl;
-      const int owner = m / p.rows_per_owner;
-      return p.owner_base[owner] + size_t(m - owner * p.rows_per_owner) * p.ldl + p.col_offset;
+      const int g = p.first_row + m, owner = g / p.rows_per_owner;
+      return p.owner_base[owner] + size_t(g - owner * p.rows_per_owner) * p.ldl + p.col_offset;
     };
     auto flush_stats = [&](int bt_of) {
       const int m = bt_of * 256 + 128 * rank + row;
@@ -1089,7 +1090,8 @@ head_fp8_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       const int n0 = tile * 128 + 32 * quad, n = n0 + lane;
       const bool in = n < p.N;
       // a store instruction writes 128 contiguous bytes of a row
-      int owner = p.rows_per_owner ? first / p.rows_per_owner : 0, left = p.rows_per_owner ? (owner + 1) * p.rows_per_owner - first : kRows;
+      const int g = p.first_row + first;
+      int owner = p.rows_per_owner ? g / p.rows_per_owner : 0, left = p.rows_per_owner ? (owner + 1) * p.rows_per_owner - g : kRows;
       float *dst = p.rows_per_owner ? p.owner_base[owner] + size_t(p.rows_per_owner - left) * p.ldl + p.col_offset + n
                                     : p.logits + size_t(first) * p.ldl + n;
 #pragma unroll
@@ -1405,12 +1407,15 @@ int run_head(const void *a_e4m3, const float *a_scale, const void *w_e4m3, const
   // Three, five ... times 128 rows: what is behind the last whole pair tile would take half of one for its own, and goes to a launch
   // by itself instead, by the kernel of its size.  One launch / two, us in a loop (128 x 256 tiles before: 289 to 317, 478 to 500, 652 to 662):
   // 257 rows 340 / 262, 352 rows 345 / 311, 384 rows 352 / 318, 513 rows 521 / 429, 640 rows 523 / 486, 770 rows 685 / 609, 880 rows
-  // 684 / 661.  (Rows of several owners stay together: an owner's rows are told apart by their place in the batch.)
-  if (M > 256 && p.rows_per_owner == 0 && ((M + 127) / 128 & 1)) {
+  // 684 / 661.  The rows of several owners are cut the same way (eight owners, with the row records, full clocks): 257 rows 307 / 246,
+  // 300 rows 308 / 260, 384 rows 311 / 288, 513 rows 466 / 392, 640 rows 468 / 436, 770 rows 611 / 551.
+  if (M > 256 && ((M + 127) / 128 & 1)) {
     const int whole = M & ~255;
     HeadArgs rest = p;
     p.M = whole; rest.M = M - whole;
-    rest.a_scale += size_t(whole) * (K / kTileK); rest.logits += size_t(whole) * p.ldl;
+    rest.a_scale += size_t(whole) * (K / kTileK);
+    if (p.rows_per_owner) rest.first_row = whole;   // (a row's owner follows from its place in the call)
+    else rest.logits += size_t(whole) * p.ldl;
     if (rest.row_stats) rest.row_stats += whole;
     const int rc = run_head(a_e4m3, a_scale, w_e4m3, w_scale, p, stream);
     return rc ? rc : run_head(static_cast<const uint8_t *>(a_e4m3) + size_t(whole) * K, rest.a_scale, w_e4m3, w_scale, rest, stream);

@@ -87,11 +87,12 @@ def test_head_argument_errors(pkg):
     assert pkg.fuse_head_fp8_workspace_bytes(4, 100) == 0
 
 
-@pytest.mark.parametrize("M,owners", [(5, 2), (64, 4), (200, 8), (130, 3)])
+@pytest.mark.parametrize("M,owners", [(5, 2), (64, 4), (200, 8), (130, 3), (256, 8), (257, 3), (280, 5), (300, 8), (640, 4)])
 def test_head_scatter_to_row_owners(pkg, oracle, M, owners):
     """Vocabulary-sharded head with the row exchange in its epilogue: every "rank" (all emulated on one GPU, one
     launch each over its vocabulary slice) stores row m into owner m / rows_per_owner; the owners' buffers together
-    must equal the unsharded head bit for bit."""
+    must equal the unsharded head bit for bit.  (From 257 rows on: the rows behind the last whole pair tile, a launch of their own, begin
+    in the middle of an owner's rows.)"""
     import importlib
     sharded = importlib.import_module("ds41_b200.sharded")
     N, K = 1000, 512
@@ -141,6 +142,39 @@ def test_head_scatter_to_row_owners(pkg, oracle, M, owners):
     low = (rec[:, 1] & np.uint64(0xffffffff)).astype(np.uint32)
     assert (unorder(~low) == w_np.min(axis=1)).all()
     assert ((rec[:, 1] >> np.uint64(32)) == 0).all()
+
+
+def kernels_of(call):
+    """How many kernels a call launches: captured, not run."""
+    from cuda.bindings import runtime
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+        call()
+    raw = runtime.cudaGraph_t(graph.raw_cuda_graph())
+    _, _, count = runtime.cudaGraphGetNodes(raw, 0)
+    _, nodes, _ = runtime.cudaGraphGetNodes(raw, count)
+    kinds = [runtime.cudaGraphNodeGetType(n)[1] for n in nodes]
+    return sum(k == runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel for k in kinds)
+
+
+@pytest.mark.parametrize("M,launches", [(128, 1), (256, 1), (257, 2), (384, 2), (385, 1), (640, 2)])
+def test_scattered_head_is_cut_into_the_plain_heads_launches(pkg, M, launches):
+    import ctypes as C
+    N, K, owners = 512, 256, 8
+    per = (M + owners - 1) // owners
+    a, a_scale = pkg.quantize_activations(torch.randn(M, K, device="cuda").to(torch.bfloat16))
+    w, w_scale = torch.zeros(N, K, dtype=torch.uint8, device="cuda"), torch.ones(N // 128, K // 128, device="cuda")
+    out, bufs = torch.empty(M, N, device="cuda"), [torch.empty(per, N, device="cuda") for _ in range(owners)]
+    flag, ptrs = torch.zeros(1, dtype=torch.int32, device="cuda"), (C.c_void_p * owners)(*[b.data_ptr() for b in bufs])
+
+    def scattered():
+        fn = pkg.lib().ds41_b200_head_fp8_scatter
+        fn.argtypes = [C.c_void_p] * 4 + [C.POINTER(C.c_void_p), C.c_int, C.c_int, C.c_int64] + [C.c_int] * 4 + [C.c_void_p] * 2
+        assert fn(a.data_ptr(), a_scale.data_ptr(), w.data_ptr(), w_scale.data_ptr(), ptrs, owners, per, N, 0, M, N, K,
+                  flag.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+
+    assert kernels_of(lambda: pkg.head_fp8(a, a_scale, w, w_scale, logits=out, error_flag=flag)) == launches
+    assert kernels_of(scattered) == launches
 
 
 def test_peer_buffer_alloc_and_view(pkg):
