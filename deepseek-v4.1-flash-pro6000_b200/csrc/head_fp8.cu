@@ -593,7 +593,7 @@ head_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 // records at 1024 rows), waits in line (around a call all sums would be spilled).  The hand-back to the leading CTA is a relaxed
 // arrival: with release semantics at cluster scope a K block took 1870 cycles instead of 840.  Tried without gain: 128 ids a tile, four
 // accumulators, 32 sums and boxes stored by TMA (829 us: 24 KB a K block of half the size); the next K block's scales, its wait or its
-// first load ahead (721 to 850: spills); sixteen columns a load (740).
+// first load ahead (721 to 850: spills); sixteen columns a load (740).  Every batch tile has rows for both CTAs (run_head).
 __global__ void __launch_bounds__(kPairThreads, 1)
 head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ HeadArgs p) {
   using Smem = PairSmem;
@@ -617,13 +617,12 @@ head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   const int rank = int(cluster_rank()), pair = int(blockIdx.x) >> 1, pairs = int(gridDim.x) >> 1;
   const int b_tiles = (p.M + 255) / 256, total_tiles = (p.N + 255) / 256 * b_tiles;
   // tile t = (vocabulary tile t / b_tiles, batch tile t % b_tiles)
-  const int active = p.M > 128 ? 2 : 1;   // CTAs of a pair that have batch rows at all
   Abort ab{abort_word};
 
   if (threadIdx.x == 0) {
     *abort_word = 0;
     for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int b = 0; b < kAccBufs; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], kEpiWarps * active); }
+    for (int b = 0; b < kAccBufs; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 2 * kEpiWarps); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {  // TMEM allocation by one full warp of each CTA; the address lands in shared memory
@@ -655,15 +654,13 @@ head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       cudaTriggerProgrammaticLaunchCompletion();
       const uint32_t leader_full = peer_addr(full, 0);
       for (int tile = pair; tile < total_tiles && !ab.set(); tile += pairs) {
-        const int id = tile / b_tiles * 256 + 128 * rank, first = tile % b_tiles * 256, mine = first + 128 * rank;
-        // (a second half without batch rows is not fetched: what the MMA makes of the rows' place nobody reads)
-        const uint32_t bytes = kStageBytes + 128 * kTileK + (first + 128 < p.M ? 128 * kTileK : 0);
+        const int id = tile / b_tiles * 256 + 128 * rank, mine = tile % b_tiles * 256 + 128 * rank;
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, ab)) break;
           unsigned char *a_dst = tiles + size_t(stage) * kStageBytes, *w_dst = a_dst + 128 * kTileK;
-          if (rank == 0) mbar_expect_tx(&full[stage], bytes);   // of both CTAs
+          if (rank == 0) mbar_expect_tx(&full[stage], 2 * kStageBytes);   // of both CTAs
           tma_load_pair(w_dst, &map_w, leader_full + 8 * stage, 0, id, kb, policy);
-          if (mine < p.M) tma_load_pair(a_dst, &map_a, leader_full + 8 * stage, 0, mine, kb, keep);
+          tma_load_pair(a_dst, &map_a, leader_full + 8 * stage, 0, mine, kb, keep);
           if (++stage == uint32_t(kStages)) { stage = 0; phase ^= 1; }
         }
       }
@@ -707,7 +704,6 @@ head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   }
   } else {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
-  if (rank < active) {
     // ------------------------------------------------------------------ epilogue: warp = (lane quadrant, column group)
     cudaGridDependencySynchronize();
     const int quad = warp & 3;          // TMEM lanes [32*quad, 32*quad+32) are readable by this warp: batch rows
@@ -864,9 +860,6 @@ head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       }
     }
     if (alive && table_bt >= 0) flush_stats(table_bt);
-  } else {
-    cudaGridDependencySynchronize();
-  }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -1405,10 +1398,11 @@ int run_head(const void *a_e4m3, const float *a_scale, const void *w_e4m3, const
   const int kblocks = K / kTileK;
   CUtensorMap mw, ma;
   // Three, five ... times 128 rows: what is behind the last whole pair tile would take half of one for its own, and goes to a launch
-  // by itself instead, by the kernel of its size.  One launch / two, us in a loop (128 x 256 tiles before: 289 to 317, 478 to 500, 652 to 662):
-  // 257 rows 340 / 262, 352 rows 345 / 311, 384 rows 352 / 318, 513 rows 521 / 429, 640 rows 523 / 486, 770 rows 685 / 609, 880 rows
-  // 684 / 661.  The rows of several owners are cut the same way (eight owners, with the row records, full clocks): 257 rows 307 / 246,
-  // 300 rows 308 / 260, 384 rows 311 / 288, 513 rows 466 / 392, 640 rows 468 / 436, 770 rows 611 / 551.
+  // by itself instead, by the kernel of its size.  One launch / two, us with the quantiser (short runs at full clocks; in brackets the
+  // 128 x 256 tiles before the pairs): 257 rows 275 / 234 (253), 300 rows 273 / 247 (253), 340 rows 277 / 266 (261), 384 rows 280 / 274
+  // (268), 513 rows 416 / 360 (396), 640 rows 423 / 409 (420), 770 rows 555 / 507 (543), 880 rows 557 / 548 (565).  The rows of several
+  // owners are cut the same way (eight owners, with the row records): 257 rows 294 / 244 (280), 384 rows 299 / 290 (289), 513 rows 452 /
+  // 384 (432), 640 rows 455 / 434 (451), 770 rows 597 / 544 (587).
   if (M > 256 && ((M + 127) / 128 & 1)) {
     const int whole = M & ~255;
     HeadArgs rest = p;
