@@ -215,13 +215,15 @@ __global__ void __launch_bounds__(kThreads, 2) verify_kernel(const __grid_consta
 
 namespace ds41 {
 namespace {
-// Up to this many rows the cluster kernel takes the statistics in one launch; beyond, the batch path's grid-wide passes do (they need
-// the scratch that begins with the 41st row).  Whole calls with either, us: 129280 ids 40 rows 61 / 51, 80 rows 91 / 66, 160 rows 155 /
-// 108; 40000 ids 40 rows 48 / 41, 80 rows 74 / 57 (they meet at 32 rows, where the clusters of eight CTAs no longer run all at a time).
+// Up to this many rows the cluster kernel takes the statistics in one launch; beyond, the batch path's kernels do.  Whole calls with
+// either, us: 129280 ids 33 rows 43 / 41, 35 rows 59 / 45, 40 rows 61 / 49; 50001 ids 33 rows 38 / 38, 35 rows 50 / 40, 40 rows 56 / 45;
+// 33000 ids 33 rows 35 / 35, 35 rows 50 / 40, 40 rows 53 / 43: beyond 33 rows the clusters of eight CTAs no longer run all at a time.
 // Up to 32768 ids, one and two CTAs a row, the cluster kernel is ahead: 24000 ids 40 rows 32 / 61, 80 rows 41 / 60, 160 rows 61 / 64.
-constexpr int kClusterStatRows = 40;
-int cluster_stat_rows(int vocab) { return vocab > 32768 ? kClusterStatRows : 160; }
-// The scratch begins with the row statistics; the replay's rows follow, then the batch path's scratch.
+int cluster_stat_rows(int vocab) { return vocab > 32768 ? kResidentRows : 160; }
+// Up to this many rows the batch path's work space lies where the replay's rows do, which are written when the batch path is done (a
+// caller is asked for no more scratch than that); beyond, behind them.
+constexpr int kSharedScratchRows = 40;
+// The scratch begins with the row statistics; the replay's rows follow, then, beyond kSharedScratchRows, the batch path's scratch.
 size_t verify_stats_bytes(int sequences, int drafts) {
   static_assert(sizeof(RowStats) % 16 == 0, "what follows is aligned");
   return size_t(sequences) * size_t(2 * drafts + 1) * sizeof(RowStats);
@@ -235,7 +237,7 @@ extern "C" size_t ds41_b200_verify_scratch_bytes_for(int sequences, int drafts, 
   if (sequences < 1 || drafts < 0 || drafts > 5 || vocab < 1 || vocab > DS41_B200_MAX_VOCAB) return 0;
   const int rows = sequences * (2 * drafts + 1);
   return verify_stats_bytes(sequences, drafts) + verify_replay_scratch_bytes() +
-         (vocab >= kFlatMinVocab && rows > kClusterStatRows ? flat_scratch_bytes(rows) : 0);
+         (vocab >= kFlatMinVocab && rows > kSharedScratchRows ? flat_scratch_bytes(rows) : 0);
 }
 extern "C" size_t ds41_b200_verify_scratch_bytes(int sequences, int drafts) {
   return ds41_b200_verify_scratch_bytes_for(sequences, drafts, DS41_B200_MAX_VOCAB);
@@ -283,7 +285,8 @@ extern "C" int ds41_b200_verify_logits(const ds41_b200_verify_args *p, cudaStrea
     f.stride = p->vocab; f.vocab = p->vocab; f.rows = stat_launch_rows;
     f.t = a.temperature; f.top_p = p->top_p; f.seeds = p->seeds; f.steps = p->steps; f.slot = a.slot; f.purpose = a.purpose;
     f.stats = pstats; f.draw_every = a.draw_every; f.bound_scale = a.bound_scale;
-    void *flat_scratch = static_cast<unsigned char *>(p->scratch) + stats_bytes + verify_replay_scratch_bytes();
+    unsigned char *flat_scratch = static_cast<unsigned char *>(p->scratch) + stats_bytes;
+    if (int(stat_rows) > kSharedScratchRows) flat_scratch += verify_replay_scratch_bytes();
     if ((e = launch_flat(f, flat_scratch, stream)) != cudaSuccess) return int(e);
     a.only_uncovered = 1;      // what it could not take
     a.pending = flat_pending(flat_scratch);

@@ -186,7 +186,7 @@ int ds41_b200_sample_logits(const ds41_b200_sample_args *args, cudaStream_t stre
  * may then be NULL).  `scratch` is caller-owned device memory of ds41_b200_verify_scratch_bytes() bytes (16-byte
  * aligned): 48 bytes of statistics per logits row, 7.3 MB for the replay of transactions whose decisions fell inside the
  * rounding bound (status bits 1 / 2 / 4 / 8: redone in the same call in the reference's order, they leave with status 0), and
- * the batch path's work space (for more than 40 logits rows of at least 16384 ids).  With less the call still works: without
+ * the batch path's work space (for more than 40 logits rows of at least 16384 ids; up to 40 it lies in the replay's share).  With less the call still works: without
  * the batch path's share every row goes through the cluster kernel; without the replay's, as without status words, the bits
  * stay. */
 typedef struct ds41_b200_verify_args {

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import __graft_entry__ as entry
+from captured import kernels_of
 
 pytestmark = pytest.mark.gpu
 
@@ -42,7 +43,7 @@ def test_sampling(pkg, oracle, rows, vocab, lead, t, top, top_k):
     assert (st.cpu().numpy() >= 0).all() and (tok.cpu().numpy() == want).all()
 
 
-@pytest.mark.parametrize("seqs,drafts,vocab", [(8, 2, 50001), (9, 2, 50001), (41, 0, 16384), (4, 5, 129280), (1, 1, 1025)])
+@pytest.mark.parametrize("seqs,drafts,vocab", [(6, 2, 50001), (3, 5, 33001), (7, 2, 33001), (8, 2, 50001), (9, 2, 50001), (41, 0, 16384), (4, 5, 129280), (1, 1, 1025)])
 @pytest.mark.parametrize("t,top,sigma", [(0.7, 0.95, 0.6), (1.0, 1.0, 1.0)])
 def test_verification(pkg, oracle, seqs, drafts, vocab, t, top, sigma):
     target = oracle.gen_logits(11 + vocab, seqs * (drafts + 1), vocab)
@@ -59,6 +60,20 @@ def test_verification(pkg, oracle, seqs, drafts, vocab, t, top, sigma):
     got = pkg.results_to_numpy(res)
     assert (st.cpu().numpy() == 0).all()
     assert all((got[f] == want[f]).all() for f in ("tokens", "emitted", "accepted_drafts", "rejected")), (got, want)
+
+
+@pytest.mark.parametrize("seqs,drafts,vocab,kernels", [(6, 2, 33001, 3), (32, 0, 33001, 3), (3, 5, 33001, 6), (8, 2, 33001, 6), (9, 2, 33001, 6),
+                                                       (32, 2, 32768, 3)])
+def test_launches_of_a_verification(pkg, seqs, drafts, vocab, kernels):
+    """Statistics by one launch of the cluster kernel, or by three of the batch path in front of it; verification; replay."""
+    rows = seqs * (drafts + 1)
+    target, draft = torch.randn(rows, vocab, device="cuda"), torch.randn(max(1, seqs * drafts), vocab, device="cuda")
+    ids = torch.zeros(max(1, seqs * drafts), dtype=torch.int32, device="cuda")
+    z = torch.zeros(seqs, dtype=torch.int64, device="cuda")
+    scratch = torch.empty(pkg.verify_scratch_bytes(seqs, drafts, vocab), dtype=torch.uint8, device="cuda")
+    out, st = pkg.verify_logits(target, draft if drafts else None, ids if drafts else None, drafts, 0.7, 0.95, z, z, scratch=scratch)
+    assert kernels_of(lambda: pkg.verify_logits(target, draft if drafts else None, ids if drafts else None, drafts, 0.7, 0.95, z, z,
+                                                scratch=scratch, results=out, status=st)) == kernels
 
 
 @pytest.mark.parametrize("rows,vocab", [(34, 700), (3, 16384), (3, 16385), (3, 32769), (3, 131072), (2, 1)])

@@ -9,6 +9,7 @@ import torch
 
 import __graft_entry__ as entry
 import oracle_lib
+from captured import kernels_of
 
 pytestmark = pytest.mark.gpu
 
@@ -142,19 +143,6 @@ def test_head_scatter_to_row_owners(pkg, oracle, M, owners):
     low = (rec[:, 1] & np.uint64(0xffffffff)).astype(np.uint32)
     assert (unorder(~low) == w_np.min(axis=1)).all()
     assert ((rec[:, 1] >> np.uint64(32)) == 0).all()
-
-
-def kernels_of(call):
-    """How many kernels a call launches: captured, not run."""
-    from cuda.bindings import runtime
-    graph = torch.cuda.CUDAGraph(keep_graph=True)
-    with torch.cuda.graph(graph, capture_error_mode="thread_local"):
-        call()
-    raw = runtime.cudaGraph_t(graph.raw_cuda_graph())
-    _, _, count = runtime.cudaGraphGetNodes(raw, 0)
-    _, nodes, _ = runtime.cudaGraphGetNodes(raw, count)
-    kinds = [runtime.cudaGraphNodeGetType(n)[1] for n in nodes]
-    return sum(k == runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel for k in kinds)
 
 
 @pytest.mark.parametrize("M,launches", [(128, 1), (256, 1), (257, 2), (384, 2), (385, 1), (640, 2)])

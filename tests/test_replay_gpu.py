@@ -59,3 +59,10 @@ def test_flagged_transactions_are_replayed_exactly(t, top):
     r = run_verify_case(1e12, 24, 129280, t, top)
     assert r["flagged_without_replay"] >= 6, r
     assert r["records_equal"] and r["status"] == [0], r
+
+
+def test_flagged_transactions_whose_scratch_is_shared():
+    """35 logits rows: the batch path's work space lies where the replay's rows are written afterwards (csrc/verify.cu)."""
+    r = run_verify_case(1e12, 7, 40000, 0.8, 0.95)
+    assert r["flagged_without_replay"] >= 2, r
+    assert r["records_equal"] and r["status"] == [0], r
