@@ -42,7 +42,9 @@ def test_every_kernel_is_found():
 
 
 REMOTE = re.compile(r"map_shared_rank|\bexchange\(c,|\bexchange_by_reading\(|\brow_body\s*<|cluster\.sync\(|\bdraw_region\(|"
-                    r"\bnucleus_row\(|\bfast_small_support\(|\bgeneral_search\(")
+                    r"\bnucleus_row\(|\bfast_small_support\(|\bgeneral_search\(|\bpeer_(?:load|store)_\w+\(|\bpeer_addr\(|"
+                    r"\bmbar_arrive_leader\(|\btma_load_pair\(|\bumma_f8_pair\b|\bumma_commit_pair\(")
+PLAIN_PTX = {"flat_front_kernel", "head_fp8_pair_kernel"}    # clusters by csrc/cluster.cuh
 
 
 def test_cluster_kernels_wait_until_every_cta_has_started():
@@ -50,12 +52,12 @@ def test_cluster_kernels_wait_until_every_cta_has_started():
     started: announced, then awaited, in the same block and without a way around it, before the first access."""
     seen = set()
     for name, kernel, _, body in kernels():
-        if not re.search(r"make_ctx\(|this_cluster\(", body):
+        if not re.search(r"make_ctx\(|this_cluster\(|\bcluster_rank\(", body):
             assert not REMOTE.search(body), (name, kernel)
             continue
         seen.add(kernel)
-        if kernel == "row_kernel":
-            continue                     # the next test
+        if kernel == "row_kernel" or kernel in PLAIN_PTX:
+            continue                     # the next tests
         assert body.count("cluster_announce();") == 1 and body.count("cluster_await();") == 1, (name, kernel)
         announced, awaited = body.index("cluster_announce();"), body.index("cluster_await();")
         assert announced < awaited < REMOTE.search(body).start(), (name, kernel)
@@ -66,7 +68,70 @@ def test_cluster_kernels_wait_until_every_cta_has_started():
             assert branch < announced and not REMOTE.search(body.replace(braced(body, branch), "")), kernel
         else:
             assert "{" not in body[:announced] and "return" not in body[:announced], (name, kernel)
-    assert seen == {"row_kernel", "verify_kernel", "verify_rows_fast_kernel", "probability_rows_kernel", "score_kernel"}
+    assert seen == {"row_kernel", "verify_kernel", "verify_rows_fast_kernel", "probability_rows_kernel", "score_kernel"} | PLAIN_PTX
+
+
+def enclosing(text, at):
+    """Where the blocks begin that hold the place `at`, the outermost first."""
+    open_ = []
+    for i, ch in enumerate(text[:at]):
+        if ch == "{":
+            open_.append(i)
+        elif ch == "}":
+            open_.pop()
+    return open_
+
+
+def test_barriers_of_the_cluster_stand_around_the_accesses_in_plain_ptx():
+    """Kernels that use csrc/cluster.cuh: before an access to another CTA's shared memory, and behind the last one, every thread of the
+    cluster passes a barrier: one in the same block or in a block around it, and no block of a barrier depends on more than the variant."""
+    seen = set()
+    for name, kernel, _, body in kernels():
+        if kernel not in PLAIN_PTX:
+            continue
+        seen.add(kernel)
+        assert "return" not in without_lambdas(body), kernel
+        barriers = [m.start() for m in re.finditer(r"\bcluster_barrier\(\);", body)]
+        variants = [i for i in (body.find("if constexpr (kKnown) {"),) if i >= 0]
+        variants = [i + len("if constexpr (kKnown) {" + braced(body, i) + "} else ") for i in variants]
+        assert all(set(enclosing(body, b)) <= set(variants) for b in barriers), kernel
+        accesses = [m.start() for m in REMOTE.finditer(body)]
+        assert len(accesses) >= 5, kernel
+        for at in accesses:
+            around = enclosing(body, at)
+            assert any(b < at and enclosing(body, b) == around[:len(enclosing(body, b))] for b in barriers), (kernel, body[at:at + 60])
+        last = [b for b in barriers if b > accesses[-1] and not enclosing(body, b)]
+        assert last, kernel
+        given_back = body.find("tcgen05.dealloc.cta_group::2")       # the pair's tensor memory: by both, neither gone
+        assert given_back < 0 or last[0] < given_back < last[-1], kernel
+    assert seen == PLAIN_PTX
+    users = {n for n in os.listdir(CSRC) if n.endswith((".cu", ".cuh")) and '#include "cluster.cuh"' in open(os.path.join(CSRC, n)).read()}
+    assert users == {"flat.cu", "head_fp8.cu"}
+
+
+def test_an_early_arrival_at_the_clusters_barrier_is_completed():
+    """The CTA that ends a row alone arrives early, behind its last access to another CTA's shared memory, and completes that barrier
+    before its next row; the others pass it as the row's end.  Nowhere else is a barrier of the cluster taken apart."""
+    fast, row = source("row_fast.cuh"), source("row_kernel.cuh")
+    text = braced(fast, fast.index("FastOutcome fast_small_support("))
+    assert text.count("cluster_arrive();") == 1 and "if (release) cluster_arrive();" in text
+    ahead, behind = text.split("if (release) cluster_arrive();")
+    assert "out.applicable = 1;\n  if (c.rank != 0) return out;" in ahead      # one CTA, and its row is decided
+    assert not enclosing(text, text.index("cluster_arrive();"))
+    assert not REMOTE.search(behind) and "lists" not in behind and "return out;" in behind and behind.count("return out;") == 1
+    body = braced(row, row.index("bool row_body("))
+    call, complete = body.index("fast_small_support("), body.index("cluster_complete();")
+    branch = "if (f.applicable) {"
+    assert body.count("cluster_complete();") == 1 and call < body.index(branch) < complete
+    taken = braced(body, body.index("if (release && c.rank == 0)"))
+    assert re.sub(r"\s+", " ", taken).strip() == "cluster_complete(); __syncthreads(); closed = true;"
+    assert body.rindex("return closed;") > complete
+    assert "if (!row_body<kMode, kPerSm>(a, c, s, row)) c.cluster.sync();" in row
+    for name in os.listdir(CSRC):
+        if name.endswith((".cu", ".cuh")):
+            text = re.sub(r"__device__ __forceinline__ void cluster_(?:arrive|complete)\(\)[^\n]*", "", source(name))
+            uses = len(re.findall(r"\bcluster_(?:arrive|complete)\(\)", text))
+            assert uses == {"row_fast.cuh": 1, "row_kernel.cuh": 1}.get(name, 0), name
 
 
 def test_first_exchange_of_a_row_reads():
@@ -89,6 +154,7 @@ def test_first_exchange_of_a_row_reads():
 
 
 WAIT = "cudaGridDependencySynchronize();"
+ROLES = {"head_fp8_kernel": 3, "head_fp8_decode_kernel": 3, "head_fp8_pair_kernel": 4}   # kernels of specialised warps: their roles
 
 
 def early_kernels():
@@ -110,6 +176,7 @@ def without_lambdas(text):
 def test_early_kernels_wait_before_they_touch_global_memory():
     early = early_kernels()
     assert {"row_kernel", "head_fp8_kernel", "flat_mass_kernel", "verify_rows_fast_kernel", "replay_sample_kernel"} <= early
+    assert PLAIN_PTX | {"head_fp8_decode_kernel"} <= early
     seen = {}
     for name, kernel, parameters, body in kernels():
         if kernel not in early:
@@ -118,10 +185,14 @@ def test_early_kernels_wait_before_they_touch_global_memory():
         text = without_lambdas(body)
         assert WAIT in text, (name, kernel)
         pointers = re.findall(r"\*\s*(?:__restrict__\s*)?(\w+)\s*(?:,|$)", parameters)
-        touch = r"__ldg\(|__ldc|load_input\(|tma_load|cp\.async\.c|\bfetch\(|stage_begin\(|\brow_body|\b[ap]\.\w+\["
+        touch = r"__ldg\(|__ldc|load_input\(|tma_load|cp\.async\.c|copy4_async\(|\bfetch(?:_scales)?\(|stage_begin\(|\brow_body|\b[ap]\.\w+\["
         touch += "".join(rf"|\b{p}\[|(?<!prefetch_l2\()\b{p} \+" for p in pointers)
-        for part in re.split(r"\} else if \(", text) if kernel == "head_fp8_kernel" else [text]:   # (its warps go separate ways)
-            before = part[:part.index(WAIT)] if WAIT in part else ""
+        parts = [text]
+        if kernel in ROLES:              # (the warps go separate ways, each with a wait of its own)
+            parts = [part for part in re.split(r"\} else (?:if \([^{]*)?\{", text) if WAIT in part]
+            assert len(parts) == text.count(WAIT) == ROLES[kernel], kernel
+        for part in parts:
+            before = part[:part.index(WAIT)]
             assert not re.search(touch, before), (name, kernel, re.search(touch, before))
     assert set(seen) == early, early - set(seen)
 
