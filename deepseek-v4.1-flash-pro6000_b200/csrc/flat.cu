@@ -845,17 +845,20 @@ __global__ void __launch_bounds__(kRT4) flat_resolve_kernel(FlatArgs a) {
   }
 }
 
-// Test hook: the weights of n logits of a row with maximum max_logit, as the FP64 pass forms them.
+// Test hook: the weights of n logits of a row with maximum max_logit, as the FP64 pass forms them (two at a time, the power of two in
+// the table's entry); NaN where the cluster kernels' form has another bit.
 __global__ void flat_weight_probe_kernel(const float *y, float max_logit, double t, double *out, int n) {
   __shared__ double table[64];
   if (threadIdx.x < 64) table[threadIdx.x] = kPow2Neg64[threadIdx.x];
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float v[1] = {y[i]};
-  double e[1];
-  row_weights<1>(v, make_weights(max_logit, kLog2e / t, float(650.0 / kLog2e * t), table), e);
-  out[i] = e[0];
+  const RowWeights w = make_weights(max_logit, kLog2e / t, float(650.0 / kLog2e * t), table);
+  const float v[2] = {y[i], y[(i + 1) % n]};
+  double e[2], f[2];
+  row_weights<2, true>(v, w, e);
+  row_weights<2>(v, w, f);
+  out[i] = __double_as_longlong(e[0]) == __double_as_longlong(f[0]) && __double_as_longlong(e[1]) == __double_as_longlong(f[1]) ? e[0] : CUDART_NAN;
 }
 
 }  // namespace

@@ -145,14 +145,15 @@ def test_same_tokens_as_cluster_kernel_at_1024_rows(pkg):
 def test_batch_weight_error_bound(pkg):
     """The FP64 pass's weight 2^-((max - y) * log2(e) / T) (64-entry table of 2^(-j/64) times a Taylor polynomial of
     degree 4) against long double: within the 1024 * 2^-53 relative that the resolve kernel's bounds allow for, over
-    temperatures, offsets and ranges up to the path's exponent limit; exactly 1 at the maximum."""
+    temperatures, offsets and ranges up to the path's exponent limit of 2^-600; exactly 1 at the maximum.  The cluster
+    kernels' form, which moves the power of two behind the polynomial, has the same bits (the hook answers NaN where not)."""
     lib = pkg.lib()
     lib.ds41_b200_test_batch_weight.argtypes = [C.c_void_p, C.c_float, C.c_double, C.c_void_p, C.c_int, C.c_void_p]
     rng = np.random.default_rng(3)
     worst = 0.0
     for t, m, span in ((0.6, 5.3125, 11.3), (1.0, -2.71875, 24.0), (0.25, 11.0, 7.5), (1.7, 0.0, 50.0),
                        (0.6, 37.5, 12.0), (0.5, 1000.0, 30.0), (1.0, -3000.0, 100.0), (0.3, 2.5, 31.0), (2.0, 0.5, 1.0),
-                       (0.1, 3.0, 41.0)):
+                       (0.1, 3.0, 41.0), (1.0, 2.0, 415.0), (0.7, -40.0, 291.0)):
         y = (np.float32(m) - (rng.random(2_000_000) * span).astype(np.float32)).astype(np.float32)
         y[0] = np.float32(m)
         yt = torch.from_numpy(y).cuda()
@@ -160,6 +161,7 @@ def test_batch_weight_error_bound(pkg):
         assert lib.ds41_b200_test_batch_weight(yt.data_ptr(), m, t, out.data_ptr(), y.size, None) == 0
         torch.cuda.synchronize()
         got = out.cpu().numpy().astype(np.longdouble)
+        assert np.isfinite(got).all()
         arg = (y.astype(np.longdouble) - np.longdouble(np.float32(m))) / np.longdouble(t)
         want = np.exp(arg)
         rel = np.abs(got - want) / want
