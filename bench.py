@@ -53,8 +53,6 @@ NCU_TRAFFIC_PER_ROW = {
 NCU_TRAFFIC_PER_LAUNCH = {
     # head_fp8_decode_kernel<64>, 64 x 129280 x 4096: 529.99 MB read + 7.70 MB written (profiles/head_fp8_kernel_b64_full_vocab.md)
     ("cfg2_b64", "head_fp8_kernel"): 537.7e6,
-    # row_kernel<0, 2>, 64 flat rows: 34.37 MB read + 0.07 MB written (profiles/row_kernel_64rows_flat.md); one read per row
-    ("cfg2_b64", "row_kernel"): 34.44e6,
 }
 
 

@@ -92,16 +92,6 @@ __device__ __forceinline__ bool mbar_try(uint64_t *bar, uint32_t parity) {
         : "memory");
   return done != 0;
 }
-// Without waiting at all.
-__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(done)
-      : "r"(smem_addr(bar)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
 // (In line: around a call the 64 sums of an epilogue thread would be spilled.)
 template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, const Abort &ab) {
@@ -1431,10 +1421,6 @@ int run_head(const void *a_e4m3, const float *a_scale, const void *w_e4m3, const
   const int most = rows == 64 ? DecodeSmem<64>::kMaxGroup : 4;
   for (int g = most; g > 1; g >>= 1)
     if (kblocks % g == 0 && ring(g) >= 2) { group = g; break; }
-  if (const char *forced = getenv("DS41_HEAD_GROUP")) {
-    const int g = atoi(forced);
-    if ((g == 1 || g == 2 || g == 4) && g <= most && kblocks % g == 0 && ring(g) >= 2) group = g;
-  }
   p.group = group;
   if (!make_map(&mw, w_e4m3, uint64_t(N), uint64_t(K), 128, uint32_t(group)) ||
       !make_map(&ma, a_e4m3, uint64_t(M), uint64_t(K), uint32_t(rows), uint32_t(group)))
