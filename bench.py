@@ -201,7 +201,7 @@ class HeadSample:
         self.kernels = {
             "head_fp8_kernel": {"bound": "hbm" if batch <= 128 else "tensor", "bytes": head_bytes,
                                 "flops": 2.0 * batch * self.vn * HIDDEN},
-            # the sampler call: flat_* kernels (batch >= 64) or row_kernel (smaller batches); one read of the logits
+            # the sampler call: flat_* kernels (from 33 rows on) or row_kernel (smaller batches); one read of the logits
             # is the algorithmic minimum
             "sampler": {"bound": "hbm", "bytes": my_rows * VOCAB * 4 + my_rows * 24, "flops": 0.0},
         }

@@ -537,10 +537,10 @@ __device__ __forceinline__ unsigned mass_sub_region(const float *x, int left, co
 }
 
 // The FP64 pass: the weight of every id, per 1024-id sub-region the sum over all ids and over the ids before the window; a
-// warp takes a sub-region at a time.  Bound by the latency of its loads, conversions and FP64 chains as much as by issue slots (38
+// warp takes a sub-region at a time.  Bound by the latency of its loads, conversions and FP64 chains as much as by issue slots (39
 // instructions per id), not by memory: eight CTAs an SM with 64 registers and two loads ahead instead of six with 80 and four
-// take the sampling call of 1024 rows from 342 to 326 us, of 256 rows from 115 to 109.  (A table of 16 entries, free of bank
-// conflicts, with one more multiply-add: 350.)
+// take the sampling call of 1024 rows from 342 (347 before the power of two moved into the table's entry, window.cuh) to 326 us, of 256 rows
+// from 115 to 109.  (A table of 16 entries, free of bank conflicts, with one more multiply-add: 350.)
 __global__ void __launch_bounds__(kFlatMassThreads, 8) flat_mass_kernel(FlatArgs a) {
   __shared__ double table[64];
   __shared__ WarpWindow windows[kFlatMassThreads / 32];

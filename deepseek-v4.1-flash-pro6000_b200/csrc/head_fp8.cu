@@ -214,6 +214,9 @@ __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigne
 }
 
 // ---- a pair of CTAs (a cluster of two) on one tile
+// An accumulator is handed back to the leading CTA.  Relaxed is enough because nothing is published: the arrival only keeps the next MMA from
+// overwriting what has been read, and it is issued once tcgen05.wait::ld has returned the values in every lane (__syncwarp), with a
+// tcgen05 fence on either side.  So nothing else may be handed over by this barrier.
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -296,7 +299,7 @@ struct HeadArgs {
   // The same records in the row-scattered variant: row m's record lies owner_stats_offset bytes behind owner_base[owner]
   // at index (first_row + m) % rows_per_owner (0: none).  Several GPUs merge into one record, so those atomics have system scope.
   long long owner_stats_offset;
-  int stages;            // shared-memory stages of the TMA ring (host: PairSmem::stages)
+  int stages;            // shared-memory stages of the TMA ring (host: stages() of the kernel's own layout)
   int group;             // K blocks per stage: every row of a weight tile is fetched as group*128 contiguous bytes
 };
 
@@ -593,7 +596,7 @@ head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   extern __shared__ __align__(1024) unsigned char smem[];
   // carve: [stages][A 16 KB | W 16 KB], then output blocks, scale tables, barriers; the same places in both CTAs
   unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~uintptr_t(1023));
-  float *out = reinterpret_cast<float *>(tiles + size_t(kStages) * kStageBytes);   // [epilogue warp][32][20]
+  float *out = reinterpret_cast<float *>(tiles + size_t(kStages) * kStageBytes);   // [epilogue warp][32][16], the 16-byte pieces of a row in an order of its own
   float4 *stats = reinterpret_cast<float4 *>(out + kEpiWarps * Smem::kOutFloats);  // [epilogue thread] maximum, minimum, its id, not finite
   float *sa = reinterpret_cast<float *>(stats + kEpiWarps * 32);                   // [K/128][128]
   const int kblocks = p.K / kTileK;
@@ -810,7 +813,8 @@ head_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         stats[et] = make_float4(st_best, st_low, __int_as_float(st_id), st_bad + st_bad1);
       }
       // Lane l holds row l of the warp's 32 x 64 block.  Sixteen ids at a time go through shared memory, so that a store instruction
-      // writes 64 contiguous bytes of eight rows (rows 80 bytes apart: neither side has a bank conflict).
+      // writes 64 contiguous bytes of eight rows.  (A row of the block is 64 bytes; its four pieces are swapped by bits 1 and 2 of the row's
+      // number, so that neither side has a bank conflict.)
       if (alive) {
         const bool plain = p.rows_per_owner == 0 && whole && p.ldl % 4 == 0 && (reinterpret_cast<uintptr_t>(p.logits) & 15u) == 0;
         const int r0 = quad * 32 + (lane >> 2), col = 4 * (lane & 3);

@@ -111,7 +111,7 @@ __device__ __forceinline__ RowWeights make_weights(float max_logit, double log2e
   return w;
 }
 // kBeside: the power of two goes to the table's entry, beside the polynomial's chain (the batch path's pass: 347 -> 342 us at 1024 rows), not
-// to the product behind it (the cluster kernels, whose registers it strains: 11 verified rows 32.9 us against 33.2).
+// to the product behind it (the cluster kernels, whose registers it strains: 11 verified rows 32.6 to 32.9 us against 33.2).
 template <int kN, bool kBeside = false>
 __device__ __forceinline__ void row_weights(const float (&y)[kN], const RowWeights &w, double (&e)[kN]) {
   double d[kN], t[kN], q[kN], tb[kN];
