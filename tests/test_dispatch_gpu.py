@@ -1,6 +1,7 @@
 """The sizes at which a sampling or verification call changes its path (csrc/sampler.cu, csrc/verify.cu): the last batch of the
 cluster kernel and the first of the grid-wide passes, rows at odd addresses, vocabularies around the cluster sizes.  Tokens
-and records against the CPU oracle; likewise the operators on probability rows (csrc/prob.cu)."""
+and records against the CPU oracle; likewise the operators on probability rows (csrc/prob.cu).  Which side a size takes is
+seen in the kernels that its call launches."""
 import numpy as np
 import pytest
 import torch
@@ -27,7 +28,9 @@ def u64(a):
 
 
 @pytest.mark.parametrize("rows,vocab,lead", [(12, 129280, 0), (13, 129280, 0), (48, 50001, 1), (49, 50001, 1), (49, 16385, 2),
-                                             (50, 16383, 3), (5, 32769, 0), (5, 131072, 0), (3, 1025, 1)])
+                                             (50, 16383, 3), (5, 32769, 0), (5, 131072, 0), (3, 1025, 1),
+                                             (32, 50001, 1), (33, 50001, 1), (256, 16385, 2), (257, 16385, 2),
+                                             (257, 16384, 0), (257, 32768, 0)])
 @pytest.mark.parametrize("t,top,top_k", [(0.7, 0.95, 0), (1.0, 1.0, 0), (0.8, 0.9, 40), (0.0, 1.0, 0)])
 def test_sampling(pkg, oracle, rows, vocab, lead, t, top, top_k):
     x = oracle.gen_logits(7 + vocab, rows, vocab)
@@ -43,7 +46,8 @@ def test_sampling(pkg, oracle, rows, vocab, lead, t, top, top_k):
     assert (st.cpu().numpy() >= 0).all() and (tok.cpu().numpy() == want).all()
 
 
-@pytest.mark.parametrize("seqs,drafts,vocab", [(6, 2, 50001), (3, 5, 33001), (7, 2, 33001), (8, 2, 50001), (9, 2, 50001), (41, 0, 16384), (4, 5, 129280), (1, 1, 1025)])
+@pytest.mark.parametrize("seqs,drafts,vocab", [(6, 2, 50001), (3, 5, 33001), (7, 2, 33001), (8, 2, 50001), (9, 2, 50001), (41, 0, 16384), (4, 5, 129280), (1, 1, 1025),
+                                               (160, 0, 16384), (161, 0, 16384), (32, 4, 24000), (54, 1, 32768)])
 @pytest.mark.parametrize("t,top,sigma", [(0.7, 0.95, 0.6), (1.0, 1.0, 1.0)])
 def test_verification(pkg, oracle, seqs, drafts, vocab, t, top, sigma):
     target = oracle.gen_logits(11 + vocab, seqs * (drafts + 1), vocab)
@@ -62,8 +66,23 @@ def test_verification(pkg, oracle, seqs, drafts, vocab, t, top, sigma):
     assert all((got[f] == want[f]).all() for f in ("tokens", "emitted", "accepted_drafts", "rejected")), (got, want)
 
 
+@pytest.mark.parametrize("rows,vocab,top_k,kernels", [(32, 50001, 0, 2), (33, 50001, 0, 5), (130, 50001, 0, 5), (131, 50001, 0, 7),
+                                                       (256, 32768, 0, 2), (257, 32768, 0, 7), (202, 50001, 40, 1), (203, 50001, 40, 3),
+                                                       (256, 32768, 40, 1), (257, 32768, 40, 3)])
+def test_launches_of_a_sampling(pkg, rows, vocab, top_k, kernels):
+    """Top-p: the cluster kernel and the replay; or the batch path's front (one launch or three), masses and resolve before them.
+    Top-k: the cluster kernel, or the streaming path's two before it."""
+    x = torch.randn(rows, vocab, device="cuda")
+    z = torch.zeros(rows, dtype=torch.int64, device="cuda")
+    scratch = torch.empty(pkg.sample_scratch_bytes(rows, vocab), dtype=torch.uint8, device="cuda")
+    call = dict(top_k=top_k, scratch=scratch, tokens=torch.empty(rows, dtype=torch.int32, device="cuda"),
+                status=torch.empty(rows, dtype=torch.int32, device="cuda"))
+    pkg.sample_logits(x, 0.7, 0.95, z, z, **call)
+    assert kernels_of(lambda: pkg.sample_logits(x, 0.7, 0.95, z, z, **call)) == kernels
+
+
 @pytest.mark.parametrize("seqs,drafts,vocab,kernels", [(6, 2, 33001, 3), (32, 0, 33001, 3), (3, 5, 33001, 6), (8, 2, 33001, 6), (9, 2, 33001, 6),
-                                                       (32, 2, 32768, 3)])
+                                                       (32, 2, 32768, 3), (160, 0, 16384, 3), (161, 0, 16384, 8)])
 def test_launches_of_a_verification(pkg, seqs, drafts, vocab, kernels):
     """Statistics by one launch of the cluster kernel, or by three of the batch path in front of it; verification; replay."""
     rows = seqs * (drafts + 1)
