@@ -171,12 +171,19 @@ namespace {
 // 148 rows 32 / 53, 256 rows 58 / 61; 32768 ids 256 rows 63 / 67.
 // Greedy (drawn for 129280 ids): 32 rows 10.0 / 10.6, 64 rows 18 / 15; 40000 ids: 32 rows 8.8 / 9.0, 48 rows 15 / 11; 16384 and 32768
 // ids: 128 rows 7.3 / 8.4 and 9.7 / 9.8.
-// Rows cut by top-k cost the cluster kernel the same at any vocabulary of eight slices, and the streaming path what their ids
-// take to read: 40000 ids 160 rows 66 / 73, 200 rows 79 / 75; 129280 ids 200 rows 94 / 119, 256 rows 117 / 133 (and the two
-// meet, from their slopes, at about 345): the limit follows the line through the two.
+// Rows cut by top-k cost the cluster kernel the same at any vocabulary of eight slices and any k; the streaming path what their ids take
+// to read and, in the end of a row, the walk over k candidates.  Top-k 1 / 10 / 20 / 40 / 64, 40000 ids: 88 rows 36 / 27, 37 / 32, 37 / 39,
+// 40 / 67, 43 / 109; 200 rows 73 / 38, 75 / 42, 76 / 51, 78 / 77, 82 / 122; 129280 ids: 88 rows 42 / 45, 42 / 50, 44 / 58, 45 / 83, 48 / 131; 200
+// rows 88 / 79, 90 / 83, 91 / 91, 94 / 118, 97 / 165; 350 rows 147 / 117, 150 / 122, 152 / 131, 155 / 158, 159 / 209.  The two meet at about
+// 40 + ids / 1500 rows with k = 10, growing with k: over 6 vocabularies, 8 k and 12 batches the side taken costs at most 5 % more than
+// the other.  (Beyond 400 rows nothing was measured.)
 constexpr int kClusterRowsGreedy = 64;
 int cluster_rows(int vocab) { return vocab > 32768 ? kResidentRows : 256; }
-int cluster_rows_topk(int vocab) { return vocab > 32768 ? 113 + vocab / 558 : 256; }
+int cluster_rows_topk(int vocab, int k) {
+  if (vocab <= 32768 || k > kCand) return 256;   // (more than kCand candidates: the cluster kernel's in any case)
+  const int limit = (40 + vocab / 1500) * (700 + 20 * k + 4 * k * k / 5) / 1000;
+  return limit < 400 ? limit : 400;
+}
 
 // One launch that decides every row, and, for rows cut by top-p alone, the replay of those it could not certify.
 int sample_by_clusters(RowArgs a, const ds41_b200_sample_args &p, cudaStream_t stream) {
@@ -227,7 +234,7 @@ extern "C" int ds41_b200_sample_logits(const ds41_b200_sample_args *p, cudaStrea
   // With scratch: small batches by the cluster kernel alone; larger ones of rows that are only cut by top-p first go through
   // the batch path, which answers the rows it fits and marks the others -8 / -9, and the paths below then only touch those.
   const bool top_p_only = p->top_k == 0 && p->temperature > 0;
-  const int by_clusters = top_p_only ? cluster_rows(p->vocab) : p->temperature > 0 ? cluster_rows_topk(p->vocab) : kClusterRowsGreedy;
+  const int by_clusters = top_p_only ? cluster_rows(p->vocab) : p->temperature > 0 ? cluster_rows_topk(p->vocab, p->top_k) : kClusterRowsGreedy;
   if (scratch_ok && p->rows <= by_clusters) return sample_by_clusters(a, *p, stream);
   const bool flat = scratch_ok && flat_shape(p->rows, p->vocab) && top_p_only && p->logits_stride != 0;
   // the streaming path covers small nuclei only: a full-vocabulary draw never fits its candidate sets
