@@ -884,12 +884,12 @@ FlatInfo *flat_info(void *scratch, int rows) {
 }
 
 // Up to this many rows flat_front_kernel takes the place of three passes and the clearing in front of them.  Some 32 rows are at work at
-// a time, each as long as a chain of barriers takes, while the passes fill the GPU whatever the batch: whole calls at 129280 ids, us,
-// front / passes: 49 rows 44 / 67, 64 48 / 58, 100 66 / 73, 120 77 / 84, 160 96 / 91, 256 148 / 130 (40000 ids: 64 rows 42 / 51);
-// verification of 45 logits rows 46 / 68, 110 rows 81 / 89, 160 rows 107 / 102; with the head's records, which spare the passes one
-// of them, a decode step of 49 rows 132 / 139, 64 141 / 143, 100 174 / 175, 128 191 / 186.  Up to 32768 ids the cluster kernel takes
-// batches of these sizes (sampler.cu).
-constexpr int kFrontMinVocab = 32768, kFrontRows = 130, kFrontRowsKnown = 100;
+// a time, each as long as a chain of barriers takes, while the passes fill the GPU whatever the batch, with half as many CTAs a row
+// from 128 rows on: whole calls, us, front / passes: 129280 ids 40 rows 40 / 59, 64 46 / 55, 100 65 / 72, 115 72 / 79, 130 78 / 75, 160 93 / 86;
+// 65536 ids 64 rows 40 / 49, 115 60 / 66, 130 64 / 60; 33000 ids 64 rows 38 / 46, 115 56 / 59, 130 58 / 53.  With the head's records, which
+// spare the passes one of them, a decode step of 40 rows 126 / 132, 64 137 / 139, 80 169 / 168, 100 179 / 178, 120 189 / 190, 128 193 / 187.  Up
+// to 32768 ids the cluster kernel takes batches of these sizes (sampler.cu).
+constexpr int kFrontMinVocab = 32768, kFrontRows = 127, kFrontRowsKnown = 100;
 
 cudaError_t launch_flat(FlatArgs a, void *scratch, cudaStream_t stream) {
   if (!a.logits2) a.split = a.rows;

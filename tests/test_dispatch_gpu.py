@@ -66,7 +66,7 @@ def test_verification(pkg, oracle, seqs, drafts, vocab, t, top, sigma):
     assert all((got[f] == want[f]).all() for f in ("tokens", "emitted", "accepted_drafts", "rejected")), (got, want)
 
 
-@pytest.mark.parametrize("rows,vocab,top_k,kernels", [(32, 50001, 0, 2), (33, 50001, 0, 5), (130, 50001, 0, 5), (131, 50001, 0, 7),
+@pytest.mark.parametrize("rows,vocab,top_k,kernels", [(32, 50001, 0, 2), (33, 50001, 0, 5), (127, 50001, 0, 5), (128, 50001, 0, 7),
                                                        (256, 32768, 0, 2), (257, 32768, 0, 7), (202, 50001, 40, 1), (203, 50001, 40, 3),
                                                        (59, 50001, 5, 1), (60, 50001, 5, 3),
                                                        (256, 32768, 40, 1), (257, 32768, 40, 3)])

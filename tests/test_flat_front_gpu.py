@@ -38,7 +38,8 @@ def records(x):
 
 
 @pytest.mark.parametrize("rows,vocab,lead", [(33, 32769, 0), (34, 33003, 1), (33, 131072, 0), (33, 129280, 2), (100, 33001, 3), (101, 33001, 0),
-                                             (130, 40000, 0), (131, 40000, 0)])
+                                             (130, 40000, 0), (131, 40000, 0),
+                                             (127, 40000, 0), (128, 40000, 0)])
 @pytest.mark.parametrize("known", [False, True])
 def test_front(pkg, oracle, rows, vocab, lead, known):
     x = oracle.gen_logits(3 + vocab, rows, vocab)
