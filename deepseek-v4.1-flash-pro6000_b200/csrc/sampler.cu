@@ -69,8 +69,10 @@ cudaError_t launch_rows(const RowArgs &a, int rows, cudaStream_t stream) {
     args.reach = float(0.999 * kFlatMaxExponent / kLog2e * a.temperature);
     args.floor_gap = float(650.0 / kLog2e * a.temperature);
   }
-  // left-over rows only: a persistent grid of two clusters per 8 SMs walks the status words
-  const int clusters = a.only_uncovered ? (rows < 74 ? rows : 74) : rows;
+  // left-over rows only: a persistent grid walks the status words.  Two clusters per 8 SMs; in rows that only the streaming path is in front
+  // of, of one CTA each, many may be left: as many as run at a time (256 flat rows of 1024 ids 397 -> 183 us, none left over the same)
+  const int most = a.vocab < kFlatMinVocab ? resident_rows(1) : 74;
+  const int clusters = a.only_uncovered && rows > most ? most : rows;
   // A grid that surely fits the GPU with one CTA per SM gets 128 registers per thread: no spills, and more of a step's loads and
   // FP64 chains in flight.  A larger one is better off with two CTAs per SM, which fill each other's waits at the barriers
   if (clusters * cl <= kOnePerSm) return launch_rows<kMode, 1>(args, clusters, cl, dev, stream);
@@ -168,7 +170,10 @@ namespace {
 // Top-p, rows of eight CTAs (beyond 32768 ids): the line is the number of such clusters that run at a time.  129280 ids: 20 rows 30 / 31,
 // 37 rows 52 / 40, 48 rows 54 / 43; 40000 ids: 20 rows 24 / 29, 37 rows 44 / 35; decode steps of 30 rows 114.5 / 119.4, of 37 rows 142 / 126.
 // With fewer ids a row takes one or two CTAs and the batch path as many launches: 16384 ids 192 rows 37 / 56, 256 rows 37 / 55; 24000 ids
-// 148 rows 32 / 53, 256 rows 58 / 61; 32768 ids 256 rows 63 / 67.
+// 148 rows 32 / 53, 256 rows 58 / 61; 32768 ids 256 rows 63 / 67.  Below 16384 ids the other path is the streaming path: 12000 ids 148 rows 27 / 70,
+// 4000 ids 24 / 43, 1500 ids 23 / 24, 128 ids 18 / 18 peaked and 18 / 39 flat.  Rows of up to kListCap ids are ordered as a whole by the cluster
+// kernel, which the streaming path spares peaked rows: 256 ids 148 rows 24 / 20, 512 ids 41 / 20, 1024 ids 98 / 23; flat rows pass through both
+// (1024 ids 148 rows 100 / 119).
 // Greedy (drawn for 129280 ids): 32 rows 10.0 / 10.6, 64 rows 18 / 15; 40000 ids: 32 rows 8.8 / 9.0, 48 rows 15 / 11; 16384 and 32768
 // ids: 128 rows 7.3 / 8.4 and 9.7 / 9.8.
 // Rows cut by top-k cost the cluster kernel the same at any vocabulary of eight slices and any k; the streaming path what their ids take
@@ -178,7 +183,11 @@ namespace {
 // 40 + ids / 1500 rows with k = 10, growing with k: over 6 vocabularies, 8 k and 12 batches the side taken costs at most 5 % more than
 // the other.  (Beyond 400 rows nothing was measured.)
 constexpr int kClusterRowsGreedy = 64;
-int cluster_rows(int vocab) { return vocab > 32768 ? kResidentRows : 256; }
+constexpr int kClusterRowsShort = 48, kShortVocab = 128;   // rows of kShortVocab + 1 .. kListCap ids
+int cluster_rows(int vocab) {
+  if (vocab > 32768) return kResidentRows;
+  return vocab > kShortVocab && vocab <= kListCap ? kClusterRowsShort : 256;
+}
 int cluster_rows_topk(int vocab, int k) {
   if (vocab <= 32768 || k > kCand) return 256;   // (more than kCand candidates: the cluster kernel's in any case)
   const int limit = (40 + vocab / 1500) * (700 + 20 * k + 4 * k * k / 5) / 1000;

@@ -69,10 +69,11 @@ def test_verification(pkg, oracle, seqs, drafts, vocab, t, top, sigma):
 @pytest.mark.parametrize("rows,vocab,top_k,kernels", [(32, 50001, 0, 2), (33, 50001, 0, 5), (127, 50001, 0, 5), (128, 50001, 0, 7),
                                                        (256, 32768, 0, 2), (257, 32768, 0, 7), (202, 50001, 40, 1), (203, 50001, 40, 3),
                                                        (59, 50001, 5, 1), (60, 50001, 5, 3),
-                                                       (256, 32768, 40, 1), (257, 32768, 40, 3)])
+                                                       (256, 32768, 40, 1), (257, 32768, 40, 3),
+                                                       (48, 1024, 0, 2), (49, 1024, 0, 3), (49, 129, 0, 3), (256, 128, 0, 2), (256, 1025, 0, 2)])
 def test_launches_of_a_sampling(pkg, rows, vocab, top_k, kernels):
     """Top-p: the cluster kernel and the replay; or the batch path's front (one launch or three), masses and resolve before them.
-    Top-k: the cluster kernel, or the streaming path's two before it."""
+    Top-k, and top-p with few ids: the cluster kernel, or the streaming path's two before it."""
     x = torch.randn(rows, vocab, device="cuda")
     z = torch.zeros(rows, dtype=torch.int64, device="cuda")
     scratch = torch.empty(pkg.sample_scratch_bytes(rows, vocab), dtype=torch.uint8, device="cuda")

@@ -24,7 +24,7 @@ def u64(a):
 
 @pytest.mark.parametrize("rows,vocab,top_k", [(37, 33001, 40), (38, 33001, 40), (80, 40000, 7), (149, 20000, 20), (297, 9000, 20),
                                               (300, 40000, 40), (32, 33001, 40), (33, 33001, 40), (34, 33001, 40), (148, 20000, 20),
-                                              (296, 9000, 20)])
+                                              (296, 9000, 20), (300, 900, 0)])
 def test_top_k_rows_that_wait_for_a_place(pkg, oracle, rows, vocab, top_k):
     x = oracle.gen_logits(5 + vocab, rows, vocab)
     x[::3, 100:400] = x[::3].max(axis=1, keepdims=True)          # more ties at the top than the streaming path keeps
