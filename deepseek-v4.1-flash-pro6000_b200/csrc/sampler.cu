@@ -292,7 +292,14 @@ extern "C" int ds41_b200_sample_logits(const ds41_b200_sample_args *p, cudaStrea
   }
   a.status = status;
   a.only_uncovered = 1;
-  return int(launch_rows<kModeSample>(a, p->rows, stream));
+  e = launch_rows<kModeSample>(a, p->rows, stream);
+  if (e != cudaSuccess || !top_p_only) return int(e);
+  // the combine's sums carry the chunks' bounds, so that rows cut by top-p alone may be left uncertified here too
+  unsigned char *behind = static_cast<unsigned char *>(p->scratch) + streaming_bytes(p->rows, p->vocab);
+  if (flat_shape(p->rows, p->vocab)) behind += flat_scratch_bytes(p->rows);
+  ReplayArgs r{p->logits, p->logits_stride, p->vocab, p->rows, a.temperature, p->top_p, p->seeds, p->steps, p->slot,
+               p->purpose, p->tokens, status, behind};
+  return int(launch_replay(r, stream));
 }
 
 namespace ds41 {

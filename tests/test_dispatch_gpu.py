@@ -46,6 +46,26 @@ def test_sampling(pkg, oracle, rows, vocab, lead, t, top, top_k):
     assert (st.cpu().numpy() >= 0).all() and (tok.cpu().numpy() == want).all()
 
 
+@pytest.mark.parametrize("rows,vocab,lead", [(49, 1000, 0), (300, 4000, 1), (64, 1024, 0)])
+def test_uncertified_rows_of_the_streaming_path_are_redone(pkg, oracle, rows, vocab, lead):
+    """Four ids share most of the mass and top-p lies 1e-9 from the sum of the first two, closer than the chunks' sums can tell: the row is
+    redone in the reference's order and certified."""
+    x = np.repeat((-9.0 - np.arange(vocab) / 1024).astype(np.float32)[None], rows, 0)
+    for r in range(rows):
+        x[r, (np.arange(4) * 31 + r) % vocab] = 0.0
+    p = np.sort(oracle.probabilities(x[0], 1.0, 1.0))[::-1]
+    assert abs(p[0] - p[3]) < 1e-15 and 0.2 < p[0] < 0.25
+    seeds, steps = np.arange(rows) * 31 + 5, np.arange(rows) * 3 + 1
+    buf = torch.zeros(rows, vocab + 5, device="cuda")
+    view = buf[:, lead: lead + vocab]
+    view.copy_(torch.from_numpy(x))
+    for top in (2 * p[0] * (1 - 1e-9), 2 * p[0] * (1 + 1e-9)):
+        want, _ = oracle.sample_rows(x, 1.0, top, seeds, steps, threads=8)
+        tok, st = pkg.sample_logits(view, 1.0, top, u64(seeds), u64(steps))
+        torch.cuda.synchronize()
+        assert (st.cpu().numpy() == 0).all() and (tok.cpu().numpy() == want).all()
+
+
 @pytest.mark.parametrize("seqs,drafts,vocab", [(6, 2, 50001), (3, 5, 33001), (7, 2, 33001), (8, 2, 50001), (9, 2, 50001), (41, 0, 16384), (4, 5, 129280), (1, 1, 1025),
                                                (160, 0, 16384), (161, 0, 16384), (32, 4, 24000), (54, 1, 32768)])
 @pytest.mark.parametrize("t,top,sigma", [(0.7, 0.95, 0.6), (1.0, 1.0, 1.0)])
@@ -70,10 +90,10 @@ def test_verification(pkg, oracle, seqs, drafts, vocab, t, top, sigma):
                                                        (256, 32768, 0, 2), (257, 32768, 0, 7), (202, 50001, 40, 1), (203, 50001, 40, 3),
                                                        (59, 50001, 5, 1), (60, 50001, 5, 3),
                                                        (256, 32768, 40, 1), (257, 32768, 40, 3),
-                                                       (48, 1024, 0, 2), (49, 1024, 0, 3), (49, 129, 0, 3), (256, 128, 0, 2), (256, 1025, 0, 2)])
+                                                       (48, 1024, 0, 2), (49, 1024, 0, 4), (49, 129, 0, 4), (256, 128, 0, 2), (256, 1025, 0, 2)])
 def test_launches_of_a_sampling(pkg, rows, vocab, top_k, kernels):
     """Top-p: the cluster kernel and the replay; or the batch path's front (one launch or three), masses and resolve before them.
-    Top-k, and top-p with few ids: the cluster kernel, or the streaming path's two before it."""
+    Top-k, and top-p with few ids (and the replay): the cluster kernel, or the streaming path's two before it."""
     x = torch.randn(rows, vocab, device="cuda")
     z = torch.zeros(rows, dtype=torch.int64, device="cuda")
     scratch = torch.empty(pkg.sample_scratch_bytes(rows, vocab), dtype=torch.uint8, device="cuda")
