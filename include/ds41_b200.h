@@ -160,7 +160,8 @@ typedef struct ds41_b200_sample_args {
   void *scratch;              /* optional device scratch of ds41_b200_sample_scratch_bytes(rows, vocab) bytes, 16-byte
                                  aligned.  With it, larger batches of rows without penalties / bitmask and with
                                  top_k <= 64 (more than 32 rows cut by top-p, 43 to 400 by top-k, growing with ids and k, 64
-                                 greedy; up to 32768 ids more than 256, greedy 64) take a
+                                 greedy; up to 32768 ids more than 256, greedy 64, and 48 cut by
+                                 top-p with 129 to 1024 ids) take a
                                  batch-parallel path before the cluster kernel: without top_k (vocab >= 16384)
                                  grid-wide kernels (histogram, window, FP64 masses, resolve), otherwise the streaming
                                  path (chunk records + a per-row combine).  Rows these cannot take, smaller batches and
