@@ -31,8 +31,9 @@ def test_product_and_records(pkg, M, N, K):
 @pytest.mark.parametrize("N,K", [(100, 128), (257, 512), (20011, 384), (40000, 256), (300, 16384)])
 @pytest.mark.parametrize("M", [127, 128, 129, 256, 257, 350, 385, 700])
 def test_larger_batches(pkg, M, N, K):
-    """Around one CTA's 128 rows and a pair's 256 (head_fp8_kernel, head_fp8_pair_kernel): a second half without rows, several batch
-    tiles, rows behind the whole pair tiles (257 and 350), vocabularies shorter than a tile, fewer K blocks than stages."""
+    """Around one CTA's 128 rows and a pair's 256 (head_fp8_kernel, head_fp8_pair_kernel): a second half with one row and with all, several
+    batch tiles, rows behind the whole pair tiles in a launch of their own (257 and 350), vocabularies shorter than a tile, fewer K blocks
+    than stages."""
     check_product_and_records(pkg, M, N, K)
 
 
